@@ -22,6 +22,10 @@ constexpr int kStackDepth = 64;     // LBVH traversal stack
 constexpr int kLongCap = 2048;      // long walks a wrap lists for its next query's warps
 constexpr int kPartialStride = 8;   // doubles per energy partial record
 
+// Sticky device errors of a wrap.
+constexpr int kErrorTraversal = 1;  // a closest-point walk overflowed its stack
+constexpr int kErrorSolveWait = 2;  // a wait inside the linear solve ran out
+
 // Device phases of one wrap.  They mirror the reference session's
 // BeginLevel / Refresh / InnerStep / CloseOuter / EndLevel
 // (src/cuda/session.cu:504-542); CloseOuter folds into the decision kernel.
@@ -54,14 +58,14 @@ struct LevelDev {
     const int32_t* pair_nodes;     // pair_count x 2
     const int32_t* pair_begin;     // pair_count + 1
     const int32_t* pair_entry;     // vertex * 64 + slot_a * 8 + slot_b
-    // off-diagonal row lists for the matvec: for each node, the blocks that
-    // touch it; entry = block * 2 + (1 if the node is the block's b side)
-    const int32_t* row_begin;      // N + 1
-    const int32_t* row_entry;      // pairs: (block * 2 + side, other node)
+    // off-diagonal row lists for the matvec, by octets of nodes: step t of an
+    // octet holds the t-th row entry of each of its eight nodes
+    const int32_t* row_begin;      // N + 1: a node's entries are counted by row_begin[n + 1] - row_begin[n]
+    const int32_t* sell_begin;     // octets + 1: first step of each octet
+    const int32_t* sell_nodes;     // steps x 8: the other node of each block (0: none)
     const int32_t* offdiag_nodes;  // offdiag_count x 2 (pair groups first, then edge-only pairs)
     const int32_t* edge_block;     // edge_count: the block edge e adds to (< pair_count) or owns
-    const int32_t* offdiag_slots;  // offdiag_count x 2: row-entry slots of B (a) and B^T (b)
-    int row_entries;               // 2 x offdiag_count
+    const int32_t* sell_slots;     // offdiag_count x 2: places (step * 8 + node of the octet) of B (a) and B^T (b)
     // warm start from the previous level (level > 0): 4 source nodes + weights
     const int32_t* transfer_nodes;   // N x 4
     const double* transfer_weights;  // N x 4
@@ -97,7 +101,7 @@ struct WrapControl {
     int final_stats;      // the next statistics pass is the final report's
     int pcg_ok;           // outcome of this tick's solve
     int pcg_iterations;
-    int error;            // sticky device error (traversal overflow, ...)
+    int error;            // sticky device errors (kError* bits)
     int steps;            // ticks that did work for this wrap
     int tick_phase;       // the phase at the start of the current tick
     int long_cur;         // the list of long walks the next query reads (0 / 1)
@@ -181,9 +185,8 @@ struct WrapDev {
     // systems: two buffers, `control.system` selects the current one
     float* diag[2];               // N x 36
     float* rhs[2];                // N x 6
-    float* offdiag[2];            // 2 x max_offdiag x 36, in row-entry order:
-                                  // slot j holds the block of row list entry j
-                                  // (B for the a side, B^T for the b side)
+    float* offdiag[2];            // most steps x 288: the blocks by octets and steps
+                                  // (see block_base; B for the a side, B^T for the b side)
     // solve scratch
     float* factor;                // N x 36: inverse of the damped diagonal block
     double* delta;                // N x 6
@@ -239,6 +242,22 @@ __host__ __device__ inline F3 cross(F3 a, F3 b) {
 __device__ inline F3 mul3f(const float* m, F3 v) {
     return {m[0] * v.x + m[1] * v.y + m[2] * v.z, m[3] * v.x + m[4] * v.y + m[5] * v.z,
             m[6] * v.x + m[7] * v.y + m[8] * v.z};
+}
+
+// Storage of the off-diagonal blocks.  A step holds eight 6x6 blocks, one for
+// each node of an octet, as three planes of 24 float4: lane 3i + p of the
+// solve's warp owns rows 2p and 2p + 1 of node i's block, twelve floats, and
+// finds float4 c of them at plane c, place 3i + p.  So a warp reads a step
+// with three loads of 384 contiguous bytes.  (Rows stored one after another
+// put each load across 8 to 16 lines of 128 bytes, and the solve was bound by
+// the L1's tag lookups.)
+constexpr int kStepFloats = 288;
+__host__ __device__ inline long block_base(int place) {  // place: step * 8 + node of the octet
+    return (long)(place >> 3) * kStepFloats + (place & 7) * 12;
+}
+__host__ __device__ inline int block_at(int r, int q) {  // entry (r, q) from the block's base
+    const int f = (r & 1) * 6 + q;
+    return (f >> 2) * 96 + (r >> 1) * 4 + (f & 3);
 }
 
 // Leaf / internal child encoding of the traversal hierarchy.

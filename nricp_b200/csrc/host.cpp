@@ -739,6 +739,24 @@ LevelLayout build_layout(const TemplateGraph& graph, int level, int V) {
             L.offdiag_slots[k * 2 + 1] = ib;   // and from b: B^T
         }
     }
+    // the same row lists by octets of nodes and steps, as the solve stores the
+    // blocks
+    const int octets = (N + 7) / 8;
+    L.sell_begin.assign(octets + 1, 0);
+    for (int o = 0; o < octets; ++o) {
+        int32_t most = 0;
+        for (int n = o * 8; n < std::min(N, o * 8 + 8); ++n)
+            most = std::max(most, L.row_begin[n + 1] - L.row_begin[n]);
+        L.sell_begin[o + 1] = L.sell_begin[o] + most;
+    }
+    L.sell_nodes.assign(static_cast<size_t>(L.sell_begin[octets]) * 8, 0);
+    L.sell_slots.assign(static_cast<size_t>(B) * 2, 0);
+    for (int n = 0; n < N; ++n)
+        for (int32_t j = L.row_begin[n]; j < L.row_begin[n + 1]; ++j) {
+            const int32_t place = (L.sell_begin[n / 8] + (j - L.row_begin[n])) * 8 + n % 8;
+            L.sell_nodes[place] = L.row_entry[j * 2 + 1];
+            L.sell_slots[L.row_entry[j * 2]] = place;  // entry code: block * 2 + side
+        }
     // warm start from the previous level (deformation.cpp:141-160): the new
     // nodes bound to the old ones with the reference's four slots
     L.transfer_nodes.assign(static_cast<size_t>(N) * 4, 0);

@@ -51,6 +51,13 @@ struct LevelLayout {
     // the off-diagonal block that holds smoothness edge e: a node pair's own
     // block when the pair shares a vertex (< pair_count), else one of its own
     std::vector<int32_t> edge_block;
+    // The solve's storage of the off-diagonal blocks: eight nodes (an octet) by
+    // steps, step t holding the t-th row entry of each node of the octet.
+    // sell_begin: octet -> first step (octets + 1); sell_nodes: the other node
+    // of each of a step's eight blocks (0 where a node has fewer entries);
+    // sell_slots: block k's places (step * 8 + node of the octet) as B in row a
+    // and as B^T in row b.
+    std::vector<int32_t> sell_begin, sell_nodes, sell_slots;
     std::vector<int32_t> transfer_nodes, transfer_counts;
     std::vector<double> transfer_weights;
 };

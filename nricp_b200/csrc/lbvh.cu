@@ -923,7 +923,7 @@ __device__ void query_vertex(const WrapDev& w, int level, int v) {
     int overflow = 0;
     const int tri = nearest_triangle(w, {q32.x, q32.y, q32.z}, load_d3(w.deformed, v), w.corr_triangle[v],
                                      &overflow);
-    if (overflow) atomicOr(&w.control->error, 1);
+    if (overflow) atomicOr(&w.control->error, kErrorTraversal);
     store_correspondence(w, level, v, tri);
 }
 
@@ -1023,7 +1023,7 @@ __global__ void __launch_bounds__(128) k_query_queue(const WrapDev* __restrict__
                                             &unfinished, &work);
             if (lane == 0) {
                 if (unfinished) tri = nearest_triangle(w, q, q64, tri, &overflow);
-                if (overflow) atomicOr(&w.control->error, 1);
+                if (overflow) atomicOr(&w.control->error, kErrorTraversal);
                 store_correspondence(w, w.control->level, v, tri);
                 if (unfinished || work > kLongWalk) list_long_walk(w, 1 - cur, v);
             }
@@ -1053,7 +1053,7 @@ __global__ void __launch_bounds__(128) k_query_queue(const WrapDev* __restrict__
         long steps = 0;
         const int tri = nearest_triangle(w, {q32.x, q32.y, q32.z}, load_d3(w.deformed, v),
                                          w.corr_triangle[v], &overflow, &steps);
-        if (overflow) atomicOr(&w.control->error, 1);
+        if (overflow) atomicOr(&w.control->error, kErrorTraversal);
         store_correspondence(w, w.control->level, v, tri);
         if (steps > kLongWalk) list_long_walk(w, 1 - cur, v);
     }

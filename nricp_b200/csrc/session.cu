@@ -45,6 +45,12 @@ double now_seconds() {
     return std::chrono::duration<double>(std::chrono::steady_clock::now().time_since_epoch()).count();
 }
 
+// What a wrap's sticky device error says.
+const char* device_error(int bits) {
+    return (bits & kErrorTraversal) ? "a closest-point traversal exceeded its stack; the hierarchy is too deep"
+                                    : "a wait inside the linear solve ran out";
+}
+
 // One device allocation carved into aligned sub-arrays.
 class Arena {
 public:
@@ -163,7 +169,7 @@ struct Wrap {
     TemplateGraph graph;
     std::vector<LevelLayout> layouts;
     int V = 0, T = 0, Vt = 0, F = 0, L = 0, levels = 0;
-    int max_nodes = 0, max_edges = 0, max_pairs = 0, max_offdiag = 0;
+    int max_nodes = 0, max_edges = 0, max_pairs = 0, max_offdiag = 0, max_steps = 0;
     double setup_seconds = 0.0, solve_started = 0.0, solve_seconds = 0.0;
     Arena arena;
     WrapDev dev{};        // host copy of the descriptor
@@ -241,6 +247,7 @@ void envelope(Wrap& w) {
         w.max_edges = std::max(w.max_edges, L.edge_count);
         w.max_pairs = std::max(w.max_pairs, L.pair_count);
         w.max_offdiag = std::max(w.max_offdiag, static_cast<int>(L.offdiag_nodes.size() / 2));
+        w.max_steps = std::max(w.max_steps, static_cast<int>(L.sell_begin.back()));
     }
 }
 
@@ -267,7 +274,7 @@ size_t bytes_of_layout(const LevelLayout& L) {
                               L.gather_entry.size() + L.node_edge_begin.size() +
                               L.node_edge_list.size() + L.edges.size() + L.pair_nodes.size() +
                               L.pair_begin.size() + L.pair_entry.size() + L.row_begin.size() +
-                              L.row_entry.size() + L.offdiag_nodes.size() + L.offdiag_slots.size() +
+                              L.sell_begin.size() + L.sell_nodes.size() + L.offdiag_nodes.size() + L.sell_slots.size() +
                               L.edge_block.size() +
                               L.transfer_nodes.size() +
                               L.transfer_counts.size());
@@ -283,7 +290,7 @@ size_t bytes_of_layout(const LevelLayout& L) {
 size_t prepare_device(Wrap& w, WrapControl* control, cudaStream_t stream, bool plan_only = false,
                       cudaMemPool_t pool = nullptr, char* staging = nullptr) {
     const NricpSolveDesc& d = w.desc;
-    const int V = w.V, N = std::max(1, w.max_nodes), B = std::max(1, w.max_offdiag);
+    const int V = w.V, N = std::max(1, w.max_nodes);
     Arena& a = w.arena;
     // template and target
     const size_t o_tpl = a.reserve(sizeof(double) * 3 * V);
@@ -315,7 +322,7 @@ size_t prepare_device(Wrap& w, WrapControl* control, cudaStream_t stream, bool p
         o_trans[i] = a.reserve(sizeof(double) * 3 * N);
         o_diag[i] = a.reserve(sizeof(float) * 36 * N);
         o_rhs[i] = a.reserve(sizeof(float) * 6 * N);
-        o_off[i] = a.reserve(sizeof(float) * 36 * 2 * B);
+        o_off[i] = a.reserve(sizeof(float) * kStepFloats * std::max(1, w.max_steps));
     }
     const size_t o_rot32 = a.reserve(sizeof(float) * 9 * N);
     const size_t o_deformed = a.reserve(sizeof(double) * 3 * V);
@@ -481,11 +488,11 @@ size_t prepare_device(Wrap& w, WrapControl* control, cudaStream_t stream, bool p
         G.pair_begin = put(L.pair_begin);
         G.pair_entry = put(L.pair_entry);
         G.row_begin = put(L.row_begin);
-        G.row_entry = put(L.row_entry);
+        G.sell_begin = put(L.sell_begin);
+        G.sell_nodes = put(L.sell_nodes);
         G.offdiag_nodes = put(L.offdiag_nodes);
-        G.offdiag_slots = put(L.offdiag_slots);
+        G.sell_slots = put(L.sell_slots);
         G.edge_block = put(L.edge_block);
-        G.row_entries = static_cast<int>(L.row_entry.size() / 2);
         G.transfer_nodes = put(L.transfer_nodes);
         G.transfer_weights = put(L.transfer_weights);
         G.transfer_counts = put(L.transfer_counts);
@@ -890,7 +897,6 @@ void Batch::solve_shape(int cluster, TickShape& shape, int*& index, std::vector<
         if (cluster > 16 || (cluster & (cluster - 1)) != 0)
             throw InvalidArgument("the solve's cluster size is a power of two from 1 to 16");
         shape.pcg_cluster = cluster;
-        shape.pcg_shared_bytes = pcg_shared_bytes(nodes.data(), W, cluster);
         if (cls_out) cls_out->assign(W, cluster);
         return;
     }
@@ -905,7 +911,6 @@ void Batch::solve_shape(int cluster, TickShape& shape, int*& index, std::vector<
         if (std::count(cls.begin(), cls.end(), c) > 0) sizes.push_back(c);
     if (sizes.size() == 1) {
         shape.pcg_cluster = sizes[0];
-        shape.pcg_shared_bytes = pcg_shared_bytes(nodes.data(), W, sizes[0]);
         return;
     }
     if (!index) check(cudaMalloc(&index, sizeof(int) * W), "cudaMalloc(solve groups)");
@@ -915,12 +920,9 @@ void Batch::solve_shape(int cluster, TickShape& shape, int*& index, std::vector<
         std::vector<int> members;
         for (int i = 0; i < W; ++i)
             if (cls[i] == sizes[g]) members.push_back(i);
-        std::vector<int> member_nodes;
-        for (int i : members) member_nodes.push_back(nodes[i]);
         order.insert(order.end(), members.begin(), members.end());
         shape.pcg_group_cluster[g] = sizes[g];
         shape.pcg_group_count[g] = static_cast<int>(members.size());
-        shape.pcg_group_shared[g] = pcg_shared_bytes(member_nodes.data(), (int)members.size(), sizes[g]);
         shape.pcg_group_index[g] = index + first;
         if (g > 0 && !pcg_streams_[g]) {
             check(cudaStreamCreateWithFlags(&pcg_streams_[g], cudaStreamNonBlocking), "stream");
@@ -934,7 +936,6 @@ void Batch::solve_shape(int cluster, TickShape& shape, int*& index, std::vector<
     check(cudaMemcpy(index, order.data(), sizeof(int) * W, cudaMemcpyHostToDevice), "solve groups");
     shape.pcg_groups = static_cast<int>(sizes.size());
     shape.pcg_cluster = sizes[0];
-    shape.pcg_shared_bytes = shape.pcg_group_shared[0];
 }
 
 bool Batch::tail_due() const {
@@ -1060,7 +1061,7 @@ void Batch::finish() {
     const double t = now_seconds();
     for (size_t i = 0; i < wraps_.size(); ++i) {
         if (host_controls_[i].error)
-            throw StateError("a closest-point traversal exceeded its stack; the hierarchy is too deep");
+            throw StateError(device_error(host_controls_[i].error));
         if (wraps_[i]->solve_seconds == 0.0) wraps_[i]->solve_seconds = t - wraps_[i]->solve_started;
     }
 }
@@ -1101,14 +1102,15 @@ void Batch::inspect(int i, NricpInspect* out) {
     out->pcg_ok = c.pcg_ok;
     out->pcg_iterations = c.pcg_iterations;
     out->pcg_residual = c.pcg_residual;
-    std::vector<float> rows(out->off_nodes && out->off_blocks ? L.row_entry.size() / 2 * 36 : 0);
+    std::vector<float> rows(out->off_nodes && out->off_blocks ? static_cast<size_t>(L.sell_begin.back()) * kStepFloats : 0);
     if (!rows.empty()) get(rows.data(), D.offdiag[c.system], sizeof(float) * rows.size());
     check(cudaStreamSynchronize(stream_), "inspect");
     for (int k = 0; k < K && !rows.empty(); ++k) {
         out->off_nodes[k * 2] = L.offdiag_nodes[k * 2];
         out->off_nodes[k * 2 + 1] = L.offdiag_nodes[k * 2 + 1];
-        const float* block = rows.data() + static_cast<size_t>(L.offdiag_slots[k * 2]) * 36;
-        std::copy(block, block + 36, out->off_blocks + static_cast<size_t>(k) * 36);
+        const float* block = rows.data() + block_base(L.sell_slots[k * 2]);
+        for (int r = 0; r < 6; ++r)
+            for (int q = 0; q < 6; ++q) out->off_blocks[static_cast<size_t>(k) * 36 + r * 6 + q] = block[block_at(r, q)];
     }
 }
 
@@ -1278,7 +1280,7 @@ namespace {
 struct TemplateEntry {
     TemplateGraph graph;
     std::vector<LevelLayout> layouts;
-    int levels = 0, max_nodes = 0, max_edges = 0, max_pairs = 0, max_offdiag = 0;
+    int levels = 0, max_nodes = 0, max_edges = 0, max_pairs = 0, max_offdiag = 0, max_steps = 0;
 };
 
 uint64_t fnv1a(const void* data, size_t bytes, uint64_t h) {
@@ -1402,6 +1404,7 @@ struct Server::Impl {
             fresh->max_edges = w.max_edges;
             fresh->max_pairs = w.max_pairs;
             fresh->max_offdiag = w.max_offdiag;
+            fresh->max_steps = w.max_steps;
             std::lock_guard<std::mutex> lk(cache_mu);
             cache.emplace(key, std::move(fresh));
             return;
@@ -1413,6 +1416,7 @@ struct Server::Impl {
         w.max_edges = entry->max_edges;
         w.max_pairs = entry->max_pairs;
         w.max_offdiag = entry->max_offdiag;
+        w.max_steps = entry->max_steps;
     }
 
     void fail(const RequestPtr& r, const std::string& why, bool invalid) {
@@ -1563,17 +1567,12 @@ struct Server::Impl {
         pcg_cluster_size(t.max_nodes, count, sms);  // enables the launch attributes
         if (class_count == 0) {
             t.pcg_cluster = cfg.pcg_cluster;
-            std::vector<int> nodes(count, t.max_nodes);  // any wrap may take any slot
-            t.pcg_shared_bytes = pcg_shared_bytes(nodes.data(), count, t.pcg_cluster);
         } else {
-            // every class launch covers `count` entries; a class's shared
-            // memory is what its largest possible member would use
+            // every class launch covers `count` entries
             for (int g = 0; g < class_count; ++g) {
                 const int cluster = class_top >> g;
-                const int nodes = std::min(t.max_nodes, class_node_bound(cluster));
                 t.pcg_group_cluster[g] = cluster;
                 t.pcg_group_count[g] = count;
-                t.pcg_group_shared[g] = pcg_shared_bytes(&nodes, 1, cluster);
                 t.pcg_group_index[g] = class_index + static_cast<size_t>(g) * cfg.max_slots;
                 t.pcg_streams[g] = class_streams[g];
                 t.pcg_join[g] = class_join[g];
@@ -1581,7 +1580,6 @@ struct Server::Impl {
             t.pcg_fork = class_fork;
             t.pcg_groups = class_count;
             t.pcg_cluster = class_top;
-            t.pcg_shared_bytes = t.pcg_group_shared[0];
         }
         cudaGraph_t g = nullptr;
         cudaGraphExec_t exec = nullptr;
@@ -1608,14 +1606,6 @@ struct Server::Impl {
         return ctas <= 3L * sms ? 0 : 1;
     }
     static int class_of(int nodes, int shift) { return std::max(1, pcg_latency_cluster(nodes) >> shift); }
-    // The most nodes a wrap of class `cluster` can have: its latency cluster
-    // is at most cluster << max_shift, which covers up to 128 nodes per CTA
-    // below 16.
-    int class_node_bound(int cluster) const {
-        const int latency = cluster << max_shift();
-        return latency >= 16 ? pcg_max_nodes() : latency * 128;
-    }
-
     // Rewrites the class rows for the running wraps in slots 0 .. count-1
     // (tick stream order: the next tick reads them).
     void upload_classes(int count) {
@@ -1797,7 +1787,7 @@ struct Server::Impl {
                 holes.push_back(i);
                 std::string why;
                 if (host_controls[i].error) {
-                    why = "a closest-point traversal exceeded its stack; the hierarchy is too deep";
+                    why = device_error(host_controls[i].error);
                 } else {
                     try {
                         retire(i, r);

@@ -226,16 +226,16 @@ __device__ inline T warp_sum(T v) {
 // and y + x round alike), so the bits are the same, with ~N shuffles instead
 // of 5N.  Afterwards this lane holds the totals of values
 // [first, first + count) in v[0 .. count).
-template <int N, int O = 16>
-__device__ __forceinline__ void warp_sum_halving(float* v, int lane, int& first, int& count) {
+template <int N, int O = 16, typename T, typename Add>
+__device__ __forceinline__ void warp_sum_halving(T* v, int lane, int& first, int& count, Add add) {
     if constexpr (O >= 1) {
         constexpr int H = (N + 1) / 2;
         const bool upper = (lane & O) != 0;
 #pragma unroll
         for (int i = 0; i < H; ++i) {
-            const float lo = v[i];
-            const float hi = i + H < N ? v[i + H] : 0.0f;
-            v[i] = (upper ? hi : lo) + __shfl_xor_sync(0xffffffffu, upper ? lo : hi, O);
+            const T lo = v[i];
+            const T hi = i + H < N ? v[i + H] : T(0);
+            v[i] = add(upper ? hi : lo, __shfl_xor_sync(0xffffffffu, upper ? lo : hi, O));
         }
         if (upper) {
             first += H;
@@ -243,8 +243,12 @@ __device__ __forceinline__ void warp_sum_halving(float* v, int lane, int& first,
         } else {
             count = count < H ? count : H;
         }
-        warp_sum_halving<H, O / 2>(v, lane, first, count);
+        warp_sum_halving<H, O / 2>(v, lane, first, count, add);
     }
+}
+template <int N>
+__device__ __forceinline__ void warp_sum_halving(float* v, int lane, int& first, int& count) {
+    warp_sum_halving<N, 16>(v, lane, first, count, [](float a, float b) { return a + b; });
 }
 // Block sum in a fixed order; every thread returns the total.
 template <int kThreadsT>
@@ -791,35 +795,51 @@ __device__ __forceinline__ double warp_sum_rnd(double v) {
     return v;
 }
 constexpr int kPcgWarps = kPcgThreads / 32;
-constexpr int kPcgOwnFloats = 78;  // per owned node: X, R (2 x 6 FP64) + Minv 36 + P, S, W 18
+// Shared floats per owned node: X, R (2 x 6 FP64), P, S, W (18), its row's
+// entry count and (one per octet each) the octet's first step and steps, padded.
+constexpr int kPcgVectorFloats = 44;
+constexpr int kPcgBlockFloats = 36;   // its damped diagonal block; and its inverse
+// Dynamic shared memory of every solve launch: all there is.  A solve CTA holds
+// its SM alone (512 threads of 128 registers), and what the vectors leave
+// holds off-diagonal blocks.
 constexpr int kPcgMaxSmemBytes = 225 * 1024;
+constexpr int kOctet = 8;             // nodes a warp multiplies at a time (24 of its lanes)
 
 __host__ __device__ inline int pcg_segments(int nodes) { return (nodes + kSegNodes - 1) / kSegNodes; }
-// FP64 slots for the segments' three partials, padded to 16 bytes
-__host__ __device__ inline int pcg_slot_doubles(int nodes) { return (3 * pcg_segments(nodes) + 1) & ~1; }
+__host__ __device__ inline int pcg_octets(int nodes) { return (nodes + kOctet - 1) / kOctet; }
+// FP64 slots for the segments' three partials (two segments per octet)
+__host__ __device__ inline int pcg_slot_doubles(int nodes) { return 6 * pcg_octets(nodes); }
 
 // Owned-node capacity of one CTA when `ranks` CTAs share the solve.
 __host__ __device__ inline int pcg_owned_capacity(int nodes, int ranks) {
-    return (pcg_segments(nodes) + ranks - 1) / ranks * kSegNodes;
+    return (pcg_octets(nodes) + ranks - 1) / ranks * kOctet;
 }
 
-// Placement for one wrap within a shared-memory budget: the segment slots
-// always, then the all-node direction copy U if it fits (the matvec reads it
-// ~10 times per row), then the owned rows' arrays if they fit.  Whatever does
-// not fit lives in the wrap's global scratch; the arithmetic is the same.
+// Placement for one wrap within the launch's shared memory, in this order:
+// the segment slots always, the all-node direction copy U if it fits (the
+// matvec reads it ~20 times per row), the owned rows' vectors, their diagonal
+// blocks, the inverses of those, and what is left for the first steps of every
+// owned octet's off-diagonal blocks.  Whatever does not fit lives in the wrap's
+// global scratch; the arithmetic is the same.
 struct PcgPlacement {
-    bool u_shared, own_shared;
-    int floats;  // shared floats this wrap uses
+    bool u_shared, vectors_shared, diagonal_shared, inverse_shared;
+    __device__ bool all() const { return u_shared && vectors_shared && diagonal_shared && inverse_shared; }
+    int floats;  // shared floats used before the blocks
 };
-__host__ __device__ inline PcgPlacement pcg_place(int nodes, int ranks, int budget_floats) {
+__device__ inline PcgPlacement pcg_place(int nodes, int ranks, int budget_floats) {
     PcgPlacement p;
-    int used = pcg_slot_doubles(nodes) * 2;  // 3 FP64 partials per segment
+    int used = pcg_slot_doubles(nodes) * 2;
     const int u = (nodes * 6 + 3) & ~3;
-    const int own = pcg_owned_capacity(nodes, ranks) * kPcgOwnFloats;
-    p.u_shared = used + u <= budget_floats;
-    if (p.u_shared) used += u;
-    p.own_shared = used + own <= budget_floats;
-    if (p.own_shared) used += own;
+    const int cap = pcg_owned_capacity(nodes, ranks);
+    auto take = [&](int floats) {
+        const bool fits = used + floats <= budget_floats;
+        if (fits) used += floats;
+        return fits;
+    };
+    p.u_shared = take(u);
+    p.vectors_shared = take(cap * kPcgVectorFloats);
+    p.diagonal_shared = take(cap * kPcgBlockFloats);
+    p.inverse_shared = take(cap * kPcgBlockFloats);
     p.floats = used;
     return p;
 }
@@ -844,19 +864,74 @@ __device__ inline void cholesky_inverse6(const float* l, float* inv) {
         }
 }
 
-__device__ inline float dot6(const float* a, const float* b) {
-    const float2* a2 = reinterpret_cast<const float2*>(a);
-    const float2* b2 = reinterpret_cast<const float2*>(b);
-    const float2 a0 = a2[0], a1 = a2[1], a3 = a2[2];
-    const float2 b0 = b2[0], b1 = b2[1], b3 = b2[2];
-    float y = a0.x * b0.x;
-    y += a0.y * b0.y;
-    y += a1.x * b1.x;
-    y += a1.y * b1.y;
-    y += a3.x * b3.x;
-    y += a3.y * b3.y;
-    return y;
+// ---- mbarriers and bulk copies ---------------------------------------------
+__device__ __forceinline__ uint32_t shared_address(const void* p) {
+    return static_cast<uint32_t>(__cvta_generic_to_shared(p));
 }
+__device__ __forceinline__ void mbar_init(void* bar, int arrivals) {
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(shared_address(bar)), "r"(arrivals) : "memory");
+    // the copies' and the other CTAs' view of the initialised barrier
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+}
+__device__ __forceinline__ void mbar_arrive_expect(void* bar, int bytes) {
+    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(shared_address(bar)), "r"(bytes)
+                 : "memory");
+}
+// Waits for the phase of this parity, with a limit (about a second): false if
+// it ran out.
+constexpr int kWaitLimit = 1 << 20;
+__device__ __forceinline__ bool mbar_wait(void* bar, int parity) {
+    const uint32_t at = shared_address(bar);
+    for (int i = 0; i < kWaitLimit; ++i) {
+        uint32_t done;
+        asm volatile("{\n.reg .pred p;\n"
+                     "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n"
+                     "selp.u32 %0, 1, 0, p;\n}"
+                     : "=r"(done)
+                     : "r"(at), "r"(parity)
+                     : "memory");
+        if (done) return true;
+    }
+    return false;
+}
+// Global to shared, both 16-byte aligned, a multiple of 16 bytes.
+__device__ __forceinline__ void bulk_to_shared(void* dst, const void* src, int bytes, void* bar) {
+    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
+                     shared_address(dst)),
+                 "l"(__cvta_generic_to_global(src)), "r"(bytes), "r"(shared_address(bar))
+                 : "memory");
+}
+
+// Rows 2p and 2p + 1 of a 6x6 block (twelve floats in three float4) times a
+// node's six values.  The order of the operations is spelt out, so that every
+// placement gives the same bits: of the first two products, a diagonal block's
+// second is fused onto its first, an off-diagonal block's first onto its
+// second; the other four follow left to right.
+struct RowPair { float a, b; };
+template <bool kDiagonal>
+__device__ __forceinline__ float row_dot(float x0, float x1, float x2, float x3, float x4, float x5, float2 u0,
+                                         float2 u1, float2 u2) {
+    float y = kDiagonal ? __fmaf_rn(x1, u0.y, __fmul_rn(x0, u0.x)) : __fmaf_rn(x0, u0.x, __fmul_rn(x1, u0.y));
+    y = __fmaf_rn(x2, u1.x, y);
+    y = __fmaf_rn(x3, u1.y, y);
+    y = __fmaf_rn(x4, u2.x, y);
+    return __fmaf_rn(x5, u2.y, y);
+}
+template <bool kDiagonal>
+__device__ __forceinline__ RowPair row_pair_dot(float4 b0, float4 b1, float4 b2, const float* u) {
+    const float2* v = reinterpret_cast<const float2*>(u);
+    const float2 u0 = v[0], u1 = v[1], u2 = v[2];
+    return {row_dot<kDiagonal>(b0.x, b0.y, b0.z, b0.w, b1.x, b1.y, u0, u1, u2),
+            row_dot<kDiagonal>(b1.z, b1.w, b2.x, b2.y, b2.z, b2.w, u0, u1, u2)};
+}
+
+// A few steps of an octet's blocks from global memory, in registers.
+constexpr int kStepsAhead = 4;
+struct StepBlocks {
+    float4 b[kStepsAhead][3];
+    int node[kStepsAhead];
+};
 
 // The damped solve (pcg_solver.cu:15-241): (A + lambda diag-scale) x = b,
 // x0 = 0, block-Jacobi preconditioner from the Cholesky factor of each damped
@@ -879,35 +954,32 @@ __device__ inline float dot6(const float* a, const float* b) {
 // through distributed shared memory, so the matvec reads u locally and its
 // only L2 traffic is the blocks (stored in row order).  Two hardware cluster
 // barriers per iteration; nothing spins.
-__global__ void __launch_bounds__(kPcgThreads) k_pcg(const WrapDev* __restrict__ wraps,
-                                                     const int* __restrict__ index,
-                                                     int budget_floats) {
+//
+// kAllShared: every array of the placement is in shared memory (the compiler
+// then addresses it as such); the other instance decides at run time.
+template <bool kAllShared>
+__device__ __forceinline__ void pcg_solve(const WrapDev& w, const WrapControl& c, const PcgPlacement& place,
+                                          int budget_floats) {
     cg::cluster_group cluster = cg::this_cluster();
-    const int slot = index ? index[blockIdx.y] : (int)blockIdx.y;
-    if (slot < 0) return;  // an empty entry of a class launch; uniform across the cluster
-    const WrapDev& w = wraps[slot];
-    const WrapControl c = *w.control;
-    if (c.tick_phase != kPhaseSolve || c.phase != kPhaseSolve) return;  // uniform across the cluster
     const LevelDev& L = w.levels[c.level];
     const int N = L.node_count;
     const int rank = (int)cluster.block_rank();
     const int ranks = (int)cluster.num_blocks();
     const int segs = pcg_segments(N);
+    const int octets = pcg_octets(N);
     const int cap = pcg_owned_capacity(N, ranks);
-    const int seg_per = cap / kSegNodes;
-    const int s0 = min(segs, rank * seg_per);
-    const int s1 = min(segs, s0 + seg_per);
-    const int n0 = s0 * kSegNodes;
-    const int n1 = min(N, s1 * kSegNodes);
+    const int o0 = min(octets, rank * (cap / kOctet));
+    const int o1 = min(octets, o0 + cap / kOctet);
+    const int n0 = o0 * kOctet;
+    const int n1 = min(N, o1 * kOctet);
     const int own = n1 > n0 ? n1 - n0 : 0;
     const int rows = own * 6;
-    const PcgPlacement place = pcg_place(N, ranks, budget_floats);
 
     extern __shared__ float4 dynamic_shared[];
     double* slots = reinterpret_cast<double*>(dynamic_shared);  // 3 per segment, every CTA
     float* cursor = reinterpret_cast<float*>(slots + pcg_slot_doubles(N));
     float* U;
-    if (place.u_shared) {
+    if (kAllShared || place.u_shared) {
         U = cursor;
         cursor += (N * 6 + 3) & ~3;
     } else {
@@ -915,26 +987,40 @@ __global__ void __launch_bounds__(kPcgThreads) k_pcg(const WrapDev* __restrict__
     }
     double *X, *R;
     float *Minv, *P, *S, *Wv;
-    if (place.own_shared) {
+    int* degrees = nullptr;  // per owned node; then per owned octet its first step and its steps
+    float* diagonal = nullptr;
+    if (kAllShared || place.vectors_shared) {
         X = reinterpret_cast<double*>(cursor);
         R = X + cap * 6;
-        Minv = reinterpret_cast<float*>(R + cap * 6);
-        P = Minv + cap * 36;
+        P = reinterpret_cast<float*>(R + cap * 6);
         S = P + cap * 6;
         Wv = S + cap * 6;
+        degrees = reinterpret_cast<int*>(Wv + cap * 6);
+        cursor += cap * kPcgVectorFloats;
     } else {
         X = w.pcg_x + n0 * 6;
         R = w.pcg_r + n0 * 6;
-        Minv = w.factor + n0 * 36;
         P = w.pcg_p + n0 * 6;
         S = w.pcg_s + n0 * 6;
         Wv = w.pcg_ap + n0 * 6;
     }
+    if (kAllShared || place.diagonal_shared) {
+        diagonal = cursor;
+        cursor += cap * kPcgBlockFloats;
+    }
+    if (kAllShared || place.inverse_shared) {
+        Minv = cursor;
+        cursor += cap * kPcgBlockFloats;
+    } else {
+        Minv = w.factor + n0 * 36;
+    }
     const float* __restrict__ D = w.diag[c.system];
-    const float* __restrict__ B = w.offdiag[c.system];
+    const float4* __restrict__ B = reinterpret_cast<const float4*>(w.offdiag[c.system]);
     const float* __restrict__ b = w.rhs[c.system];
     const int* __restrict__ row_begin = L.row_begin;
-    const int2* __restrict__ entries = reinterpret_cast<const int2*>(L.row_entry);
+    const int* __restrict__ sell_begin = L.sell_begin;
+    const int* __restrict__ sell_nodes = L.sell_nodes;
+    constexpr int kStepFloat4s = kStepFloats / 4;
     const float damping = (float)c.damping;
     const bool scaled = w.diagonal_damping != 0;
     const int max_iterations = w.pcg_max_iterations;
@@ -942,6 +1028,41 @@ __global__ void __launch_bounds__(kPcgThreads) k_pcg(const WrapDev* __restrict__
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     __shared__ double red[3][kPcgWarps];
     __shared__ double tot[3];
+    __shared__ alignas(8) unsigned long long blocks_arrived;  // mbarrier
+    __shared__ int cached_s;
+
+    // ---- the first steps of every owned octet's blocks into the shared
+    //      memory that is left, as many as fit, by bulk copies that run under
+    //      the factorisation below ----
+    if (warp == 0) {
+        int most = 0;
+        for (int o = o0 + lane; o < o1; o += 32) most = max(most, sell_begin[o + 1] - sell_begin[o]);
+        most = __reduce_max_sync(0xffffffffu, most);
+        const int left = budget_floats - place.floats;
+        const int cached = o1 > o0 ? min(most, left / ((o1 - o0) * (kStepFloats + kOctet))) : 0;
+        if (lane == 0) {
+            cached_s = cached;
+            mbar_init(&blocks_arrived, 1);
+        }
+        __syncwarp();
+        int bytes = 0;
+        for (int o = o0 + lane; o < o1; o += 32)
+            bytes += min(cached, sell_begin[o + 1] - sell_begin[o]) * (int)sizeof(float) * (kStepFloats + kOctet);
+        bytes = __reduce_add_sync(0xffffffffu, bytes);
+        if (lane == 0) mbar_arrive_expect(&blocks_arrived, bytes);
+        __syncwarp();
+        float* block_room = cursor;
+        float* node_room = cursor + (long)(o1 - o0) * cached * kStepFloats;
+        for (int o = o0 + lane; o < o1; o += 32) {
+            const int first = sell_begin[o], count = min(cached, sell_begin[o + 1] - first);
+            if (count <= 0) continue;
+            const int at = (o - o0) * cached;
+            bulk_to_shared(block_room + (long)at * kStepFloats, B + (long)first * kStepFloat4s,
+                           count * kStepFloats * (int)sizeof(float), &blocks_arrived);
+            bulk_to_shared(node_room + at * kOctet, sell_nodes + (long)first * kOctet,
+                           count * kOctet * (int)sizeof(float), &blocks_arrived);
+        }
+    }
 
     // ---- damped diagonal blocks and their inverses (route A's damped():
     //      scale = max(D_rr, 1e-12)); Cholesky with the reference's jitter ----
@@ -950,6 +1071,16 @@ __global__ void __launch_bounds__(kPcgThreads) k_pcg(const WrapDev* __restrict__
         float blk[36];
         for (int i = 0; i < 36; ++i) blk[i] = D[n * 36 + i];
         for (int r = 0; r < 6; ++r) blk[r * 7] += damping * (scaled ? fmaxf(blk[r * 7], 1e-12f) : 1.0f);
+        if (kAllShared) {  // stored as a step's block
+            float* to = diagonal + block_base(m);
+            for (int i = 0; i < 36; ++i) to[block_at(i / 6, i % 6)] = blk[i];
+            degrees[m] = row_begin[n + 1] - row_begin[n];
+            if (m % kOctet == 0) {
+                const int first = sell_begin[n / kOctet];
+                degrees[cap + m / kOctet * 2] = first;
+                degrees[cap + m / kOctet * 2 + 1] = sell_begin[n / kOctet + 1] - first;
+            }
+        }
         float jitter = 0.0f;
         bool ok = false;
         for (int attempt = 0; attempt < 8 && !ok; ++attempt) {
@@ -984,7 +1115,7 @@ __global__ void __launch_bounds__(kPcgThreads) k_pcg(const WrapDev* __restrict__
             for (int q = 0; q < 6; ++q) z += mi[q] * (float)R[m * 6 + q];
             U[n0 * 6 + i] = z;
         }
-        if (place.u_shared && ranks > 1) {
+        if ((kAllShared || place.u_shared) && ranks > 1) {
             __syncthreads();
             const float4* src = reinterpret_cast<const float4*>(U + n0 * 6);
             const int vec = rows / 4;  // rows = 6 * own, own a multiple of 4 except at the end
@@ -996,54 +1127,119 @@ __global__ void __launch_bounds__(kPcgThreads) k_pcg(const WrapDev* __restrict__
                 for (int k = vec * 4 + threadIdx.x; k < rows; k += blockDim.x) dst_tail[k] = U[n0 * 6 + k];
             }
         }
-        if (!place.u_shared) __threadfence();  // the global copy: visible device-wide first
+        if (!kAllShared && !place.u_shared) __threadfence();  // the global copy: visible device-wide first
     };
     precondition_and_share();
     cluster.sync();
+
+    const int cached = cached_s;
+    const float4* cached_blocks = reinterpret_cast<const float4*>(cursor);
+    const int* cached_nodes = reinterpret_cast<const int*>(cursor + (long)(o1 - o0) * cached * kStepFloats);
+    if (!mbar_wait(&blocks_arrived, 0)) atomicOr(&w.control->error, kErrorSolveWait);
 
     double gamma_prev = 0.0, alpha_prev = 0.0, bnorm = 0.0, residual = 0.0;
     int iterations = 0;
     bool converged = false;
     for (int it = 0;; ++it) {
-        // ---- w = A u for the owned rows; per-segment partials of (r,u), (w,u), (r,r) ----
-        for (int sl = warp; sl < s1 - s0; sl += kPcgWarps) {
-            const int seg = s0 + sl;
-            const int sn0 = seg * kSegNodes;
-            const int seg_rows = (min(N, sn0 + kSegNodes) - sn0) * 6;
-            double g = 0.0, d = 0.0, rr = 0.0;
-            for (int k = lane; k < seg_rows; k += 32) {
-                const int n = sn0 + k / 6, r = k % 6;
-                const int i = (sn0 - n0) * 6 + k;
-                const float* drow = D + n * 36 + r * 6;
-                const float* un = U + n * 6;
-                const float dd = drow[r] + damping * (scaled ? fmaxf(drow[r], 1e-12f) : 1.0f);
-                float y = 0.0f;
-                for (int q = 0; q < 6; ++q) y += (q == r ? dd : drow[q]) * un[q];
-                const int e1 = row_begin[n + 1];
-                int e = row_begin[n];
-                for (; e + 4 <= e1; e += 4) {
-                    int nb[4];
-                    for (int u = 0; u < 4; ++u) nb[u] = entries[e + u].y;
-                    float part[4];
-                    for (int u = 0; u < 4; ++u) part[u] = dot6(B + (long)(e + u) * 36 + r * 6, U + nb[u] * 6);
-                    for (int u = 0; u < 4; ++u) y += part[u];
-                }
-                for (; e < e1; ++e) y += dot6(B + (long)e * 36 + r * 6, U + entries[e].y * 6);
-                Wv[i] = y;
-                const double ui = (double)un[r];
-                const double ri = R[i];
-                g = rnd(g + rnd(ri * ui));
-                d = rnd(d + rnd((double)y * ui));
-                rr = rnd(rr + rnd(ri * ri));
+        // ---- w = A u for the owned rows, an octet per warp at a time: lane
+        //      3i + p multiplies rows 2p and 2p + 1 of the octet's node i ----
+        for (int o = o0 + warp; o < o1; o += kPcgWarps) {
+            const int i = lane / 3, p = lane - i * 3;
+            const int n = o * kOctet + i;
+            const bool on = lane < 24 && n < N;
+            int first, steps, degree = 0;
+            if (kAllShared) {
+                first = degrees[cap + (o - o0) * 2];
+                steps = degrees[cap + (o - o0) * 2 + 1];
+                if (on) degree = degrees[n - n0];
+            } else {
+                first = sell_begin[o];
+                steps = sell_begin[o + 1] - first;
+                if (on) degree = row_begin[n + 1] - row_begin[n];
             }
-            g = warp_sum_rnd(g);
-            d = warp_sum_rnd(d);
-            rr = warp_sum_rnd(rr);
+            const int kept = min(cached, steps);  // steps in shared memory
+            StepBlocks ahead;
+            auto fetch = [&](int t) {
+#pragma unroll
+                for (int k = 0; k < kStepsAhead; ++k)
+                    if (t + k < degree) {
+                        const float4* at = B + (long)(first + t + k) * kStepFloat4s + lane;
+                        ahead.node[k] = __ldg(sell_nodes + (long)(first + t + k) * kOctet + i);
+                        ahead.b[k][0] = __ldg(at);
+                        ahead.b[k][1] = __ldg(at + 24);
+                        ahead.b[k][2] = __ldg(at + 48);
+                    }
+            };
+            fetch(kept);
+            RowPair y = {0.0f, 0.0f};
+            if (kAllShared) {
+                if (on) {
+                    const float4* at = reinterpret_cast<const float4*>(diagonal) + (long)(o - o0) * kStepFloat4s + lane;
+                    y = row_pair_dot<true>(at[0], at[24], at[48], U + n * 6);
+                }
+            } else if (on) {
+                const float4* d4 = reinterpret_cast<const float4*>(D + (long)n * 36) + p * 3;
+                float4 q0 = __ldg(d4), q1 = __ldg(d4 + 1), q2 = __ldg(d4 + 2);
+                auto damp = [&](float& x) { x += damping * (scaled ? fmaxf(x, 1e-12f) : 1.0f); };
+                damp(p == 0 ? q0.x : (p == 1 ? q0.z : q1.x));  // (2p, 2p) and (2p + 1, 2p + 1)
+                damp(p == 0 ? q1.w : (p == 1 ? q2.y : q2.w));
+                y = row_pair_dot<true>(q0, q1, q2, U + n * 6);
+            }
+            {
+                const float4* at = cached_blocks + (long)(o - o0) * cached * kStepFloat4s + lane;
+                const int* node = cached_nodes + (o - o0) * cached * kOctet + i;
+                const int end = min(kept, degree);
+#pragma unroll 4
+                for (int t = 0; t < end; ++t) {
+                    const RowPair part = row_pair_dot<false>(at[t * kStepFloat4s], at[t * kStepFloat4s + 24],
+                                                      at[t * kStepFloat4s + 48], U + node[t * kOctet] * 6);
+                    y.a += part.a;
+                    y.b += part.b;
+                }
+            }
+            for (int t = kept; t < degree; t += kStepsAhead) {
+                RowPair part[kStepsAhead];
+#pragma unroll
+                for (int k = 0; k < kStepsAhead; ++k)
+                    if (t + k < degree)
+                        part[k] = row_pair_dot<false>(ahead.b[k][0], ahead.b[k][1], ahead.b[k][2], U + ahead.node[k] * 6);
+#pragma unroll
+                for (int k = 0; k < kStepsAhead; ++k)
+                    if (t + k < degree) {
+                        y.a += part[k].a;
+                        y.b += part[k].b;
+                    }
+                fetch(t + kStepsAhead);
+            }
+            const int first_row = (o * kOctet - n0) * 6;
+            if (on) *reinterpret_cast<float2*>(Wv + first_row + 2 * lane) = make_float2(y.a, y.b);
+            __syncwarp();
+            // the two segments' partials of (r,u), (w,u), (r,r), a row per
+            // lane; the six sums end in lanes 0, 4, 8, 16, 20 and 24
+            double v[6];
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                const int k = first_row + h * 24 + lane;
+                double ui = 0.0, ri = 0.0, wi = 0.0;
+                if (lane < 24 && k < rows) {
+                    ui = (double)U[n0 * 6 + k];
+                    ri = R[k];
+                    wi = (double)Wv[k];
+                }
+                v[3 * h] = rnd(ri * ui);
+                v[3 * h + 1] = rnd(wi * ui);
+                v[3 * h + 2] = rnd(ri * ri);
+            }
+            int held = 0, count = 6;
+            warp_sum_halving<6, 16>(v, lane, held, count, [](double x, double z) { return rnd(x + z); });
+            double partial[6];
+#pragma unroll
+            for (int k = 0; k < 6; ++k)
+                partial[k] = __shfl_sync(0xffffffffu, v[0], (k >= 3 ? 16 : 0) + (k % 3) * 4);
             if (lane < ranks) {  // lane q stores the partials in CTA q's slots
-                double* dst = cluster.map_shared_rank(slots, lane) + 3 * seg;
-                dst[0] = g;
-                dst[1] = d;
-                dst[2] = rr;
+                double* dst = cluster.map_shared_rank(slots, lane) + 6 * o;
+#pragma unroll
+                for (int k = 0; k < 6; ++k) dst[k] = partial[k];
             }
         }
         cluster.sync();
@@ -1126,6 +1322,23 @@ __global__ void __launch_bounds__(kPcgThreads) k_pcg(const WrapDev* __restrict__
     }
     // no CTA may exit while another can still write into its shared memory
     cluster.sync();
+}
+
+__global__ void __launch_bounds__(kPcgThreads) k_pcg(const WrapDev* __restrict__ wraps,
+                                                     const int* __restrict__ index,
+                                                     int budget_floats) {
+    const int slot = index ? index[blockIdx.y] : (int)blockIdx.y;
+    if (slot < 0) return;  // an empty entry of a class launch; uniform across the cluster
+    const WrapDev& w = wraps[slot];
+    const WrapControl c = *w.control;
+    if (c.tick_phase != kPhaseSolve || c.phase != kPhaseSolve) return;  // uniform across the cluster
+    const PcgPlacement place =
+        pcg_place(w.levels[c.level].node_count, (int)cg::this_cluster().num_blocks(), budget_floats);
+    if (place.all()) {
+        pcg_solve<true>(w, c, place, budget_floats);
+    } else {
+        pcg_solve<false>(w, c, place, budget_floats);
+    }
 }
 
 // ---------------------------------------------------------------------------
@@ -1434,27 +1647,27 @@ __global__ void __launch_bounds__(kNodeThreads, 3) k_node_assemble(const WrapDev
         [&](int wi, int bx) { k_node_assemble_body(wraps[wi], part, bx); });
 }
 
-// Writes block k of the system twice, in row-entry order: B where the row
-// list of node a references it, B^T where node b's does.
+// Writes block k of the system twice: B where the row list of node a holds it,
+// B^T where node b's does.
 __device__ inline void store_block_pair(float* out, const LevelDev& L, int k, const float* blk) {
-    float* A = out + (long)L.offdiag_slots[k * 2] * 36;
-    float* T = out + (long)L.offdiag_slots[k * 2 + 1] * 36;
+    float* A = out + block_base(L.sell_slots[k * 2]);
+    float* T = out + block_base(L.sell_slots[k * 2 + 1]);
     for (int r = 0; r < 6; ++r)
         for (int q = 0; q < 6; ++q) {
-            A[r * 6 + q] = blk[r * 6 + q];
-            T[q * 6 + r] = blk[r * 6 + q];
+            A[block_at(r, q)] = blk[r * 6 + q];
+            T[block_at(q, r)] = blk[r * 6 + q];
         }
 }
 
 // Adds block k into the system, both ways (the smoothness edge of a node pair
 // whose shared-vertex block is already there).
 __device__ inline void add_block_pair(float* out, const LevelDev& L, int k, const float* blk) {
-    float* A = out + (long)L.offdiag_slots[k * 2] * 36;
-    float* T = out + (long)L.offdiag_slots[k * 2 + 1] * 36;
+    float* A = out + block_base(L.sell_slots[k * 2]);
+    float* T = out + block_base(L.sell_slots[k * 2 + 1]);
     for (int r = 0; r < 6; ++r)
         for (int q = 0; q < 6; ++q) {
-            A[r * 6 + q] += blk[r * 6 + q];
-            T[q * 6 + r] += blk[r * 6 + q];
+            A[block_at(r, q)] += blk[r * 6 + q];
+            T[block_at(q, r)] += blk[r * 6 + q];
         }
 }
 
@@ -1510,15 +1723,15 @@ __device__ __forceinline__ void k_pair_assemble_body(const WrapDev& w, int part,
     // what it holds, both ways
     int first = 0, count = 36;
     warp_sum_halving<36>(blk, lane, first, count);
-    float* A = w.offdiag[1 - c.system] + (long)L.offdiag_slots[p * 2] * 36;
-    float* T = w.offdiag[1 - c.system] + (long)L.offdiag_slots[p * 2 + 1] * 36;
+    float* A = w.offdiag[1 - c.system] + block_base(L.sell_slots[p * 2]);
+    float* T = w.offdiag[1 - c.system] + block_base(L.sell_slots[p * 2 + 1]);
 #pragma unroll
     for (int i = 0; i < 2; ++i) {
         if (i >= count) break;
         const int j = first + i, r = j / 6, q = j - r * 6;
         const float value = (c.route == 1 && (r < 3 || q < 3)) ? 0.0f : blk[i];
-        A[r * 6 + q] = value;
-        T[q * 6 + r] = value;
+        A[block_at(r, q)] = value;
+        T[block_at(q, r)] = value;
     }
 }
 
@@ -1835,11 +2048,11 @@ void launch_tick(const WrapDev* wraps, const TickShape& s, cudaStream_t stream,
         k_c_rhs<<<grids.c_rhs, kNodeThreads, virtual_smem, stream>>>(wraps, W, solve_part);
     }
     if (timed) cudaEventRecord(timers->pcg_begin, stream);
-    auto launch_pcg = [&](int cluster, int count, int shared, const int* index, cudaStream_t on) {
+    auto launch_pcg = [&](int cluster, int count, const int* index, cudaStream_t on) {
         cudaLaunchConfig_t config = {};
         config.gridDim = dim3(cluster, count);
         config.blockDim = dim3(kPcgThreads);
-        config.dynamicSmemBytes = shared;
+        config.dynamicSmemBytes = kPcgMaxSmemBytes;
         config.stream = on;
         cudaLaunchAttribute attribute[1];
         attribute[0].id = cudaLaunchAttributeClusterDimension;
@@ -1848,21 +2061,19 @@ void launch_tick(const WrapDev* wraps, const TickShape& s, cudaStream_t stream,
         attribute[0].val.clusterDim.z = 1;
         config.attrs = attribute;
         config.numAttrs = 1;
-        cudaLaunchKernelEx(&config, k_pcg, wraps, index, (int)(shared / sizeof(float)));
+        cudaLaunchKernelEx(&config, k_pcg, wraps, index, kPcgMaxSmemBytes / (int)sizeof(float));
     };
     if (s.pcg_groups <= 0) {
-        launch_pcg(s.pcg_cluster, W, s.pcg_shared_bytes, nullptr, stream);
+        launch_pcg(s.pcg_cluster, W, nullptr, stream);
     } else {
         // fork: every class launch after everything before it on `stream`
         cudaEventRecord(s.pcg_fork, stream);
         for (int g = 1; g < s.pcg_groups; ++g) {
             cudaStreamWaitEvent(s.pcg_streams[g], s.pcg_fork, 0);
-            launch_pcg(s.pcg_group_cluster[g], s.pcg_group_count[g], s.pcg_group_shared[g],
-                       s.pcg_group_index[g], s.pcg_streams[g]);
+            launch_pcg(s.pcg_group_cluster[g], s.pcg_group_count[g], s.pcg_group_index[g], s.pcg_streams[g]);
             cudaEventRecord(s.pcg_join[g], s.pcg_streams[g]);
         }
-        launch_pcg(s.pcg_group_cluster[0], s.pcg_group_count[0], s.pcg_group_shared[0],
-                   s.pcg_group_index[0], stream);
+        launch_pcg(s.pcg_group_cluster[0], s.pcg_group_count[0], s.pcg_group_index[0], stream);
         for (int g = 1; g < s.pcg_groups; ++g) cudaStreamWaitEvent(stream, s.pcg_join[g], 0);
     }
     if (timed) cudaEventRecord(timers->pcg_end, stream);
@@ -1919,15 +2130,6 @@ int pcg_cluster_size(int max_nodes, int wraps, int sm_count) {
     int ranks = pcg_latency_cluster(max_nodes);
     while (ranks > 1 && (long)ranks * wraps > sm_count) ranks /= 2;
     return ranks;
-}
-
-// Dynamic shared memory of the solve launch: what the largest wrap would use
-// at this cluster size, at most the per-CTA maximum.
-int pcg_shared_bytes(const int* max_nodes, int wraps, int cluster) {
-    int floats = 0;
-    for (int i = 0; i < wraps; ++i)
-        floats = max(floats, pcg_place(max_nodes[i], cluster, 1 << 30).floats);
-    return min(floats * (int)sizeof(float), kPcgMaxSmemBytes);
 }
 
 int pcg_max_nodes() { return 32768; }
