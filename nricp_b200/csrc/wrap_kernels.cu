@@ -818,7 +818,7 @@ __host__ __device__ inline int pcg_owned_capacity(int nodes, int ranks) {
 // Placement for one wrap within the launch's shared memory, in this order:
 // the segment slots always, the all-node direction copy U if it fits (the
 // matvec reads it ~20 times per row), the owned rows' vectors, their diagonal
-// blocks, the inverses of those, and what is left for the first steps of every
+// blocks, the inverses of those, and what is left for the last steps of every
 // owned octet's off-diagonal blocks.  Whatever does not fit lives in the wrap's
 // global scratch; the arithmetic is the same.
 struct PcgPlacement {
@@ -874,6 +874,9 @@ __device__ __forceinline__ void mbar_init(void* bar, int arrivals) {
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
 }
+__device__ __forceinline__ void mbar_arrive(void* bar) {
+    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(shared_address(bar)) : "memory");
+}
 __device__ __forceinline__ void mbar_arrive_expect(void* bar, int bytes) {
     asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(shared_address(bar)), "r"(bytes)
                  : "memory");
@@ -900,6 +903,27 @@ __device__ __forceinline__ void bulk_to_shared(void* dst, const void* src, int b
     asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
                      shared_address(dst)),
                  "l"(__cvta_generic_to_global(src)), "r"(bytes), "r"(shared_address(bar))
+                 : "memory");
+}
+
+// The same shared-memory address in another CTA of the cluster.
+__device__ __forceinline__ uint32_t peer_address(const void* p, int rank) {
+    uint32_t out;
+    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(out) : "r"(shared_address(p)), "r"(rank));
+    return out;
+}
+// This CTA's shared memory to a peer's, completing on the peer's mbarrier;
+// 16-byte aligned, a multiple of 16 bytes.
+__device__ __forceinline__ void bulk_to_peer(uint32_t dst, const void* src, int bytes, uint32_t bar) {
+    asm volatile("cp.async.bulk.shared::cluster.shared::cta.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
+                     dst),
+                 "r"(shared_address(src)), "r"(bytes), "r"(bar)
+                 : "memory");
+}
+// Two doubles into a peer's shared memory, completing on its mbarrier.
+__device__ __forceinline__ void store_to_peer(uint32_t dst, double a, double b, uint32_t bar) {
+    asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.v2.b64 [%0], {%1, %2}, [%3];" ::"r"(dst),
+                 "l"(__double_as_longlong(a)), "l"(__double_as_longlong(b)), "r"(bar)
                  : "memory");
 }
 
@@ -949,11 +973,13 @@ struct StepBlocks {
 //   p = u + beta p;  s = w + beta s;  x += alpha p;  r -= alpha s.
 //
 // FP32 blocks, matvec, p, s, u and w; FP64 x, r, the inner products and the
-// scalars.  Each CTA writes its slice of u once into its own shared copy and
-// then copies the slice, 16 bytes at a time, into every other CTA's copy
-// through distributed shared memory, so the matvec reads u locally and its
-// only L2 traffic is the blocks (stored in row order).  Two hardware cluster
-// barriers per iteration; nothing spins.
+// scalars.  Each CTA sends its slice of u as one bulk copy per peer through
+// distributed shared memory, and each octet's partial sums with asynchronous
+// stores; both complete on an mbarrier of the receiver, so a CTA waits only for
+// its data, and the loop has no cluster barrier.  What is received is not
+// overwritten early: a peer sends its next u after it has every CTA's sums,
+// which each CTA sends after reading u; and its next sums after it has every
+// CTA's u, which each CTA sends after reading the sums.
 //
 // kAllShared: every array of the placement is in shared memory (the compiler
 // then addresses it as such); the other instance decides at run time.
@@ -1027,11 +1053,12 @@ __device__ __forceinline__ void pcg_solve(const WrapDev& w, const WrapControl& c
     const double tolerance = w.pcg_tolerance;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     __shared__ double red[3][kPcgWarps];
-    __shared__ double tot[3];
-    __shared__ alignas(8) unsigned long long blocks_arrived;  // mbarrier
+    // mbarriers: the cached blocks; an iteration's partial sums; its u
+    __shared__ alignas(8) unsigned long long blocks_arrived, sums_arrived, u_arrived;
     __shared__ int cached_s;
+    bool timed_out = false;  // a wait of this thread ran out
 
-    // ---- the first steps of every owned octet's blocks into the shared
+    // ---- the last steps of every owned octet's blocks into the shared
     //      memory that is left, as many as fit, by bulk copies that run under
     //      the factorisation below ----
     if (warp == 0) {
@@ -1043,6 +1070,8 @@ __device__ __forceinline__ void pcg_solve(const WrapDev& w, const WrapControl& c
         if (lane == 0) {
             cached_s = cached;
             mbar_init(&blocks_arrived, 1);
+            mbar_init(&sums_arrived, kPcgWarps);
+            mbar_init(&u_arrived, 1);
         }
         __syncwarp();
         int bytes = 0;
@@ -1054,7 +1083,8 @@ __device__ __forceinline__ void pcg_solve(const WrapDev& w, const WrapControl& c
         float* block_room = cursor;
         float* node_room = cursor + (long)(o1 - o0) * cached * kStepFloats;
         for (int o = o0 + lane; o < o1; o += 32) {
-            const int first = sell_begin[o], count = min(cached, sell_begin[o + 1] - first);
+            const int count = min(cached, sell_begin[o + 1] - sell_begin[o]);
+            const int first = sell_begin[o + 1] - count;
             if (count <= 0) continue;
             const int at = (o - o0) * cached;
             bulk_to_shared(block_room + (long)at * kStepFloats, B + (long)first * kStepFloat4s,
@@ -1102,75 +1132,119 @@ __device__ __forceinline__ void pcg_solve(const WrapDev& w, const WrapControl& c
         P[i] = 0.0f;
         S[i] = 0.0f;
     }
-    __syncthreads();
-
-    // u = M^-1 r for the owned rows into this CTA's copy, then the slice into
-    // every other CTA's copy (16-byte stores; the slice starts on a segment,
-    // so at a multiple of 96 bytes)
-    auto precondition_and_share = [&]() {
-        for (int i = threadIdx.x; i < rows; i += blockDim.x) {
-            const int m = i / 6, r = i - m * 6;
-            const float* mi = Minv + m * 36 + r * 6;
-            float z = 0.0f;
-            for (int q = 0; q < 6; ++q) z += mi[q] * (float)R[m * 6 + q];
-            U[n0 * 6 + i] = z;
-        }
-        if ((kAllShared || place.u_shared) && ranks > 1) {
-            __syncthreads();
-            const float4* src = reinterpret_cast<const float4*>(U + n0 * 6);
-            const int vec = rows / 4;  // rows = 6 * own, own a multiple of 4 except at the end
-            for (int q = 1; q < ranks; ++q) {
-                const int dst_rank = (rank + q) % ranks;
-                float4* dst = reinterpret_cast<float4*>(cluster.map_shared_rank(U, dst_rank) + n0 * 6);
-                for (int k = threadIdx.x; k < vec; k += blockDim.x) dst[k] = src[k];
-                float* dst_tail = cluster.map_shared_rank(U, dst_rank) + n0 * 6;
-                for (int k = vec * 4 + threadIdx.x; k < rows; k += blockDim.x) dst_tail[k] = U[n0 * 6 + k];
-            }
-        }
-        if (!kAllShared && !place.u_shared) __threadfence();  // the global copy: visible device-wide first
-    };
-    precondition_and_share();
+    // every CTA's rows and mbarriers are ready
     cluster.sync();
 
     const int cached = cached_s;
     const float4* cached_blocks = reinterpret_cast<const float4*>(cursor);
     const int* cached_nodes = reinterpret_cast<const int*>(cursor + (long)(o1 - o0) * cached * kStepFloats);
-    if (!mbar_wait(&blocks_arrived, 0)) atomicOr(&w.control->error, kErrorSolveWait);
+    if (!mbar_wait(&blocks_arrived, 0)) timed_out = true;
 
-    double gamma_prev = 0.0, alpha_prev = 0.0, bnorm = 0.0, residual = 0.0;
+    // The CTAs that own rows; the others only wait at the end.  (Where u is
+    // global the loop meets at cluster barriers, and a graph that large gives
+    // every CTA rows.)
+    const int active = (octets * kOctet + cap - 1) / cap;
+    const bool u_shared = kAllShared || place.u_shared;
+    const int u_bytes = ((N * 6 + 3) & ~3) * (int)sizeof(float);  // of every row
+    const int own_bytes = (rank == active - 1 ? u_bytes : n1 * 24) - n0 * 24;
+    const int peer = min(lane, active - 1);
+    const uint32_t peer_slots = peer_address(slots, peer), peer_sums_arrived = peer_address(&sums_arrived, peer);
+
+    // One segment's rows per warp at a time: `update` forms r[i], then
+    // u = M^-1 r into this CTA's copy.
+    auto segment_rows = [&](auto update) {
+        for (int sl = warp; sl * 24 < rows; sl += kPcgWarps) {
+            const int i = sl * 24 + lane;
+            const bool on = lane < 24 && i < rows;
+            if (on) update(i);
+            __syncwarp();
+            if (on) {
+                const int m = sl * 4 + lane / 6, r = lane % 6;
+                const float* mi = Minv + m * 36 + r * 6;
+                float z = 0.0f;
+                for (int q = 0; q < 6; ++q) z += mi[q] * (float)R[m * 6 + q];
+                U[n0 * 6 + i] = z;
+            }
+        }
+    };
+    // The slice of u into every other CTA's copy: one bulk copy per peer,
+    // which completes on the peer's mbarrier.
+    auto share_u = [&]() {
+        if (!u_shared) {
+            __threadfence();  // the global copy: visible device-wide first
+            cluster.sync();
+            return;
+        }
+        if (active > 1) asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+        __syncthreads();
+        if (active > 1 && warp == 0) {
+            if (lane == 0) mbar_arrive_expect(&u_arrived, u_bytes - own_bytes);
+            if (lane < active && lane != rank)
+                bulk_to_peer(peer_address(U, lane) + n0 * 24, U + n0 * 6, own_bytes, peer_address(&u_arrived, lane));
+        }
+    };
+    // A few streamed steps of octet o (its first `streamed`) into registers.
+    const int i_node = lane / 3, p_row = lane - i_node * 3;
+    StepBlocks ahead;
+    auto fetch = [&](int first, int t, int end) {
+#pragma unroll
+        for (int k = 0; k < kStepsAhead; ++k)
+            if (t + k < end) {
+                const float4* at = B + (long)(first + t + k) * kStepFloat4s + lane;
+                ahead.node[k] = __ldg(sell_nodes + (long)(first + t + k) * kOctet + i_node);
+                ahead.b[k][0] = __ldg(at);
+                ahead.b[k][1] = __ldg(at + 24);
+                ahead.b[k][2] = __ldg(at + 48);
+            }
+    };
+    struct OctetShape { int first, streamed, degree; };
+    auto octet_shape = [&](int o) {
+        OctetShape x;
+        const int n = o * kOctet + i_node;
+        const bool on = lane < 24 && n < N;
+        int steps;
+        x.degree = 0;
+        if (kAllShared) {
+            x.first = degrees[cap + (o - o0) * 2];
+            steps = degrees[cap + (o - o0) * 2 + 1];
+            if (on) x.degree = degrees[n - n0];
+        } else {
+            x.first = sell_begin[o];
+            steps = sell_begin[o + 1] - x.first;
+            if (on) x.degree = row_begin[n + 1] - row_begin[n];
+        }
+        x.streamed = max(0, steps - cached);
+        return x;
+    };
+    // The warp's first streamed steps do not depend on u: they are fetched
+    // before the wait for it.
+    OctetShape shape = {0, 0, 0};
+    auto fetch_first = [&]() {
+        if (o0 + warp < o1) {
+            shape = octet_shape(o0 + warp);
+            fetch(shape.first, 0, min(shape.streamed, shape.degree));
+        }
+    };
+    if (own > 0) {
+        segment_rows([](int) {});
+        share_u();
+        fetch_first();
+    }
+
+    double gamma_prev = 0.0, alpha_prev = 0.0, bnorm = 0.0, residual = 0.0, surely_above = 0.0;
     int iterations = 0;
     bool converged = false;
-    for (int it = 0;; ++it) {
+    for (int it = 0; own > 0; ++it) {
+        if (u_shared && active > 1 && !mbar_wait(&u_arrived, it & 1)) timed_out = true;
         // ---- w = A u for the owned rows, an octet per warp at a time: lane
         //      3i + p multiplies rows 2p and 2p + 1 of the octet's node i ----
         for (int o = o0 + warp; o < o1; o += kPcgWarps) {
-            const int i = lane / 3, p = lane - i * 3;
-            const int n = o * kOctet + i;
+            const int n = o * kOctet + i_node;
             const bool on = lane < 24 && n < N;
-            int first, steps, degree = 0;
-            if (kAllShared) {
-                first = degrees[cap + (o - o0) * 2];
-                steps = degrees[cap + (o - o0) * 2 + 1];
-                if (on) degree = degrees[n - n0];
-            } else {
-                first = sell_begin[o];
-                steps = sell_begin[o + 1] - first;
-                if (on) degree = row_begin[n + 1] - row_begin[n];
+            if (o != o0 + warp) {
+                shape = octet_shape(o);
+                fetch(shape.first, 0, min(shape.streamed, shape.degree));
             }
-            const int kept = min(cached, steps);  // steps in shared memory
-            StepBlocks ahead;
-            auto fetch = [&](int t) {
-#pragma unroll
-                for (int k = 0; k < kStepsAhead; ++k)
-                    if (t + k < degree) {
-                        const float4* at = B + (long)(first + t + k) * kStepFloat4s + lane;
-                        ahead.node[k] = __ldg(sell_nodes + (long)(first + t + k) * kOctet + i);
-                        ahead.b[k][0] = __ldg(at);
-                        ahead.b[k][1] = __ldg(at + 24);
-                        ahead.b[k][2] = __ldg(at + 48);
-                    }
-            };
-            fetch(kept);
             RowPair y = {0.0f, 0.0f};
             if (kAllShared) {
                 if (on) {
@@ -1178,38 +1252,49 @@ __device__ __forceinline__ void pcg_solve(const WrapDev& w, const WrapControl& c
                     y = row_pair_dot<true>(at[0], at[24], at[48], U + n * 6);
                 }
             } else if (on) {
-                const float4* d4 = reinterpret_cast<const float4*>(D + (long)n * 36) + p * 3;
+                const float4* d4 = reinterpret_cast<const float4*>(D + (long)n * 36) + p_row * 3;
                 float4 q0 = __ldg(d4), q1 = __ldg(d4 + 1), q2 = __ldg(d4 + 2);
                 auto damp = [&](float& x) { x += damping * (scaled ? fmaxf(x, 1e-12f) : 1.0f); };
-                damp(p == 0 ? q0.x : (p == 1 ? q0.z : q1.x));  // (2p, 2p) and (2p + 1, 2p + 1)
-                damp(p == 0 ? q1.w : (p == 1 ? q2.y : q2.w));
+                damp(p_row == 0 ? q0.x : (p_row == 1 ? q0.z : q1.x));  // (2p, 2p) and (2p + 1, 2p + 1)
+                damp(p_row == 0 ? q1.w : (p_row == 1 ? q2.y : q2.w));
                 y = row_pair_dot<true>(q0, q1, q2, U + n * 6);
             }
             {
-                const float4* at = cached_blocks + (long)(o - o0) * cached * kStepFloat4s + lane;
-                const int* node = cached_nodes + (o - o0) * cached * kOctet + i;
-                const int end = min(kept, degree);
-#pragma unroll 4
-                for (int t = 0; t < end; ++t) {
-                    const RowPair part = row_pair_dot<false>(at[t * kStepFloat4s], at[t * kStepFloat4s + 24],
-                                                      at[t * kStepFloat4s + 48], U + node[t * kOctet] * 6);
-                    y.a += part.a;
-                    y.b += part.b;
+                const int end = min(shape.streamed, shape.degree);
+                for (int t = 0; t < end; t += kStepsAhead) {
+                    RowPair part[kStepsAhead];
+#pragma unroll
+                    for (int k = 0; k < kStepsAhead; ++k)
+                        if (t + k < end)
+                            part[k] = row_pair_dot<false>(ahead.b[k][0], ahead.b[k][1], ahead.b[k][2], U + ahead.node[k] * 6);
+#pragma unroll
+                    for (int k = 0; k < kStepsAhead; ++k)
+                        if (t + k < end) {
+                            y.a += part[k].a;
+                            y.b += part[k].b;
+                        }
+                    fetch(shape.first, t + kStepsAhead, end);
                 }
             }
-            for (int t = kept; t < degree; t += kStepsAhead) {
-                RowPair part[kStepsAhead];
+            {
+                const float4* at = cached_blocks + (long)(o - o0) * cached * kStepFloat4s + lane;
+                const int* node = cached_nodes + (o - o0) * cached * kOctet + i_node;
+                const int end = shape.degree - shape.streamed;
+                for (int t = 0; t < end; t += kStepsAhead) {
+                    RowPair part[kStepsAhead];
 #pragma unroll
-                for (int k = 0; k < kStepsAhead; ++k)
-                    if (t + k < degree)
-                        part[k] = row_pair_dot<false>(ahead.b[k][0], ahead.b[k][1], ahead.b[k][2], U + ahead.node[k] * 6);
-#pragma unroll
-                for (int k = 0; k < kStepsAhead; ++k)
-                    if (t + k < degree) {
-                        y.a += part[k].a;
-                        y.b += part[k].b;
+                    for (int k = 0; k < kStepsAhead; ++k) {
+                        const int tk = min(t + k, end - 1);  // past the end: the last one again, not added
+                        part[k] = row_pair_dot<false>(at[tk * kStepFloat4s], at[tk * kStepFloat4s + 24],
+                                                      at[tk * kStepFloat4s + 48], U + node[tk * kOctet] * 6);
                     }
-                fetch(t + kStepsAhead);
+#pragma unroll
+                    for (int k = 0; k < kStepsAhead; ++k)
+                        if (t + k < end) {
+                            y.a += part[k].a;
+                            y.b += part[k].b;
+                        }
+                }
             }
             const int first_row = (o * kOctet - n0) * 6;
             if (on) *reinterpret_cast<float2*>(Wv + first_row + 2 * lane) = make_float2(y.a, y.b);
@@ -1236,61 +1321,87 @@ __device__ __forceinline__ void pcg_solve(const WrapDev& w, const WrapControl& c
 #pragma unroll
             for (int k = 0; k < 6; ++k)
                 partial[k] = __shfl_sync(0xffffffffu, v[0], (k >= 3 ? 16 : 0) + (k % 3) * 4);
-            if (lane < ranks) {  // lane q stores the partials in CTA q's slots
-                double* dst = cluster.map_shared_rank(slots, lane) + 6 * o;
-#pragma unroll
-                for (int k = 0; k < 6; ++k) dst[k] = partial[k];
+            if (active == 1) {
+                if (lane == 0)
+                    for (int k = 0; k < 6; ++k) slots[6 * o + k] = partial[k];
+            } else if (lane < active) {  // lane q stores the partials in CTA q's slots
+                const uint32_t dst = peer_slots + 48 * o;
+                store_to_peer(dst, partial[0], partial[1], peer_sums_arrived);
+                store_to_peer(dst + 16, partial[2], partial[3], peer_sums_arrived);
+                store_to_peer(dst + 32, partial[4], partial[5], peer_sums_arrived);
             }
         }
-        cluster.sync();
-        // ---- totals over every segment, in one fixed order in every CTA ----
+        __syncwarp();
+        if (threadIdx.x == 0) {
+            mbar_arrive_expect(&sums_arrived, active > 1 ? 48 * octets : 0);
+        } else if (lane == 0) {
+            mbar_arrive(&sums_arrived);
+        }
+        if (!mbar_wait(&sums_arrived, it & 1)) timed_out = true;
+        // ---- totals over every segment, in one fixed order in every CTA:
+        //      each warp its stride of the segments, then every warp the same
+        //      butterfly over the warps' sums ----
+        double gamma, delta, rr_total;
         {
-            double g = 0.0, d = 0.0, rr = 0.0;
-            for (int sg = threadIdx.x; sg < segs; sg += blockDim.x) {
-                g = rnd(g + slots[3 * sg]);
-                d = rnd(d + slots[3 * sg + 1]);
-                rr = rnd(rr + slots[3 * sg + 2]);
+            double v[3] = {0.0, 0.0, 0.0};
+            if (warp * 32 < segs) {
+                for (int sg = threadIdx.x; sg < segs; sg += blockDim.x)
+                    for (int k = 0; k < 3; ++k) v[k] = rnd(v[k] + slots[3 * sg + k]);
+                int held = 0, count = 3;
+                warp_sum_halving<3, 16>(v, lane, held, count, [](double x, double z) { return rnd(x + z); });
             }
-            g = warp_sum_rnd(g);
-            d = warp_sum_rnd(d);
-            rr = warp_sum_rnd(rr);
-            if (lane == 0) { red[0][warp] = g; red[1][warp] = d; red[2][warp] = rr; }
-            __syncthreads();
-            if (warp == 0) {
-                for (int k = 0; k < 3; ++k) {
-                    double v = lane < kPcgWarps ? red[k][lane] : 0.0;
-                    v = warp_sum_rnd(v);
-                    if (lane == 0) tot[k] = v;
-                }
+            // the sums end in lanes 0, 8 and 16
+            if (lane == 0 || lane == 8 || lane == 16) red[lane >> 3][warp] = v[0];
+            const bool failed = __syncthreads_or(timed_out);
+            double a = red[lane >> 4][lane & 15], b2 = red[2][lane & 15];
+            static_assert(kPcgWarps == 16, "a half warp per sum");
+            for (int o = 8; o > 0; o >>= 1) {
+                a = rnd(a + __shfl_xor_sync(0xffffffffu, a, o));
+                b2 = rnd(b2 + __shfl_xor_sync(0xffffffffu, b2, o));
             }
-            __syncthreads();
+            gamma = __shfl_sync(0xffffffffu, a, 0);
+            delta = __shfl_sync(0xffffffffu, a, 16);
+            rr_total = b2;
+            if (failed) {  // uniform over the CTA; its peers' waits run out in turn
+                if (threadIdx.x == 0) atomicOr(&w.control->error, kErrorSolveWait);
+                for (int i = 0; i < 256; ++i) __nanosleep(10000);  // the copies in flight
+                break;
+            }
         }
-        const double gamma = tot[0], delta = tot[1], rr_total = tot[2];
         if (it == 0) {
             bnorm = rnd(sqrt(rr_total));
             if (!(bnorm > 0.0)) { converged = true; residual = 0.0; break; }
+            // |r|^2 above this is surely not converged: the comparison below
+            // without its root and quotient
+            const double limit = tolerance * bnorm;
+            surely_above = limit > 1e-140 ? limit * limit * (1.0 + 1e-6) : 1e300;
         }
-        residual = rnd(rnd(sqrt(rr_total)) / bnorm);
-        if (residual <= tolerance) { converged = true; break; }
-        if (it >= max_iterations) break;
+        const bool capped = it >= max_iterations;
+        if (capped || !(rr_total > surely_above)) {
+            residual = rnd(rnd(sqrt(rr_total)) / bnorm);
+            if (residual <= tolerance) { converged = true; break; }
+            if (capped) break;
+        }
         const double beta = it == 0 ? 0.0 : rnd(gamma / gamma_prev);
         const double denominator = it == 0 ? delta : rnd(delta - rnd(rnd(beta * gamma) / alpha_prev));
-        if (!(fabs(denominator) > 1e-300)) break;
+        if (!(fabs(denominator) > 1e-300)) {
+            residual = rnd(rnd(sqrt(rr_total)) / bnorm);
+            break;
+        }
         const double alpha = rnd(gamma / denominator);
         gamma_prev = gamma;
         alpha_prev = alpha;
         // ---- p, s, x, r for the owned rows; then u = M^-1 r, shared ----
-        for (int i = threadIdx.x; i < rows; i += blockDim.x) {
+        segment_rows([&](int i) {
             const float pn = (float)((double)U[n0 * 6 + i] + rnd(beta * (double)P[i]));
             const float sn = (float)((double)Wv[i] + rnd(beta * (double)S[i]));
             P[i] = pn;
             S[i] = sn;
             X[i] = rnd(X[i] + rnd(alpha * (double)pn));
             R[i] = rnd(R[i] - rnd(alpha * (double)sn));
-        }
-        __syncthreads();
-        precondition_and_share();
-        cluster.sync();
+        });
+        share_u();
+        fetch_first();
         iterations = it + 1;
     }
     if (rank == 0 && threadIdx.x == 0) {
