@@ -10,12 +10,14 @@
 // stored in its parent (64 B per internal node = one L2 line pair), so a
 // visit costs one 64-byte load instead of three dependent ones.
 //
-// Query (thread per template vertex): the previous correspondence's triangle
+// Query (a group of lanes per template vertex): the previous correspondence's triangle
 // seeds the search radius, the traversal prunes FP32 boxes with a fixed-depth
 // stack whose overflow is reported (never silently pruned), and every
 // triangle it reaches is measured with the reference's FP64 closest-point
 // routine (src/geometry/closest_point.cpp:24-121), so the winner, its point,
 // normal and distance are those of an FP64 brute-force scan.
+#include <type_traits>
+
 #include "common.cuh"
 #include "kernels.cuh"
 
@@ -736,120 +738,147 @@ __device__ int nearest_triangle(const WrapDev& w, F3 q, D3 q64, int seed, int* o
 // or above the fan of slivers at a lat-long pole, stays far from the nearest
 // triangles and walks hundreds to thousands of steps query after query).
 constexpr long kLongWalk = 256;
-// A warp's stack: 32 entries for each of 32 levels of pending subtrees.
+// Lanes per query for `total` queries on a grid of `resident` threads: the
+// widest groups that keep the grid about as busy.  A walk's time is its chain of
+// dependent rounds, so a few queries want wide groups; many queries fill the
+// device anyway, and narrower groups visit fewer subtrees that a bound found
+// meanwhile would have pruned.
+__host__ __device__ inline int group_lanes(long total, long resident) {
+    return total * 16 <= resident * 2 ? 16 : (total * 8 <= resident * 4 ? 8 : 4);
+}
+
+// The warps' stacks of pending subtrees: 1,024 entries per warp, shared by its
+// groups of G lanes.
 constexpr int kWarpStack = 1024;
 
-// The nearest triangle for `q` found by the 32 lanes of a warp together: the
-// same pruning and the same winner rule as `nearest_triangle`, so the same
-// answer, with up to 32 pending subtrees taken from the stack at a time, so
-// that a walk of thousands of steps takes tens to a hundred dependent rounds.
-// `nodes` / `dists` are the warp's stack.  Should the stack not hold a
-// round's children, the rest of the walk is left to one lane
-// (`*unfinished`), seeded with the winner so far, which is returned.  Every
-// lane returns the same triangle; `*work` is the entries taken.
-__device__ int nearest_triangle_warp(const WrapDev& w, F3 q, D3 q64, int seed, uint32_t* nodes,
-                                     float* dists, int* overflow, bool* unfinished, long* work) {
-    const int lane = threadIdx.x & 31;
-    const double slack = (double)w.rank_window;
+// The nearest triangle for `q` found by a group of G lanes of a warp (each
+// group its own query): the same pruning and the same winner rule as
+// `nearest_triangle`, so the same answer, with up to G pending subtrees taken
+// from the stack at a time, so that a walk takes several times fewer dependent
+// rounds.  All 32 lanes call it together, and a warp's groups run their rounds
+// side by side until the last is done; `on` is false for a group without a
+// query.  `nodes` / `dists` are the group's stack (kWarpStack * G / 32
+// entries).  Should the stack not hold a round's children, the rest of the
+// walk is left to one lane (`*unfinished`), seeded with the winner so far,
+// which is returned.  Every lane of a group returns the same triangle; `*work`
+// is the entries taken.
+template <int G>
+__device__ int nearest_triangle_group(const WrapDev& w, bool on, F3 q, D3 q64, int seed, uint32_t* nodes,
+                                      float* dists, int* overflow, bool* unfinished, long* work) {
+    constexpr int kStack = kWarpStack * G / 32;
+    const int lane = threadIdx.x & 31, at_group = lane & (G - 1);
+    const uint32_t group = (G == 32 ? 0xffffffffu : ((1u << (G & 31)) - 1u)) << (lane - at_group);
+    const uint32_t below = group & ((1u << lane) - 1u);
+    const double slack = on ? (double)w.rank_window : 0.0;
     double best = 1e300;
     int best_tri = -1;
     float bound = 3.4e38f;
-    if (seed >= 0 && seed < w.F) {
+    if (on && seed >= 0 && seed < w.F) {
         best = triangle_distance_fp64(w, q64, seed);
         best_tri = seed;
         const double r = sqrt(best) + slack;
         bound = __double2float_ru(r * r);
     }
-    if (lane == 0) {
-        nodes[0] = (uint32_t)w.bvh_root;
-        dists[0] = 0.0f;
+    // The stack holds pending internal nodes from its bottom up and pending
+    // leaves from its top down; a round takes one kind for the whole warp, so
+    // that the FP64 measurement and the box tests do not run by turns under
+    // half-empty masks.
+    const uint32_t root = on ? (uint32_t)w.bvh_root : 0;
+    if (on && at_group == 0) {
+        nodes[(root & kLeafBit) ? kStack - 1 : 0] = root;
+        dists[(root & kLeafBit) ? kStack - 1 : 0] = 0.0f;
     }
-    int sp = 1;  // warp-uniform
-    const long round_limit = 4L * (long)w.F + 1024;
+    int inner = on && !(root & kLeafBit) ? 1 : 0;  // the same in a group's lanes
+    int leaves = on && (root & kLeafBit) ? 1 : 0;
+    const long round_limit = on ? 4L * (long)w.F + 1024 : 0;
     long rounds = 0, taken = 0;
     *unfinished = false;
     __syncwarp();
-    while (sp > 0) {
-        if (++rounds > round_limit) {  // a corrupt hierarchy: report, do not loop
+    while (__any_sync(0xffffffffu, inner + leaves > 0)) {
+        if (inner + leaves > 0 && ++rounds > round_limit) {  // a corrupt hierarchy: report, do not loop
             *overflow = 1;
-            break;
+            inner = leaves = 0;
         }
-        const int take = sp < 32 ? sp : 32;
-        sp -= take;
+        // leaves once some group can fill its lanes with them, or nothing else is left
+        if (__any_sync(0xffffffffu, leaves >= G) || !__any_sync(0xffffffffu, inner > 0)) {
+            // FP64 distances, then the group's winner under the exact rule
+            const int take = leaves < G ? leaves : G;
+            const int first = kStack - leaves;
+            leaves -= take;
+            taken += take;
+            double d = 1e300;
+            int tri = 0x7fffffff;
+            if (at_group < take && dists[first + at_group] < bound) {
+                int t;
+                const double x = leaf_distance(w, (int)(nodes[first + at_group] & ~kLeafBit), q64, &t);
+                if (t != seed) {
+                    d = x;
+                    tri = t;
+                }
+            }
+            for (int o = G / 2; o > 0; o >>= 1) {
+                const double od = __shfl_xor_sync(0xffffffffu, d, o);
+                const int ot = __shfl_xor_sync(0xffffffffu, tri, o);
+                if (od < d || (od == d && ot < tri)) {
+                    d = od;
+                    tri = ot;
+                }
+            }
+            if (d < best || (d == best && tri < best_tri)) {
+                best = d;
+                best_tri = tri;
+                const double r = sqrt(best) + slack;
+                bound = __double2float_ru(r * r);
+            }
+            continue;
+        }
+        const int take = inner < G ? inner : G;
+        inner -= take;
         taken += take;
-        uint32_t node = 0;
-        bool live = false;
-        if (lane < take) {
-            node = nodes[sp + lane];
-            live = dists[sp + lane] < bound;
+        bool push[2] = {false, false};  // left, right child
+        uint32_t child[2] = {0, 0};
+        float dist[2] = {0.0f, 0.0f};
+        if (at_group < take && dists[inner + at_group] < bound) {
+            const float4* nd = w.bvh_nodes + (long)nodes[inner + at_group] * 4;
+            const float4 n0 = __ldg(nd), n1 = __ldg(nd + 1), n2 = __ldg(nd + 2), n3 = __ldg(nd + 3);
+            dist[0] = box_distance(q, n0.x, n0.y, n0.z, n0.w, n1.x, n1.y);
+            dist[1] = box_distance(q, n1.z, n1.w, n2.x, n2.y, n2.z, n2.w);
+            child[0] = __float_as_uint(n3.x);
+            child[1] = __float_as_uint(n3.y);
+            // the nearer child second: it is taken first
+            if (dist[0] < dist[1]) {
+                const float x = dist[0]; dist[0] = dist[1]; dist[1] = x;
+                const uint32_t y = child[0]; child[0] = child[1]; child[1] = y;
+            }
+            push[0] = dist[0] < bound;
+            push[1] = dist[1] < bound;
         }
         __syncwarp();
-        // leaves: FP64 distance, then the warp's winner under the exact rule
-        double d = 1e300;
-        int tri = 0x7fffffff;
-        if (live && (node & kLeafBit)) {
-            int t;
-            const double x = leaf_distance(w, (int)(node & ~kLeafBit), q64, &t);
-            if (t != seed) {
-                d = x;
-                tri = t;
-            }
+        // each kind's place: the lanes' farther children, then their nearer ones
+        int new_inner = 0, new_leaves = 0, place[2] = {0, 0};
+#pragma unroll
+        for (int k = 0; k < 2; ++k) {
+            const bool leaf = (child[k] & kLeafBit) != 0;
+            const uint32_t to_inner = __ballot_sync(0xffffffffu, push[k] && !leaf) & group;
+            const uint32_t to_leaves = __ballot_sync(0xffffffffu, push[k] && leaf) & group;
+            place[k] = leaf ? kStack - 1 - (leaves + new_leaves + __popc(to_leaves & below))
+                            : inner + new_inner + __popc(to_inner & below);
+            new_inner += __popc(to_inner);
+            new_leaves += __popc(to_leaves);
         }
-        for (int o = 16; o > 0; o >>= 1) {
-            const double od = __shfl_xor_sync(0xffffffffu, d, o);
-            const int ot = __shfl_xor_sync(0xffffffffu, tri, o);
-            if (od < d || (od == d && ot < tri)) {
-                d = od;
-                tri = ot;
-            }
-        }
-        if (d < best || (d == best && tri < best_tri)) {
-            best = d;
-            best_tri = tri;
-            const double r = sqrt(best) + slack;
-            bound = __double2float_ru(r * r);
-        }
-        // internal nodes: the children that can still hold something closer,
-        // the nearer one pushed last (taken first)
-        uint32_t push[2] = {0, 0};
-        float push_d[2] = {0.0f, 0.0f};
-        int pushes = 0;
-        if (live && !(node & kLeafBit)) {
-            const float4* nd = w.bvh_nodes + (long)node * 4;
-            const float4 n0 = __ldg(nd), n1 = __ldg(nd + 1), n2 = __ldg(nd + 2), n3 = __ldg(nd + 3);
-            const float dl = box_distance(q, n0.x, n0.y, n0.z, n0.w, n1.x, n1.y);
-            const float dr = box_distance(q, n1.z, n1.w, n2.x, n2.y, n2.z, n2.w);
-            const uint32_t cl = __float_as_uint(n3.x), cr = __float_as_uint(n3.y);
-            const bool hl = dl < bound, hr = dr < bound;
-            const bool left_first = dl <= dr;
-            if (hl && hr) {
-                push[0] = left_first ? cr : cl;
-                push_d[0] = left_first ? dr : dl;
-                push[1] = left_first ? cl : cr;
-                push_d[1] = left_first ? dl : dr;
-                pushes = 2;
-            } else if (hl || hr) {
-                push[0] = hl ? cl : cr;
-                push_d[0] = hl ? dl : dr;
-                pushes = 1;
-            }
-        }
-        int at = pushes;  // inclusive prefix over the lanes, then exclusive
-        for (int o = 1; o < 32; o <<= 1) {
-            const int y = __shfl_up_sync(0xffffffffu, at, o);
-            if (lane >= o) at += y;
-        }
-        const int total = __shfl_sync(0xffffffffu, at, 31);
-        at -= pushes;
-        if (sp + total > kWarpStack) {  // the rest by one lane, from the winner so far
+        if (inner + new_inner + leaves + new_leaves > kStack) {  // the rest by one lane, from the winner so far
             *unfinished = true;
-            break;
+            inner = leaves = 0;
+        } else {
+#pragma unroll
+            for (int k = 0; k < 2; ++k)
+                if (push[k]) {
+                    nodes[place[k]] = child[k];
+                    dists[place[k]] = dist[k];
+                }
+            inner += new_inner;
+            leaves += new_leaves;
         }
-        for (int k = 0; k < pushes; ++k) {
-            nodes[sp + at + k] = push[k];
-            dists[sp + at + k] = push_d[k];
-        }
-        sp += total;
         __syncwarp();
     }
     *work = taken;
@@ -913,30 +942,6 @@ __device__ inline void store_masked(const WrapDev& w, int v) {
     w.robust[v] = 1.0;
 }
 
-// The correspondence of template vertex v, found by one thread.
-__device__ void query_vertex(const WrapDev& w, int level, int v) {
-    if (w.mask && !w.mask[v]) {
-        store_masked(w, v);
-        return;
-    }
-    const float4 q32 = w.deformed32[v];
-    int overflow = 0;
-    const int tri = nearest_triangle(w, {q32.x, q32.y, q32.z}, load_d3(w.deformed, v), w.corr_triangle[v],
-                                     &overflow);
-    if (overflow) atomicOr(&w.control->error, kErrorTraversal);
-    store_correspondence(w, level, v, tri);
-}
-
-// Thread per vertex, block row per wrap.
-__global__ void k_query(const WrapDev* __restrict__ wraps) {
-    const WrapDev& w = wraps[blockIdx.y];
-    const WrapControl c = *w.control;
-    if (!queries(c.tick_phase)) return;
-    const int v = blockIdx.x * blockDim.x + threadIdx.x;
-    if (v >= w.V) return;
-    query_vertex(w, c.level, v);
-}
-
 // Puts vertex v on the wrap's list of long walks for its next query (list
 // 1 - long_cur), unless the list is full.
 __device__ inline void list_long_walk(const WrapDev& w, int next, int v) {
@@ -947,15 +952,16 @@ __device__ inline void list_long_walk(const WrapDev& w, int next, int v) {
     }
 }
 
-// The same work as queues over a grid that fits on the device at once.
-// First, the vertices whose walk was long at the wrap's previous query (its
-// list), a warp each.  Then every other vertex of every querying wrap, in
-// wrap then vertex order, handed out 32 at a time to whichever warp is free
-// (a walk's length varies a lot from vertex to vertex, so fixed blocks would
-// hold an SM until their slowest warp ends).  A launch lasts as long as its
-// longest walks: the warps take those at its start, in tens of dependent
-// rounds, beside the threads' walks instead of after them.  A walk longer
-// than kLongWalk steps lists its vertex for the wrap's next query.
+// The closest points of every querying wrap, as queues over a grid that fits on
+// the device at once.  First, the vertices whose walk was long at the wrap's
+// previous query (its list), a warp each.  Then every other vertex of every
+// querying wrap, in wrap then vertex order, handed out to whichever warp is
+// free, a group of 4, 8 or 16 lanes per vertex (group_lanes).  A thread per
+// vertex left a launch waiting for a chain of a few hundred dependent fetches
+// with a few lanes of each warp alive; groups cut the chain and share its
+// fetches: the queries of a 25,000-vertex wrap onto 394,000 triangles took
+// 18.7 ms, now 5.8; of 16 uneven wraps in a batch 70 ms, now 32.  A walk longer
+// than kLongWalk lists its vertex for the wrap's next query.
 // counter[0]: the vertices' queue head; counter[1]: the long walks'; both
 // start at 0.
 __global__ void __launch_bounds__(128) k_query_queue(const WrapDev* __restrict__ wraps, int wrap_count,
@@ -999,11 +1005,11 @@ __global__ void __launch_bounds__(128) k_query_queue(const WrapDev* __restrict__
         }
         return lo;
     };
+    uint32_t* const warp_nodes = stack_nodes + (threadIdx.x >> 5) * kWarpStack;
+    float* const warp_dists = stack_dists + (threadIdx.x >> 5) * kWarpStack;
     // ---- the listed long walks, a warp each ----
     {
         const int total = first_long[wrap_count];
-        uint32_t* nodes = stack_nodes + (threadIdx.x >> 5) * kWarpStack;
-        float* dists = stack_dists + (threadIdx.x >> 5) * kWarpStack;
         while (true) {
             int item = 0;
             if (lane == 0) item = atomicAdd(counter + 1, 1);
@@ -1019,8 +1025,8 @@ __global__ void __launch_bounds__(128) k_query_queue(const WrapDev* __restrict__
             int overflow = 0;
             bool unfinished = false;
             long work = 0;
-            int tri = nearest_triangle_warp(w, q, q64, w.corr_triangle[v], nodes, dists, &overflow,
-                                            &unfinished, &work);
+            int tri = nearest_triangle_group<32>(w, true, q, q64, w.corr_triangle[v], warp_nodes, warp_dists,
+                                                 &overflow, &unfinished, &work);
             if (lane == 0) {
                 if (unfinished) tri = nearest_triangle(w, q, q64, tri, &overflow);
                 if (overflow) atomicOr(&w.control->error, kErrorTraversal);
@@ -1030,48 +1036,84 @@ __global__ void __launch_bounds__(128) k_query_queue(const WrapDev* __restrict__
             __syncwarp();
         }
     }
-    // ---- every other vertex, a thread each ----
+    // ---- every other vertex, a group of lanes each ----
     const int total = first[wrap_count];
-    while (true) {
-        int base = 0;
-        if (lane == 0) base = atomicAdd(counter, 32);
-        base = __shfl_sync(0xffffffffu, base, 0);
-        if (base >= total) break;
-        const int item = base + lane;
-        if (item >= total) continue;
-        const int wi = wrap_of(first, item);
-        const WrapDev& w = wraps[wi];
-        const int v = item - first[wi];
-        if (w.mask && !w.mask[v]) {
-            store_masked(w, v);
-            continue;
+    auto others = [&](auto lanes) {
+        constexpr int G = decltype(lanes)::value;
+        constexpr int kGroups = 32 / G;
+        const int group = lane / G;
+        while (true) {
+            int base = 0;
+            if (lane == 0) base = atomicAdd(counter, kGroups);
+            base = __shfl_sync(0xffffffffu, base, 0);
+            if (base >= total) break;
+            const int item = min(base + group, total - 1);
+            const int wi = wrap_of(first, item);
+            const WrapDev& w = wraps[wi];
+            const int v = item - first[wi];
+            const int cur = w.control->long_cur;
+            const bool mine = base + group < total;
+            const bool masked = w.mask && !w.mask[v];
+            const bool on = mine && !masked && !w.long_flag[(long)cur * w.V + v];  // flagged: a warp's walk, above
+            const float4 q32 = w.deformed32[v];
+            const F3 q = {q32.x, q32.y, q32.z};
+            const D3 q64 = load_d3(w.deformed, v);
+            int overflow = 0;
+            bool unfinished = false;
+            long work = 0;
+            int tri = nearest_triangle_group<G>(w, on, q, q64, w.corr_triangle[v],
+                                                warp_nodes + group * (kWarpStack / kGroups),
+                                                warp_dists + group * (kWarpStack / kGroups), &overflow, &unfinished,
+                                                &work);
+            if (lane % G == 0) {
+                if (on) {
+                    if (unfinished) tri = nearest_triangle(w, q, q64, tri, &overflow);
+                    if (overflow) atomicOr(&w.control->error, kErrorTraversal);
+                    store_correspondence(w, w.control->level, v, tri);
+                    if (unfinished || work > kLongWalk) list_long_walk(w, 1 - cur, v);
+                } else if (mine && masked) {
+                    store_masked(w, v);
+                }
+            }
+            __syncwarp();
         }
-        const int cur = w.control->long_cur;
-        if (w.long_flag[(long)cur * w.V + v]) continue;  // a warp's walk, above
-        const float4 q32 = w.deformed32[v];
-        int overflow = 0;
-        long steps = 0;
-        const int tri = nearest_triangle(w, {q32.x, q32.y, q32.z}, load_d3(w.deformed, v),
-                                         w.corr_triangle[v], &overflow, &steps);
-        if (overflow) atomicOr(&w.control->error, kErrorTraversal);
-        store_correspondence(w, w.control->level, v, tri);
-        if (steps > kLongWalk) list_long_walk(w, 1 - cur, v);
+    };
+    const int lanes = group_lanes(total, (long)gridDim.x * blockDim.x);
+    if (lanes == 16) {
+        others(std::integral_constant<int, 16>{});
+    } else if (lanes == 8) {
+        others(std::integral_constant<int, 8>{});
+    } else {
+        others(std::integral_constant<int, 4>{});
     }
 }
 
 // Stand-alone query over a prepared hierarchy (parity tests and the
-// `closest_points` entry point): FP32 ranking, FP64 winner.
-__global__ void k_closest_points(const WrapDev* __restrict__ wraps, const double* __restrict__ queries,
-                                 int count, double* __restrict__ out_points,
-                                 double* __restrict__ out_normals, double* __restrict__ out_distances,
-                                 int32_t* __restrict__ out_triangles, int* __restrict__ overflow_flag) {
+// `closest_points` entry point): a group of G lanes per query.
+template <int G>
+__global__ void __launch_bounds__(128) k_closest_points(const WrapDev* __restrict__ wraps,
+                                                       const double* __restrict__ queries, int count,
+                                                       double* __restrict__ out_points,
+                                                       double* __restrict__ out_normals,
+                                                       double* __restrict__ out_distances,
+                                                       int32_t* __restrict__ out_triangles,
+                                                       int* __restrict__ overflow_flag) {
+    __shared__ uint32_t stack_nodes[4 * kWarpStack];
+    __shared__ float stack_dists[4 * kWarpStack];
     const WrapDev& w = wraps[0];
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= count) return;
-    const D3 q = load_d3(queries, i);
+    const int group = threadIdx.x / G;
+    const int i = blockIdx.x * (128 / G) + group;
+    const bool on = i < count;
+    const D3 q = on ? load_d3(queries, i) : D3{0.0, 0.0, 0.0};
+    const F3 q32 = {__double2float_rn(q.x), __double2float_rn(q.y), __double2float_rn(q.z)};
     int overflow = 0;
-    const int tri = nearest_triangle(w, {__double2float_rn(q.x), __double2float_rn(q.y),
-                                         __double2float_rn(q.z)}, q, -1, &overflow);
+    bool unfinished = false;
+    long work = 0;
+    constexpr int kStack = kWarpStack * G / 32;
+    int tri = nearest_triangle_group<G>(w, on, q32, q, -1, stack_nodes + group * kStack, stack_dists + group * kStack,
+                                        &overflow, &unfinished, &work);
+    if (!on || threadIdx.x % G != 0) return;
+    if (unfinished) tri = nearest_triangle(w, q32, q, tri, &overflow);
     if (overflow) atomicOr(overflow_flag, 1);
     D3 point = {0, 0, 0}, normal = {0, 0, 0};
     double distance = 0.0;
@@ -1092,12 +1134,7 @@ __global__ void k_closest_points(const WrapDev* __restrict__ wraps, const double
     out_triangles[i] = tri;
 }
 
-void launch_query(const WrapDev* wraps, int wrap_count, int max_vertices, cudaStream_t stream, int* counter) {
-    if (!counter) {
-        dim3 grid(blocks_for(max_vertices, 128), wrap_count);
-        k_query<<<grid, 128, 0, stream>>>(wraps);
-        return;
-    }
+void launch_query(const WrapDev* wraps, int wrap_count, cudaStream_t stream, int* counter) {
     // the warps' stacks, then two scans over the wraps (1024 at most)
     constexpr size_t kStackBytes = (sizeof(uint32_t) + sizeof(float)) * kWarpStack * 4;
     static const int resident = [] {  // blocks of the queue that fit on the device at once
@@ -1117,8 +1154,25 @@ void launch_query(const WrapDev* wraps, int wrap_count, int max_vertices, cudaSt
 void launch_closest_points(const WrapDev* wrap, const double* queries, int count,
                            double* points, double* normals, double* distances, int32_t* triangles,
                            int* overflow, cudaStream_t stream) {
-    k_closest_points<<<blocks_for(count, 128), 128, 0, stream>>>(
-        wrap, queries, count, points, normals, distances, triangles, overflow);
+    static const long resident = [] {
+        int device = 0, sms = 148, per_sm = 0;
+        cudaGetDevice(&device);
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_closest_points<8>, 128, 0);
+        return 128L * sms * (per_sm > 0 ? per_sm : 1);
+    }();
+    auto launch = [&](auto kernel, int lanes) {
+        kernel<<<blocks_for((long)count * lanes, 128), 128, 0, stream>>>(wrap, queries, count, points, normals, distances,
+                                                                   triangles, overflow);
+    };
+    const int lanes = group_lanes(count, resident);
+    if (lanes == 16) {
+        launch(k_closest_points<16>, 16);
+    } else if (lanes == 8) {
+        launch(k_closest_points<8>, 8);
+    } else {
+        launch(k_closest_points<4>, 4);
+    }
 }
 
 }  // namespace nricp_b200

@@ -2198,7 +2198,7 @@ void launch_tick(const WrapDev* wraps, const TickShape& s, cudaStream_t stream,
     k_evaluate<<<grids.evaluate, kVertexThreads, virtual_smem, refresh>>>(wraps, W, refresh_part);
     k_normals<<<grids.normals, kVertexThreads, virtual_smem, refresh>>>(wraps, W, refresh_part);
     if (timed) cudaEventRecord(timers->query_begin, refresh);
-    launch_query(wraps, W, s.max_vertices, refresh, s.query_counter);
+    launch_query(wraps, W, refresh, s.query_counter);
     if (timed) cudaEventRecord(timers->query_end, refresh);
     k_stats<<<dim3(1, W), kStatsThreads, 0, refresh>>>(wraps, 1);
     assemble_and_decide(refresh_part, refresh);
