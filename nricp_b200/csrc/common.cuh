@@ -64,7 +64,7 @@ struct LevelDev {
     const int32_t* sell_begin;     // octets + 1: first step of each octet
     const int32_t* sell_nodes;     // steps x 8: the other node of each block (0: none)
     const int32_t* offdiag_nodes;  // offdiag_count x 2 (pair groups first, then edge-only pairs)
-    const int32_t* edge_block;     // edge_count: the block edge e adds to (< pair_count) or owns
+    const int32_t* block_edge;     // offdiag_count: the smoothness edge that adds to the block, or -1
     const int32_t* sell_slots;     // offdiag_count x 2: places (step * 8 + node of the octet) of B (a) and B^T (b)
     // warm start from the previous level (level > 0): 4 source nodes + weights
     const int32_t* transfer_nodes;   // N x 4
@@ -181,7 +181,8 @@ struct WrapDev {
     float4* resid_aux32;          // V: (n.x, n.y, n.z, p2p scale)
     float4* lm_resid32;           // V: landmark offset (xyz), w
     float4* offsets32;            // V x kMaxSlots: each binding's node-local offset R (p - g), FP32,
-                                  // for the tick's assembly (xyz, unused)
+                                  // and its FP32 weight, for the tick's assembly
+    float* anchor32;              // N x 12: each node's anchor term of the system
     // systems: two buffers, `control.system` selects the current one
     float* diag[2];               // N x 36
     float* rhs[2];                // N x 6

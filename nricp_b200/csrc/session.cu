@@ -275,7 +275,7 @@ size_t bytes_of_layout(const LevelLayout& L) {
                               L.node_edge_list.size() + L.edges.size() + L.pair_nodes.size() +
                               L.pair_begin.size() + L.pair_entry.size() + L.row_begin.size() +
                               L.sell_begin.size() + L.sell_nodes.size() + L.offdiag_nodes.size() + L.sell_slots.size() +
-                              L.edge_block.size() +
+                              L.offdiag_nodes.size() / 2 +
                               L.transfer_nodes.size() +
                               L.transfer_counts.size());
 }
@@ -341,6 +341,7 @@ size_t prepare_device(Wrap& w, WrapControl* control, cudaStream_t stream, bool p
     const size_t o_r1 = a.reserve(sizeof(float4) * V);
     const size_t o_r2 = a.reserve(sizeof(float4) * V);
     const size_t o_off32 = a.reserve(sizeof(float4) * kMaxSlots * V);
+    const size_t o_anchor = a.reserve(sizeof(float) * 12 * N);
     const size_t o_factor = a.reserve(sizeof(float) * 36 * N);
     const size_t o_delta = a.reserve(sizeof(double) * 6 * N);
     const size_t o_x = a.reserve(sizeof(double) * 6 * N);
@@ -492,7 +493,11 @@ size_t prepare_device(Wrap& w, WrapControl* control, cudaStream_t stream, bool p
         G.sell_nodes = put(L.sell_nodes);
         G.offdiag_nodes = put(L.offdiag_nodes);
         G.sell_slots = put(L.sell_slots);
-        G.edge_block = put(L.edge_block);
+        {
+            std::vector<int32_t> block_edge(L.offdiag_nodes.size() / 2, -1);
+            for (int e = 0; e < L.edge_count; ++e) block_edge[L.edge_block[e]] = e;
+            G.block_edge = put(block_edge);
+        }
         G.transfer_nodes = put(L.transfer_nodes);
         G.transfer_weights = put(L.transfer_weights);
         G.transfer_counts = put(L.transfer_counts);
@@ -521,6 +526,7 @@ size_t prepare_device(Wrap& w, WrapControl* control, cudaStream_t stream, bool p
     D.resid_aux32 = a.at<float4>(o_r1);
     D.lm_resid32 = a.at<float4>(o_r2);
     D.offsets32 = a.at<float4>(o_off32);
+    D.anchor32 = a.at<float>(o_anchor);
     D.factor = a.at<float>(o_factor);
     D.delta = a.at<double>(o_delta);
     D.pcg_x = a.at<double>(o_x);

@@ -26,7 +26,7 @@ namespace {
 
 constexpr int kVertexThreads = 256;
 constexpr int kNodeThreads = 256;   // 8 warps = 8 nodes per block
-constexpr int kEdgeThreads = 128;
+constexpr int kEdgeSums = 128;      // edges per partial sum of the smoothness energy
 constexpr int kPcgThreads = 512;
 constexpr int kStatsThreads = 512;
 
@@ -250,6 +250,20 @@ template <int N>
 __device__ __forceinline__ void warp_sum_halving(float* v, int lane, int& first, int& count) {
     warp_sum_halving<N, 16>(v, lane, first, count, [](float a, float b) { return a + b; });
 }
+// Where warp_sum_halving leaves the totals, without the sums.
+template <int N, int O = 16>
+__device__ __forceinline__ void halving_place(int lane, int& first, int& count) {
+    if constexpr (O >= 1) {
+        constexpr int H = (N + 1) / 2;
+        if (lane & O) {
+            first += H;
+            count = count > H ? count - H : 0;
+        } else {
+            count = count < H ? count : H;
+        }
+        halving_place<H, O / 2>(lane, first, count);
+    }
+}
 // Block sum in a fixed order; every thread returns the total.
 template <int kThreadsT>
 __device__ inline double block_sum(double v, double* scratch) {
@@ -265,6 +279,20 @@ __device__ inline double block_sum(double v, double* scratch) {
     }
     __syncthreads();
     return scratch[32];
+}
+
+// The same block sum of N values with two barriers for all of them; thread 0
+// holds the totals.  `scratch` is kThreadsT / 32 x N doubles.
+template <int kThreadsT, int N>
+__device__ inline void block_sums(double* v, double* scratch) {
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    for (int k = 0; k < N; ++k) v[k] = warp_sum(v[k]);
+    __syncthreads();
+    if (lane == 0)
+        for (int k = 0; k < N; ++k) scratch[warp * N + k] = v[k];
+    __syncthreads();
+    if (warp == 0)
+        for (int k = 0; k < N; ++k) v[k] = warp_sum(lane < kThreadsT / 32 ? scratch[lane * N + k] : 0.0);
 }
 
 // ---- symmetric 6x6 accumulation in the upper triangle ----------------------
@@ -1456,13 +1484,8 @@ __global__ void __launch_bounds__(kPcgThreads) k_pcg(const WrapDev* __restrict__
 // deformation evaluation (deformation.cpp:55-68) and the deformed template's
 // vertex normals (mesh.cpp:71-88)
 // ---------------------------------------------------------------------------
-__device__ __forceinline__ void k_evaluate_body(const WrapDev& w, int part, int bx) {
-    const WrapControl c = *w.control;
-    if (!in_part(c, part)) return;
-    if (c.phase == kPhaseDone || !has_candidate(c)) return;
-    const int v = bx * blockDim.x + threadIdx.x;
-    if (v >= w.V) return;
-    const LevelDev& L = w.levels[c.level];
+// The deformed position of vertex v under the state being evaluated.
+__device__ __forceinline__ D3 evaluate_vertex(const WrapDev& w, const LevelDev& L, const WrapControl& c, int v) {
     const int buf = eval_buffer(c);
     const double* R = w.rot[buf];
     const double* T = w.trans[buf];
@@ -1479,6 +1502,15 @@ __device__ __forceinline__ void k_evaluate_body(const WrapDev& w, int part, int 
     if (count == 0) sum = p;
     store_d3(w.deformed, v, sum);
     w.deformed32[v] = make_float4((float)sum.x, (float)sum.y, (float)sum.z, 0.0f);
+    return sum;
+}
+
+__device__ __forceinline__ void k_evaluate_body(const WrapDev& w, int part, int bx) {
+    const WrapControl c = *w.control;
+    if (!in_part(c, part)) return;
+    if (c.phase == kPhaseDone || !has_candidate(c)) return;
+    const int v = bx * blockDim.x + threadIdx.x;
+    if (v < w.V) evaluate_vertex(w, w.levels[c.level], c, v);
 }
 
 __global__ void k_evaluate(const WrapDev* __restrict__ wraps, int wrap_count, int part) {
@@ -1531,19 +1563,66 @@ __device__ inline F3 node_offset32(const WrapDev& w, const LevelDev& L, int node
     return mul3f(w.rot32 + node * 9, {(float)p.x, (float)p.y, (float)p.z});
 }
 
+// A node's anchor term (energy.cpp:239-271): its energy, and what it adds to
+// the node's diagonal block and right-hand side (twelve floats: the upper
+// triangle of the rotation block, the rotation half, the translation half).
+__device__ __forceinline__ void anchor_term(const WrapDev& w, const WrapControl& c, int node) {
+    const double weight = w.weights[c.level][3];
+    double energy = 0.0;
+    if (weight > 0.0) {
+        const int buf = eval_buffer(c);
+        const D3 om = log_so3(w.rot[buf] + node * 9);
+        const D3 t = load_d3(w.trans[buf], node);
+        const double sc = sqrt(weight);
+        const double vals[6] = {sc * om.x, sc * om.y, sc * om.z, sc * t.x, sc * t.y, sc * t.z};
+        for (int k = 0; k < 6; ++k) energy += vals[k] * vals[k];
+        if (assembles(c)) {
+            double J[9];
+            left_jacobian_inverse(om, J);
+            float* out = w.anchor32 + node * 12;
+            int at = 0;
+            for (int r = 0; r < 3; ++r)
+                for (int q = r; q < 3; ++q) {
+                    double s = 0.0;
+                    for (int k = 0; k < 3; ++k) s += J[k * 3 + r] * J[k * 3 + q];
+                    out[at++] = (float)(weight * s);
+                }
+            for (int r = 0; r < 3; ++r) {
+                double s = 0.0;
+                for (int k = 0; k < 3; ++k) s += J[k * 3 + r] * (k == 0 ? om.x : k == 1 ? om.y : om.z);
+                out[at++] = (float)(weight * s);
+            }
+            out[9] = (float)(weight * t.x);
+            out[10] = (float)(weight * t.y);
+            out[11] = (float)(weight * t.z);
+        }
+    }
+    w.node_partials[node] = energy;  // the decision kernel sums them
+}
+
+// kEvaluate: the vertex is deformed first (the solve chain; the refresh chain
+// has deformed it before its query).  The blocks past the vertices' take the
+// nodes' anchor terms, a thread each: FP64 logarithms and Jacobians of several
+// thousand cycles, which in the node assembly held a whole warp per node.
+template <bool kEvaluate>
 __device__ __forceinline__ void k_residual_body(const WrapDev& w, int part, int bx) {
     const WrapControl c = *w.control;
     if (!in_part(c, part)) return;
     if (!computes_energy(c)) return;
-    if ((long)bx * blockDim.x >= w.V) return;
+    const LevelDev& L = w.levels[c.level];
+    const int vertex_blocks = blocks_of_dev(w.V, kVertexThreads);
+    if (bx >= vertex_blocks) {
+        const int node = (bx - vertex_blocks) * kVertexThreads + threadIdx.x;
+        if (node < L.node_count) anchor_term(w, c, node);
+        return;
+    }
     const int v = bx * blockDim.x + threadIdx.x;
     const double* wt = w.weights[c.level];
-    const LevelDev& L = w.levels[c.level];
-    double e_p2p = 0.0, e_plane = 0.0, e_lm = 0.0;
+    double e[3] = {0.0, 0.0, 0.0};  // point to point, plane, landmark
     if (v < w.V) {
         float4 r0 = make_float4(0.f, 0.f, 0.f, 0.f), r1 = r0, r2 = r0;
         const bool bound = L.bind_counts[v] > 0;
-        const D3 q = load_d3(w.deformed, v);
+        const D3 q = kEvaluate ? evaluate_vertex(w, L, c, v) : load_d3(w.deformed, v);
         if (bound && w.corr_code[v] == 0) {
             const D3 y = load_d3(w.corr_point, v);
             const D3 o = rsub(q, y);
@@ -1552,7 +1631,7 @@ __device__ __forceinline__ void k_residual_body(const WrapDev& w, int part, int 
             if (wt[0] > 0.0) {
                 const double s = sqrt(wt[0] * u);
                 const D3 so = rmul(o, s);
-                e_p2p = da(da(dm(so.x, so.x), dm(so.y, so.y)), dm(so.z, so.z));
+                e[0] = da(da(dm(so.x, so.x), dm(so.y, so.y)), dm(so.z, so.z));
                 r0 = make_float4((float)o.x, (float)o.y, (float)o.z, (float)(wt[0] * u));
             } else {
                 r0 = make_float4((float)o.x, (float)o.y, (float)o.z, 0.0f);
@@ -1560,7 +1639,7 @@ __device__ __forceinline__ void k_residual_body(const WrapDev& w, int part, int 
             if (wt[1] > 0.0) {
                 const double s = sqrt(wt[1] * u);
                 const double value = dm(s, rdot(n, o));
-                e_plane = dm(value, value);
+                e[1] = dm(value, value);
                 r1 = make_float4((float)n.x, (float)n.y, (float)n.z, (float)(wt[1] * u));
             }
         }
@@ -1568,57 +1647,72 @@ __device__ __forceinline__ void k_residual_body(const WrapDev& w, int part, int 
             const D3 o = rsub(q, load_d3(w.lm_target, v));
             const double s = sqrt(wt[4]);
             const D3 so = rmul(o, s);
-            e_lm = da(da(dm(so.x, so.x), dm(so.y, so.y)), dm(so.z, so.z));
+            e[2] = da(da(dm(so.x, so.x), dm(so.y, so.y)), dm(so.z, so.z));
             r2 = make_float4((float)o.x, (float)o.y, (float)o.z, (float)wt[4]);
         }
-        w.residual32[v] = r0;
-        w.resid_aux32[v] = r1;
-        w.lm_resid32[v] = r2;
-        // each binding's offset, once for the node and pair assembly that follow
-        if (bound && assembles(c))
-            for (int k = 0; k < L.bind_counts[v]; ++k) {
-                const int node = L.bind_nodes[v * kMaxSlots + k];
-                if (node < 0) continue;
-                const F3 a = node_offset32(w, L, node, v);
-                w.offsets32[v * kMaxSlots + k] = make_float4(a.x, a.y, a.z, 0.0f);
-            }
+        if (assembles(c)) {
+            w.residual32[v] = r0;
+            w.resid_aux32[v] = r1;
+            if (w.L > 0) w.lm_resid32[v] = r2;
+            // each binding's offset and FP32 weight, once for the node and pair
+            // assembly that follow
+            if (bound)
+                for (int k = 0; k < L.bind_counts[v]; ++k) {
+                    const int node = L.bind_nodes[v * kMaxSlots + k];
+                    if (node < 0) continue;
+                    const F3 a = node_offset32(w, L, node, v);
+                    w.offsets32[v * kMaxSlots + k] =
+                        make_float4(a.x, a.y, a.z, (float)L.bind_weights[v * kMaxSlots + k]);
+                }
+        }
     }
-    __shared__ double scratch[33];
-    const double s0 = block_sum<kVertexThreads>(e_p2p, scratch);
-    const double s1 = block_sum<kVertexThreads>(e_plane, scratch);
-    const double s4 = block_sum<kVertexThreads>(e_lm, scratch);
+    __shared__ double scratch[kVertexThreads / 32 * 3];
+    block_sums<kVertexThreads, 3>(e, scratch);
     if (threadIdx.x == 0) {
         double* p = w.partials + (long)bx * kPartialStride;
-        p[0] = s0; p[1] = s1; p[2] = s4;
+        p[0] = e[0]; p[1] = e[1]; p[2] = e[2];
     }
 }
 
+template <bool kEvaluate>
 __global__ void __launch_bounds__(kVertexThreads) k_residual(const WrapDev* __restrict__ wraps, int wrap_count, int part) {
     over_virtual_blocks<true>(
         wraps, wrap_count,
         [&](const WrapDev& w) {
             const WrapControl c = *w.control;
-            return in_part(c, part) ? (computes_energy(c) ? blocks_of_dev(w.V, kVertexThreads) : 0) : 0;
+            if (!in_part(c, part) || !computes_energy(c)) return 0;
+            return blocks_of_dev(w.V, kVertexThreads) + blocks_of_dev(w.levels[c.level].node_count, kVertexThreads);
         },
-        [&](int wi, int bx) { k_residual_body(wraps[wi], part, bx); });
+        [&](int wi, int bx) { k_residual_body<kEvaluate>(wraps[wi], part, bx); });
 }
 
 // ---------------------------------------------------------------------------
-// Gauss-Newton blocks: warp per node for the diagonal block and the
-// right-hand side (data, landmark, incident smoothness edges, anchor), thread
-// per node pair for the cross blocks of shared vertices, thread per edge for
-// the smoothness blocks.  Closed forms of sum_rows J^T J for an offset
+// Gauss-Newton blocks in one launch: a warp per node for the diagonal block and
+// the right-hand side (data, landmark, incident smoothness edges, anchor), then
+// a warp per off-diagonal block (the vertices its node pair shares, and the
+// smoothness edge between them).  Closed forms of sum_rows J^T J for an offset
 // residual replace the reference's row-by-row outer products.
 // ---------------------------------------------------------------------------
 
-__device__ __forceinline__ void k_node_assemble_body(const WrapDev& w, int part, int bx) {
-    const WrapControl c = *w.control;
-    if (!in_part(c, part)) return;
-    if (!computes_energy(c)) return;
+// What one binding or one shared vertex adds is read through an index, so each
+// lane keeps the next entry's data and the index after it in flight while it
+// adds the current one.
+struct NodeEntry {
+    float4 a, r0, r1, r2;
+};
+__device__ __forceinline__ NodeEntry load_entry(const WrapDev& w, int entry, bool landmarks) {
+    NodeEntry x;
+    const int v = entry / kMaxSlots;
+    x.a = __ldg(w.offsets32 + entry);
+    x.r0 = __ldg(w.residual32 + v);
+    x.r1 = __ldg(w.resid_aux32 + v);
+    x.r2 = landmarks ? __ldg(w.lm_resid32 + v) : make_float4(0.f, 0.f, 0.f, 0.f);
+    return x;
+}
+
+__device__ __forceinline__ void assemble_node(const WrapDev& w, const WrapControl& c, int node) {
     const bool build = assembles(c);
     const LevelDev& L = w.levels[c.level];
-    if ((long)bx * (kNodeThreads / 32) >= L.node_count) return;
-    const int node = (bx * blockDim.x + threadIdx.x) >> 5;
     const int lane = threadIdx.x & 31;
     const double* wt = w.weights[c.level];
     const int buf = eval_buffer(c);
@@ -1626,296 +1720,256 @@ __device__ __forceinline__ void k_node_assemble_body(const WrapDev& w, int part,
     float d[21], g[6];
     for (int i = 0; i < 21; ++i) d[i] = 0.0f;
     for (int i = 0; i < 6; ++i) g[i] = 0.0f;
-    double e_anchor = 0.0;
-    if (node < L.node_count) {
-        if (build) {
-            for (int i = L.gather_begin[node] + lane; i < L.gather_begin[node + 1]; i += 32) {
-                const int entry = L.gather_entry[i];
-                const int v = entry / kMaxSlots;
-                const float wgt = (float)L.bind_weights[entry];
-                const float4 a4 = w.offsets32[entry];
-                const F3 a = {a4.x, a4.y, a4.z};
-                const float4 r0 = w.residual32[v];
-                const float4 r1 = w.resid_aux32[v];
-                const float4 r2 = w.lm_resid32[v];
-                if (r0.w > 0.0f) {  // point to point
-                    const F3 o = {r0.x, r0.y, r0.z};
-                    add_offset_block(d, a, r0.w * wgt * wgt);
-                    const F3 ao = cross(a, o);
-                    const float s = r0.w * wgt;
-                    g[0] -= s * ao.x; g[1] -= s * ao.y; g[2] -= s * ao.z;
-                    g[3] -= s * o.x; g[4] -= s * o.y; g[5] -= s * o.z;
-                }
-                if (r1.w > 0.0f) {  // point to plane
-                    const F3 n = {r1.x, r1.y, r1.z};
-                    const F3 an = cross(a, n);
-                    const float u[6] = {an.x, an.y, an.z, n.x, n.y, n.z};
-                    add_rank_one(d, u, r1.w * wgt * wgt);
-                    const float pv = dot(n, F3{r0.x, r0.y, r0.z});
-                    const float s = r1.w * wgt * pv;
-                    for (int k = 0; k < 6; ++k) g[k] -= s * u[k];
-                }
-                if (r2.w > 0.0f) {  // landmark
-                    const F3 o = {r2.x, r2.y, r2.z};
-                    add_offset_block(d, a, r2.w * wgt * wgt);
-                    const F3 ao = cross(a, o);
-                    const float s = r2.w * wgt;
-                    g[0] -= s * ao.x; g[1] -= s * ao.y; g[2] -= s * ao.z;
-                    g[3] -= s * o.x; g[4] -= s * o.y; g[5] -= s * o.z;
-                }
+    if (build) {
+        const int end = L.gather_begin[node + 1];
+        const bool landmarks = w.L > 0;
+        int i = L.gather_begin[node] + lane;
+        int after = i + 32 < end ? L.gather_entry[i + 32] : 0;
+        NodeEntry ahead;
+        if (i < end) ahead = load_entry(w, L.gather_entry[i], landmarks);
+        for (; i < end; i += 32) {
+            const NodeEntry x = ahead;
+            if (i + 32 < end) ahead = load_entry(w, after, landmarks);
+            if (i + 64 < end) after = L.gather_entry[i + 64];
+            const float wgt = x.a.w;
+            const F3 a = {x.a.x, x.a.y, x.a.z};
+            if (x.r0.w > 0.0f) {  // point to point
+                const F3 o = {x.r0.x, x.r0.y, x.r0.z};
+                add_offset_block(d, a, x.r0.w * wgt * wgt);
+                const F3 ao = cross(a, o);
+                const float s = x.r0.w * wgt;
+                g[0] -= s * ao.x; g[1] -= s * ao.y; g[2] -= s * ao.z;
+                g[3] -= s * o.x; g[4] -= s * o.y; g[5] -= s * o.z;
             }
-            if (wt[2] > 0.0) {
-                const float ws = (float)wt[2];
-                const double* R = w.rot[buf];
-                const double* T = w.trans[buf];
-                for (int i = L.node_edge_begin[node] + lane; i < L.node_edge_begin[node + 1]; i += 32) {
-                    const int e = L.node_edge_list[i];
-                    const int a = L.edges[e * 2], b = L.edges[e * 2 + 1];
-                    const D3 ga = load_d3(L.rest, a), gb = load_d3(L.rest, b);
-                    const D3 gd = gb - ga;
-                    const D3 diff = radd(radd(rmat(R + a * 9, gd), ga), load_d3(T, a)) -
-                                    (gb + load_d3(T, b));
-                    const F3 dv = {(float)diff.x, (float)diff.y, (float)diff.z};
-                    if (a == node) {
-                        const F3 cv = mul3f(w.rot32 + a * 9, {(float)gd.x, (float)gd.y, (float)gd.z});
-                        add_offset_block(d, cv, ws);
-                        const F3 cd = cross(cv, dv);
-                        g[0] -= ws * cd.x; g[1] -= ws * cd.y; g[2] -= ws * cd.z;
-                        g[3] -= ws * dv.x; g[4] -= ws * dv.y; g[5] -= ws * dv.z;
-                    } else {
-                        d[tri_index(3, 3)] += ws; d[tri_index(4, 4)] += ws; d[tri_index(5, 5)] += ws;
-                        g[3] += ws * dv.x; g[4] += ws * dv.y; g[5] += ws * dv.z;
-                    }
-                }
+            if (x.r1.w > 0.0f) {  // point to plane
+                const F3 n = {x.r1.x, x.r1.y, x.r1.z};
+                const F3 an = cross(a, n);
+                const float u[6] = {an.x, an.y, an.z, n.x, n.y, n.z};
+                add_rank_one(d, u, x.r1.w * wgt * wgt);
+                const float pv = dot(n, F3{x.r0.x, x.r0.y, x.r0.z});
+                const float s = x.r1.w * wgt * pv;
+                for (int k = 0; k < 6; ++k) g[k] -= s * u[k];
             }
-        }
-        if (lane == 0 && wt[3] > 0.0) {  // anchor (energy.cpp:239-271)
-            const double* R = w.rot[buf] + node * 9;
-            const D3 om = log_so3(R);
-            const D3 t = load_d3(w.trans[buf], node);
-            const double sc = sqrt(wt[3]);
-            const double vals[6] = {sc * om.x, sc * om.y, sc * om.z, sc * t.x, sc * t.y, sc * t.z};
-            for (int k = 0; k < 6; ++k) e_anchor += vals[k] * vals[k];
-            if (build) {
-                double J[9];
-                left_jacobian_inverse(om, J);
-                for (int r = 0; r < 3; ++r)
-                    for (int q = r; q < 3; ++q) {
-                        double s = 0.0;
-                        for (int k = 0; k < 3; ++k) s += J[k * 3 + r] * J[k * 3 + q];
-                        d[tri_index(r, q)] += (float)(wt[3] * s);
-                    }
-                for (int r = 0; r < 3; ++r) {
-                    double s = 0.0;
-                    for (int k = 0; k < 3; ++k) s += J[k * 3 + r] * (k == 0 ? om.x : k == 1 ? om.y : om.z);
-                    g[r] -= (float)(wt[3] * s);
-                }
-                d[tri_index(3, 3)] += (float)wt[3]; d[tri_index(4, 4)] += (float)wt[3];
-                d[tri_index(5, 5)] += (float)wt[3];
-                g[3] -= (float)(wt[3] * t.x); g[4] -= (float)(wt[3] * t.y); g[5] -= (float)(wt[3] * t.z);
-            }
-        }
-        if (build) {
-            // the 21 upper-triangle sums and the 6 of the rhs, spread over the
-            // lanes; each lane stores what it holds
-            float v[27];
-            for (int i = 0; i < 21; ++i) v[i] = d[i];
-            for (int i = 0; i < 6; ++i) v[21 + i] = g[i];
-            int first = 0, count = 27;
-            warp_sum_halving<27>(v, lane, first, count);
-            if (count > 0) {
-                float* D = w.diag[next] + node * 36;
-                float* G = w.rhs[next] + node * 6;
-                const bool restricted = c.route == 1;
-                const int j = first;
-                if (j < 21) {
-                    int r = 0;
-                    while (tri_index(r + 1, r + 1) <= j) ++r;  // row of upper-triangle entry j
-                    const int q = j - tri_index(r, r) + r;
-                    float value = v[0];
-                    if (restricted && (r < 3 || q < 3)) value = (r == q) ? 1.0f : 0.0f;
-                    D[r * 6 + q] = value;
-                    D[q * 6 + r] = value;
-                } else {
-                    const int k = j - 21;
-                    G[k] = (restricted && k < 3) ? 0.0f : v[0];
-                }
+            if (x.r2.w > 0.0f) {  // landmark
+                const F3 o = {x.r2.x, x.r2.y, x.r2.z};
+                add_offset_block(d, a, x.r2.w * wgt * wgt);
+                const F3 ao = cross(a, o);
+                const float s = x.r2.w * wgt;
+                g[0] -= s * ao.x; g[1] -= s * ao.y; g[2] -= s * ao.z;
+                g[3] -= s * o.x; g[4] -= s * o.y; g[5] -= s * o.z;
             }
         }
     }
-    // the node's anchor energy; the decision kernel sums them as a block sum
-    // over this block's warps would (no block barrier here)
-    if (lane == 0 && node < L.node_count) w.node_partials[node] = e_anchor;
-}
-
-__global__ void __launch_bounds__(kNodeThreads, 3) k_node_assemble(const WrapDev* __restrict__ wraps, int wrap_count, int part) {
-    over_virtual_blocks<false>(
-        wraps, wrap_count,
-        [&](const WrapDev& w) {
-            const WrapControl c = *w.control;
-            return in_part(c, part) ? (computes_energy(c) ? blocks_of_dev(w.levels[c.level].node_count * 32, kNodeThreads) : 0) : 0;
-        },
-        [&](int wi, int bx) { k_node_assemble_body(wraps[wi], part, bx); });
-}
-
-// Writes block k of the system twice: B where the row list of node a holds it,
-// B^T where node b's does.
-__device__ inline void store_block_pair(float* out, const LevelDev& L, int k, const float* blk) {
-    float* A = out + block_base(L.sell_slots[k * 2]);
-    float* T = out + block_base(L.sell_slots[k * 2 + 1]);
-    for (int r = 0; r < 6; ++r)
-        for (int q = 0; q < 6; ++q) {
-            A[block_at(r, q)] = blk[r * 6 + q];
-            T[block_at(q, r)] = blk[r * 6 + q];
+    // the incident smoothness edges; each edge's energy is its first node's
+    // to store (the decision kernel sums them)
+    const float ws = (float)wt[2];
+    const double sc = sqrt(wt[2]);
+    const double* R = w.rot[buf];
+    const double* T = w.trans[buf];
+    for (int i = L.node_edge_begin[node] + lane; i < L.node_edge_begin[node + 1]; i += 32) {
+        const int e = L.node_edge_list[i];
+        const int a = L.edges[e * 2], b = L.edges[e * 2 + 1];
+        double energy = 0.0;
+        if (wt[2] > 0.0) {
+            const D3 ga = load_d3(L.rest, a), gb = load_d3(L.rest, b);
+            const D3 gd = rsub(gb, ga);
+            const D3 field_a = radd(radd(rmat(R + a * 9, gd), ga), load_d3(T, a));
+            const D3 field_b = radd(gb, load_d3(T, b));
+            const D3 diff = rsub(field_a, field_b);
+            const D3 scaled = rmul(diff, sc);
+            energy = da(da(dm(scaled.x, scaled.x), dm(scaled.y, scaled.y)), dm(scaled.z, scaled.z));
+            if (build) {
+                const F3 dv = {(float)diff.x, (float)diff.y, (float)diff.z};
+                if (a == node) {
+                    const F3 cv = mul3f(w.rot32 + a * 9, {(float)gd.x, (float)gd.y, (float)gd.z});
+                    add_offset_block(d, cv, ws);
+                    const F3 cd = cross(cv, dv);
+                    g[0] -= ws * cd.x; g[1] -= ws * cd.y; g[2] -= ws * cd.z;
+                    g[3] -= ws * dv.x; g[4] -= ws * dv.y; g[5] -= ws * dv.z;
+                } else {
+                    d[tri_index(3, 3)] += ws; d[tri_index(4, 4)] += ws; d[tri_index(5, 5)] += ws;
+                    g[3] += ws * dv.x; g[4] += ws * dv.y; g[5] += ws * dv.z;
+                }
+            }
         }
-}
-
-// Adds block k into the system, both ways (the smoothness edge of a node pair
-// whose shared-vertex block is already there).
-__device__ inline void add_block_pair(float* out, const LevelDev& L, int k, const float* blk) {
-    float* A = out + block_base(L.sell_slots[k * 2]);
-    float* T = out + block_base(L.sell_slots[k * 2 + 1]);
-    for (int r = 0; r < 6; ++r)
-        for (int q = 0; q < 6; ++q) {
-            A[block_at(r, q)] += blk[r * 6 + q];
-            T[block_at(q, r)] += blk[r * 6 + q];
+        if (a == node) w.edge_partials[e] = energy;
+    }
+    if (!build) return;
+    if (lane == 0 && wt[3] > 0.0) {  // the anchor term, formed with the residuals
+        const float* x = w.anchor32 + node * 12;
+        int at = 0;
+        for (int r = 0; r < 3; ++r)
+            for (int q = r; q < 3; ++q) d[tri_index(r, q)] += x[at++];
+        for (int r = 0; r < 3; ++r) g[r] -= x[at++];
+        d[tri_index(3, 3)] += (float)wt[3]; d[tri_index(4, 4)] += (float)wt[3];
+        d[tri_index(5, 5)] += (float)wt[3];
+        g[3] -= x[9]; g[4] -= x[10]; g[5] -= x[11];
+    }
+    // the 21 upper-triangle sums and the 6 of the rhs, spread over the
+    // lanes; each lane stores what it holds
+    float v[27];
+    for (int i = 0; i < 21; ++i) v[i] = d[i];
+    for (int i = 0; i < 6; ++i) v[21 + i] = g[i];
+    int first = 0, count = 27;
+    warp_sum_halving<27>(v, lane, first, count);
+    if (count > 0) {
+        float* D = w.diag[next] + node * 36;
+        float* G = w.rhs[next] + node * 6;
+        const bool restricted = c.route == 1;
+        const int j = first;
+        if (j < 21) {
+            int r = 0;
+            while (tri_index(r + 1, r + 1) <= j) ++r;  // row of upper-triangle entry j
+            const int q = j - tri_index(r, r) + r;
+            float value = v[0];
+            if (restricted && (r < 3 || q < 3)) value = (r == q) ? 1.0f : 0.0f;
+            D[r * 6 + q] = value;
+            D[q * 6 + r] = value;
+        } else {
+            const int k = j - 21;
+            G[k] = (restricted && k < 3) ? 0.0f : v[0];
         }
+    }
 }
 
-// Warp per node pair: lanes stride over the vertices the two nodes share,
-// each lane keeps a 6x6 block in registers, one butterfly reduction.
-__device__ __forceinline__ void k_pair_assemble_body(const WrapDev& w, int part, int bx) {
-    const WrapControl c = *w.control;
-    if (!in_part(c, part)) return;
-    if (!assembles(c)) return;
+// Off-diagonal block k: the lanes stride over the vertices its node pair
+// shares (none past pair_count), each with a 6x6 block in registers, then one
+// halving reduction; the smoothness edge of the pair is added to the sums (it
+// took a kernel of its own before, which read and wrote the blocks again with
+// a thread per edge: 28 us of latency in every tick).
+struct PairEntry {
+    float4 a, b, r0, r1;
+    float lm;
+};
+__device__ __forceinline__ PairEntry load_pair(const WrapDev& w, int code, bool landmarks) {
+    PairEntry x;
+    const int v = code >> 6, sa = (code >> 3) & 7, sb = code & 7;
+    x.a = __ldg(w.offsets32 + v * kMaxSlots + sa);
+    x.b = __ldg(w.offsets32 + v * kMaxSlots + sb);
+    x.r0 = __ldg(w.residual32 + v);
+    x.r1 = __ldg(w.resid_aux32 + v);
+    x.lm = landmarks ? __ldg(&w.lm_resid32[v].w) : 0.0f;
+    return x;
+}
+
+__device__ __forceinline__ void assemble_block(const WrapDev& w, const WrapControl& c, int k) {
     const LevelDev& L = w.levels[c.level];
-    const int p = (bx * blockDim.x + threadIdx.x) >> 5;
     const int lane = threadIdx.x & 31;
-    if (p >= L.pair_count) return;
     float blk[36];
     for (int i = 0; i < 36; ++i) blk[i] = 0.0f;
-    for (int i = L.pair_begin[p] + lane; i < L.pair_begin[p + 1]; i += 32) {
-        const int code = L.pair_entry[i];
-        const int v = code >> 6, sa = (code >> 3) & 7, sb = code & 7;
-        const float wa = (float)L.bind_weights[v * kMaxSlots + sa];
-        const float wb = (float)L.bind_weights[v * kMaxSlots + sb];
-        const float4 a4 = w.offsets32[v * kMaxSlots + sa], b4 = w.offsets32[v * kMaxSlots + sb];
-        const F3 aa = {a4.x, a4.y, a4.z};
-        const F3 ab = {b4.x, b4.y, b4.z};
-        const float4 r0 = w.residual32[v], r1 = w.resid_aux32[v], r2 = w.lm_resid32[v];
-        const float coef = (r0.w + r2.w) * wa * wb;  // p2p and landmark share the form
-        if (coef > 0.0f) {
-            // [ (aa.ab) I - ab aa^T, [aa]x ; [ab]x^T, I ]
-            const float dp = dot(aa, ab);
-            const float av[3] = {aa.x, aa.y, aa.z}, bv[3] = {ab.x, ab.y, ab.z};
-            for (int r = 0; r < 3; ++r)
-                for (int q = 0; q < 3; ++q)
-                    blk[r * 6 + q] += coef * ((r == q ? dp : 0.0f) - bv[r] * av[q]);
-            blk[0 * 6 + 4] += -coef * aa.z; blk[0 * 6 + 5] += coef * aa.y;
-            blk[1 * 6 + 3] += coef * aa.z;  blk[1 * 6 + 5] += -coef * aa.x;
-            blk[2 * 6 + 3] += -coef * aa.y; blk[2 * 6 + 4] += coef * aa.x;
-            // [ab]x^T = -[ab]x in rows 3-5, columns 0-2
-            blk[3 * 6 + 1] += coef * ab.z;  blk[3 * 6 + 2] += -coef * ab.y;
-            blk[4 * 6 + 0] += -coef * ab.z; blk[4 * 6 + 2] += coef * ab.x;
-            blk[5 * 6 + 0] += coef * ab.y;  blk[5 * 6 + 1] += -coef * ab.x;
-            blk[3 * 6 + 3] += coef; blk[4 * 6 + 4] += coef; blk[5 * 6 + 5] += coef;
+    const bool pair = k < L.pair_count;
+    if (pair) {
+        const int end = L.pair_begin[k + 1];
+        const bool landmarks = w.L > 0;
+        int i = L.pair_begin[k] + lane;
+        int after = i + 32 < end ? L.pair_entry[i + 32] : 0;
+        PairEntry ahead;
+        if (i < end) ahead = load_pair(w, L.pair_entry[i], landmarks);
+        for (; i < end; i += 32) {
+            const PairEntry x = ahead;
+            if (i + 32 < end) ahead = load_pair(w, after, landmarks);
+            if (i + 64 < end) after = L.pair_entry[i + 64];
+            const float wa = x.a.w, wb = x.b.w;
+            const F3 aa = {x.a.x, x.a.y, x.a.z};
+            const F3 ab = {x.b.x, x.b.y, x.b.z};
+            const float coef = (x.r0.w + x.lm) * wa * wb;  // p2p and landmark share the form
+            if (coef > 0.0f) {
+                // [ (aa.ab) I - ab aa^T, [aa]x ; [ab]x^T, I ]
+                const float dp = dot(aa, ab);
+                const float av[3] = {aa.x, aa.y, aa.z}, bv[3] = {ab.x, ab.y, ab.z};
+                for (int r = 0; r < 3; ++r)
+                    for (int q = 0; q < 3; ++q)
+                        blk[r * 6 + q] += coef * ((r == q ? dp : 0.0f) - bv[r] * av[q]);
+                blk[0 * 6 + 4] += -coef * aa.z; blk[0 * 6 + 5] += coef * aa.y;
+                blk[1 * 6 + 3] += coef * aa.z;  blk[1 * 6 + 5] += -coef * aa.x;
+                blk[2 * 6 + 3] += -coef * aa.y; blk[2 * 6 + 4] += coef * aa.x;
+                // [ab]x^T = -[ab]x in rows 3-5, columns 0-2
+                blk[3 * 6 + 1] += coef * ab.z;  blk[3 * 6 + 2] += -coef * ab.y;
+                blk[4 * 6 + 0] += -coef * ab.z; blk[4 * 6 + 2] += coef * ab.x;
+                blk[5 * 6 + 0] += coef * ab.y;  blk[5 * 6 + 1] += -coef * ab.x;
+                blk[3 * 6 + 3] += coef; blk[4 * 6 + 4] += coef; blk[5 * 6 + 5] += coef;
+            }
+            if (x.r1.w > 0.0f) {
+                const F3 n = {x.r1.x, x.r1.y, x.r1.z};
+                const F3 ca = cross(aa, n), cb = cross(ab, n);
+                const float ua[6] = {ca.x, ca.y, ca.z, n.x, n.y, n.z};
+                const float ub[6] = {cb.x, cb.y, cb.z, n.x, n.y, n.z};
+                const float s = x.r1.w * wa * wb;
+                for (int r = 0; r < 6; ++r)
+                    for (int q = 0; q < 6; ++q) blk[r * 6 + q] += s * ua[r] * ub[q];
+            }
         }
-        if (r1.w > 0.0f) {
-            const F3 n = {r1.x, r1.y, r1.z};
-            const F3 ca = cross(aa, n), cb = cross(ab, n);
-            const float ua[6] = {ca.x, ca.y, ca.z, n.x, n.y, n.z};
-            const float ub[6] = {cb.x, cb.y, cb.z, n.x, n.y, n.z};
-            const float s = r1.w * wa * wb;
-            for (int r = 0; r < 6; ++r)
-                for (int q = 0; q < 6; ++q) blk[r * 6 + q] += s * ua[r] * ub[q];
-        }
+    }
+    // the smoothness edge's term, ws * [[0, -[c]x], [0, -I]], c = R_a (g_b - g_a)
+    const int edge = L.block_edge[k];
+    const float ws = edge >= 0 && w.weights[c.level][2] > 0.0 ? (float)w.weights[c.level][2] : 0.0f;
+    F3 cv = {0.0f, 0.0f, 0.0f};
+    if (ws > 0.0f && c.route == 0) {
+        const int a = L.edges[edge * 2], b = L.edges[edge * 2 + 1];
+        const D3 gd = rsub(load_d3(L.rest, b), load_d3(L.rest, a));
+        cv = mul3f(w.rot32 + a * 9, {(float)gd.x, (float)gd.y, (float)gd.z});
     }
     // the 36 sums spread over the lanes (two each at most); each lane stores
     // what it holds, both ways
     int first = 0, count = 36;
-    warp_sum_halving<36>(blk, lane, first, count);
-    float* A = w.offdiag[1 - c.system] + block_base(L.sell_slots[p * 2]);
-    float* T = w.offdiag[1 - c.system] + block_base(L.sell_slots[p * 2 + 1]);
+    if (pair) warp_sum_halving<36>(blk, lane, first, count);
+    else halving_place<36>(lane, first, count);
+    float* A = w.offdiag[1 - c.system] + block_base(L.sell_slots[k * 2]);
+    float* T = w.offdiag[1 - c.system] + block_base(L.sell_slots[k * 2 + 1]);
 #pragma unroll
     for (int i = 0; i < 2; ++i) {
         if (i >= count) break;
         const int j = first + i, r = j / 6, q = j - r * 6;
-        const float value = (c.route == 1 && (r < 3 || q < 3)) ? 0.0f : blk[i];
+        float value = (c.route == 1 && (r < 3 || q < 3)) ? 0.0f : blk[i];
+        if (edge >= 0) {
+            float term = 0.0f;
+            if (r >= 3) {
+                if (r == q) term = -ws;
+            } else if (q >= 3 && q - 3 != r) {
+                // row r, column q of -[c]x: c's remaining component, its sign
+                // alternating around the cycle
+                const int other = 3 - r - (q - 3);
+                const float x = other == 0 ? cv.x : (other == 1 ? cv.y : cv.z);
+                term = (q - 3 == (r + 1) % 3) ? ws * x : -ws * x;
+            }
+            value = pair ? value + term : term;
+        }
         A[block_at(r, q)] = value;
         T[block_at(q, r)] = value;
     }
 }
 
-__global__ void __launch_bounds__(kNodeThreads, 3) k_pair_assemble(const WrapDev* __restrict__ wraps, int wrap_count, int part) {
-    over_virtual_blocks<false>(
-        wraps, wrap_count,
-        [&](const WrapDev& w) {
-            const WrapControl c = *w.control;
-            return in_part(c, part) ? (assembles(c) ? blocks_of_dev(w.levels[c.level].pair_count * 32, kNodeThreads) : 0) : 0;
-        },
-        [&](int wi, int bx) { k_pair_assemble_body(wraps[wi], part, bx); });
-}
-
-__device__ __forceinline__ void k_edge_assemble_body(const WrapDev& w, int part, int bx) {
+// Blocks of eight warps: the nodes', then the off-diagonal blocks'.
+__device__ __forceinline__ void k_assemble_body(const WrapDev& w, int part, int bx) {
     const WrapControl c = *w.control;
     if (!in_part(c, part)) return;
     if (!computes_energy(c)) return;
     const LevelDev& L = w.levels[c.level];
-    if ((long)bx * blockDim.x >= L.edge_count) return;
-    const int e = bx * blockDim.x + threadIdx.x;
-    const double* wt = w.weights[c.level];
-    const int buf = eval_buffer(c);
-    double energy = 0.0;
-    if (e < L.edge_count) {
-        const int a = L.edges[e * 2], b = L.edges[e * 2 + 1];
-        const D3 ga = load_d3(L.rest, a), gb = load_d3(L.rest, b);
-        const D3 gd = rsub(gb, ga);
-        const double* R = w.rot[buf];
-        const double* T = w.trans[buf];
-        if (wt[2] > 0.0) {
-            const double sc = sqrt(wt[2]);
-            const D3 field_a = radd(radd(rmat(R + a * 9, gd), ga), load_d3(T, a));
-            const D3 field_b = radd(gb, load_d3(T, b));
-            const D3 diff = rmul(rsub(field_a, field_b), sc);
-            energy = da(da(dm(diff.x, diff.x), dm(diff.y, diff.y)), dm(diff.z, diff.z));
-        }
-        if (assembles(c)) {
-            float blk[36];
-            for (int i = 0; i < 36; ++i) blk[i] = 0.0f;
-            if (wt[2] > 0.0) {
-                const float ws = (float)wt[2];
-                const F3 cv = mul3f(w.rot32 + a * 9, {(float)gd.x, (float)gd.y, (float)gd.z});
-                // ws * [[0, -[c]x], [0, -I]]
-                if (c.route == 0) {
-                    blk[0 * 6 + 4] = ws * cv.z;  blk[0 * 6 + 5] = -ws * cv.y;
-                    blk[1 * 6 + 3] = -ws * cv.z; blk[1 * 6 + 5] = ws * cv.x;
-                    blk[2 * 6 + 3] = ws * cv.y;  blk[2 * 6 + 4] = -ws * cv.x;
-                }
-                blk[3 * 6 + 3] = -ws; blk[4 * 6 + 4] = -ws; blk[5 * 6 + 5] = -ws;
-            }
-            // into the pair's block when the pair shares a vertex (the pair
-            // assembly, launched before on the same stream, wrote it this tick)
-            const int k = L.edge_block[e];
-            if (k < L.pair_count) {
-                add_block_pair(w.offdiag[1 - c.system], L, k, blk);
-            } else {
-                store_block_pair(w.offdiag[1 - c.system], L, k, blk);
-            }
-        }
+    const int node_blocks = blocks_of_dev((long)L.node_count * 32, kNodeThreads);
+    const int warp = threadIdx.x >> 5;
+    if (bx < node_blocks) {
+        const int node = bx * (kNodeThreads / 32) + warp;
+        if (node < L.node_count) assemble_node(w, c, node);
+    } else if (assembles(c)) {
+        const int k = (bx - node_blocks) * (kNodeThreads / 32) + warp;
+        if (k < L.offdiag_count) assemble_block(w, c, k);
     }
-    // the edge's smoothness energy; the decision kernel sums them as a block
-    // sum over this block would (no block barrier here)
-    if (e < L.edge_count) w.edge_partials[e] = energy;
 }
 
-__global__ void __launch_bounds__(kEdgeThreads) k_edge_assemble(const WrapDev* __restrict__ wraps, int wrap_count, int part) {
+// Two blocks per SM (127 registers, no spills): three spill (80 registers; a
+// batch of 16 wraps 54 against 46 ms of assembly), one leaves too few warps
+// (68 ms).
+__global__ void __launch_bounds__(kNodeThreads, 2) k_assemble(const WrapDev* __restrict__ wraps, int wrap_count, int part) {
     over_virtual_blocks<false>(
         wraps, wrap_count,
         [&](const WrapDev& w) {
             const WrapControl c = *w.control;
-            return in_part(c, part) ? (computes_energy(c) ? blocks_of_dev(w.levels[c.level].edge_count, kEdgeThreads) : 0) : 0;
+            if (!in_part(c, part) || !computes_energy(c)) return 0;
+            const LevelDev& L = w.levels[c.level];
+            return blocks_of_dev((long)L.node_count * 32, kNodeThreads) +
+                   (assembles(c) ? blocks_of_dev((long)L.offdiag_count * 32, kNodeThreads) : 0);
         },
-        [&](int wi, int bx) { k_edge_assemble_body(wraps[wi], part, bx); });
+        [&](int wi, int bx) { k_assemble_body(wraps[wi], part, bx); });
 }
 
 // ---------------------------------------------------------------------------
@@ -1926,67 +1980,67 @@ __device__ inline double relative_change(double before, double after) {  // rout
     return (before - after) / fmax(fabs(before), 1e-12);
 }
 
-__global__ void k_decide(const WrapDev* __restrict__ wraps, int part) {
+constexpr int kDecideThreads = 256;
+constexpr int kMaxEdgeSums = 512;  // a multiple of kDecideThreads
+__global__ void __launch_bounds__(kDecideThreads) k_decide(const WrapDev* __restrict__ wraps, int part) {
     const WrapDev& w = wraps[blockIdx.x];
     WrapControl* ctl = w.control;
     if (part != 0 && (part == 1) != (ctl->tick_phase == kPhaseSolve)) return;
     const int phase = ctl->phase;
     if (phase == kPhaseDone) return;
-    __shared__ double scratch[33];
+    constexpr int kWarps = kDecideThreads / 32;
+    __shared__ double scratch[kWarps * kEnergyKinds];
+    __shared__ double edge_sums[kMaxEdgeSums];
     __shared__ double parts_s[kEnergyKinds];
     const WrapControl c0 = *ctl;
     if (computes_energy(c0)) {
         const LevelDev& L = w.levels[c0.level];
         const int vb = (w.V + kVertexThreads - 1) / kVertexThreads;
-        const int eb = (L.edge_count + kEdgeThreads - 1) / kEdgeThreads;
+        const int eb = (L.edge_count + kEdgeSums - 1) / kEdgeSums;
         const int nb = (L.node_count + kNodeThreads / 32 - 1) / (kNodeThreads / 32);
-        double s0 = 0, s1 = 0, s4 = 0, s2 = 0, s3 = 0;
+        double s[kEnergyKinds] = {0, 0, 0, 0, 0};
         for (int i = threadIdx.x; i < vb; i += blockDim.x) {
-            s0 += w.partials[(long)i * kPartialStride];
-            s1 += w.partials[(long)i * kPartialStride + 1];
-            s4 += w.partials[(long)i * kPartialStride + 2];
+            s[0] += w.partials[(long)i * kPartialStride];
+            s[1] += w.partials[(long)i * kPartialStride + 1];
+            s[4] += w.partials[(long)i * kPartialStride + 2];
         }
-        for (int i = threadIdx.x; i < eb; i += blockDim.x) {
-            // edge block i's smoothness energy, summed in the order of a block
-            // sum over its 128 threads: a butterfly within each warp (lane l
-            // holds edge 128i + 32j + l, zero past the last edge), then the
-            // four warps' sums, ((w0 + w2) + (w1 + w3)); the zeros the other
-            // lanes add change nothing (energies are non-negative)
-            static_assert(kEdgeThreads == 4 * 32, "four warps per edge block");
-            double warp_total[4];
-            for (int j = 0; j < 4; ++j) {
-                double x[32];
-                for (int l = 0; l < 32; ++l) {
-                    const int e = i * kEdgeThreads + j * 32 + l;
-                    x[l] = e < L.edge_count ? w.edge_partials[e] : 0.0;
+        // Each 128 edges' smoothness energy, summed in the order of a block
+        // sum over 128 threads: a butterfly within each 32 (zero past the last
+        // edge), then ((w0 + w2) + (w1 + w3)).  A warp takes 128 edges at a
+        // time with coalesced loads; thread i then adds sum i, i + 256, ...
+        // (one thread per 128 edges, summing 128 values of its own, took 6 us).
+        const int lane = threadIdx.x & 31;
+        for (int base = 0; base < eb; base += kMaxEdgeSums) {
+            const int here = min(kMaxEdgeSums, eb - base);
+            for (int i = threadIdx.x >> 5; i < here; i += kWarps) {
+                double x[4];
+                for (int j = 0; j < 4; ++j) {
+                    const int e = (base + i) * kEdgeSums + j * 32 + lane;
+                    x[j] = e < L.edge_count ? w.edge_partials[e] : 0.0;
                 }
                 for (int o = 16; o > 0; o >>= 1)
-                    for (int l = 0; l < o; ++l) x[l] = x[l] + x[l + o];
-                warp_total[j] = x[0];
+                    for (int j = 0; j < 4; ++j) x[j] += __shfl_xor_sync(0xffffffffu, x[j], o);
+                if (lane == 0) edge_sums[i] = (x[0] + x[2]) + (x[1] + x[3]);
             }
-            s2 += (warp_total[0] + warp_total[2]) + (warp_total[1] + warp_total[3]);
+            __syncthreads();
+            for (int i = threadIdx.x; i < here; i += blockDim.x) s[2] += edge_sums[i];
+            __syncthreads();
         }
         for (int i = threadIdx.x; i < nb; i += blockDim.x) {
             // node block i's anchor energy, summed in the order of a block sum
-            // over its 8 warps (lane 0 of warp j holds node 8i + j; the other
-            // lanes add zeros, which change nothing)
-            static_assert(kNodeThreads == 8 * 32, "eight nodes per node block");
+            // over 8 warps (node 8i + j in lane 0 of warp j; the other lanes'
+            // zeros change nothing)
+            static_assert(kNodeThreads == 8 * 32, "eight nodes per partial sum");
             double v[8];
             for (int j = 0; j < 8; ++j) {
                 const int n = i * 8 + j;
                 v[j] = n < L.node_count ? w.node_partials[n] : 0.0;
             }
-            s3 += ((v[0] + v[4]) + (v[2] + v[6])) + ((v[1] + v[5]) + (v[3] + v[7]));
+            s[3] += ((v[0] + v[4]) + (v[2] + v[6])) + ((v[1] + v[5]) + (v[3] + v[7]));
         }
-        const double t0 = block_sum<256>(s0, scratch);
-        const double t1 = block_sum<256>(s1, scratch);
-        const double t2 = block_sum<256>(s2, scratch);
-        const double t3 = block_sum<256>(s3, scratch);
-        const double t4 = block_sum<256>(s4, scratch);
-        if (threadIdx.x == 0) {
-            parts_s[0] = t0; parts_s[1] = t1; parts_s[2] = t2; parts_s[3] = t3; parts_s[4] = t4;
-        }
-        __syncthreads();
+        block_sums<kDecideThreads, kEnergyKinds>(s, scratch);
+        if (threadIdx.x == 0)
+            for (int k = 0; k < kEnergyKinds; ++k) parts_s[k] = s[k];
     }
     // the long walks this tick's query took from its list are done: clear
     // their flags and empty the list, which the next query but one fills
@@ -2094,7 +2148,7 @@ __global__ void k_decide(const WrapDev* __restrict__ wraps, int part) {
 // Grids of the virtual-block kernels: as many blocks as fit on the device
 // at once (occupancy of each kernel at its block size, times the SMs).
 struct VirtualGrids {
-    int prologue, c_fit, c_rhs, evaluate, normals, residual, node, pair, edge;
+    int prologue, c_fit, c_rhs, evaluate, normals, residual, candidate, assemble;
 };
 const VirtualGrids& virtual_grids() {
     static const VirtualGrids grids = [] {
@@ -2112,10 +2166,9 @@ const VirtualGrids& virtual_grids() {
         g.c_rhs = fit(k_c_rhs, kNodeThreads);
         g.evaluate = fit(k_evaluate, kVertexThreads);
         g.normals = fit(k_normals, kVertexThreads);
-        g.residual = fit(k_residual, kVertexThreads);
-        g.node = fit(k_node_assemble, kNodeThreads);
-        g.pair = fit(k_pair_assemble, kNodeThreads);
-        g.edge = fit(k_edge_assemble, kEdgeThreads);
+        g.residual = fit(k_residual<false>, kVertexThreads);
+        g.candidate = fit(k_residual<true>, kVertexThreads);
+        g.assemble = fit(k_assemble, kNodeThreads);
         return g;
     }();
     return grids;
@@ -2139,14 +2192,18 @@ void launch_tick(const WrapDev* wraps, const TickShape& s, cudaStream_t stream,
     const bool split = s.side_stream != nullptr && !timed;
     const int solve_part = split ? 1 : 0, refresh_part = split ? 2 : 0;
     cudaStream_t refresh = split ? s.side_stream : stream;
-    auto assemble_and_decide = [&](int part, cudaStream_t on) {
+    // evaluate: the solve chain's kernel deforms the candidate's vertices too
+    // (a timed tick's refresh chain has done it, for either kind of wrap)
+    auto assemble_and_decide = [&](int part, bool evaluate, cudaStream_t on) {
         if (timed) cudaEventRecord(timers->assemble_begin, on);
-        k_residual<<<grids.residual, kVertexThreads, virtual_smem, on>>>(wraps, W, part);
-        k_node_assemble<<<grids.node, kNodeThreads, virtual_smem, on>>>(wraps, W, part);
-        if (s.max_pairs > 0) k_pair_assemble<<<grids.pair, kNodeThreads, virtual_smem, on>>>(wraps, W, part);
-        k_edge_assemble<<<grids.edge, kEdgeThreads, virtual_smem, on>>>(wraps, W, part);
+        if (evaluate) {
+            k_residual<true><<<grids.candidate, kVertexThreads, virtual_smem, on>>>(wraps, W, part);
+        } else {
+            k_residual<false><<<grids.residual, kVertexThreads, virtual_smem, on>>>(wraps, W, part);
+        }
+        k_assemble<<<grids.assemble, kNodeThreads, virtual_smem, on>>>(wraps, W, part);
         if (timed) cudaEventRecord(timers->assemble_end, on);
-        k_decide<<<W, 256, 0, on>>>(wraps, part);
+        k_decide<<<W, kDecideThreads, 0, on>>>(wraps, part);
     };
     if (split) {
         cudaEventRecord(s.side_fork, stream);
@@ -2188,10 +2245,7 @@ void launch_tick(const WrapDev* wraps, const TickShape& s, cudaStream_t stream,
         for (int g = 1; g < s.pcg_groups; ++g) cudaStreamWaitEvent(stream, s.pcg_join[g], 0);
     }
     if (timed) cudaEventRecord(timers->pcg_end, stream);
-    if (split) {
-        k_evaluate<<<grids.evaluate, kVertexThreads, virtual_smem, stream>>>(wraps, W, solve_part);
-        assemble_and_decide(solve_part, stream);
-    }
+    if (split) assemble_and_decide(solve_part, true, stream);
 
     // ---- the refresh chain ----
     k_prologue<<<grids.prologue, 128, virtual_smem, refresh>>>(wraps, W, refresh_part);
@@ -2201,7 +2255,7 @@ void launch_tick(const WrapDev* wraps, const TickShape& s, cudaStream_t stream,
     launch_query(wraps, W, refresh, s.query_counter);
     if (timed) cudaEventRecord(timers->query_end, refresh);
     k_stats<<<dim3(1, W), kStatsThreads, 0, refresh>>>(wraps, 1);
-    assemble_and_decide(refresh_part, refresh);
+    assemble_and_decide(refresh_part, false, refresh);
     if (split) {
         cudaEventRecord(s.side_join, refresh);
         cudaStreamWaitEvent(stream, s.side_join, 0);
@@ -2209,10 +2263,10 @@ void launch_tick(const WrapDev* wraps, const TickShape& s, cudaStream_t stream,
 }
 
 int tick_kernel_launches(const TickShape& s, bool timed) {
-    // an untimed tick with a side stream assembles and decides in each branch
-    const int per_chain = (s.max_pairs > 0 ? 5 : 4) + 1;  // residual, node, pair, edge, decide; evaluate
-    return (s.max_pairs > 0 ? 14 : 13) - (s.route_c ? 0 : 2) + (s.pcg_groups > 0 ? s.pcg_groups : 1) +
-           (s.side_stream && !timed ? per_chain : 0);
+    // stats twice, [fit, rhs,] solve launches, prologue, evaluate, normals,
+    // query, residual, assembly, decision; an untimed tick with a side stream
+    // runs the last three in each branch
+    return 9 + (s.route_c ? 2 : 0) + (s.pcg_groups > 0 ? s.pcg_groups : 1) + (s.side_stream && !timed ? 3 : 0);
 }
 
 // Cluster size of the solve for one wrap of `nodes` nodes on its own: a
