@@ -21,6 +21,8 @@ size_t lbvh_scratch_bytes(int triangle_count);
 uint32_t lbvh_build(const double* points, const int32_t* faces, int triangle_count,
                     void* scratch, float4* nodes, float4* leaves, cudaStream_t stream,
                     LbvhExport* out);
+// Kernels one hierarchy build launches.
+int lbvh_build_launches(int triangle_count);
 // The target's ingestion on the device, once after its upload in the caller's
 // units: its points normalised in place ((p - center) * scale) and its
 // area-weighted vertex normals, both bit-identical to the host's.

@@ -3,11 +3,10 @@
 // Build (once per target, all on the device): FP32 triangle centroids and
 // scene bounds, 30-bit Morton codes with the reference's quantisation
 // (src/cuda/lbvh.cu:146-168), a stable LSD radix sort of (code, index) written
-// here (4-bit digits, per-tile ranking in shared memory), Karras' split search
+// here (8-bit digits, warps ranking their keys by ballots), Karras' split search
 // with index tie-breaking (lbvh.cu:177-245), and a bottom-up box fit with the
 // fence + arrival-counter protocol (no waiting: the second child to arrive
-// merges).  The hierarchy is then packed for traversal with each child's box
-// stored in its parent (64 B per internal node = one L2 line pair), so a
+// merges), straight into the traversal layout, with each child's box stored in its parent (64 B per internal node = one L2 line pair), so a
 // visit costs one 64-byte load instead of three dependent ones.
 //
 // Query (a group of lanes per template vertex): the previous correspondence's triangle
@@ -28,8 +27,13 @@ namespace {
 constexpr int kThreads = 256;
 constexpr int kSortItems = 8;                       // keys per thread per tile
 constexpr int kSortTile = kThreads * kSortItems;    // 2048 keys
-constexpr int kRadixBits = 4;
-constexpr int kRadix = 1 << kRadixBits;             // 16 bins
+constexpr int kRadixBits = 8;
+constexpr int kRadix = 1 << kRadixBits;             // 256 bins, one per thread
+// Up to this many tiles every tile's block sums the tiles' counts itself; past
+// it a scan kernel does (each block's sum would pass 10 us).
+constexpr int kTilesSummed = 128;
+
+int blocks_for(long n, int threads = kThreads) { return (int)((n + threads - 1) / threads); }
 
 __device__ inline uint32_t expand_bits(uint32_t v) {  // lbvh.cu:132-139
     v &= 0x000003ffu;
@@ -40,171 +44,259 @@ __device__ inline uint32_t expand_bits(uint32_t v) {  // lbvh.cu:132-139
     return v;
 }
 
-// FP32 copies of the target corners, triangle centroids ((a+b+c)/3 with each
-// operation rounded on its own, as lbvh.cu:44-45 evaluates it).
+// Floats as integers in the same order (negative ones flipped), so that the
+// scene bounds are integer atomics: minima and maxima are exact in any order.
+__device__ inline uint32_t ordered_bits(float x) {
+    const uint32_t b = __float_as_uint(x);
+    return (b & 0x80000000u) ? ~b : (b | 0x80000000u);
+}
+__device__ inline float ordered_float(uint32_t o) {
+    return __uint_as_float((o & 0x80000000u) ? (o & 0x7fffffffu) : ~o);
+}
+
+// Triangle centroids from FP32 copies of the corners ((a+b+c)/3 with each
+// operation rounded on its own, as lbvh.cu:44-45 evaluates it), and their
+// bounds: three ordered minima, then three ordered maxima, complemented so
+// that all six start from 0xff bytes.  (Folding the blocks' partial bounds in
+// one thread took 85 to 108 us, a third of a hierarchy export.)
 __global__ void k_centroids(const double* __restrict__ points, const int32_t* __restrict__ faces,
-                            int count, float* __restrict__ centroids) {
-    const int t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= count) return;
-    const int32_t* f = faces + (long)t * 3;
-    for (int k = 0; k < 3; ++k) {
-        const float a = __double2float_rn(points[(long)f[0] * 3 + k]);
-        const float b = __double2float_rn(points[(long)f[1] * 3 + k]);
-        const float c = __double2float_rn(points[(long)f[2] * 3 + k]);
-        centroids[(long)t * 3 + k] = __fdiv_rn(__fadd_rn(__fadd_rn(a, b), c), 3.0f);
-    }
-}
-
-// Scene bounds of the centroids: per-block partials, then one block folds
-// them.  min/max are exact, so the order does not matter.
-__global__ void k_bounds_partial(const float* __restrict__ centroids, int count,
-                                 float* __restrict__ partial) {
-    __shared__ float lo[3][kThreads], hi[3][kThreads];
-    float l[3] = {3.4e38f, 3.4e38f, 3.4e38f}, h[3] = {-3.4e38f, -3.4e38f, -3.4e38f};
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < count; i += gridDim.x * blockDim.x)
+                            int count, float* __restrict__ centroids, uint32_t* __restrict__ ordered) {
+    // bounds start at +-3.4e38, and a centroid that is no number does not count
+    const uint32_t start = ordered_bits(3.4e38f), start_max = ~ordered_bits(-3.4e38f);
+    uint32_t best[6] = {start, start, start, start_max, start_max, start_max};
+    for (long t = (long)blockIdx.x * blockDim.x + threadIdx.x; t < count; t += (long)gridDim.x * blockDim.x) {
+        const int32_t* f = faces + t * 3;
         for (int k = 0; k < 3; ++k) {
-            l[k] = fminf(l[k], centroids[(long)i * 3 + k]);
-            h[k] = fmaxf(h[k], centroids[(long)i * 3 + k]);
+            const float a = __double2float_rn(points[(long)f[0] * 3 + k]);
+            const float b = __double2float_rn(points[(long)f[1] * 3 + k]);
+            const float c = __double2float_rn(points[(long)f[2] * 3 + k]);
+            const float m = __fdiv_rn(__fadd_rn(__fadd_rn(a, b), c), 3.0f);
+            centroids[t * 3 + k] = m;
+            if (m != m) continue;
+            const uint32_t o = ordered_bits(m);
+            best[k] = min(best[k], o);
+            best[3 + k] = min(best[3 + k], ~o);
         }
-    for (int k = 0; k < 3; ++k) { lo[k][threadIdx.x] = l[k]; hi[k][threadIdx.x] = h[k]; }
+    }
+    for (int k = 0; k < 6; ++k) best[k] = __reduce_min_sync(0xffffffffu, best[k]);
+    __shared__ uint32_t warp_best[6][kThreads / 32];
+    if ((threadIdx.x & 31) == 0)
+        for (int k = 0; k < 6; ++k) warp_best[k][threadIdx.x >> 5] = best[k];
     __syncthreads();
-    for (int s = blockDim.x / 2; s > 0; s >>= 1) {
-        if (threadIdx.x < s)
-            for (int k = 0; k < 3; ++k) {
-                lo[k][threadIdx.x] = fminf(lo[k][threadIdx.x], lo[k][threadIdx.x + s]);
-                hi[k][threadIdx.x] = fmaxf(hi[k][threadIdx.x], hi[k][threadIdx.x + s]);
-            }
-        __syncthreads();
+    if (threadIdx.x < 6) {
+        uint32_t x = warp_best[threadIdx.x][0];
+        for (int i = 1; i < kThreads / 32; ++i) x = min(x, warp_best[threadIdx.x][i]);
+        atomicMin(ordered + threadIdx.x, x);
     }
-    if (threadIdx.x == 0)
-        for (int k = 0; k < 3; ++k) {
-            partial[blockIdx.x * 6 + k] = lo[k][0];
-            partial[blockIdx.x * 6 + 3 + k] = hi[k][0];
-        }
 }
 
-__global__ void k_bounds_final(const float* __restrict__ partial, int blocks,
-                               float* __restrict__ bounds) {
-    if (threadIdx.x != 0) return;
-    float l[3] = {3.4e38f, 3.4e38f, 3.4e38f}, h[3] = {-3.4e38f, -3.4e38f, -3.4e38f};
-    for (int b = 0; b < blocks; ++b)
-        for (int k = 0; k < 3; ++k) {
-            l[k] = fminf(l[k], partial[b * 6 + k]);
-            h[k] = fmaxf(h[k], partial[b * 6 + 3 + k]);
-        }
-    for (int k = 0; k < 3; ++k) { bounds[k] = l[k]; bounds[3 + k] = h[k]; }
-}
-
-__global__ void k_morton(const float* __restrict__ centroids, int count,
-                         const float* __restrict__ bounds, uint32_t* __restrict__ codes,
-                         uint32_t* __restrict__ order) {
-    const int t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= count) return;
-    uint32_t q[3];
-    for (int k = 0; k < 3; ++k) {
-        const float extent = __fsub_rn(bounds[3 + k], bounds[k]);
-        const float scale = extent > 1e-10f ? __fdiv_rn(1023.0f, extent) : 0.0f;
-        const float v = __fmul_rn(__fsub_rn(centroids[(long)t * 3 + k], bounds[k]), scale);
-        q[k] = (uint32_t)fminf(1023.0f, fmaxf(0.0f, v));
-    }
-    codes[t] = (expand_bits(q[2]) << 2) | (expand_bits(q[1]) << 1) | expand_bits(q[0]);
-    order[t] = (uint32_t)t;
-}
-
-// ---- stable LSD radix sort of (key, value), 4-bit digits --------------------
-
-__global__ void k_radix_histogram(const uint32_t* __restrict__ keys, int count, int shift,
-                                  uint32_t* __restrict__ counts, int tiles) {
+// Morton codes in the caller's numbering, the identity permutation, the bounds
+// as floats, and the first sort pass's digit counts: a block per sort tile.
+__global__ void k_morton(const float* __restrict__ centroids, int count, const uint32_t* __restrict__ ordered,
+                         float* __restrict__ bounds_out, uint32_t* __restrict__ codes, uint32_t* __restrict__ order,
+                         uint32_t* __restrict__ counts) {
     __shared__ uint32_t bins[kRadix];
-    if (threadIdx.x < kRadix) bins[threadIdx.x] = 0;
+    bins[threadIdx.x] = 0;
+    __syncthreads();
+    float lo[3], scale[3];
+    for (int k = 0; k < 3; ++k) {
+        lo[k] = ordered_float(ordered[k]);
+        const float hi = ordered_float(~ordered[3 + k]);
+        const float extent = __fsub_rn(hi, lo[k]);
+        scale[k] = extent > 1e-10f ? __fdiv_rn(1023.0f, extent) : 0.0f;
+        if (blockIdx.x == 0 && threadIdx.x == 0) {
+            bounds_out[k] = lo[k];
+            bounds_out[3 + k] = hi;
+        }
+    }
+    const long base = (long)blockIdx.x * kSortTile;
+    for (int i = threadIdx.x; i < kSortTile; i += kThreads) {
+        const long t = base + i;
+        if (t >= count) break;
+        uint32_t q[3];
+        for (int k = 0; k < 3; ++k)
+            q[k] = (uint32_t)fminf(1023.0f, fmaxf(0.0f, __fmul_rn(__fsub_rn(centroids[t * 3 + k], lo[k]), scale[k])));
+        const uint32_t code = (expand_bits(q[2]) << 2) | (expand_bits(q[1]) << 1) | expand_bits(q[0]);
+        codes[t] = code;
+        order[t] = (uint32_t)t;
+        atomicAdd(&bins[code & (kRadix - 1)], 1u);
+    }
+    __syncthreads();
+    counts[(long)blockIdx.x * kRadix + threadIdx.x] = bins[threadIdx.x];
+}
+
+// ---- stable LSD radix sort of (key, value), 8-bit digits ---------------------
+//
+// Per pass: each 2,048-key tile's digit counts (tile-major), then a scatter
+// whose block finds its tile's place for every digit by summing the tiles'
+// counts, a thread per digit -- or, past kTilesSummed tiles, reads the sums a
+// scan kernel left.  Eight-bit digits sort 30-bit codes in four passes; with
+// 4-bit digits it was eight passes of three kernels each, 60 % of the build.
+
+__global__ void k_radix_counts(const uint32_t* __restrict__ keys, long count, int shift,
+                               uint32_t* __restrict__ counts) {
+    __shared__ uint32_t bins[kRadix];
+    bins[threadIdx.x] = 0;
     __syncthreads();
     const long base = (long)blockIdx.x * kSortTile;
-    for (int i = threadIdx.x; i < kSortTile; i += blockDim.x) {
-        const long at = base + i;
-        if (at < count) atomicAdd(&bins[(keys[at] >> shift) & (kRadix - 1)], 1u);
-    }
+    for (int i = threadIdx.x; i < kSortTile; i += kThreads)
+        if (base + i < count) atomicAdd(&bins[(keys[base + i] >> shift) & (kRadix - 1)], 1u);
     __syncthreads();
-    if (threadIdx.x < kRadix) counts[threadIdx.x * tiles + blockIdx.x] = bins[threadIdx.x];
+    counts[(long)blockIdx.x * kRadix + threadIdx.x] = bins[threadIdx.x];
 }
 
-// Exclusive scan of the digit-major count matrix in one block.
-__global__ void k_radix_scan(uint32_t* __restrict__ counts, int total) {
-    __shared__ uint32_t sums[1024];
-    const int per = (total + blockDim.x - 1) / blockDim.x;
-    const int begin = threadIdx.x * per;
-    uint32_t local = 0;
-    for (int i = begin; i < begin + per && i < total; ++i) local += counts[i];
-    sums[threadIdx.x] = local;
-    __syncthreads();
-    for (int s = 1; s < blockDim.x; s <<= 1) {
-        const uint32_t v = threadIdx.x >= s ? sums[threadIdx.x - s] : 0;
+// A block per digit: its counts over the tiles become exclusive sums, the
+// digit's total goes after the last tile's row.
+__global__ void k_radix_sums(uint32_t* __restrict__ counts, int tiles) {
+    __shared__ uint32_t warp_sum[kThreads / 32];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    uint32_t running = 0;
+    for (int base = 0; base < tiles; base += kThreads) {
+        const int t = base + threadIdx.x;
+        const uint32_t c = t < tiles ? counts[(long)t * kRadix + blockIdx.x] : 0;
+        uint32_t x = c;
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
+            if (lane >= o) x += y;
+        }
+        if (lane == 31) warp_sum[warp] = x;
         __syncthreads();
-        sums[threadIdx.x] += v;
+        uint32_t before = 0, all = 0;
+        for (int i = 0; i < kThreads / 32; ++i) {
+            if (i < warp) before += warp_sum[i];
+            all += warp_sum[i];
+        }
+        if (t < tiles) counts[(long)t * kRadix + blockIdx.x] = running + before + x - c;
+        running += all;
         __syncthreads();
     }
-    uint32_t running = threadIdx.x == 0 ? 0 : sums[threadIdx.x - 1];
-    for (int i = begin; i < begin + per && i < total; ++i) {
-        const uint32_t c = counts[i];
-        counts[i] = running;
-        running += c;
-    }
+    if (threadIdx.x == 0) counts[(long)tiles * kRadix + blockIdx.x] = running;
 }
 
-// Each thread owns kSortItems consecutive keys of the tile, so ranking by
-// (digit, thread, position) preserves the input order within a digit.
-__global__ void k_radix_scatter(const uint32_t* __restrict__ keys_in,
-                                const uint32_t* __restrict__ values_in, int count, int shift,
-                                const uint32_t* __restrict__ offsets, int tiles,
-                                uint32_t* __restrict__ keys_out,
-                                uint32_t* __restrict__ values_out) {
-    __shared__ uint32_t grid_counts[kRadix * kThreads];  // [digit][thread]
-    __shared__ uint32_t partial[kThreads];
-    const long base = (long)blockIdx.x * kSortTile + (long)threadIdx.x * kSortItems;
-    uint32_t k[kSortItems], v[kSortItems];
-    int digit[kSortItems];
-    uint32_t mine[kRadix];
-    for (int d = 0; d < kRadix; ++d) mine[d] = 0;
-    for (int i = 0; i < kSortItems; ++i) {
-        const long at = base + i;
-        digit[i] = -1;
-        if (at < count) {
-            k[i] = keys_in[at];
-            v[i] = values_in[at];
-            digit[i] = (k[i] >> shift) & (kRadix - 1);
-            mine[digit[i]]++;
+// Each warp owns 256 consecutive keys of the tile and ranks them 32 at a time
+// in order, so equal digits keep their input order.
+__global__ void __launch_bounds__(kThreads) k_radix_scatter(
+    const uint32_t* __restrict__ keys_in, const uint32_t* __restrict__ values_in, long count, int shift,
+    const uint32_t* __restrict__ counts, int tiles, int summed, uint32_t* __restrict__ keys_out,
+    uint32_t* __restrict__ values_out) {
+    constexpr int kWarps = kThreads / 32;
+    __shared__ uint32_t held[kWarps][kRadix];  // a warp's keys of each digit so far; then its place for the digit
+    __shared__ uint32_t warp_sum[kWarps];
+    __shared__ alignas(16) uint32_t part[2][4][kRadix];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, digit = threadIdx.x;
+    for (int i = 0; i < kWarps; ++i) held[i][digit] = 0;
+    // this tile's keys before it per digit, and the digit's total
+    uint32_t before = 0, total = 0;
+    if (summed) {
+        before = counts[(long)blockIdx.x * kRadix + digit];
+        total = counts[(long)tiles * kRadix + digit];
+    } else {
+        // four digits and every fourth tile per thread
+        const int quad = threadIdx.x & 63, row = threadIdx.x >> 6;
+        uint4 b4 = make_uint4(0, 0, 0, 0), t4 = b4;
+#pragma unroll 8
+        for (int t = row; t < tiles; t += 4) {
+            const uint4 c = reinterpret_cast<const uint4*>(counts + (long)t * kRadix)[quad];
+            t4.x += c.x; t4.y += c.y; t4.z += c.z; t4.w += c.w;
+            if (t < (int)blockIdx.x) { b4.x += c.x; b4.y += c.y; b4.z += c.z; b4.w += c.w; }
+        }
+        reinterpret_cast<uint4*>(part[0][row])[quad] = b4;
+        reinterpret_cast<uint4*>(part[1][row])[quad] = t4;
+        __syncthreads();
+        for (int i = 0; i < 4; ++i) {
+            before += part[0][i][digit];
+            total += part[1][i][digit];
         }
     }
-    for (int d = 0; d < kRadix; ++d) grid_counts[d * kThreads + threadIdx.x] = mine[d];
-    __syncthreads();
-    // exclusive scan of the [digit][thread] matrix: each thread sums a run of
-    // kRadix consecutive entries, a block scan of the runs, then write-back.
-    uint32_t run = 0;
-    for (int i = 0; i < kRadix; ++i) run += grid_counts[threadIdx.x * kRadix + i];
-    partial[threadIdx.x] = run;
-    __syncthreads();
-    for (int s = 1; s < kThreads; s <<= 1) {
-        const uint32_t add = threadIdx.x >= s ? partial[threadIdx.x - s] : 0;
-        __syncthreads();
-        partial[threadIdx.x] += add;
-        __syncthreads();
+    uint32_t x = total;  // exclusive scan of the totals over the digits
+    for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
+        if (lane >= o) x += y;
     }
-    uint32_t running = threadIdx.x == 0 ? 0 : partial[threadIdx.x - 1];
-    for (int i = 0; i < kRadix; ++i) {
-        const uint32_t c = grid_counts[threadIdx.x * kRadix + i];
-        grid_counts[threadIdx.x * kRadix + i] = running;
-        running += c;
-    }
+    if (lane == 31) warp_sum[warp] = x;
     __syncthreads();
-    uint32_t local[kRadix];
-    for (int d = 0; d < kRadix; ++d)
-        local[d] = grid_counts[d * kThreads + threadIdx.x] - grid_counts[d * kThreads] +
-                   offsets[d * tiles + blockIdx.x];
+    uint32_t place = before + x - total;
+    for (int i = 0; i < warp; ++i) place += warp_sum[i];
+    // ranks within the warp's keys
+    const long base = (long)blockIdx.x * kSortTile + warp * (kSortTile / kWarps) + lane;
+    uint32_t k[kSortItems], v[kSortItems], rank[kSortItems];
+#pragma unroll
     for (int i = 0; i < kSortItems; ++i) {
-        if (digit[i] < 0) continue;
-        const uint32_t at = local[digit[i]]++;
+        const long at = base + i * 32;
+        k[i] = at < count ? keys_in[at] : 0xffffffffu;
+        v[i] = at < count ? values_in[at] : 0;
+    }
+#pragma unroll
+    for (int i = 0; i < kSortItems; ++i) {
+        const bool on = base + i * 32 < count;
+        const uint32_t d = (k[i] >> shift) & (kRadix - 1);
+        uint32_t same = __ballot_sync(0xffffffffu, on);  // the lanes with this digit
+#pragma unroll
+        for (int bit = 0; bit < kRadixBits; ++bit) {
+            const uint32_t set = __ballot_sync(0xffffffffu, (d >> bit) & 1u);
+            same &= ((d >> bit) & 1u) ? set : ~set;
+        }
+        const uint32_t ahead = on ? held[warp][d] : 0;
+        rank[i] = ahead + __popc(same & ((1u << lane) - 1u));
+        __syncwarp();
+        if (on && (same >> lane) == 1u) held[warp][d] = rank[i] + 1;  // its last lane
+        __syncwarp();
+    }
+    __syncthreads();
+    // each warp's place for the digit
+    for (int i = 0; i < kWarps; ++i) {
+        const uint32_t c = held[i][digit];
+        held[i][digit] = place;
+        place += c;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int i = 0; i < kSortItems; ++i) {
+        if (base + i * 32 >= count) continue;
+        const uint32_t at = held[warp][(k[i] >> shift) & (kRadix - 1)] + rank[i];
         keys_out[at] = k[i];
         values_out[at] = v[i];
     }
+}
+
+size_t radix_count_bytes(long n) {
+    return sizeof(uint32_t) * kRadix * (size_t)((n + kSortTile - 1) / kSortTile + 1);
+}
+
+// Sorts by the low `bits` bits between the two buffer pairs; returns the pair
+// that holds the result.  `counted`: the first pass's counts are there.
+int radix_sort(uint32_t* const keys[2], uint32_t* const values[2], long n, int bits, bool counted, uint32_t* counts,
+               cudaStream_t stream) {
+    const int tiles = (int)((n + kSortTile - 1) / kSortTile);
+    const int summed = tiles > kTilesSummed ? 1 : 0;
+    int cur = 0;
+    for (int shift = 0; shift < bits; shift += kRadixBits) {
+        if (shift > 0 || !counted) k_radix_counts<<<tiles, kThreads, 0, stream>>>(keys[cur], n, shift, counts);
+        if (summed) k_radix_sums<<<kRadix, kThreads, 0, stream>>>(counts, tiles);
+        k_radix_scatter<<<tiles, kThreads, 0, stream>>>(keys[cur], values[cur], n, shift, counts, tiles, summed,
+                                                        keys[1 - cur], values[1 - cur]);
+        cur = 1 - cur;
+    }
+    return cur;
+}
+
+int radix_sort_launches(long n, int bits, bool counted) {
+    const int passes = (bits + kRadixBits - 1) / kRadixBits;
+    return passes * ((n + kSortTile - 1) / kSortTile > kTilesSummed ? 3 : 2) - (counted ? 1 : 0);
+}
+
+constexpr int kCodeBits = 30;
+
+// Centroids, bounds, codes and the sort, shared by the build and the export:
+// returns the buffer pair with the sorted codes (with 30-bit codes the first).
+int sorted_codes(const double* points, const int32_t* faces, int n, float* centroids, uint32_t* ordered, float* bounds,
+                 uint32_t* const keys[2], uint32_t* const values[2], uint32_t* counts, cudaStream_t stream) {
+    const int blocks = blocks_for(n);
+    cudaMemsetAsync(ordered, 0xff, sizeof(uint32_t) * 6, stream);
+    k_centroids<<<blocks < 592 ? blocks : 592, kThreads, 0, stream>>>(points, faces, n, centroids, ordered);
+    k_morton<<<blocks_for(n, kSortTile), kThreads, 0, stream>>>(centroids, n, ordered, bounds, keys[0], values[0],
+                                                                counts);
+    return radix_sort(keys, values, n, kCodeBits, true, counts, stream);
 }
 
 // ---- Karras build --------------------------------------------------------
@@ -218,7 +310,9 @@ __device__ inline int lcp(const uint32_t* codes, int n, int i, int j) {
 
 // Internal node i covers a range and splits it (lbvh.cu:190-245).  Children
 // are written in the reference's numbering: a leaf is its sorted position
-// (< n), an internal node is n + index.
+// (< n), an internal node is n + index.  `left` and `right` are for exports
+// (may be null); `parent` (may be null) holds, for every child, twice its
+// parent's index, plus one for a right child, and -1 for the root.
 __global__ void k_karras(const uint32_t* __restrict__ codes, int n, int32_t* __restrict__ left,
                          int32_t* __restrict__ right, int32_t* __restrict__ parent) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -243,114 +337,84 @@ __global__ void k_karras(const uint32_t* __restrict__ codes, int n, int32_t* __r
     const int split = rl + offset;
     const int lc = rl == split ? rl : n + split;
     const int rc = split + 1 == rr ? rr : n + split + 1;
-    left[i] = lc;
-    right[i] = rc;
-    parent[lc] = n + i;
-    parent[rc] = n + i;
+    if (left) {
+        left[i] = lc;
+        right[i] = rc;
+    }
+    if (parent) {
+        parent[lc] = 2 * i;
+        parent[rc] = 2 * i + 1;
+        if (i == 0) parent[n] = -1;
+    }
 }
 
-struct Box { float lo[3], hi[3]; };
-
-// Leaf boxes from the FP32 corners, then the bottom-up merge: the fence makes
-// a child's box visible before its arrival is counted, and only the second
-// arrival at a parent carries on -- nothing ever waits.
+// The traversal layout, bottom up in one pass.  A leaf is packed (80 bytes: its
+// FP64 corners and triangle) and its box taken from the FP32 corners; then each
+// child writes its box and code into its half of its parent's node (4 float4:
+// left box lo and hi, right box lo and hi, the two children), and the second to
+// arrive goes on with the union.  The fence makes a half visible before its
+// arrival is counted, and nothing ever waits.  (Boxes in an array of their own,
+// packed by two more kernels, took 190 us at 494,000 triangles,
+// now 103.)
 __global__ void k_refit(const double* __restrict__ points, const int32_t* __restrict__ faces,
-                        const uint32_t* __restrict__ order, int n,
-                        const int32_t* __restrict__ left, const int32_t* __restrict__ right,
-                        const int32_t* __restrict__ parent, uint32_t* __restrict__ arrivals,
-                        float* __restrict__ boxes) {
+                        const uint32_t* __restrict__ order, int n, const int32_t* __restrict__ parent,
+                        uint32_t* __restrict__ arrivals, float4* __restrict__ nodes, float4* __restrict__ leaves) {
     const int leaf = blockIdx.x * blockDim.x + threadIdx.x;
     if (leaf >= n) return;
-    const int32_t* f = faces + (long)order[leaf] * 3;
-    Box b;
-    for (int k = 0; k < 3; ++k) {
-        const float x = __double2float_rn(points[(long)f[0] * 3 + k]);
-        const float y = __double2float_rn(points[(long)f[1] * 3 + k]);
-        const float z = __double2float_rn(points[(long)f[2] * 3 + k]);
-        b.lo[k] = fminf(x, fminf(y, z));
-        b.hi[k] = fmaxf(x, fmaxf(y, z));
-    }
-    for (int k = 0; k < 3; ++k) {
-        boxes[(long)leaf * 6 + k] = b.lo[k];
-        boxes[(long)leaf * 6 + 3 + k] = b.hi[k];
-    }
-    int node = leaf;
-    for (int depth = 0; depth < 2 * n + 2; ++depth) {
-        const int p = parent[node];
-        if (p < 0) return;
-        __threadfence();
-        if (atomicAdd(&arrivals[p - n], 1u) != 1u) return;
-        __threadfence();
-        const int l = left[p - n], r = right[p - n];
-        for (int k = 0; k < 3; ++k) {
-            const float a = __ldcg(&boxes[(long)l * 6 + k]);
-            const float c = __ldcg(&boxes[(long)r * 6 + k]);
-            boxes[(long)p * 6 + k] = fminf(a, c);
-            const float a2 = __ldcg(&boxes[(long)l * 6 + 3 + k]);
-            const float c2 = __ldcg(&boxes[(long)r * 6 + 3 + k]);
-            boxes[(long)p * 6 + 3 + k] = fmaxf(a2, c2);
-        }
-        node = p;
-    }
-}
-
-
-__device__ inline uint32_t encode_child(int child, int n) {
-    return child < n ? (kLeafBit | (uint32_t)child) : (uint32_t)(child - n);
-}
-
-// Traversal layout: internal node i = 4 float4 = (left box lo, left hi.x),
-// (left hi.yz, right lo.xy), (right lo.z, right hi), (children, unused).
-__global__ void k_pack_nodes(const int32_t* __restrict__ left, const int32_t* __restrict__ right,
-                             const float* __restrict__ boxes, int n, float4* __restrict__ nodes) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n - 1) return;
-    const int l = left[i], r = right[i];
-    const float* bl = boxes + (long)l * 6;
-    const float* br = boxes + (long)r * 6;
-    nodes[(long)i * 4 + 0] = make_float4(bl[0], bl[1], bl[2], bl[3]);
-    nodes[(long)i * 4 + 1] = make_float4(bl[4], bl[5], br[0], br[1]);
-    nodes[(long)i * 4 + 2] = make_float4(br[2], br[3], br[4], br[5]);
-    nodes[(long)i * 4 + 3] = make_float4(__uint_as_float(encode_child(l, n)),
-                                         __uint_as_float(encode_child(r, n)), 0.0f, 0.0f);
-}
-
-__global__ void k_pack_leaves(const double* __restrict__ points, const int32_t* __restrict__ faces,
-                              const uint32_t* __restrict__ order, int n,
-                              float4* __restrict__ leaves) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    const int tri = (int)order[i];
+    const int tri = (int)order[leaf];
     const int32_t* f = faces + (long)tri * 3;
     double c[9];
     for (int k = 0; k < 3; ++k)
         for (int a = 0; a < 3; ++a) c[k * 3 + a] = points[(long)f[k] * 3 + a];
-    double2* l = reinterpret_cast<double2*>(leaves) + (long)i * kLeafFloat4s;
+    double2* l = reinterpret_cast<double2*>(leaves) + (long)leaf * kLeafFloat4s;
     l[0] = make_double2(c[0], c[1]);
     l[1] = make_double2(c[2], c[3]);
     l[2] = make_double2(c[4], c[5]);
     l[3] = make_double2(c[6], c[7]);
     l[4] = make_double2(c[8], __longlong_as_double((long long)tri));
+    if (n == 1) return;
+    float lo[3], hi[3];
+    for (int k = 0; k < 3; ++k) {
+        const float x = __double2float_rn(c[k]), y = __double2float_rn(c[3 + k]), z = __double2float_rn(c[6 + k]);
+        lo[k] = fminf(x, fminf(y, z));
+        hi[k] = fmaxf(x, fmaxf(y, z));
+    }
+    uint32_t code = kLeafBit | (uint32_t)leaf;
+    int up = parent[leaf];
+    for (int depth = 0; depth < 2 * n + 2 && up >= 0; ++depth) {
+        const int p = up >> 1, side = up & 1;
+        float* node = reinterpret_cast<float*>(nodes + (long)p * 4);
+        float2* mine = reinterpret_cast<float2*>(node + side * 6);
+        mine[0] = make_float2(lo[0], lo[1]);
+        mine[1] = make_float2(lo[2], hi[0]);
+        mine[2] = make_float2(hi[1], hi[2]);
+        node[12 + side] = __uint_as_float(code);
+        __threadfence();
+        if (atomicAdd(&arrivals[p], 1u) != 1u) return;
+        __threadfence();
+        const float2* other = reinterpret_cast<const float2*>(node + (1 - side) * 6);
+        const float2 o0 = __ldcg(other), o1 = __ldcg(other + 1), o2 = __ldcg(other + 2);
+        lo[0] = fminf(lo[0], o0.x); lo[1] = fminf(lo[1], o0.y); lo[2] = fminf(lo[2], o1.x);
+        hi[0] = fmaxf(hi[0], o1.y); hi[1] = fmaxf(hi[1], o2.x); hi[2] = fmaxf(hi[2], o2.y);
+        code = (uint32_t)p;
+        up = parent[n + p];
+    }
 }
-
-int blocks_for(long n, int threads = kThreads) { return (int)((n + threads - 1) / threads); }
 
 }  // namespace
 
 size_t lbvh_scratch_bytes(int n) {
     // the carve sequence of lbvh_build, each piece rounded up to 256 bytes
-    const size_t tiles = (size_t)((n + kSortTile - 1) / kSortTile);
     const size_t pieces[] = {
         sizeof(float) * 3 * (size_t)n,                 // centroids
-        sizeof(float) * 6 * 1024,                      // bound partials
+        64,                                            // bounds, ordered
         64,                                            // bounds
         sizeof(uint32_t) * (size_t)n, sizeof(uint32_t) * (size_t)n,  // keys x2
         sizeof(uint32_t) * (size_t)n, sizeof(uint32_t) * (size_t)n,  // values x2
-        sizeof(uint32_t) * kRadix * (tiles + 1),       // digit counts
-        sizeof(int32_t) * (size_t)n, sizeof(int32_t) * (size_t)n,    // left, right
+        radix_count_bytes(n),                          // digit counts
+        sizeof(int32_t) * (size_t)n, sizeof(int32_t) * (size_t)n,    // left, right (export)
         sizeof(int32_t) * 2 * (size_t)n,               // parent
         sizeof(uint32_t) * (size_t)n,                  // arrivals
-        sizeof(float) * 6 * 2 * (size_t)n,             // boxes
     };
     size_t total = 0;
     for (size_t bytes : pieces) total += (bytes + 255) & ~size_t(255);
@@ -370,44 +434,27 @@ uint32_t lbvh_build(const double* points, const int32_t* faces, int n, void* scr
         return p;
     };
     float* centroids = reinterpret_cast<float*>(carve(sizeof(float) * 3 * n));
-    float* bound_partial = reinterpret_cast<float*>(carve(sizeof(float) * 6 * 1024));
+    uint32_t* ordered = reinterpret_cast<uint32_t*>(carve(64));
     float* bounds = reinterpret_cast<float*>(carve(64));
     uint32_t* keys[2] = {reinterpret_cast<uint32_t*>(carve(sizeof(uint32_t) * n)),
                          reinterpret_cast<uint32_t*>(carve(sizeof(uint32_t) * n))};
     uint32_t* values[2] = {reinterpret_cast<uint32_t*>(carve(sizeof(uint32_t) * n)),
                            reinterpret_cast<uint32_t*>(carve(sizeof(uint32_t) * n))};
-    const int tiles = (n + kSortTile - 1) / kSortTile;
-    uint32_t* counts = reinterpret_cast<uint32_t*>(carve(sizeof(uint32_t) * kRadix * (tiles + 1)));
+    uint32_t* counts = reinterpret_cast<uint32_t*>(carve(radix_count_bytes(n)));
     int32_t* left = reinterpret_cast<int32_t*>(carve(sizeof(int32_t) * n));
     int32_t* right = reinterpret_cast<int32_t*>(carve(sizeof(int32_t) * n));
     int32_t* parent = reinterpret_cast<int32_t*>(carve(sizeof(int32_t) * 2 * n));
     uint32_t* arrivals = reinterpret_cast<uint32_t*>(carve(sizeof(uint32_t) * n));
-    float* boxes = reinterpret_cast<float*>(carve(sizeof(float) * 6 * 2 * n));
 
-    k_centroids<<<blocks_for(n), kThreads, 0, stream>>>(points, faces, n, centroids);
-    const int bound_blocks = blocks_for(n) < 1024 ? blocks_for(n) : 1024;
-    k_bounds_partial<<<bound_blocks, kThreads, 0, stream>>>(centroids, n, bound_partial);
-    k_bounds_final<<<1, 32, 0, stream>>>(bound_partial, bound_blocks, bounds);
-    k_morton<<<blocks_for(n), kThreads, 0, stream>>>(centroids, n, bounds, keys[0], values[0]);
-    int cur = 0;
-    for (int shift = 0; shift < 32; shift += kRadixBits) {
-        k_radix_histogram<<<tiles, kThreads, 0, stream>>>(keys[cur], n, shift, counts, tiles);
-        k_radix_scan<<<1, 1024, 0, stream>>>(counts, kRadix * tiles);
-        k_radix_scatter<<<tiles, kThreads, 0, stream>>>(keys[cur], values[cur], n, shift, counts,
-                                                        tiles, keys[1 - cur], values[1 - cur]);
-        cur = 1 - cur;
-    }
+    const int cur = sorted_codes(points, faces, n, centroids, ordered, bounds, keys, values, counts, stream);
     const uint32_t* codes = keys[cur];
     const uint32_t* order = values[cur];
-    cudaMemsetAsync(parent, 0xff, sizeof(int32_t) * 2 * n, stream);
-    cudaMemsetAsync(arrivals, 0, sizeof(uint32_t) * n, stream);
     if (n > 1) {
-        k_karras<<<blocks_for(n - 1), kThreads, 0, stream>>>(codes, n, left, right, parent);
+        cudaMemsetAsync(arrivals, 0, sizeof(uint32_t) * n, stream);
+        k_karras<<<blocks_for(n - 1), kThreads, 0, stream>>>(codes, n, out ? left : nullptr, out ? right : nullptr,
+                                                             parent);
     }
-    k_refit<<<blocks_for(n), kThreads, 0, stream>>>(points, faces, order, n, left, right, parent,
-                                                    arrivals, boxes);
-    if (n > 1) k_pack_nodes<<<blocks_for(n - 1), kThreads, 0, stream>>>(left, right, boxes, n, nodes);
-    k_pack_leaves<<<blocks_for(n), kThreads, 0, stream>>>(points, faces, order, n, leaves);
+    k_refit<<<blocks_for(n), kThreads, 0, stream>>>(points, faces, order, n, parent, arrivals, nodes, leaves);
     if (out) {
         cudaMemcpyAsync(out->codes, codes, sizeof(uint32_t) * n, cudaMemcpyDeviceToHost, stream);
         cudaMemcpyAsync(out->order, order, sizeof(uint32_t) * n, cudaMemcpyDeviceToHost, stream);
@@ -419,6 +466,8 @@ uint32_t lbvh_build(const double* points, const int32_t* faces, int n, void* scr
     }
     return n > 1 ? 0u : (kLeafBit | 0u);
 }
+
+int lbvh_build_launches(int n) { return 2 + radix_sort_launches(n, kCodeBits, true) + (n > 1 ? 2 : 1); }
 
 // ---------------------------------------------------------------------------
 // Target ingestion: normalisation and vertex normals on the device
@@ -491,30 +540,29 @@ __global__ void k_target_normals(const double* __restrict__ p, int n, const int3
     }
 }
 
-// Radix passes that cover vertex indices below n, rounded up to an even
-// count so that the sorted arrays end in the first buffer.
-int corner_sort_passes(int n) {
+// Key bits that cover vertex indices below n.
+int corner_key_bits(int n) {
     int bits = 1;
     while (bits < 32 && (1u << bits) < (uint32_t)n) ++bits;
-    const int passes = (bits + kRadixBits - 1) / kRadixBits;
-    return passes + (passes & 1);
+    return bits;
 }
 
 }  // namespace
 
 size_t ingest_scratch_bytes(int n, int F) {
     const size_t corners = (size_t)F * 3;
-    const size_t tiles = (corners + kSortTile - 1) / kSortTile;
     const size_t pieces[] = {sizeof(uint32_t) * corners, sizeof(uint32_t) * corners,
                              sizeof(uint32_t) * corners, sizeof(uint32_t) * corners,
-                             sizeof(uint32_t) * kRadix * (tiles + 1)};
+                             radix_count_bytes((long)corners)};
     size_t total = 0;
     for (size_t bytes : pieces) total += (bytes + 255) & ~size_t(255);
     (void)n;
     return total + 256;
 }
 
-int ingest_launches(int n, int F) { return 2 + 3 * corner_sort_passes(n) + (F > 0 ? 1 : 0); }
+int ingest_launches(int n, int F) {
+    return 2 + (F > 0 ? 1 + radix_sort_launches((long)F * 3, corner_key_bits(n), false) : 0);
+}
 
 void ingest_target(double* points, int n, const int32_t* faces, int F, const double center[3], double scale,
                    double* normals, void* scratch, cudaStream_t stream) {
@@ -531,22 +579,13 @@ void ingest_target(double* points, int n, const int32_t* faces, int F, const dou
                          reinterpret_cast<uint32_t*>(carve(sizeof(uint32_t) * corners))};
     uint32_t* values[2] = {reinterpret_cast<uint32_t*>(carve(sizeof(uint32_t) * corners)),
                            reinterpret_cast<uint32_t*>(carve(sizeof(uint32_t) * corners))};
-    const int tiles = (int)((corners + kSortTile - 1) / kSortTile);
-    uint32_t* counts = reinterpret_cast<uint32_t*>(carve(sizeof(uint32_t) * kRadix * (tiles + 1)));
+    uint32_t* counts = reinterpret_cast<uint32_t*>(carve(radix_count_bytes(corners)));
+    int cur = 0;
     if (F > 0) {
         k_corner_keys<<<blocks_for(corners), kThreads, 0, stream>>>(faces, corners, keys[0], values[0]);
-        int cur = 0;
-        const int passes = corner_sort_passes(n);
-        for (int pass = 0; pass < passes; ++pass) {
-            const int shift = pass * kRadixBits;
-            k_radix_histogram<<<tiles, kThreads, 0, stream>>>(keys[cur], (int)corners, shift, counts, tiles);
-            k_radix_scan<<<1, 1024, 0, stream>>>(counts, kRadix * tiles);
-            k_radix_scatter<<<tiles, kThreads, 0, stream>>>(keys[cur], values[cur], (int)corners, shift,
-                                                            counts, tiles, keys[1 - cur], values[1 - cur]);
-            cur = 1 - cur;
-        }
+        cur = radix_sort(keys, values, corners, corner_key_bits(n), false, counts, stream);
     }
-    k_target_normals<<<blocks_for(n), kThreads, 0, stream>>>(points, n, faces, keys[0], values[0], corners,
+    k_target_normals<<<blocks_for(n), kThreads, 0, stream>>>(points, n, faces, keys[cur], values[cur], corners,
                                                              normals);
 }
 
@@ -1196,14 +1235,12 @@ __global__ void k_check_faces(const int32_t* __restrict__ faces, int count, int 
 void check(cudaError_t status, const char* what);  // throws CudaError (session.cu)
 
 size_t lbvh_export_scratch_bytes(int n) {
-    const size_t tiles = (size_t)((n + kSortTile - 1) / kSortTile);
     const size_t pieces[] = {
         sizeof(float) * 3 * (size_t)n,            // centroids
-        sizeof(float) * 6 * 1024,                 // bound partials
+        64,                                       // bounds, ordered
         sizeof(uint32_t) * (size_t)n,             // second key buffer
         sizeof(uint32_t) * (size_t)n,             // second value buffer
-        sizeof(uint32_t) * kRadix * (tiles + 1),  // digit counts
-        sizeof(int32_t) * 2 * (size_t)n,          // parent links (written by the split pass)
+        radix_count_bytes(n),                     // digit counts
         256,                                      // validation flag
     };
     size_t total = 0;
@@ -1227,12 +1264,10 @@ bool lbvh_export_to_device(const double* points, int vertex_count, const int32_t
         return p;
     };
     float* centroids = reinterpret_cast<float*>(carve(sizeof(float) * 3 * n));
-    float* bound_partial = reinterpret_cast<float*>(carve(sizeof(float) * 6 * 1024));
+    uint32_t* ordered = reinterpret_cast<uint32_t*>(carve(64));
     uint32_t* keys[2] = {codes, reinterpret_cast<uint32_t*>(carve(sizeof(uint32_t) * n))};
     uint32_t* values[2] = {order, reinterpret_cast<uint32_t*>(carve(sizeof(uint32_t) * n))};
-    const int tiles = (n + kSortTile - 1) / kSortTile;
-    uint32_t* counts = reinterpret_cast<uint32_t*>(carve(sizeof(uint32_t) * kRadix * (tiles + 1)));
-    int32_t* parent = reinterpret_cast<int32_t*>(carve(sizeof(int32_t) * 2 * n));
+    uint32_t* counts = reinterpret_cast<uint32_t*>(carve(radix_count_bytes(n)));
     int* flag = reinterpret_cast<int*>(carve(256));
 
     // the array keeps the previous call's contents: clear what starts at zero
@@ -1246,23 +1281,10 @@ bool lbvh_export_to_device(const double* points, int vertex_count, const int32_t
     check(cudaStreamSynchronize(stream), "hierarchy export: face check");
     if (host_flag) return false;
 
-    k_centroids<<<blocks_for(n), kThreads, 0, stream>>>(points, faces, n, centroids);
-    const int bound_blocks = blocks_for(n) < 1024 ? blocks_for(n) : 1024;
-    k_bounds_partial<<<bound_blocks, kThreads, 0, stream>>>(centroids, n, bound_partial);
-    k_bounds_final<<<1, 32, 0, stream>>>(bound_partial, bound_blocks, bounds);
-    k_morton<<<blocks_for(n), kThreads, 0, stream>>>(centroids, n, bounds, keys[0], values[0]);
-    int cur = 0;
-    for (int shift = 0; shift < 32; shift += kRadixBits) {
-        k_radix_histogram<<<tiles, kThreads, 0, stream>>>(keys[cur], n, shift, counts, tiles);
-        k_radix_scan<<<1, 1024, 0, stream>>>(counts, kRadix * tiles);
-        k_radix_scatter<<<tiles, kThreads, 0, stream>>>(keys[cur], values[cur], n, shift, counts,
-                                                        tiles, keys[1 - cur], values[1 - cur]);
-        cur = 1 - cur;
-    }
-    // eight passes: the sorted arrays are back in the caller's buffers
-    check(cudaMemsetAsync(parent, 0xff, sizeof(int32_t) * 2 * n, stream),
-          "hierarchy export: clearing the parent links");
-    if (n > 1) k_karras<<<blocks_for(n - 1), kThreads, 0, stream>>>(keys[cur], n, left, right, parent);
+    // an even number of passes: the sorted arrays are back in the caller's buffers
+    static_assert((kCodeBits + kRadixBits - 1) / kRadixBits % 2 == 0, "the result is in the first pair");
+    sorted_codes(points, faces, n, centroids, ordered, bounds, keys, values, counts, stream);
+    if (n > 1) k_karras<<<blocks_for(n - 1), kThreads, 0, stream>>>(codes, n, left, right, nullptr);
     return true;
 }
 

@@ -594,10 +594,6 @@ size_t build_scratch_bytes(const Wrap& w) {
     return std::max(lbvh_scratch_bytes(w.F), ingest_scratch_bytes(w.Vt, w.F));
 }
 
-// Kernels one hierarchy build launches (lbvh_build): centroids, two bound
-// passes, Morton codes, 8 radix passes of 3 kernels, Karras, refit, 2 packs.
-int lbvh_build_launches(int n) { return 4 + 8 * 3 + (n > 1 ? 1 : 0) + 1 + (n > 1 ? 2 : 1); }
-
 // Kernels the target structures of a wrap launch per reset: the hierarchy.
 int target_build_launches(const Wrap& w) { return lbvh_build_launches(w.F); }
 

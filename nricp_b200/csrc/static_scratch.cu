@@ -40,7 +40,7 @@ bool lbvh_export_to_device(const double* points, int vertex_count, const int32_t
 namespace {
 
 constexpr int kStaticTriangles = 262144;
-// the export's intermediates for kStaticTriangles triangles (7.04 MiB), rounded up
+// the export's intermediates for kStaticTriangles triangles (5.1 MiB), rounded up
 constexpr size_t kStaticScratchBytes = 8u * 1024u * 1024u;
 
 static __device__ __align__(256) unsigned char g_static_scratch[kStaticScratchBytes];
