@@ -357,6 +357,23 @@ int nricp_template_graph_level(const double* points, int count, int levels,
                                int32_t* edges, int edge_capacity, int* edge_count,
                                int use_device);
 
+/* build_template_graph(...) (bindings.cpp:886-925), every level from one
+ * build: `out` holds one entry per level (nricp_plan's count), whose buffers
+ * are the caller's, sized as nricp_template_graph_level's. */
+typedef struct NricpGraphLevel {
+    int32_t* template_indices;
+    double* node_positions;
+    int32_t* bind_nodes;
+    double* bind_weights;
+    int32_t* bind_counts;
+    int32_t* edges;
+    int edge_capacity; /* in */
+    int edge_count;    /* out */
+} NricpGraphLevel;
+int nricp_template_graph(const double* points, int count, int levels, int nodes_initial, int growth,
+                         int max_nodes, int edge_neighbours, double* center, double* scale,
+                         NricpGraphLevel* out, int use_device);
+
 /* farthest_point_seeds(points, count, first_index) (bindings.cpp:796-804,
  * src/core/sampling.cpp:47-88): deterministic farthest-point sampling, ties
  * to the lower index; first_index is clamped into range.  Writes

@@ -132,6 +132,15 @@ class Inspect(C.Structure):
     ]
 
 
+class GraphLevel(C.Structure):
+    _fields_ = [
+        ("template_indices", C.POINTER(C.c_int32)), ("node_positions", C.POINTER(C.c_double)),
+        ("bind_nodes", C.POINTER(C.c_int32)), ("bind_weights", C.POINTER(C.c_double)),
+        ("bind_counts", C.POINTER(C.c_int32)), ("edges", C.POINTER(C.c_int32)),
+        ("edge_capacity", C.c_int), ("edge_count", C.c_int),
+    ]
+
+
 class ServerConfig(C.Structure):
     _fields_ = [
         ("memory_budget_bytes", C.c_size_t), ("max_slots", C.c_int), ("prep_threads", C.c_int),

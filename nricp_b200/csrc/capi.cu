@@ -19,6 +19,7 @@
 #include "host.hpp"
 #include "kernels.cuh"
 #include "graph_build.hpp"
+#include "resources.hpp"
 #include "session.hpp"
 
 using namespace nricp_b200;
@@ -346,6 +347,42 @@ int nricp_batch_solve(const NricpSolveDesc* descs, int count, NricpResult* resul
 
 // ---- components ----------------------------------------------------------------
 
+namespace {
+
+TemplateGraph template_graph(const double* points, int count, int levels, int nodes_initial, int growth, int max_nodes,
+                             int edge_neighbours, bool use_device) {
+    if (count <= 0) throw InvalidArgument("invalid mesh: mesh has no vertices");
+    if (max_nodes > NRICP_MAX_SLOTS) throw InvalidArgument("max_nodes_per_vertex exceeds 8");
+    if (use_device && device_graph_supported(edge_neighbours)) {
+        require_device();
+        const StreamLease stream = StreamLease::take();
+        return std::move(device_template_graphs(
+            {GraphRequest{points, count, levels, nodes_initial, growth, max_nodes, edge_neighbours}}, stream)[0]);
+    }
+    return build_template_graph(points, count, levels, nodes_initial, growth, max_nodes, edge_neighbours);
+}
+
+void copy_level(const GraphLevel& L, int count, int32_t* template_indices, double* node_positions,
+                int32_t* bind_nodes, double* bind_weights, int32_t* bind_counts, int32_t* edges, int edge_capacity,
+                int* edge_count) {
+    const int N = L.node_count();
+    std::memcpy(template_indices, L.template_index.data(), sizeof(int32_t) * N);
+    std::memcpy(node_positions, L.rest.data(), sizeof(double) * 3 * N);
+    for (int v = 0; v < count; ++v) {
+        for (int s = 0; s < NRICP_MAX_SLOTS; ++s) {
+            bind_nodes[v * NRICP_MAX_SLOTS + s] = L.bindings[v].nodes[s];
+            bind_weights[v * NRICP_MAX_SLOTS + s] = L.bindings[v].weights[s];
+        }
+        bind_counts[v] = L.bindings[v].count;
+    }
+    const int E = static_cast<int>(L.edges.size() / 2);
+    *edge_count = E;
+    if (E > edge_capacity) throw InvalidArgument("edge buffer too small");
+    std::memcpy(edges, L.edges.data(), sizeof(int32_t) * 2 * E);
+}
+
+}  // namespace
+
 int nricp_template_graph_level(const double* points, int count, int levels, int nodes_initial,
                                int growth, int max_nodes, int edge_neighbours, int level,
                                double* center, double* scale, int32_t* template_indices,
@@ -353,45 +390,29 @@ int nricp_template_graph_level(const double* points, int count, int levels, int 
                                int32_t* bind_counts, int32_t* edges, int edge_capacity,
                                int* edge_count, int use_device) {
     return guarded([&] {
-        if (count <= 0) throw InvalidArgument("invalid mesh: mesh has no vertices");
-        if (max_nodes > NRICP_MAX_SLOTS) throw InvalidArgument("max_nodes_per_vertex exceeds 8");
-        TemplateGraph g;
-        if (use_device && device_graph_supported(edge_neighbours)) {
-            require_device();
-            cudaStream_t stream;
-            check(cudaStreamCreateWithFlags(&stream, cudaStreamNonBlocking), "stream");
-            try {
-                g = std::move(device_template_graphs(
-                    {GraphRequest{points, count, levels, nodes_initial, growth, max_nodes, edge_neighbours}},
-                    stream)[0]);
-            } catch (...) {
-                cudaStreamDestroy(stream);
-                throw;
-            }
-            cudaStreamDestroy(stream);
-        } else {
-            g = build_template_graph(points, count, levels, nodes_initial, growth, max_nodes,
-                                     edge_neighbours);
-        }
+        const TemplateGraph g =
+            template_graph(points, count, levels, nodes_initial, growth, max_nodes, edge_neighbours, use_device != 0);
         if (level < 0 || level >= static_cast<int>(g.levels.size()))
             throw InvalidArgument("level out of range");
-        const GraphLevel& L = g.levels[level];
         for (int k = 0; k < 3; ++k) center[k] = g.center[k];
         *scale = g.scale;
-        const int N = L.node_count();
-        std::memcpy(template_indices, L.template_index.data(), sizeof(int32_t) * N);
-        std::memcpy(node_positions, L.rest.data(), sizeof(double) * 3 * N);
-        for (int v = 0; v < count; ++v) {
-            for (int s = 0; s < NRICP_MAX_SLOTS; ++s) {
-                bind_nodes[v * NRICP_MAX_SLOTS + s] = L.bindings[v].nodes[s];
-                bind_weights[v * NRICP_MAX_SLOTS + s] = L.bindings[v].weights[s];
-            }
-            bind_counts[v] = L.bindings[v].count;
+        copy_level(g.levels[level], count, template_indices, node_positions, bind_nodes, bind_weights, bind_counts,
+                   edges, edge_capacity, edge_count);
+    });
+}
+
+int nricp_template_graph(const double* points, int count, int levels, int nodes_initial, int growth, int max_nodes,
+                         int edge_neighbours, double* center, double* scale, NricpGraphLevel* out, int use_device) {
+    return guarded([&] {
+        const TemplateGraph g =
+            template_graph(points, count, levels, nodes_initial, growth, max_nodes, edge_neighbours, use_device != 0);
+        for (int k = 0; k < 3; ++k) center[k] = g.center[k];
+        *scale = g.scale;
+        for (size_t l = 0; l < g.levels.size(); ++l) {
+            NricpGraphLevel& o = out[l];
+            copy_level(g.levels[l], count, o.template_indices, o.node_positions, o.bind_nodes, o.bind_weights,
+                       o.bind_counts, o.edges, o.edge_capacity, &o.edge_count);
         }
-        const int E = static_cast<int>(L.edges.size() / 2);
-        *edge_count = E;
-        if (E > edge_capacity) throw InvalidArgument("edge buffer too small");
-        std::memcpy(edges, L.edges.data(), sizeof(int32_t) * 2 * E);
     });
 }
 
@@ -442,18 +463,12 @@ int nricp_fit_rigid(const double* source_points, const double* target_points, co
         require_device();
         const size_t n = static_cast<size_t>(count);
         const size_t bytes = sizeof(double) * (7 * std::max<size_t>(1, n) + 12);
-        char* base = nullptr;
-        check(cudaMalloc(&base, bytes), "cudaMalloc(rigid fit)");
-        std::unique_ptr<char, void (*)(char*)> guard(base, [](char* p) { cudaFree(p); });
-        double* src = reinterpret_cast<double*>(base);
+        const StreamLease stream = StreamLease::take();
+        const PoolBuffer memory(bytes, stream, "cudaMallocFromPoolAsync(rigid fit)");
+        double* src = reinterpret_cast<double*>(memory.data());
         double* dst = src + 3 * std::max<size_t>(1, n);
         double* w = dst + 3 * std::max<size_t>(1, n);
         double* out = w + std::max<size_t>(1, n);
-        cudaStream_t stream;
-        check(cudaStreamCreateWithFlags(&stream, cudaStreamNonBlocking), "stream");
-        std::unique_ptr<CUstream_st, void (*)(cudaStream_t)> stream_guard(stream, [](cudaStream_t s) {
-            cudaStreamDestroy(s);
-        });
         if (n > 0) {
             check(cudaMemcpyAsync(src, source_points, sizeof(double) * 3 * n, cudaMemcpyHostToDevice, stream), "upload");
             check(cudaMemcpyAsync(dst, target_points, sizeof(double) * 3 * n, cudaMemcpyHostToDevice, stream), "upload");
@@ -476,14 +491,13 @@ int nricp_closest_points(const double* target_points, int vertex_count, const in
     return guarded([&] {
         validate_mesh(target_points, vertex_count, faces, face_count, "target");
         require_device();
-        cudaStream_t stream;
-        check(cudaStreamCreateWithFlags(&stream, cudaStreamNonBlocking), "stream");
-        const std::vector<double> pts(target_points, target_points + (size_t)vertex_count * 3);
-        const std::vector<double> normals = vertex_normals(pts, faces, face_count);
+        const StreamLease stream = StreamLease::take();
+        const double* pts = target_points;
+        const size_t point_bytes = sizeof(double) * 3 * vertex_count;
         size_t bytes = 0;
         auto reserve = [&bytes](size_t n) { size_t at = bytes; bytes += (n + 255) & ~size_t(255); return at; };
-        const size_t o_p = reserve(sizeof(double) * pts.size());
-        const size_t o_n = reserve(sizeof(double) * normals.size());
+        const size_t o_p = reserve(point_bytes);
+        const size_t o_n = reserve(point_bytes);
         const size_t o_f = reserve(sizeof(int32_t) * 3 * face_count);
         const size_t o_nodes = reserve(sizeof(float4) * 4 * std::max(1, face_count - 1));
         const size_t o_leaves = reserve(sizeof(float4) * kLeafFloat4s * face_count);
@@ -494,10 +508,10 @@ int nricp_closest_points(const double* target_points, int vertex_count, const in
         const size_t o_ot = reserve(sizeof(int32_t) * std::max(1, query_count));
         const size_t o_flag = reserve(sizeof(int));
         const size_t o_wrap = reserve(sizeof(WrapDev));
-        const size_t o_scratch = reserve(lbvh_scratch_bytes(face_count));
-        char* base = nullptr;
-        check(cudaMalloc(&base, bytes), "cudaMalloc(closest points)");
-        std::unique_ptr<char, void (*)(char*)> guard(base, [](char* p) { cudaFree(p); });
+        const size_t o_scratch =
+            reserve(std::max(lbvh_scratch_bytes(face_count), ingest_scratch_bytes(vertex_count, face_count)));
+        const PoolBuffer memory(bytes, stream, "cudaMallocFromPoolAsync(closest points)");
+        char* const base = memory.data();
         WrapDev w;
         std::memset(&w, 0, sizeof w);
         w.Vt = vertex_count;
@@ -519,12 +533,15 @@ int nricp_closest_points(const double* target_points, int vertex_count, const in
                                        (hi[2] - lo[2]) * (hi[2] - lo[2]));
             w.rank_window = static_cast<float>(4e-6 * d);
         }
-        check(cudaMemcpyAsync(base + o_p, pts.data(), sizeof(double) * pts.size(), cudaMemcpyHostToDevice, stream), "upload");
-        check(cudaMemcpyAsync(base + o_n, normals.data(), sizeof(double) * normals.size(), cudaMemcpyHostToDevice, stream), "upload");
+        check(cudaMemcpyAsync(base + o_p, pts, point_bytes, cudaMemcpyHostToDevice, stream), "upload");
         check(cudaMemcpyAsync(base + o_f, faces, sizeof(int32_t) * 3 * face_count, cudaMemcpyHostToDevice, stream), "upload");
         if (query_count > 0)
             check(cudaMemcpyAsync(base + o_q, queries, sizeof(double) * 3 * query_count, cudaMemcpyHostToDevice, stream), "upload");
         check(cudaMemsetAsync(base + o_flag, 0, sizeof(int), stream), "flag");
+        // the vertex normals, to the host's bits (the frame is the caller's own)
+        const double origin[3] = {0.0, 0.0, 0.0};
+        ingest_target(const_cast<double*>(w.tgt_points), vertex_count, w.tgt_faces, face_count, origin, 1.0,
+                      const_cast<double*>(w.tgt_normals), base + o_scratch, stream);
         w.bvh_root = static_cast<int>(lbvh_build(w.tgt_points, w.tgt_faces, face_count, base + o_scratch,
                                                  const_cast<float4*>(w.bvh_nodes),
                                                  const_cast<float4*>(w.bvh_leaves), stream, nullptr));
@@ -546,7 +563,6 @@ int nricp_closest_points(const double* target_points, int vertex_count, const in
         int flag = 0;
         check(cudaMemcpyAsync(&flag, base + o_flag, sizeof(int), cudaMemcpyDeviceToHost, stream), "download");
         check(cudaStreamSynchronize(stream), "closest points");
-        cudaStreamDestroy(stream);
         if (flag) throw StateError("a closest-point traversal exceeded its stack");
     });
 }
@@ -557,9 +573,7 @@ int nricp_lbvh_export(const double* target_points, int vertex_count, const int32
     return guarded([&] {
         validate_mesh(target_points, vertex_count, faces, face_count, "target");
         require_device();
-        cudaStream_t stream;
-        check(cudaStreamCreateWithFlags(&stream, cudaStreamNonBlocking), "stream");
-        char* base = nullptr;
+        const StreamLease stream = StreamLease::take();
         size_t bytes = 0;
         auto reserve = [&bytes](size_t n) { size_t at = bytes; bytes += (n + 255) & ~size_t(255); return at; };
         const size_t o_p = reserve(sizeof(double) * 3 * vertex_count);
@@ -567,8 +581,8 @@ int nricp_lbvh_export(const double* target_points, int vertex_count, const int32
         const size_t o_nodes = reserve(sizeof(float4) * 4 * std::max(1, face_count - 1));
         const size_t o_leaves = reserve(sizeof(float4) * kLeafFloat4s * face_count);
         const size_t o_scratch = reserve(lbvh_scratch_bytes(face_count));
-        check(cudaMalloc(&base, bytes), "cudaMalloc(lbvh)");
-        std::unique_ptr<char, void (*)(char*)> guard(base, [](char* p) { cudaFree(p); });
+        const PoolBuffer memory(bytes, stream, "cudaMallocFromPoolAsync(lbvh)");
+        char* const base = memory.data();
         check(cudaMemcpyAsync(base + o_p, target_points, sizeof(double) * 3 * vertex_count, cudaMemcpyHostToDevice, stream), "upload");
         check(cudaMemcpyAsync(base + o_f, faces, sizeof(int32_t) * 3 * face_count, cudaMemcpyHostToDevice, stream), "upload");
         LbvhExport out{codes, order, left, right, bounds};
@@ -577,7 +591,6 @@ int nricp_lbvh_export(const double* target_points, int vertex_count, const int32
                    reinterpret_cast<float4*>(base + o_leaves), stream, &out);
         check(cudaGetLastError(), "lbvh build");
         check(cudaStreamSynchronize(stream), "lbvh build");
-        cudaStreamDestroy(stream);
     });
 }
 

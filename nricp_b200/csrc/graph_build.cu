@@ -10,12 +10,14 @@
 #include <algorithm>
 #include <climits>
 #include <cmath>
+#include <cstring>
 #include <vector>
 
 #include <cooperative_groups.h>
 
 #include "async.cuh"
 #include "graph_build.hpp"
+#include "resources.hpp"
 #include "session.hpp"
 #include "staging.hpp"
 
@@ -459,15 +461,21 @@ __global__ void __launch_bounds__(kBindThreads) k_neighbours(const double* __res
 
 int blocks(long n, int threads) { return static_cast<int>((n + threads - 1) / threads); }
 
-template <typename T>
-T* to_device(const std::vector<T>& v, std::vector<void*>& owned, cudaStream_t stream) {
-    T* d = nullptr;
-    check(cudaMalloc(&d, sizeof(T) * std::max<size_t>(1, v.size())), "cudaMalloc(graph build)");
-    owned.push_back(d);
-    if (!v.empty())
-        check(cudaMemcpyAsync(d, v.data(), sizeof(T) * v.size(), cudaMemcpyHostToDevice, stream), "upload");
-    return d;
-}
+// Small host arrays that go up in one copy: each at a 256-byte offset.
+class Packed {
+public:
+    template <typename T>
+    size_t add(const std::vector<T>& v) {
+        const size_t at = bytes_.size();
+        bytes_.resize((at + sizeof(T) * std::max<size_t>(1, v.size()) + 255) & ~size_t(255));
+        if (!v.empty()) std::memcpy(bytes_.data() + at, v.data(), sizeof(T) * v.size());
+        return at;
+    }
+    const std::vector<char>& bytes() const { return bytes_; }
+
+private:
+    std::vector<char> bytes_;
+};
 
 }  // namespace
 
@@ -479,7 +487,6 @@ std::vector<TemplateGraph> device_template_graphs(const std::vector<GraphRequest
     std::vector<TemplateGraph> out(W);
     if (W == 0) return out;
     // host: normalisation (mesh.cpp:174-187) and the sizes of every level
-    std::vector<double> points;
     std::vector<long> point_offset(W), seed_offset(W);
     std::vector<int> point_count(W), seed_count(W);
     std::vector<std::vector<int>> level_sizes(W);
@@ -503,32 +510,6 @@ std::vector<TemplateGraph> device_template_graphs(const std::vector<GraphRequest
         max_levels = std::max(max_levels, levels);
         max_points = std::max(max_points, r.count);
     }
-    // every template normalised on its own host thread, into its place
-    points.resize(static_cast<size_t>(total_points) * 3);
-#pragma omp parallel for schedule(dynamic, 1) if (W > 1)
-    for (int t = 0; t < W; ++t) {
-        const GraphRequest& r = requests[t];
-        TemplateGraph& g = out[t];
-        compute_normalization(r.points, r.count, g.center, &g.scale);
-        const std::vector<double> norm = normalized(r.points, r.count, g.center, g.scale);
-        std::copy(norm.begin(), norm.end(), points.begin() + point_offset[t] * 3);
-    }
-    std::vector<void*> owned;
-    double* d_points = to_device(points, owned, stream);
-    long* d_point_offset = to_device(point_offset, owned, stream);
-    int* d_point_count = to_device(point_count, owned, stream);
-    int* d_seed_count = to_device(seed_count, owned, stream);
-    long* d_seed_offset = to_device(seed_offset, owned, stream);
-    double* d_nearest = nullptr;
-    int* d_seeds = nullptr;
-    check(cudaMalloc(&d_nearest, sizeof(double) * std::max<long>(1, total_points)), "cudaMalloc(graph build)");
-    owned.push_back(d_nearest);
-    check(cudaMalloc(&d_seeds, sizeof(int) * std::max<long>(1, total_seeds)), "cudaMalloc(graph build)");
-    owned.push_back(d_seeds);
-    int* d_failed = nullptr;
-    check(cudaMalloc(&d_failed, sizeof(int)), "cudaMalloc(graph build)");
-    owned.push_back(d_failed);
-    int failed = 0;
     // every level's sizes, on the host
     struct LevelPlan {
         std::vector<int> nodes, support, taken;
@@ -559,53 +540,108 @@ std::vector<TemplateGraph> device_template_graphs(const std::vector<GraphRequest
         all_edges = edge_base[l + 1];
     }
 
-    // the downloads land in page-locked memory: seeds, then per level the
-    // bindings' nodes and weights, then every level's neighbour lists
+    // Every template normalised on its own host thread, into page-locked
+    // memory, where the downloads land too: the points and the small arrays,
+    // the seeds, then per level the bindings' nodes and weights, then every
+    // level's neighbour lists.
     const long bind_entries = std::max<long>(1, total_points * NRICP_MAX_SLOTS);
-    const size_t seed_bytes = (sizeof(int) * std::max<long>(1, total_seeds) + 255) & ~size_t(255);
+    auto rounded = [](size_t bytes) { return (bytes + 255) & ~size_t(255); };
+    const size_t point_bytes = rounded(sizeof(double) * 3 * std::max<long>(1, total_points));
+    const size_t seed_bytes = rounded(sizeof(int) * std::max<long>(1, total_seeds));
     const size_t level_bytes = (sizeof(int32_t) + sizeof(double)) * bind_entries;
-    StagingLease lease(seed_bytes + level_bytes * max_levels + sizeof(int) * all_edges);
-    int* seeds = reinterpret_cast<int*>(lease.data());
-    auto host_nodes = [&](int l) {
-        return reinterpret_cast<int32_t*>(lease.data() + seed_bytes + level_bytes * l);
-    };
+    StagingLease lease(point_bytes + seed_bytes + level_bytes * max_levels + sizeof(int) * all_edges);
+    double* points = reinterpret_cast<double*>(lease.data());
+    char* const down = lease.data() + point_bytes;
+    int* seeds = reinterpret_cast<int*>(down);
+    auto host_nodes = [&](int l) { return reinterpret_cast<int32_t*>(down + seed_bytes + level_bytes * l); };
     auto host_weights = [&](int l) {
-        return reinterpret_cast<double*>(lease.data() + seed_bytes + level_bytes * l + sizeof(int32_t) * bind_entries);
+        return reinterpret_cast<double*>(down + seed_bytes + level_bytes * l + sizeof(int32_t) * bind_entries);
     };
-    int* host_neigh = reinterpret_cast<int*>(lease.data() + seed_bytes + level_bytes * max_levels);
+    int* host_neigh = reinterpret_cast<int*>(down + seed_bytes + level_bytes * max_levels);
+#pragma omp parallel for schedule(dynamic, 1) if (W > 1)
+    for (int t = 0; t < W; ++t) {
+        const GraphRequest& r = requests[t];
+        TemplateGraph& g = out[t];
+        compute_normalization(r.points, r.count, g.center, &g.scale);
+        normalized_into(r.points, r.count, g.center, g.scale, points + point_offset[t] * 3);
+    }
 
     // seeds: a cluster of 1-16 CTAs per template, at most two points per
     // thread while every template's CTAs fit on the device at once, else four
     // (a CTA takes its SM); past 16 CTAs up to eight; one block beyond 131,072
     // points.  One launch per cluster size and points per thread; the launches
     // touch different templates, so each runs on a stream of its own.
-    {
-        int device = 0, sms = 148;
-        check(cudaGetDevice(&device), "device");
-        check(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device), "device");
-        auto cluster_log2 = [](int n, int per) {
-            int g = 0;
-            while (g < 4 && (1 << g) * kFpsThreads * per < n) ++g;
-            return g;
-        };
-        long ctas = 0;
-        for (int t = 0; t < W; ++t) ctas += 1 << cluster_log2(point_count[t], 2);
-        const int target = ctas <= sms ? 2 : 4;
-        constexpr int kClasses = 5 * 4;  // cluster 1 .. 16 by 1, 2, 4, 8 points per thread
-        std::vector<std::vector<int>> by_class(kClasses);
-        std::vector<int> single, chunk(kClasses, 0);
-        for (int t = 0; t < W; ++t) {
-            if (point_count[t] > kFpsClusterPoints) {
-                single.push_back(t);
-                continue;
-            }
-            const int g = cluster_log2(point_count[t], target);
-            const int here = (point_count[t] + (1 << g) - 1) >> g;
-            int per = 0;
-            while ((1 << per) * kFpsThreads < here) ++per;
-            by_class[g * 4 + per].push_back(t);
-            chunk[g * 4 + per] = std::max(chunk[g * 4 + per], here);
+    int device = 0, sms = 148;
+    check(cudaGetDevice(&device), "device");
+    check(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device), "device");
+    auto cluster_log2 = [](int n, int per) {
+        int g = 0;
+        while (g < 4 && (1 << g) * kFpsThreads * per < n) ++g;
+        return g;
+    };
+    long ctas = 0;
+    for (int t = 0; t < W; ++t) ctas += 1 << cluster_log2(point_count[t], 2);
+    const int target = ctas <= sms ? 2 : 4;
+    constexpr int kClasses = 5 * 4;  // cluster 1 .. 16 by 1, 2, 4, 8 points per thread
+    std::vector<std::vector<int>> by_class(kClasses);
+    std::vector<int> single, chunk(kClasses, 0);
+    for (int t = 0; t < W; ++t) {
+        if (point_count[t] > kFpsClusterPoints) {
+            single.push_back(t);
+            continue;
         }
+        const int g = cluster_log2(point_count[t], target);
+        const int here = (point_count[t] + (1 << g) - 1) >> g;
+        int per = 0;
+        while ((1 << per) * kFpsThreads < here) ++per;
+        by_class[g * 4 + per].push_back(t);
+        chunk[g * 4 + per] = std::max(chunk[g * 4 + per], here);
+    }
+    // the small arrays and the points go up in two copies
+    Packed packed;
+    const size_t o_point_offset = packed.add(point_offset), o_point_count = packed.add(point_count);
+    const size_t o_seed_count = packed.add(seed_count), o_seed_offset = packed.add(seed_offset);
+    std::vector<long> bind_offset(W);
+    for (int t = 0; t < W; ++t) bind_offset[t] = point_offset[t] * NRICP_MAX_SLOTS;
+    const size_t o_bind_offset = packed.add(bind_offset), o_single = packed.add(single);
+    std::vector<size_t> o_class(kClasses), o_nodes(max_levels), o_support(max_levels), o_taken(max_levels),
+        o_eoff(max_levels);
+    for (int k = 0; k < kClasses; ++k) o_class[k] = packed.add(by_class[k]);
+    for (int l = 0; l < max_levels; ++l) {
+        o_nodes[l] = packed.add(plan[l].nodes);
+        o_support[l] = packed.add(plan[l].support);
+        o_taken[l] = packed.add(plan[l].taken);
+        o_eoff[l] = packed.add(plan[l].eoff);
+    }
+    size_t device_bytes = 0;
+    auto piece = [&](size_t bytes) {
+        const size_t at = device_bytes;
+        device_bytes += rounded(bytes);
+        return at;
+    };
+    const size_t o_packed = piece(packed.bytes().size()), o_points = piece(point_bytes), o_seeds = piece(seed_bytes);
+    const size_t o_failed = piece(sizeof(int));
+    const size_t o_nearest = piece(single.empty() ? 0 : sizeof(double) * total_points);
+    const size_t o_bind_nodes = piece(sizeof(int32_t) * bind_entries * max_levels);
+    const size_t o_bind_weights = piece(sizeof(double) * bind_entries * max_levels);
+    const size_t o_neigh = piece(sizeof(int) * all_edges);
+    PoolBuffer memory(device_bytes, stream, "cudaMallocFromPoolAsync(graph build)");
+    const char* meta = memory.data() + o_packed;
+    auto ints = [&](size_t at) { return reinterpret_cast<const int*>(meta + at); };
+    auto longs = [&](size_t at) { return reinterpret_cast<const long*>(meta + at); };
+    double* d_points = reinterpret_cast<double*>(memory.data() + o_points);
+    int* d_seeds = reinterpret_cast<int*>(memory.data() + o_seeds);
+    int* d_failed = reinterpret_cast<int*>(memory.data() + o_failed);
+    double* d_nearest = reinterpret_cast<double*>(memory.data() + o_nearest);
+    int32_t* d_bind_nodes = reinterpret_cast<int32_t*>(memory.data() + o_bind_nodes);
+    double* d_bind_weights = reinterpret_cast<double*>(memory.data() + o_bind_weights);
+    int* d_neigh = reinterpret_cast<int*>(memory.data() + o_neigh);
+    int failed = 0;
+    check(cudaMemcpyAsync(memory.data() + o_packed, packed.bytes().data(), packed.bytes().size(),
+                          cudaMemcpyHostToDevice, stream), "upload");
+    check(cudaMemcpyAsync(d_points, points, sizeof(double) * 3 * total_points, cudaMemcpyHostToDevice, stream),
+          "upload");
+    {
         using FpsKernel = decltype(&k_fps<1>);
         static const FpsKernel kernels[4] = {k_fps<1>, k_fps<2>, k_fps<4>, k_fps<8>};
         static const bool enabled = [] {
@@ -617,25 +653,21 @@ std::vector<TemplateGraph> device_template_graphs(const std::vector<GraphRequest
             return true;
         }();
         (void)enabled;
-        const int* d_class[kClasses] = {};
-        for (int k = 0; k < kClasses; ++k)
-            if (!by_class[k].empty()) d_class[k] = to_device(by_class[k], owned, stream);
-        const int* d_single = single.empty() ? nullptr : to_device(single, owned, stream);
         check(cudaMemsetAsync(d_failed, 0, sizeof(int), stream), "farthest-point seeds");
         cudaEvent_t fork = nullptr;
         check(cudaEventCreateWithFlags(&fork, cudaEventDisableTiming), "event");
         check(cudaEventRecord(fork, stream), "event");
+        std::vector<StreamLease> lanes;
         auto beside = [&](auto&& launch) {  // on a stream of its own, joined afterwards
-            cudaStream_t lane;
+            lanes.push_back(StreamLease::take());
+            const cudaStream_t lane = lanes.back();
             cudaEvent_t join;
-            check(cudaStreamCreateWithFlags(&lane, cudaStreamNonBlocking), "stream");
             check(cudaEventCreateWithFlags(&join, cudaEventDisableTiming), "event");
             check(cudaStreamWaitEvent(lane, fork, 0), "wait");
             launch(lane);
             check(cudaEventRecord(join, lane), "event");
             check(cudaStreamWaitEvent(stream, join, 0), "wait");
-            cudaStreamDestroy(lane);  // released once its work is done
-            cudaEventDestroy(join);
+            cudaEventDestroy(join);  // released once its work is done
         };
         for (int k = 0; k < kClasses; ++k) {
             if (by_class[k].empty()) continue;
@@ -653,17 +685,16 @@ std::vector<TemplateGraph> device_template_graphs(const std::vector<GraphRequest
                 config.attrs = attribute;
                 config.numAttrs = 1;
                 check(cudaLaunchKernelEx(&config, kernels[k % 4], (const double*)d_points,
-                                         (const long*)d_point_offset, (const int*)d_point_count,
-                                         (const int*)d_seed_count, (const long*)d_seed_offset, d_class[k], d_seeds,
-                                         d_failed),
+                                         longs(o_point_offset), ints(o_point_count), ints(o_seed_count),
+                                         longs(o_seed_offset), ints(o_class[k]), d_seeds, d_failed),
                       "farthest-point seeds");
             });
         }
         if (!single.empty())
             beside([&](cudaStream_t lane) {
                 k_fps_block<<<static_cast<int>(single.size()), kFpsThreads, 0, lane>>>(
-                    d_points, d_point_offset, d_point_count, d_seed_count, d_seed_offset, d_single, d_nearest,
-                    d_seeds);
+                    d_points, longs(o_point_offset), ints(o_point_count), ints(o_seed_count), longs(o_seed_offset),
+                    ints(o_single), d_nearest, d_seeds);
             });
         cudaEventDestroy(fork);
     }
@@ -672,34 +703,19 @@ std::vector<TemplateGraph> device_template_graphs(const std::vector<GraphRequest
                           stream), "download seeds");
 
     // per level: bindings and neighbour lists of every template in one launch each
-    int32_t* d_bind_nodes = nullptr;
-    double* d_bind_weights = nullptr;
-    int* d_neigh = nullptr;
-    check(cudaMalloc(&d_bind_nodes, sizeof(int32_t) * bind_entries * max_levels), "cudaMalloc(graph build)");
-    owned.push_back(d_bind_nodes);
-    check(cudaMalloc(&d_bind_weights, sizeof(double) * bind_entries * max_levels), "cudaMalloc(graph build)");
-    owned.push_back(d_bind_weights);
-    check(cudaMalloc(&d_neigh, sizeof(int) * all_edges), "cudaMalloc(graph build)");
-    owned.push_back(d_neigh);
-    std::vector<long> bind_offset(W);
-    for (int t = 0; t < W; ++t) bind_offset[t] = point_offset[t] * NRICP_MAX_SLOTS;
-    long* d_bind_offset = to_device(bind_offset, owned, stream);
     for (int l = 0; l < max_levels; ++l) {
         const LevelPlan& p = plan[l];
-        int* d_nodes = to_device(p.nodes, owned, stream);
-        int* d_support = to_device(p.support, owned, stream);
-        int* d_taken = to_device(p.taken, owned, stream);
-        long* d_eoff = to_device(p.eoff, owned, stream);
         int32_t* level_nodes = d_bind_nodes + bind_entries * l;
         double* level_weights = d_bind_weights + bind_entries * l;
         int* level_neigh = d_neigh + edge_base[l];
         k_bind<<<dim3(blocks(max_points, kBindThreads / kBindLanes), W), kBindThreads, 0, stream>>>(
-            d_points, d_point_offset, d_point_count, d_seeds, d_seed_offset, d_nodes, d_support,
-            d_bind_offset, level_nodes, level_weights);
+            d_points, longs(o_point_offset), ints(o_point_count), d_seeds, longs(o_seed_offset), ints(o_nodes[l]),
+            ints(o_support[l]), longs(o_bind_offset), level_nodes, level_weights);
         check(cudaGetLastError(), "bindings");
         if (p.max_nodes > 0)
             k_neighbours<<<dim3(blocks(p.max_nodes, kBindThreads / 32), W), kBindThreads, 0, stream>>>(
-                d_points, d_point_offset, d_seeds, d_seed_offset, d_nodes, d_taken, d_eoff, level_neigh);
+                d_points, longs(o_point_offset), d_seeds, longs(o_seed_offset), ints(o_nodes[l]), ints(o_taken[l]),
+                longs(o_eoff[l]), level_neigh);
         check(cudaGetLastError(), "node edges");
         check(cudaMemcpyAsync(host_nodes(l), level_nodes, sizeof(int32_t) * bind_entries, cudaMemcpyDeviceToHost,
                               stream), "download bindings");
@@ -711,7 +727,6 @@ std::vector<TemplateGraph> device_template_graphs(const std::vector<GraphRequest
     }
     check(cudaMemcpyAsync(&failed, d_failed, sizeof(int), cudaMemcpyDeviceToHost, stream), "download");
     check(cudaStreamSynchronize(stream), "graph build");
-    for (void* p : owned) cudaFree(p);
     if (failed) throw StateError("a wait inside the farthest-point seeds ran out");
 
     // host: the graphs in the host build's form, one template per thread

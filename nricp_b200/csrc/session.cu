@@ -26,6 +26,7 @@
 #include "host.hpp"
 #include "graph_build.hpp"
 #include "kernels.cuh"
+#include "resources.hpp"
 #include "session.hpp"
 #include "staging.hpp"
 
@@ -132,28 +133,6 @@ struct InputSink {
         }
     }
 };
-
-// Device memory of batches: a stream-ordered pool per device that keeps up
-// to 8 GB between batches, so that repeated batches allocate and free their
-// arenas without waiting for the device.
-cudaMemPool_t batch_pool(int device) {
-    static std::mutex mu;
-    static std::map<int, cudaMemPool_t> pools;
-    std::lock_guard<std::mutex> lk(mu);
-    auto it = pools.find(device);
-    if (it != pools.end()) return it->second;
-    cudaMemPoolProps props = {};
-    props.allocType = cudaMemAllocationTypePinned;
-    props.location.type = cudaMemLocationTypeDevice;
-    props.location.id = device;
-    cudaMemPool_t pool = nullptr;
-    check(cudaMemPoolCreate(&pool, &props), "cudaMemPoolCreate");
-    uint64_t keep = 8ull << 30;
-    check(cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep), "pool");
-    pools[device] = pool;
-    return pool;
-}
-
 
 }  // namespace
 
@@ -602,40 +581,26 @@ int target_build_launches(const Wrap& w) { return lbvh_build_launches(w.F); }
 // ---------------------------------------------------------------------------
 // Batch
 // ---------------------------------------------------------------------------
-Batch::Batch() {
-    check(cudaStreamCreateWithFlags(&stream_, cudaStreamNonBlocking), "cudaStreamCreate");
-}
+Batch::Batch() : stream_(StreamLease::take()) {}
 
 Batch::~Batch() {
     if (graph_exec_) cudaGraphExecDestroy(graph_exec_);
     if (tail_graph_) cudaGraphExecDestroy(tail_graph_);
-    if (tail_index_) cudaFree(tail_index_);
-    if (stream_) cudaStreamSynchronize(stream_);
-    if (pool_) {  // back to the pool in stream order, without a device-wide wait
-        for (auto& w : wraps_) w->arena.release_async(stream_);
-        for (int k = 0; k < kBuildStreams; ++k)
-            if (build_scratch_[k]) cudaFreeAsync(build_scratch_[k], stream_);
-    }
-    for (int k = 0; k < kBuildStreams; ++k) {
-        if (build_streams_[k]) cudaStreamDestroy(build_streams_[k]);
+    cudaStreamSynchronize(stream_);
+    // back to the pool in stream order, without a device-wide wait
+    for (auto& w : wraps_) w->arena.release_async(stream_);
+    for (int k = 0; k < kBuildStreams; ++k)
+        if (build_scratch_[k]) cudaFreeAsync(build_scratch_[k], stream_);
+    if (device_block_) cudaFreeAsync(device_block_, stream_);
+    for (int k = 0; k < kBuildStreams; ++k)
         if (build_done_[k]) cudaEventDestroy(build_done_[k]);
-    }
     if (build_fork_) cudaEventDestroy(build_fork_);
     wraps_.clear();
-    if (query_counter_) cudaFree(query_counter_);
-    if (side_stream_) cudaStreamDestroy(side_stream_);
     if (side_fork_) cudaEventDestroy(side_fork_);
     if (side_join_) cudaEventDestroy(side_join_);
-    if (dev_wraps_) cudaFree(dev_wraps_);
-    if (dev_controls_) cudaFree(dev_controls_);
-    if (pcg_index_) cudaFree(pcg_index_);
-    for (int g = 0; g < 5; ++g) {
-        if (pcg_streams_[g]) cudaStreamDestroy(pcg_streams_[g]);
+    for (int g = 0; g < 5; ++g)
         if (pcg_join_[g]) cudaEventDestroy(pcg_join_[g]);
-    }
     if (pcg_fork_) cudaEventDestroy(pcg_fork_);
-    if (host_controls_) cudaFreeHost(host_controls_);
-    if (stream_) cudaStreamDestroy(stream_);
 }
 
 
@@ -741,14 +706,31 @@ void Batch::upload_all(LbvhExport* lbvh_out) {
     int device = 0;
     check(cudaGetDevice(&device), "device");
     pool_ = batch_pool(device);
-    check(cudaMalloc(&dev_controls_, sizeof(WrapControl) * W), "cudaMalloc(controls)");
-    check(cudaMallocHost(&host_controls_, sizeof(WrapControl) * W), "cudaMallocHost(controls)");
+    // descriptors, controls, the query queues' heads and the solve classes'
+    // lists, one block
+    size_t block_bytes = 0;
+    auto piece = [&block_bytes](size_t bytes) {
+        const size_t at = block_bytes;
+        block_bytes += (bytes + 255) & ~size_t(255);
+        return at;
+    };
+    const size_t o_wraps = piece(sizeof(WrapDev) * W), o_controls = piece(sizeof(WrapControl) * W);
+    const size_t o_counter = piece(2 * sizeof(int)), o_index = piece(sizeof(int) * W), o_tail = piece(sizeof(int) * W);
+    check(cudaMallocFromPoolAsync(&device_block_, block_bytes, pool_, stream_), "cudaMallocFromPoolAsync(batch)");
+    char* block = static_cast<char*>(device_block_);
+    dev_wraps_ = reinterpret_cast<WrapDev*>(block + o_wraps);
+    dev_controls_ = reinterpret_cast<WrapControl*>(block + o_controls);
+    query_counter_ = reinterpret_cast<int*>(block + o_counter);
+    pcg_index_ = reinterpret_cast<int*>(block + o_index);
+    tail_index_ = reinterpret_cast<int*>(block + o_tail);
+    host_block_ = PinnedLease(sizeof(WrapControl) * W);
+    host_controls_ = static_cast<WrapControl*>(host_block_.data());
     size_t scratch_bytes = 0;
     for (const auto& w : wraps_) scratch_bytes = std::max(scratch_bytes, build_scratch_bytes(*w));
     for (int k = 0; k < kBuildStreams; ++k) {
         check(cudaMallocFromPoolAsync(&build_scratch_[k], scratch_bytes, pool_, stream_),
               "cudaMallocFromPoolAsync(scratch)");
-        check(cudaStreamCreateWithFlags(&build_streams_[k], cudaStreamNonBlocking), "stream");
+        build_streams_[k] = StreamLease::take();
         check(cudaEventCreateWithFlags(&build_done_[k], cudaEventDisableTiming), "event");
     }
     check(cudaEventCreateWithFlags(&build_fork_, cudaEventDisableTiming), "event");
@@ -773,10 +755,9 @@ void Batch::upload_all(LbvhExport* lbvh_out) {
         if (!failure[i].empty()) throw std::runtime_error(failure[i]);
     shape_ = TickShape{};
     shape_.wraps = W;
-    check(cudaMalloc(&query_counter_, 2 * sizeof(int)), "cudaMalloc(query queues)");
     shape_.query_counter = query_counter_;
     if (!side_stream_) {
-        check(cudaStreamCreateWithFlags(&side_stream_, cudaStreamNonBlocking), "stream");
+        side_stream_ = StreamLease::take();
         check(cudaEventCreateWithFlags(&side_fork_, cudaEventDisableTiming), "event");
         check(cudaEventCreateWithFlags(&side_join_, cudaEventDisableTiming), "event");
     }
@@ -794,7 +775,6 @@ void Batch::upload_all(LbvhExport* lbvh_out) {
         if (w.desc.route == NRICP_ROUTE_C) shape_.route_c = 1;
     }
     set_pcg_cluster(default_pcg_cluster());
-    check(cudaMalloc(&dev_wraps_, sizeof(WrapDev) * W), "cudaMalloc(wraps)");
     std::vector<WrapDev> host(W);
     for (int i = 0; i < W; ++i) host[i] = wraps_[i]->dev;
     check(cudaMemcpyAsync(dev_wraps_, host.data(), sizeof(WrapDev) * W, cudaMemcpyHostToDevice, stream_),
@@ -890,7 +870,7 @@ void Batch::set_pcg_cluster(int cluster) {
     }
 }
 
-void Batch::solve_shape(int cluster, TickShape& shape, int*& index, std::vector<int>* cls_out) {
+void Batch::solve_shape(int cluster, TickShape& shape, int* index, std::vector<int>* cls_out) {
     const int W = static_cast<int>(wraps_.size());
     std::vector<int> nodes(W);
     for (int i = 0; i < W; ++i) nodes[i] = wraps_[i]->max_nodes;
@@ -915,7 +895,6 @@ void Batch::solve_shape(int cluster, TickShape& shape, int*& index, std::vector<
         shape.pcg_cluster = sizes[0];
         return;
     }
-    if (!index) check(cudaMalloc(&index, sizeof(int) * W), "cudaMalloc(solve groups)");
     std::vector<int> order;
     for (size_t g = 0; g < sizes.size(); ++g) {
         const int first = static_cast<int>(order.size());
@@ -927,7 +906,7 @@ void Batch::solve_shape(int cluster, TickShape& shape, int*& index, std::vector<
         shape.pcg_group_count[g] = static_cast<int>(members.size());
         shape.pcg_group_index[g] = index + first;
         if (g > 0 && !pcg_streams_[g]) {
-            check(cudaStreamCreateWithFlags(&pcg_streams_[g], cudaStreamNonBlocking), "stream");
+            pcg_streams_[g] = StreamLease::take();
             check(cudaEventCreateWithFlags(&pcg_join_[g], cudaEventDisableTiming), "event");
         }
         shape.pcg_streams[g] = pcg_streams_[g];
@@ -935,7 +914,8 @@ void Batch::solve_shape(int cluster, TickShape& shape, int*& index, std::vector<
     }
     if (!pcg_fork_) check(cudaEventCreateWithFlags(&pcg_fork_, cudaEventDisableTiming), "event");
     shape.pcg_fork = pcg_fork_;
-    check(cudaMemcpy(index, order.data(), sizeof(int) * W, cudaMemcpyHostToDevice), "solve groups");
+    check(cudaMemcpyAsync(index, order.data(), sizeof(int) * W, cudaMemcpyHostToDevice, stream_), "solve groups");
+    check(cudaStreamSynchronize(stream_), "solve groups");
     shape.pcg_groups = static_cast<int>(sizes.size());
     shape.pcg_cluster = sizes[0];
 }

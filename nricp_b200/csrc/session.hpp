@@ -11,6 +11,7 @@
 #include "../../include/nricp_b200.h"
 #include "common.cuh"
 #include "kernels.cuh"
+#include "resources.hpp"
 
 namespace nricp_b200 {
 
@@ -98,7 +99,8 @@ private:
                                       const std::vector<double>& trans, int level) const;
 
     std::vector<std::unique_ptr<Wrap>> wraps_;
-    cudaStream_t stream_ = nullptr;
+    StreamLease stream_;
+    void* device_block_ = nullptr;  // holds the five device arrays below
     WrapDev* dev_wraps_ = nullptr;
     WrapControl* dev_controls_ = nullptr;
     // Start states and target hierarchies are built on kBuildStreams side
@@ -106,24 +108,24 @@ private:
     // target), forked from and joined back into stream_.
     static constexpr int kBuildStreams = 4;
     void reset_all(const char* staging, const std::vector<size_t>* offset, LbvhExport* lbvh_out);
-    cudaStream_t build_streams_[kBuildStreams] = {};
+    StreamLease build_streams_[kBuildStreams];
     cudaEvent_t build_fork_ = nullptr, build_done_[kBuildStreams] = {};
     void* build_scratch_[kBuildStreams] = {};
     cudaMemPool_t pool_ = nullptr;  // the arenas' and the scratch's (batch_pool)
     int* query_counter_ = nullptr;  // the query queues' heads (vertices, long walks)
-    cudaStream_t side_stream_ = nullptr;  // the tick's refresh branch
+    StreamLease side_stream_;  // the tick's refresh branch
     cudaEvent_t side_fork_ = nullptr, side_join_ = nullptr;
     int* pcg_index_ = nullptr;      // wraps ordered by solve class (device)
-    cudaStream_t pcg_streams_[5] = {};
+    StreamLease pcg_streams_[5];
     cudaEvent_t pcg_join_[5] = {};
     cudaEvent_t pcg_fork_ = nullptr;
-    WrapControl* host_controls_ = nullptr;
+    PinnedLease host_block_;
+    WrapControl* host_controls_ = nullptr;  // in host_block_
     TickShape shape_{};
     cudaGraphExec_t graph_exec_ = nullptr;
     // Solve launch fields of `shape` for the cluster setting `cluster` (as
-    // set_pcg_cluster takes it), its class lists in `index` (device, made
-    // here when needed); `cls` (if given) receives each wrap's cluster size.
-    void solve_shape(int cluster, TickShape& shape, int*& index, std::vector<int>* cls);
+    // set_pcg_cluster takes it), its class lists in `index` (device); `cls` (if given) receives each wrap's cluster size.
+    void solve_shape(int cluster, TickShape& shape, int* index, std::vector<int>* cls);
     cudaGraphExec_t capture(const TickShape& shape);
     // The batch's tail.  With halved classes, once the wraps still running
     // would fit on the SMs in one round at one halving less, their ticks run

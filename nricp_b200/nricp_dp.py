@@ -428,10 +428,7 @@ def _points(a, name):
 
 
 def _faces(a, name):
-    out = np.asarray(a)
-    if out.ndim != 2 or out.shape[1] != 3:
-        raise ValueError(f"{name} must have shape (n, 3)")
-    return np.ascontiguousarray(out.astype(np.int64).astype(np.int32))
+    return _abi._faces(a, name)
 
 
 def bounding_box_diagonal(points) -> float:
@@ -792,37 +789,34 @@ def build_template_graph(points, faces, levels: int = 4, nodes_initial: int = 10
     report = validate_mesh(p, f)
     if not report["ok"]:
         raise ValueError("invalid mesh: " + "; ".join(report["problems"]))
-    lib = load()
     n = len(p)
     level_count = max(1, int(levels))
-    out_levels = []
     center = np.zeros(3)
     scale = C.c_double()
+    P = lambda a, t: a.ctypes.data_as(C.POINTER(t))  # noqa: E731
+    buffers, structs = [], (_abi.GraphLevel * level_count)()
     for level in range(level_count):
         g = float(max(1, growth)) ** level
         nodes = min(max(1, int(math.floor(nodes_initial * g + 0.5))), n)
-        idx = np.zeros(nodes, dtype=np.int32)
-        pos = np.zeros((nodes, 3))
-        bn = np.zeros((n, _abi.MAX_SLOTS), dtype=np.int32)
-        bw = np.zeros((n, _abi.MAX_SLOTS))
-        bc = np.zeros(n, dtype=np.int32)
         cap = max(1, nodes * max(1, edge_neighbours))
-        edges = np.zeros((cap, 2), dtype=np.int32)
-        count = C.c_int()
-        P = lambda a, t: a.ctypes.data_as(C.POINTER(t))  # noqa: E731
-        check(lib.nricp_template_graph_level(
-            P(p, C.c_double), n, level_count, nodes_initial, growth, max_nodes_per_vertex,
-            edge_neighbours, level, P(center, C.c_double), C.byref(scale), P(idx, C.c_int32),
-            P(pos, C.c_double), P(bn, C.c_int32), P(bw, C.c_double), P(bc, C.c_int32),
-            P(edges, C.c_int32), cap, C.byref(count), int(bool(use_device))))
-        support = max(4, int(max_nodes_per_vertex))
-        out_levels.append({
-            "node_positions": pos,
-            "node_template_indices": idx.astype(np.int64),
-            "bindings": {"nodes": bn[:, :support].astype(np.int64), "weights": bw[:, :support],
-                         "counts": bc.astype(np.int64)},
-            "edges": edges[:count.value].astype(np.int64),
-        })
+        b = {"indices": np.empty(nodes, dtype=np.int32), "positions": np.empty((nodes, 3)),
+             "nodes": np.empty((n, _abi.MAX_SLOTS), dtype=np.int32), "weights": np.empty((n, _abi.MAX_SLOTS)),
+             "counts": np.empty(n, dtype=np.int32), "edges": np.empty((cap, 2), dtype=np.int32)}
+        structs[level] = _abi.GraphLevel(P(b["indices"], C.c_int32), P(b["positions"], C.c_double),
+                                         P(b["nodes"], C.c_int32), P(b["weights"], C.c_double),
+                                         P(b["counts"], C.c_int32), P(b["edges"], C.c_int32), cap, 0)
+        buffers.append(b)
+    check(load().nricp_template_graph(P(p, C.c_double), n, level_count, nodes_initial, growth,
+                                      max_nodes_per_vertex, edge_neighbours, P(center, C.c_double),
+                                      C.byref(scale), structs, int(bool(use_device))))
+    support = max(4, int(max_nodes_per_vertex))
+    out_levels = [{
+        "node_positions": b["positions"],
+        "node_template_indices": b["indices"].astype(np.int64),
+        "bindings": {"nodes": b["nodes"][:, :support].astype(np.int64), "weights": b["weights"][:, :support],
+                     "counts": b["counts"].astype(np.int64)},
+        "edges": b["edges"][:s.edge_count].astype(np.int64),
+    } for b, s in zip(buffers, structs)]
     return {"normalization": {"center": center[None, :].copy(), "scale": scale.value},
             "levels": out_levels}
 
