@@ -265,25 +265,8 @@ __device__ __forceinline__ void halving_place(int lane, int& first, int& count) 
         halving_place<H, O / 2>(lane, first, count);
     }
 }
-// Block sum in a fixed order; every thread returns the total.
-template <int kThreadsT>
-__device__ inline double block_sum(double v, double* scratch) {
-    v = warp_sum(v);
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    __syncthreads();
-    if (lane == 0) scratch[warp] = v;
-    __syncthreads();
-    if (warp == 0) {
-        double x = lane < kThreadsT / 32 ? scratch[lane] : 0.0;
-        x = warp_sum(x);
-        if (lane == 0) scratch[32] = x;
-    }
-    __syncthreads();
-    return scratch[32];
-}
-
-// The same block sum of N values with two barriers for all of them; thread 0
-// holds the totals.  `scratch` is kThreadsT / 32 x N doubles.
+// Block sums of N values in a fixed order, two barriers for all of them; the
+// first warp's lanes hold the totals.  `scratch` is kThreadsT / 32 x N doubles.
 template <int kThreadsT, int N>
 __device__ inline void block_sums(double* v, double* scratch) {
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -324,9 +307,11 @@ __device__ inline void add_rank_one(float* d, const float* u, float coef) {
 // ---------------------------------------------------------------------------
 // statistics (deform_ops.cu:135-182 / correspondence.cpp:82-94)
 // ---------------------------------------------------------------------------
+constexpr int kStatsBins = 2048;
+constexpr int kStatsKept = 2048;
 // The statistics pass at a tick's start (final_mode 0) also takes the tick's
 // phase snapshot.
-__global__ void k_stats(const WrapDev* __restrict__ wraps, int final_mode) {
+__global__ void __launch_bounds__(kStatsThreads) k_stats(const WrapDev* __restrict__ wraps, int final_mode) {
     const WrapDev& w = wraps[blockIdx.y * gridDim.x + blockIdx.x];
     const WrapControl c = *w.control;
     if (!final_mode && threadIdx.x == 0) w.control->tick_phase = c.phase;
@@ -340,74 +325,126 @@ __global__ void k_stats(const WrapDev* __restrict__ wraps, int final_mode) {
         level = c.stats_pending - 1;
         target = w.level_stats + level;
     }
-    __shared__ double scratch[33];
-    __shared__ int hist[256];
-    __shared__ unsigned long long prefix_s;
-    __shared__ int rank_s;
-    int counts[5] = {0, 0, 0, 0, 0};
-    double sum = 0.0, maximum = 0.0;
-    for (int v = threadIdx.x; v < w.V; v += blockDim.x) {
+    constexpr int kWarps = kStatsThreads / 32;
+    __shared__ double scratch[kWarps * 7];
+    __shared__ int hist[kStatsBins];
+    __shared__ unsigned long long kept[kStatsKept];
+    __shared__ double totals_s[6];
+    __shared__ unsigned long long low_s, high_s, maximum_s;
+    __shared__ int warp_count[kWarps], bin_s, rank_s, count_s;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    // counts per outcome, and the accepted distances' sum and extremes (a
+    // distance is never negative, so its bits order like the distance)
+    double sums[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
+    unsigned long long low = ~0ull, high = 0ull;
+    double maximum = 0.0;
+#pragma unroll 4
+    for (int v = threadIdx.x; v < w.V; v += kStatsThreads) {
         const int code = w.corr_code[v];
-        if (code >= 0 && code < 5) counts[code]++;
+        const double d = w.corr_distance[v];
+        for (int k = 0; k < 5; ++k)
+            if (code == k) sums[k] += 1.0;
         if (code == 0) {
-            const double d = w.corr_distance[v];
-            sum += d;
+            sums[5] += d;
+            const unsigned long long bits = (unsigned long long)__double_as_longlong(d);
+            low = min(low, bits);
+            high = max(high, bits);
             maximum = fmax(maximum, d);
         }
     }
-    int totals[5];
-    for (int k = 0; k < 5; ++k) totals[k] = (int)block_sum<kStatsThreads>((double)counts[k], scratch);
-    const double total_sum = block_sum<kStatsThreads>(sum, scratch);
-    // max via the same fixed tree on negated values is not needed: max is exact
-    double m = maximum;
-    for (int o = 16; o > 0; o >>= 1) m = fmax(m, __shfl_xor_sync(0xffffffffu, m, o));
-    __syncthreads();
-    if ((threadIdx.x & 31) == 0) scratch[threadIdx.x >> 5] = m;
-    __syncthreads();
     if (threadIdx.x == 0) {
-        double mm = 0.0;
-        for (int i = 0; i < kStatsThreads / 32; ++i) mm = fmax(mm, scratch[i]);
-        scratch[32] = mm;
+        low_s = ~0ull;
+        high_s = maximum_s = 0ull;
     }
+    block_sums<kStatsThreads, 6>(sums, scratch);
+    for (int o = 16; o > 0; o >>= 1) {
+        low = min(low, __shfl_xor_sync(0xffffffffu, low, o));
+        high = max(high, __shfl_xor_sync(0xffffffffu, high, o));
+        maximum = fmax(maximum, __shfl_xor_sync(0xffffffffu, maximum, o));
+    }
+    if (lane == 0) {
+        atomicMin(&low_s, low);
+        atomicMax(&high_s, high);
+        atomicMax(&maximum_s, (unsigned long long)__double_as_longlong(maximum));
+    }
+    if (threadIdx.x == 0)
+        for (int k = 0; k < 6; ++k) totals_s[k] = sums[k];
     __syncthreads();
-    const double total_max = scratch[32];
+    int totals[5];
+    for (int k = 0; k < 5; ++k) totals[k] = (int)totals_s[k];
+    const double total_sum = totals_s[5];
     const int accepted = totals[0];
-    // p95 = the floor(0.95 (n - 1))-th smallest accepted distance, found by a
-    // radix select over the IEEE bits (non-negative doubles order like their
-    // bit patterns).
+    const double total_max = __longlong_as_double((long long)maximum_s);
+    // p95 = the floor(0.95 (n - 1))-th smallest accepted distance: the range
+    // of the bits that holds it, split into 2,048 equal bins and narrowed to
+    // the rank's bin until a bin is one value; once a bin's distances fit in
+    // shared memory they are kept there.  (Eight passes of 8 bits over the
+    // vertices, the first two counting into a few bins only, took 750 us for
+    // 100,000 vertices.)
     double p95 = 0.0;
     if (accepted > 0) {
         double pi = 0.95 * (double)(accepted - 1);
         if (pi > (double)(accepted - 1)) pi = (double)(accepted - 1);
-        if (threadIdx.x == 0) { prefix_s = 0ull; rank_s = (int)pi; }
-        __syncthreads();
-        unsigned long long mask = 0ull;
-        for (int shift = 56; shift >= 0; shift -= 8) {
-            for (int i = threadIdx.x; i < 256; i += blockDim.x) hist[i] = 0;
+        int rank = (int)pi, in_shared = -1;
+        unsigned long long from = low_s, span = high_s - low_s;  // the value lies in [from, from + span]
+        while (span > 0) {
+            const int bits = 64 - __clzll((long long)span);
+            const int shift = bits > 11 ? bits - 11 : 0;
+            for (int i = threadIdx.x; i < kStatsBins; i += kStatsThreads) hist[i] = 0;
             __syncthreads();
-            const unsigned long long prefix = prefix_s;
-            for (int v = threadIdx.x; v < w.V; v += blockDim.x) {
-                if (w.corr_code[v] != 0) continue;
-                const unsigned long long bits = (unsigned long long)__double_as_longlong(w.corr_distance[v]);
-                if ((bits & mask) != prefix) continue;
-                atomicAdd(&hist[(bits >> shift) & 255ull], 1);
-            }
-            __syncthreads();
-            if (threadIdx.x == 0) {
-                int rank = rank_s;
-                int digit = 0;
-                for (; digit < 256; ++digit) {
-                    if (rank < hist[digit]) break;
-                    rank -= hist[digit];
+            // every accepted distance's place in the range, or every kept one's
+            auto each = [&](auto&& body) {
+                if (in_shared >= 0) {
+                    for (int i = threadIdx.x; i < in_shared; i += kStatsThreads) body(kept[i] - from, kept[i]);
+                } else {
+#pragma unroll 4
+                    for (int v = threadIdx.x; v < w.V; v += kStatsThreads) {
+                        const int code = w.corr_code[v];
+                        const unsigned long long b = (unsigned long long)__double_as_longlong(w.corr_distance[v]);
+                        if (code == 0 && b >= from) body(b - from, b);
+                    }
                 }
-                if (digit > 255) digit = 255;
-                rank_s = rank;
-                prefix_s = prefix | ((unsigned long long)digit << shift);
+            };
+            each([&](unsigned long long at, unsigned long long) {
+                if (at <= span) atomicAdd(&hist[at >> shift], 1);
+            });
+            __syncthreads();
+            // the bin of the rank: each thread four bins, a scan over the threads
+            constexpr int kPer = kStatsBins / kStatsThreads;
+            int mine = 0;
+            for (int k = 0; k < kPer; ++k) mine += hist[threadIdx.x * kPer + k];
+            int before = mine;
+            for (int o = 1; o < 32; o <<= 1) {
+                const int y = __shfl_up_sync(0xffffffffu, before, o);
+                if (lane >= o) before += y;
             }
-            mask |= 255ull << shift;
+            if (lane == 31) warp_count[warp] = before;
+            __syncthreads();
+            before -= mine;
+            for (int i = 0; i < warp; ++i) before += warp_count[i];
+            if (rank >= before && rank < before + mine) {  // one thread's
+                int at = rank - before, k = 0;
+                while (at >= hist[threadIdx.x * kPer + k]) at -= hist[threadIdx.x * kPer + k++];
+                bin_s = threadIdx.x * kPer + k;
+                rank_s = at;
+                count_s = 0;
+            }
+            __syncthreads();
+            const unsigned long long next = from + ((unsigned long long)bin_s << shift);
+            const unsigned long long width = (1ull << shift) - 1;  // the bin's last value, from its first
+            const int there = hist[bin_s];
+            if (width > 0 && in_shared < 0 && there <= kStatsKept) {
+                each([&](unsigned long long, unsigned long long b) {
+                    if (b >= next && b - next <= width) kept[atomicAdd(&count_s, 1)] = b;
+                });
+                in_shared = there;
+            }
+            rank = rank_s;
+            from = next;
+            span = width;
             __syncthreads();
         }
-        p95 = __longlong_as_double((long long)prefix_s);
+        p95 = __longlong_as_double((long long)from);
     }
     if (threadIdx.x == 0) {
         CorrStats s;
@@ -575,33 +612,37 @@ __global__ void __launch_bounds__(kRigidThreads) k_fit_rigid(const double* __res
                                                             const double* __restrict__ dst,
                                                             const double* __restrict__ weights, int n,
                                                             double* __restrict__ out) {
-    __shared__ double scratch[33];
+    __shared__ double scratch[kRigidThreads / 32 * 9];
+    __shared__ double total[9];
     double sums[7] = {0, 0, 0, 0, 0, 0, 0};  // w, w p, w q
-    for (int i = threadIdx.x; i < n; i += blockDim.x) {
+    for (int i = threadIdx.x; i < n; i += kRigidThreads) {
         const double w = fmax(0.0, weights[i]);
         sums[0] += w;
         for (int k = 0; k < 3; ++k) {
-            sums[1 + k] += src[i * 3 + k] * w;
-            sums[4 + k] += dst[i * 3 + k] * w;
+            sums[1 + k] += src[(long)i * 3 + k] * w;
+            sums[4 + k] += dst[(long)i * 3 + k] * w;
         }
     }
-    for (int k = 0; k < 7; ++k) sums[k] = block_sum<kRigidThreads>(sums[k], scratch);
+    block_sums<kRigidThreads, 7>(sums, scratch);
+    if (threadIdx.x == 0)
+        for (int k = 0; k < 7; ++k) total[k] = sums[k];
+    __syncthreads();
     double R[9] = {1, 0, 0, 0, 1, 0, 0, 0, 1};
-    if (!(sums[0] > 0.0)) {
+    if (!(total[0] > 0.0)) {
         if (threadIdx.x == 0)
             for (int k = 0; k < 12; ++k) out[k] = k < 9 ? R[k] : 0.0;
         return;
     }
-    const double cp[3] = {sums[1] / sums[0], sums[2] / sums[0], sums[3] / sums[0]};
-    const double cq[3] = {sums[4] / sums[0], sums[5] / sums[0], sums[6] / sums[0]};
+    const double cp[3] = {total[1] / total[0], total[2] / total[0], total[3] / total[0]};
+    const double cq[3] = {total[4] / total[0], total[5] / total[0], total[6] / total[0]};
     double S[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
-    for (int i = threadIdx.x; i < n; i += blockDim.x) {
+    for (int i = threadIdx.x; i < n; i += kRigidThreads) {
         const double w = fmax(0.0, weights[i]);
         if (w == 0.0) continue;
         for (int r = 0; r < 3; ++r)
-            for (int q = 0; q < 3; ++q) S[r * 3 + q] += w * (src[i * 3 + r] - cp[r]) * (dst[i * 3 + q] - cq[q]);
+            for (int q = 0; q < 3; ++q) S[r * 3 + q] += w * (src[(long)i * 3 + r] - cp[r]) * (dst[(long)i * 3 + q] - cq[q]);
     }
-    for (int k = 0; k < 9; ++k) S[k] = block_sum<kRigidThreads>(S[k], scratch);
+    block_sums<kRigidThreads, 9>(S, scratch);
     if (threadIdx.x == 0) {
         horn_rotation(S, R);
         for (int k = 0; k < 9; ++k) out[k] = R[k];
@@ -1461,20 +1502,45 @@ __global__ void k_evaluate(const WrapDev* __restrict__ wraps, int wrap_count, in
         [&](int wi, int bx) { k_evaluate_body(wraps[wi], part, bx); });
 }
 
+// A thread per vertex; a vertex of more faces than kWideFan (the poles of a
+// lat-long template have hundreds) is its warp's: the lanes form the faces'
+// normals, which are then added in face order, as the thread's loop would.
+// (One thread's loop over a pole's 224 faces held the kernel for 68 us.)
+constexpr int kWideFan = 24;
+__device__ __forceinline__ D3 face_normal(const WrapDev& w, int i) {
+    const int32_t* f = w.tpl_faces + (long)w.vf_faces[i] * 3;
+    const D3 a = load_d3(w.deformed, f[0]);
+    const D3 b = load_d3(w.deformed, f[1]);
+    const D3 c = load_d3(w.deformed, f[2]);
+    return rcross(rsub(b, a), rsub(c, a));
+}
 __device__ __forceinline__ void k_normals_body(const WrapDev& w, int part, int bx) {
     const WrapControl c = *w.control;
     if (!in_part(c, part)) return;
     if (!refresh_like(c.phase)) return;
-    const int v = bx * blockDim.x + threadIdx.x;
-    if (v >= w.V) return;
+    const int v = bx * blockDim.x + threadIdx.x, lane = threadIdx.x & 31;
+    const int begin = v < w.V ? w.vf_begin[v] : 0, end = v < w.V ? w.vf_begin[v + 1] : 0;
+    const bool wide = end - begin > kWideFan;
     D3 n = {0.0, 0.0, 0.0};
-    for (int i = w.vf_begin[v]; i < w.vf_begin[v + 1]; ++i) {
-        const int32_t* f = w.tpl_faces + (long)w.vf_faces[i] * 3;
-        const D3 a = load_d3(w.deformed, f[0]);
-        const D3 b = load_d3(w.deformed, f[1]);
-        const D3 cc = load_d3(w.deformed, f[2]);
-        n = radd(n, rcross(rsub(b, a), rsub(cc, a)));
+    if (!wide)
+        for (int i = begin; i < end; ++i) n = radd(n, face_normal(w, i));
+    uint32_t fans = __ballot_sync(0xffffffffu, wide);
+    while (fans) {
+        const int owner = __ffs(fans) - 1;
+        fans &= fans - 1;
+        const int b = __shfl_sync(0xffffffffu, begin, owner), e = __shfl_sync(0xffffffffu, end, owner);
+        D3 sum = {0.0, 0.0, 0.0};
+        for (int base = b; base < e; base += 32) {
+            D3 x = {0.0, 0.0, 0.0};
+            if (base + lane < e) x = face_normal(w, base + lane);
+            const int here = min(32, e - base);
+            for (int k = 0; k < here; ++k)
+                sum = radd(sum, {__shfl_sync(0xffffffffu, x.x, k), __shfl_sync(0xffffffffu, x.y, k),
+                                 __shfl_sync(0xffffffffu, x.z, k)});
+        }
+        if (lane == owner) n = sum;
     }
+    if (v >= w.V) return;
     const double len = __dsqrt_rn(rdot(n, n));
     if (len > 0.0) n = {__ddiv_rn(n.x, len), __ddiv_rn(n.y, len), __ddiv_rn(n.z, len)};
     else n = {0.0, 0.0, 0.0};
