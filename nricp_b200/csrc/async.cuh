@@ -15,6 +15,9 @@ __device__ __forceinline__ void mbar_init(void* bar, int arrivals) {
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
 }
+__device__ __forceinline__ void mbar_invalidate(void* bar) {
+    asm volatile("mbarrier.inval.shared::cta.b64 [%0];" ::"r"(shared_address(bar)) : "memory");
+}
 __device__ __forceinline__ void mbar_arrive(void* bar) {
     asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(shared_address(bar)) : "memory");
 }

@@ -196,7 +196,9 @@ struct WrapDev {
     float* pcg_p;                 // N x 6: direction p
     float* pcg_ap;                // N x 6: w = A u
     float* pcg_s;                 // N x 6: s = A p (by recurrence)
-    float* pcg_u;                 // N x 6: u = M^-1 r, every node
+    float* pcg_u;                 // N x 8: u = M^-1 r, every node (six floats a node, eight in a grid solve)
+    double* pcg_sums;             // 6 per octet: a grid solve's partial sums
+    unsigned* grid_arrivals;      // its CTAs' meetings this tick
     // reductions
     double* partials;             // energy_blocks x kPartialStride
     double* edge_partials;        // edges: each edge's smoothness energy (the decision kernel sums them)

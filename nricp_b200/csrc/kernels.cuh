@@ -59,6 +59,8 @@ struct TickShape {
     const int* pcg_group_index[5];       // device: wrap indices of the group
     cudaStream_t pcg_streams[5];         // branch streams (index 0 unused)
     cudaEvent_t pcg_fork, pcg_join[5];
+    int grid_nodes;  // graphs above this may be solved by the whole device (0: no such launch)
+    int grid_ctas;
     int* query_counter;                  // device: the query queues' heads, 2 ints
     // The refresh chain's branch (null: one chain on the tick's stream).
     cudaStream_t side_stream;
@@ -81,6 +83,8 @@ void launch_tick(const WrapDev* wraps, const TickShape& shape, cudaStream_t stre
 int tick_kernel_launches(const TickShape& shape, bool timed = false);
 int pcg_latency_cluster(int nodes);
 int pcg_cluster_size(int max_nodes, int wraps, int sm_count);
+// Sets the shape's grid solve from its wraps and max_nodes.
+void grid_solve_shape(TickShape& shape);
 int pcg_max_nodes();
 // The weighted rigid fit of n point pairs (device arrays); out = R (row-major
 // 3x3), t.

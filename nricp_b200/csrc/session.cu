@@ -328,7 +328,9 @@ size_t prepare_device(Wrap& w, WrapControl* control, cudaStream_t stream, bool p
     const size_t o_p = a.reserve(sizeof(float) * 6 * N);
     const size_t o_ap = a.reserve(sizeof(float) * 6 * N);
     const size_t o_s = a.reserve(sizeof(float) * 6 * N);
-    const size_t o_u = a.reserve(sizeof(float) * 6 * N);
+    const size_t o_u = a.reserve(sizeof(float) * 8 * N);
+    const size_t o_sums = a.reserve(sizeof(double) * 6 * ((N + 7) / 8));
+    const size_t o_arrivals = a.reserve(sizeof(unsigned));
     const int vblocks = (V + 255) / 256;
     const size_t o_part = a.reserve(sizeof(double) * kPartialStride * std::max(1, vblocks));
     const size_t o_epart = a.reserve(sizeof(double) * std::max(1, w.max_edges));
@@ -514,6 +516,8 @@ size_t prepare_device(Wrap& w, WrapControl* control, cudaStream_t stream, bool p
     D.pcg_ap = a.at<float>(o_ap);
     D.pcg_s = a.at<float>(o_s);
     D.pcg_u = a.at<float>(o_u);
+    D.pcg_sums = a.at<double>(o_sums);
+    D.grid_arrivals = a.at<unsigned>(o_arrivals);
     D.partials = a.at<double>(o_part);
     D.edge_partials = a.at<double>(o_epart);
     D.node_partials = a.at<double>(o_npart);
@@ -862,6 +866,7 @@ void Batch::set_pcg_cluster(int cluster) {
             *g = nullptr;
         }
     tail_ready_ = tail_on_ = false;
+    grid_solve_shape(shape_);
     solve_shape(cluster, shape_, pcg_index_, nullptr);
     if (cluster < 0) {  // halved classes: halved once less for the tail
         tail_shape_ = shape_;
@@ -1545,6 +1550,7 @@ struct Server::Impl {
         if (it != graphs.end()) return it->second;
         TickShape t = shape;
         t.wraps = count;
+        grid_solve_shape(t);
         t.pcg_groups = 0;
         pcg_cluster_size(t.max_nodes, count, sms);  // enables the launch attributes
         if (class_count == 0) {

@@ -314,7 +314,10 @@ constexpr int kStatsKept = 2048;
 __global__ void __launch_bounds__(kStatsThreads) k_stats(const WrapDev* __restrict__ wraps, int final_mode) {
     const WrapDev& w = wraps[blockIdx.y * gridDim.x + blockIdx.x];
     const WrapControl c = *w.control;
-    if (!final_mode && threadIdx.x == 0) w.control->tick_phase = c.phase;
+    if (!final_mode && threadIdx.x == 0) {
+        w.control->tick_phase = c.phase;
+        *w.grid_arrivals = 0;  // the grid solve's meetings of this tick
+    }
     CorrStats* target = nullptr;
     int level = -1;
     if (final_mode) {
@@ -957,6 +960,33 @@ __device__ __forceinline__ RowPair row_pair_dot(float4 b0, float4 b1, float4 b2,
             row_dot<kDiagonal>(b1.z, b1.w, b2.x, b2.y, b2.z, b2.w, u0, u1, u2)};
 }
 
+// Sixteen bytes from global memory (past the L1) to shared memory, and the wait
+// for all that the thread has under way.
+__device__ __forceinline__ void copy_16_async(void* dst, const void* src) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(shared_address(dst)),
+                 "l"(__cvta_generic_to_global(src))
+                 : "memory");
+}
+__device__ __forceinline__ void wait_copies() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+constexpr int kGatherSteps = 16;  // steps whose u a warp of a grid solve gathers at a time
+
+// One thread's part of a meeting of a cooperative grid's CTAs: counts its CTA
+// in and waits, with a limit (about a second), until `target` have come.
+__device__ __forceinline__ bool grid_arrive_and_wait(unsigned* arrivals, unsigned target) {
+    // the release covers what the CTA's threads wrote before the block barrier;
+    // the polls are plain, and one fence after the last orders what follows
+    asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(arrivals) : "memory");
+    for (int i = 0; i < kWaitLimit; ++i) {
+        unsigned seen;
+        asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(seen) : "l"(arrivals) : "memory");
+        if (seen >= target) {
+            asm volatile("fence.acq_rel.gpu;" ::: "memory");
+            return true;
+        }
+    }
+    return false;
+}
+
 // A few steps of an octet's blocks from global memory, in registers.
 constexpr int kStepsAhead = 4;
 struct StepBlocks {
@@ -990,14 +1020,21 @@ struct StepBlocks {
 //
 // kAllShared: every array of the placement is in shared memory (the compiler
 // then addresses it as such); the other instance decides at run time.
-template <bool kAllShared>
+//
+// kGrid: the CTAs are a cooperative grid over the whole device instead of a
+// cluster, for a graph whose rows are worth more SMs than a cluster has.  u
+// (eight floats a node) and the segments' sums are then in global memory, and
+// the CTAs meet at a counter in global memory twice per iteration; a CTA holds
+// so few rows that its own arrays are always in shared memory.
+template <bool kAllShared, bool kGrid>
 __device__ __forceinline__ void pcg_solve(const WrapDev& w, const WrapControl& c, const PcgPlacement& place,
                                           int budget_floats) {
+    static_assert(kAllShared || !kGrid, "the grid's own rows fit");
     cg::cluster_group cluster = cg::this_cluster();
     const LevelDev& L = w.levels[c.level];
     const int N = L.node_count;
-    const int rank = (int)cluster.block_rank();
-    const int ranks = (int)cluster.num_blocks();
+    const int rank = kGrid ? (int)blockIdx.x : (int)cluster.block_rank();
+    const int ranks = kGrid ? (int)gridDim.x : (int)cluster.num_blocks();
     const int segs = pcg_segments(N);
     const int octets = pcg_octets(N);
     const int cap = pcg_owned_capacity(N, ranks);
@@ -1009,14 +1046,28 @@ __device__ __forceinline__ void pcg_solve(const WrapDev& w, const WrapControl& c
     const int rows = own * 6;
 
     extern __shared__ float4 dynamic_shared[];
-    double* slots = reinterpret_cast<double*>(dynamic_shared);  // 3 per segment, every CTA
-    float* cursor = reinterpret_cast<float*>(slots + pcg_slot_doubles(N));
-    float* U;
-    if (kAllShared || place.u_shared) {
-        U = cursor;
-        cursor += (N * 6 + 3) & ~3;
-    } else {
+    double* slots;  // 3 per segment, in every CTA
+    float* cursor;
+    float *U, *own_u;  // u of every node; of the owned rows
+    float* gathered = nullptr;
+    if (kGrid) {
+        slots = w.pcg_sums;
         U = w.pcg_u;
+        cursor = reinterpret_cast<float*>(dynamic_shared);
+        own_u = cursor;
+        cursor += cap * 6;
+        gathered = cursor;  // a warp's steps' u
+        cursor += kPcgWarps * kGatherSteps * 64;
+    } else {
+        slots = reinterpret_cast<double*>(dynamic_shared);
+        cursor = reinterpret_cast<float*>(slots + pcg_slot_doubles(N));
+        if (kAllShared || place.u_shared) {
+            U = cursor;
+            cursor += (N * 6 + 3) & ~3;
+        } else {
+            U = w.pcg_u;
+        }
+        own_u = U + n0 * 6;
     }
     double *X, *R;
     float *Minv, *P, *S, *Wv;
@@ -1062,7 +1113,7 @@ __device__ __forceinline__ void pcg_solve(const WrapDev& w, const WrapControl& c
     __shared__ double red[3][kPcgWarps];
     // mbarriers: the cached blocks; an iteration's partial sums; its u
     __shared__ alignas(8) unsigned long long blocks_arrived, sums_arrived, u_arrived;
-    __shared__ int cached_s;
+    __shared__ int cached_s, listed_s;
     bool timed_out = false;  // a wait of this thread ran out
 
     // ---- the last steps of every owned octet's blocks into the shared
@@ -1072,42 +1123,56 @@ __device__ __forceinline__ void pcg_solve(const WrapDev& w, const WrapControl& c
         int most = 0;
         for (int o = o0 + lane; o < o1; o += 32) most = max(most, sell_begin[o + 1] - sell_begin[o]);
         most = __reduce_max_sync(0xffffffffu, most);
-        const int left = budget_floats - place.floats;
-        const int cached = o1 > o0 ? min(most, left / ((o1 - o0) * (kStepFloats + kOctet))) : 0;
+        // a grid keeps the other nodes of every step if they fit (a node of very
+        // many neighbours may prevent it), a cluster of the cached ones
+        const int room = budget_floats - place.floats;
+        const bool list_all = kGrid && (long)(o1 - o0) * most * kOctet <= room;
+        const int left = list_all ? room - (o1 - o0) * most * kOctet : room;
+        const int each = kGrid ? kStepFloats : kStepFloats + kOctet;
+        const int cached = o1 > o0 ? max(0, min(most, left / ((o1 - o0) * each))) : 0;
+        const int listed = kGrid ? (list_all ? most : 0) : cached;  // steps whose nodes are kept
         if (lane == 0) {
             cached_s = cached;
+            listed_s = listed;
             mbar_init(&blocks_arrived, 1);
             mbar_init(&sums_arrived, kPcgWarps);
             mbar_init(&u_arrived, 1);
         }
         __syncwarp();
         int bytes = 0;
-        for (int o = o0 + lane; o < o1; o += 32)
-            bytes += min(cached, sell_begin[o + 1] - sell_begin[o]) * (int)sizeof(float) * (kStepFloats + kOctet);
+        for (int o = o0 + lane; o < o1; o += 32) {
+            const int steps = sell_begin[o + 1] - sell_begin[o];
+            bytes += (min(cached, steps) * kStepFloats + min(listed, steps) * kOctet) * (int)sizeof(float);
+        }
         bytes = __reduce_add_sync(0xffffffffu, bytes);
         if (lane == 0) mbar_arrive_expect(&blocks_arrived, bytes);
         __syncwarp();
         float* block_room = cursor;
         float* node_room = cursor + (long)(o1 - o0) * cached * kStepFloats;
         for (int o = o0 + lane; o < o1; o += 32) {
-            const int count = min(cached, sell_begin[o + 1] - sell_begin[o]);
-            const int first = sell_begin[o + 1] - count;
-            if (count <= 0) continue;
-            const int at = (o - o0) * cached;
-            bulk_to_shared(block_room + (long)at * kStepFloats, B + (long)first * kStepFloat4s,
-                           count * kStepFloats * (int)sizeof(float), &blocks_arrived);
-            bulk_to_shared(node_room + at * kOctet, sell_nodes + (long)first * kOctet,
-                           count * kOctet * (int)sizeof(float), &blocks_arrived);
+            const int end = sell_begin[o + 1], steps = end - sell_begin[o];
+            const int count = min(cached, steps), nodes = min(listed, steps);
+            if (count > 0)
+                bulk_to_shared(block_room + (long)(o - o0) * cached * kStepFloats, B + (long)(end - count) * kStepFloat4s,
+                               count * kStepFloats * (int)sizeof(float), &blocks_arrived);
+            if (nodes > 0)
+                bulk_to_shared(node_room + (o - o0) * listed * kOctet, sell_nodes + (long)(end - nodes) * kOctet,
+                               nodes * kOctet * (int)sizeof(float), &blocks_arrived);
         }
     }
 
+    // a diagonal entry damped (spelt out, so that every instance rounds alike)
+    auto damped = [&](float x) {
+        const float scale = scaled ? fmaxf(x, 1e-12f) : 1.0f;
+        return __fmaf_rn(damping, scale, x);
+    };
     // ---- damped diagonal blocks and their inverses (route A's damped():
     //      scale = max(D_rr, 1e-12)); Cholesky with the reference's jitter ----
     for (int m = threadIdx.x; m < own; m += blockDim.x) {
         const int n = n0 + m;
         float blk[36];
         for (int i = 0; i < 36; ++i) blk[i] = D[n * 36 + i];
-        for (int r = 0; r < 6; ++r) blk[r * 7] += damping * (scaled ? fmaxf(blk[r * 7], 1e-12f) : 1.0f);
+        for (int r = 0; r < 6; ++r) blk[r * 7] = damped(blk[r * 7]);
         if (kAllShared) {  // stored as a step's block
             float* to = diagonal + block_base(m);
             for (int i = 0; i < 36; ++i) to[block_at(i / 6, i % 6)] = blk[i];
@@ -1140,9 +1205,10 @@ __device__ __forceinline__ void pcg_solve(const WrapDev& w, const WrapControl& c
         S[i] = 0.0f;
     }
     // every CTA's rows and mbarriers are ready
-    cluster.sync();
+    if (kGrid) __syncthreads();
+    else cluster.sync();
 
-    const int cached = cached_s;
+    const int cached = cached_s, listed = listed_s;
     const float4* cached_blocks = reinterpret_cast<const float4*>(cursor);
     const int* cached_nodes = reinterpret_cast<const int*>(cursor + (long)(o1 - o0) * cached * kStepFloats);
     if (!mbar_wait(&blocks_arrived, 0)) timed_out = true;
@@ -1151,11 +1217,20 @@ __device__ __forceinline__ void pcg_solve(const WrapDev& w, const WrapControl& c
     // global the loop meets at cluster barriers, and a graph that large gives
     // every CTA rows.)
     const int active = (octets * kOctet + cap - 1) / cap;
-    const bool u_shared = kAllShared || place.u_shared;
+    const bool u_shared = !kGrid && (kAllShared || place.u_shared);
     const int u_bytes = ((N * 6 + 3) & ~3) * (int)sizeof(float);  // of every row
     const int own_bytes = (rank == active - 1 ? u_bytes : n1 * 24) - n0 * 24;
-    const int peer = min(lane, active - 1);
-    const uint32_t peer_slots = peer_address(slots, peer), peer_sums_arrived = peer_address(&sums_arrived, peer);
+    const int peer = kGrid ? 0 : min(lane, active - 1);
+    const uint32_t peer_slots = kGrid ? 0 : peer_address(slots, peer);
+    const uint32_t peer_sums_arrived = kGrid ? 0 : peer_address(&sums_arrived, peer);
+    unsigned meetings = 0;  // the grid's, so far
+    auto meet = [&]() {     // every active CTA's writes before it are visible after it
+        __syncthreads();
+        ++meetings;
+        if (threadIdx.x == 0 && !grid_arrive_and_wait(w.grid_arrivals, meetings * (unsigned)active)) timed_out = true;
+        // the other threads learn of a wait that ran out at the totals' barrier
+        __syncthreads();
+    };
 
     // One segment's rows per warp at a time: `update` forms r[i], then
     // u = M^-1 r into this CTA's copy.
@@ -1170,13 +1245,18 @@ __device__ __forceinline__ void pcg_solve(const WrapDev& w, const WrapControl& c
                 const float* mi = Minv + m * 36 + r * 6;
                 float z = 0.0f;
                 for (int q = 0; q < 6; ++q) z += mi[q] * (float)R[m * 6 + q];
-                U[n0 * 6 + i] = z;
+                own_u[i] = z;
+                if (kGrid) __stcg(U + (long)(n0 + m) * 8 + r, z);
             }
         }
     };
     // The slice of u into every other CTA's copy: one bulk copy per peer,
     // which completes on the peer's mbarrier.
     auto share_u = [&]() {
+        if (kGrid) {
+            meet();
+            return;
+        }
         if (!u_shared) {
             __threadfence();  // the global copy: visible device-wide first
             cluster.sync();
@@ -1198,13 +1278,13 @@ __device__ __forceinline__ void pcg_solve(const WrapDev& w, const WrapControl& c
         for (int k = 0; k < kStepsAhead; ++k)
             if (t + k < end) {
                 const float4* at = B + (long)(first + t + k) * kStepFloat4s + lane;
-                ahead.node[k] = __ldg(sell_nodes + (long)(first + t + k) * kOctet + i_node);
+                if (!kGrid) ahead.node[k] = __ldg(sell_nodes + (long)(first + t + k) * kOctet + i_node);
                 ahead.b[k][0] = __ldg(at);
                 ahead.b[k][1] = __ldg(at + 24);
                 ahead.b[k][2] = __ldg(at + 48);
             }
     };
-    struct OctetShape { int first, streamed, degree; };
+    struct OctetShape { int first, steps, streamed, degree; };
     auto octet_shape = [&](int o) {
         OctetShape x;
         const int n = o * kOctet + i_node;
@@ -1220,16 +1300,17 @@ __device__ __forceinline__ void pcg_solve(const WrapDev& w, const WrapControl& c
             steps = sell_begin[o + 1] - x.first;
             if (on) x.degree = row_begin[n + 1] - row_begin[n];
         }
+        x.steps = steps;
         x.streamed = max(0, steps - cached);
         return x;
     };
     // The warp's first streamed steps do not depend on u: they are fetched
     // before the wait for it.
-    OctetShape shape = {0, 0, 0};
+    OctetShape shape = {0, 0, 0, 0};
     auto fetch_first = [&]() {
         if (o0 + warp < o1) {
             shape = octet_shape(o0 + warp);
-            fetch(shape.first, 0, min(shape.streamed, shape.degree));
+            if (!kGrid) fetch(shape.first, 0, min(shape.streamed, shape.degree));
         }
     };
     if (own > 0) {
@@ -1250,58 +1331,92 @@ __device__ __forceinline__ void pcg_solve(const WrapDev& w, const WrapControl& c
             const bool on = lane < 24 && n < N;
             if (o != o0 + warp) {
                 shape = octet_shape(o);
-                fetch(shape.first, 0, min(shape.streamed, shape.degree));
+                if (!kGrid) fetch(shape.first, 0, min(shape.streamed, shape.degree));
             }
             RowPair y = {0.0f, 0.0f};
             if (kAllShared) {
                 if (on) {
                     const float4* at = reinterpret_cast<const float4*>(diagonal) + (long)(o - o0) * kStepFloat4s + lane;
-                    y = row_pair_dot<true>(at[0], at[24], at[48], U + n * 6);
+                    y = row_pair_dot<true>(at[0], at[24], at[48], own_u + (n - n0) * 6);
                 }
             } else if (on) {
                 const float4* d4 = reinterpret_cast<const float4*>(D + (long)n * 36) + p_row * 3;
                 float4 q0 = __ldg(d4), q1 = __ldg(d4 + 1), q2 = __ldg(d4 + 2);
-                auto damp = [&](float& x) { x += damping * (scaled ? fmaxf(x, 1e-12f) : 1.0f); };
+                auto damp = [&](float& x) { x = damped(x); };
                 damp(p_row == 0 ? q0.x : (p_row == 1 ? q0.z : q1.x));  // (2p, 2p) and (2p + 1, 2p + 1)
                 damp(p_row == 0 ? q1.w : (p_row == 1 ? q2.y : q2.w));
                 y = row_pair_dot<true>(q0, q1, q2, U + n * 6);
             }
-            {
-                const int end = min(shape.streamed, shape.degree);
-                for (int t = 0; t < end; t += kStepsAhead) {
-                    RowPair part[kStepsAhead];
+            const float4* const cached_at = cached_blocks + (long)(o - o0) * cached * kStepFloat4s + lane;
+            const int* const listed_at = cached_nodes + (o - o0) * listed * kOctet;
+            // steps [t, t + kStepsAhead) below `end`, added in order: dot(k)
+            // gives the products of step t + k
+            auto add_steps = [&](int t, int end, auto&& dot) {
+                RowPair part[kStepsAhead];
 #pragma unroll
-                    for (int k = 0; k < kStepsAhead; ++k)
-                        if (t + k < end)
-                            part[k] = row_pair_dot<false>(ahead.b[k][0], ahead.b[k][1], ahead.b[k][2], U + ahead.node[k] * 6);
+                for (int k = 0; k < kStepsAhead; ++k) part[k] = dot(k);
 #pragma unroll
-                    for (int k = 0; k < kStepsAhead; ++k)
-                        if (t + k < end) {
-                            y.a += part[k].a;
-                            y.b += part[k].b;
-                        }
-                    fetch(shape.first, t + kStepsAhead, end);
-                }
-            }
-            {
-                const float4* at = cached_blocks + (long)(o - o0) * cached * kStepFloat4s + lane;
-                const int* node = cached_nodes + (o - o0) * cached * kOctet + i_node;
-                const int end = shape.degree - shape.streamed;
-                for (int t = 0; t < end; t += kStepsAhead) {
-                    RowPair part[kStepsAhead];
-#pragma unroll
-                    for (int k = 0; k < kStepsAhead; ++k) {
-                        const int tk = min(t + k, end - 1);  // past the end: the last one again, not added
-                        part[k] = row_pair_dot<false>(at[tk * kStepFloat4s], at[tk * kStepFloat4s + 24],
-                                                      at[tk * kStepFloat4s + 48], U + node[tk * kOctet] * 6);
+                for (int k = 0; k < kStepsAhead; ++k)
+                    if (t + k < end) {
+                        y.a += part[k].a;
+                        y.b += part[k].b;
                     }
+            };
+            if constexpr (kGrid) {
+                // kGatherSteps steps at a time: the warp copies all their u
+                // from global memory at once (one latency instead of one per
+                // group of steps), then multiplies from shared memory
+                float* const room = gathered + warp * kGatherSteps * 64;
+                for (int base = 0; base < shape.steps; base += kGatherSteps) {
+                    const int last = min(shape.degree, base + kGatherSteps);
+                    const int streamed = min(shape.streamed, last);
+                    fetch(shape.first, base, streamed);
 #pragma unroll
-                    for (int k = 0; k < kStepsAhead; ++k)
-                        if (t + k < end) {
-                            y.a += part[k].a;
-                            y.b += part[k].b;
+                    for (int j = 0; j < kGatherSteps / 2; ++j) {
+                        const int step = 2 * j + (lane >> 4), half = lane & 1, node = (lane >> 1) & 7;
+                        if (base + step < shape.steps)
+                        {
+                            const int at = (base + step) * kOctet + node;
+                            const int id = listed > 0 ? listed_at[at] : __ldg(sell_nodes + (long)shape.first * kOctet + at);
+                            copy_16_async(room + step * 64 + node * 8 + half * 4, U + (long)id * 8 + half * 4);
                         }
+                    }
+                    wait_copies();
+                    __syncwarp();
+                    const float* const mine = room + i_node * 8;
+                    for (int t = base; t < streamed; t += kStepsAhead) {
+                        add_steps(t, streamed, [&](int k) {
+                            return row_pair_dot<false>(ahead.b[k][0], ahead.b[k][1], ahead.b[k][2],
+                                                       mine + min(t + k - base, kGatherSteps - 1) * 64);
+                        });
+                        fetch(shape.first, t + kStepsAhead, streamed);
+                    }
+                    for (int t = max(base, shape.streamed); t < last; t += kStepsAhead)
+                        add_steps(t, last, [&](int k) {
+                            const int tk = min(t + k, last - 1);  // past the end: the last one again, not added
+                            const float4* at = cached_at + (long)(tk - shape.streamed) * kStepFloat4s;
+                            return row_pair_dot<false>(at[0], at[24], at[48], mine + (tk - base) * 64);
+                        });
+                    __syncwarp();  // read before the next steps' copies
                 }
+            } else {
+                const int streamed = min(shape.streamed, shape.degree);
+                for (int t = 0; t < streamed; t += kStepsAhead) {
+                    add_steps(t, streamed, [&](int k) {
+                        return t + k < streamed ? row_pair_dot<false>(ahead.b[k][0], ahead.b[k][1], ahead.b[k][2],
+                                                                      U + ahead.node[k] * 6)
+                                                : RowPair{0.0f, 0.0f};
+                    });
+                    fetch(shape.first, t + kStepsAhead, streamed);
+                }
+                const int* const node = listed_at + i_node;
+                const int end = shape.degree - shape.streamed;
+                for (int t = 0; t < end; t += kStepsAhead)
+                    add_steps(t, end, [&](int k) {
+                        const int tk = min(t + k, end - 1);  // past the end: the last one again, not added
+                        return row_pair_dot<false>(cached_at[tk * kStepFloat4s], cached_at[tk * kStepFloat4s + 24],
+                                                   cached_at[tk * kStepFloat4s + 48], U + node[tk * kOctet] * 6);
+                    });
             }
             const int first_row = (o * kOctet - n0) * 6;
             if (on) *reinterpret_cast<float2*>(Wv + first_row + 2 * lane) = make_float2(y.a, y.b);
@@ -1314,7 +1429,7 @@ __device__ __forceinline__ void pcg_solve(const WrapDev& w, const WrapControl& c
                 const int k = first_row + h * 24 + lane;
                 double ui = 0.0, ri = 0.0, wi = 0.0;
                 if (lane < 24 && k < rows) {
-                    ui = (double)U[n0 * 6 + k];
+                    ui = (double)own_u[k];
                     ri = R[k];
                     wi = (double)Wv[k];
                 }
@@ -1324,27 +1439,36 @@ __device__ __forceinline__ void pcg_solve(const WrapDev& w, const WrapControl& c
             }
             int held = 0, count = 6;
             warp_sum_halving<6, 16>(v, lane, held, count, [](double x, double z) { return rnd(x + z); });
-            double partial[6];
+            if constexpr (kGrid) {
+                const int third = (lane >> 2) & 3;  // lanes 0, 4, 8, 16, 20, 24 hold sums 0 .. 5
+                if ((lane & 3) == 0 && third < 3) __stcg(slots + 6 * o + (lane >> 4) * 3 + third, v[0]);
+            } else {
+                double partial[6];
 #pragma unroll
-            for (int k = 0; k < 6; ++k)
-                partial[k] = __shfl_sync(0xffffffffu, v[0], (k >= 3 ? 16 : 0) + (k % 3) * 4);
-            if (active == 1) {
-                if (lane == 0)
-                    for (int k = 0; k < 6; ++k) slots[6 * o + k] = partial[k];
-            } else if (lane < active) {  // lane q stores the partials in CTA q's slots
-                const uint32_t dst = peer_slots + 48 * o;
-                store_to_peer(dst, partial[0], partial[1], peer_sums_arrived);
-                store_to_peer(dst + 16, partial[2], partial[3], peer_sums_arrived);
-                store_to_peer(dst + 32, partial[4], partial[5], peer_sums_arrived);
+                for (int k = 0; k < 6; ++k)
+                    partial[k] = __shfl_sync(0xffffffffu, v[0], (k >= 3 ? 16 : 0) + (k % 3) * 4);
+                if (active == 1) {
+                    if (lane == 0)
+                        for (int k = 0; k < 6; ++k) slots[6 * o + k] = partial[k];
+                } else if (lane < active) {  // lane q stores the partials in CTA q's slots
+                    const uint32_t dst = peer_slots + 48 * o;
+                    store_to_peer(dst, partial[0], partial[1], peer_sums_arrived);
+                    store_to_peer(dst + 16, partial[2], partial[3], peer_sums_arrived);
+                    store_to_peer(dst + 32, partial[4], partial[5], peer_sums_arrived);
+                }
             }
         }
-        __syncwarp();
-        if (threadIdx.x == 0) {
-            mbar_arrive_expect(&sums_arrived, active > 1 ? 48 * octets : 0);
-        } else if (lane == 0) {
-            mbar_arrive(&sums_arrived);
+        if (kGrid) {
+            meet();
+        } else {
+            __syncwarp();
+            if (threadIdx.x == 0) {
+                mbar_arrive_expect(&sums_arrived, active > 1 ? 48 * octets : 0);
+            } else if (lane == 0) {
+                mbar_arrive(&sums_arrived);
+            }
+            if (!mbar_wait(&sums_arrived, it & 1)) timed_out = true;
         }
-        if (!mbar_wait(&sums_arrived, it & 1)) timed_out = true;
         // ---- totals over every segment, in one fixed order in every CTA:
         //      each warp its stride of the segments, then every warp the same
         //      butterfly over the warps' sums ----
@@ -1352,8 +1476,10 @@ __device__ __forceinline__ void pcg_solve(const WrapDev& w, const WrapControl& c
         {
             double v[3] = {0.0, 0.0, 0.0};
             if (warp * 32 < segs) {
-                for (int sg = threadIdx.x; sg < segs; sg += blockDim.x)
-                    for (int k = 0; k < 3; ++k) v[k] = rnd(v[k] + slots[3 * sg + k]);
+#pragma unroll 4
+                for (int sg = threadIdx.x; sg < segs; sg += kPcgThreads)
+                    for (int k = 0; k < 3; ++k)
+                        v[k] = rnd(v[k] + (kGrid ? __ldcg(slots + 3 * sg + k) : slots[3 * sg + k]));
                 int held = 0, count = 3;
                 warp_sum_halving<3, 16>(v, lane, held, count, [](double x, double z) { return rnd(x + z); });
             }
@@ -1400,7 +1526,7 @@ __device__ __forceinline__ void pcg_solve(const WrapDev& w, const WrapControl& c
         alpha_prev = alpha;
         // ---- p, s, x, r for the owned rows; then u = M^-1 r, shared ----
         segment_rows([&](int i) {
-            const float pn = (float)((double)U[n0 * 6 + i] + rnd(beta * (double)P[i]));
+            const float pn = (float)((double)own_u[i] + rnd(beta * (double)P[i]));
             const float sn = (float)((double)Wv[i] + rnd(beta * (double)S[i]));
             P[i] = pn;
             S[i] = sn;
@@ -1439,23 +1565,62 @@ __device__ __forceinline__ void pcg_solve(const WrapDev& w, const WrapControl& c
         }
     }
     // no CTA may exit while another can still write into its shared memory
-    cluster.sync();
+    if (!kGrid) {
+        cluster.sync();
+    } else {
+        __syncthreads();
+        if (threadIdx.x == 0)  // initialised again for the block's next wrap
+            for (void* bar : {(void*)&blocks_arrived, (void*)&sums_arrived, (void*)&u_arrived}) mbar_invalidate(bar);
+    }
 }
 
-__global__ void __launch_bounds__(kPcgThreads) k_pcg(const WrapDev* __restrict__ wraps,
+// Whether the grid kernel takes a wrap's solve this tick (both kernels ask):
+// its graph has more than `grid_nodes` nodes for every wrap that the grid would
+// take one after the other, and no smaller solve needs SMs at the same time.
+__device__ inline bool grid_takes(const WrapDev* wraps, int wrap_count, int nodes, int grid_nodes) {
+    if (grid_nodes <= 0 || nodes <= grid_nodes) return false;
+    int solving = 0, large = 0;
+    for (int i = 0; i < wrap_count; ++i) {
+        const WrapControl* c = wraps[i].control;
+        if (c->tick_phase != kPhaseSolve || c->phase != kPhaseSolve) continue;
+        ++solving;
+        large += wraps[i].levels[c->level].node_count > grid_nodes ? 1 : 0;
+    }
+    return solving == large && nodes > grid_nodes * large;
+}
+
+// The wraps the grid takes, one after the other over the whole device.
+__global__ void __launch_bounds__(kPcgThreads, 1) k_pcg_grid(const WrapDev* __restrict__ wraps, int wrap_count,
+                                                          int grid_nodes, int budget_floats) {
+    for (int i = 0; i < wrap_count; ++i) {
+        const WrapDev& w = wraps[i];
+        const WrapControl c = *w.control;
+        if (c.tick_phase != kPhaseSolve || c.phase != kPhaseSolve) continue;
+        const int N = w.levels[c.level].node_count;
+        if (!grid_takes(wraps, wrap_count, N, grid_nodes)) continue;
+        PcgPlacement place = {};
+        place.floats = pcg_owned_capacity(N, (int)gridDim.x) * (6 + kPcgVectorFloats + 2 * kPcgBlockFloats) +
+                       kPcgWarps * kGatherSteps * 64;
+        pcg_solve<true, true>(w, c, place, budget_floats);
+        __syncthreads();  // shared memory of one wrap before the next
+    }
+}
+
+__global__ void __launch_bounds__(kPcgThreads, 1) k_pcg(const WrapDev* __restrict__ wraps,
                                                      const int* __restrict__ index,
-                                                     int budget_floats) {
+                                                     int budget_floats, int wrap_count, int grid_nodes) {
     const int slot = index ? index[blockIdx.y] : (int)blockIdx.y;
     if (slot < 0) return;  // an empty entry of a class launch; uniform across the cluster
     const WrapDev& w = wraps[slot];
     const WrapControl c = *w.control;
     if (c.tick_phase != kPhaseSolve || c.phase != kPhaseSolve) return;  // uniform across the cluster
+    if (grid_takes(wraps, wrap_count, w.levels[c.level].node_count, grid_nodes)) return;
     const PcgPlacement place =
         pcg_place(w.levels[c.level].node_count, (int)cg::this_cluster().num_blocks(), budget_floats);
     if (place.all()) {
-        pcg_solve<true>(w, c, place, budget_floats);
+        pcg_solve<true, false>(w, c, place, budget_floats);
     } else {
-        pcg_solve<false>(w, c, place, budget_floats);
+        pcg_solve<false, false>(w, c, place, budget_floats);
     }
 }
 
@@ -2233,8 +2398,21 @@ void launch_tick(const WrapDev* wraps, const TickShape& s, cudaStream_t stream,
         attribute[0].val.clusterDim.z = 1;
         config.attrs = attribute;
         config.numAttrs = 1;
-        cudaLaunchKernelEx(&config, k_pcg, wraps, index, kPcgMaxSmemBytes / (int)sizeof(float));
+        cudaLaunchKernelEx(&config, k_pcg, wraps, index, kPcgMaxSmemBytes / (int)sizeof(float), W, s.grid_nodes);
     };
+    if (s.grid_nodes > 0) {
+        cudaLaunchConfig_t config = {};
+        config.gridDim = dim3(s.grid_ctas);
+        config.blockDim = dim3(kPcgThreads);
+        config.dynamicSmemBytes = kPcgMaxSmemBytes;
+        config.stream = stream;
+        cudaLaunchAttribute attribute[1];
+        attribute[0].id = cudaLaunchAttributeCooperative;
+        attribute[0].val.cooperative = 1;
+        config.attrs = attribute;
+        config.numAttrs = 1;
+        cudaLaunchKernelEx(&config, k_pcg_grid, wraps, W, s.grid_nodes, kPcgMaxSmemBytes / (int)sizeof(float));
+    }
     if (s.pcg_groups <= 0) {
         launch_pcg(s.pcg_cluster, W, nullptr, stream);
     } else {
@@ -2270,7 +2448,7 @@ int tick_kernel_launches(const TickShape& s, bool timed) {
     // stats twice, [fit, rhs,] solve launches, prologue, evaluate, normals,
     // query, residual, assembly, decision; an untimed tick with a side stream
     // runs the last three in each branch
-    return 9 + (s.route_c ? 2 : 0) + (s.pcg_groups > 0 ? s.pcg_groups : 1) + (s.side_stream && !timed ? 3 : 0);
+    return 9 + (s.route_c ? 2 : 0) + (s.grid_nodes > 0 ? 1 : 0) + (s.pcg_groups > 0 ? s.pcg_groups : 1) + (s.side_stream && !timed ? 3 : 0);
 }
 
 // Cluster size of the solve for one wrap of `nodes` nodes on its own: a
@@ -2286,6 +2464,7 @@ void pcg_enable() {
     static const bool enabled = [] {  // once per process, thread-safe
         cudaFuncSetAttribute(k_pcg, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
         cudaFuncSetAttribute(k_pcg, cudaFuncAttributeMaxDynamicSharedMemorySize, kPcgMaxSmemBytes);
+        cudaFuncSetAttribute(k_pcg_grid, cudaFuncAttributeMaxDynamicSharedMemorySize, kPcgMaxSmemBytes);
         return true;
     }();
     (void)enabled;
@@ -2299,6 +2478,33 @@ int pcg_cluster_size(int max_nodes, int wraps, int sm_count) {
     int ranks = pcg_latency_cluster(max_nodes);
     while (ranks > 1 && (long)ranks * wraps > sm_count) ranks /= 2;
     return ranks;
+}
+
+// Graphs above this many nodes (per wrap the grid takes) are solved by the
+// whole device.  An iteration of a 16-CTA cluster grows with the rows per CTA,
+// the grid's is mostly its two meetings: 6.9 against 9.9 us at 1,000 nodes with
+// 6 bindings, 10.2 against 10.3 at 2,000; with 8 bindings 8.7 against 10.8 at
+// 1,250, 16 against 12.5 at 2,500, 34 against 14 at 5,000, 73 against 18 at
+// 10,000.
+constexpr int kGridNodes = 2000;
+// Wraps a tick may hold with the grid solve among its launches: it is of use to
+// few large wraps only, and a launch without work costs each tick 3 us.
+constexpr int kGridWraps = 8;
+void grid_solve_shape(TickShape& shape) {
+    shape.grid_nodes = shape.max_nodes > kGridNodes && shape.wraps <= kGridWraps ? kGridNodes : 0;
+    shape.grid_ctas = 0;
+    if (!shape.grid_nodes) return;
+    pcg_enable();
+    int device = 0, sms = 0, cooperative = 0, per_sm = 0;
+    cudaGetDevice(&device);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
+    cudaDeviceGetAttribute(&cooperative, cudaDevAttrCooperativeLaunch, device);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_pcg_grid, kPcgThreads, kPcgMaxSmemBytes);
+    if (!cooperative || per_sm < 1) {
+        shape.grid_nodes = 0;
+        return;
+    }
+    shape.grid_ctas = sms;
 }
 
 int pcg_max_nodes() { return 32768; }

@@ -1,8 +1,8 @@
 """The linear solve at the edges of its partition (nricp_b200/csrc/
 wrap_kernels.cu, `pcg_solve`): octets of eight nodes that are full, one short
 and one over, CTAs without rows, blocks that fit in shared memory and blocks
-that are streamed, and graphs whose vectors do not fit.  Every cluster size
-gives the same bits, and the increment satisfies the damped system that the
+that are streamed, and graphs whose vectors do not fit, solved by a cluster
+and by the whole device.  Every one of these gives the same bits, and the increment satisfies the damped system that the
 device assembled to the bar of test_gpu_solve_stats.
 """
 
@@ -39,6 +39,11 @@ def test_solves_at_every_partition_edge(dp, device, nodes):
             reference = got
         assert np.array_equal(reference["vertices"], got["vertices"]), cluster
         assert np.array_equal(reference["rotations"], got["rotations"]), cluster
+    if nodes > 2_000:  # alone a large graph is the whole device's, among equals a cluster's
+        many = dp.WrapBatch([(*case.args(), case.options)] * (nodes // 2_000 + 1))
+        many.run()
+        assert np.array_equal(reference["vertices"], many.result(0)["vertices"])
+        assert np.array_equal(reference["rotations"], many.result(0)["rotations"])
     session = dp.RouteBSession(*case.args(), **case.options)
     checked = 0
     while not session.finished() and checked < 2:
