@@ -1273,16 +1273,19 @@ __device__ __forceinline__ void pcg_solve(const WrapDev& w, const WrapControl& c
     // A few streamed steps of octet o (its first `streamed`) into registers.
     const int i_node = lane / 3, p_row = lane - i_node * 3;
     StepBlocks ahead;
+    // Past the end they are zeros: values left over from an earlier fetch would
+    // hold their registers through the whole iteration.
     auto fetch = [&](int first, int t, int end) {
 #pragma unroll
-        for (int k = 0; k < kStepsAhead; ++k)
-            if (t + k < end) {
-                const float4* at = B + (long)(first + t + k) * kStepFloat4s + lane;
-                if (!kGrid) ahead.node[k] = __ldg(sell_nodes + (long)(first + t + k) * kOctet + i_node);
-                ahead.b[k][0] = __ldg(at);
-                ahead.b[k][1] = __ldg(at + 24);
-                ahead.b[k][2] = __ldg(at + 48);
-            }
+        for (int k = 0; k < kStepsAhead; ++k) {
+            const bool there = t + k < end;
+            const float4* at = B + (long)(first + t + k) * kStepFloat4s + lane;
+            const float4 zero = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+            if (!kGrid) ahead.node[k] = there ? __ldg(sell_nodes + (long)(first + t + k) * kOctet + i_node) : 0;
+            ahead.b[k][0] = there ? __ldg(at) : zero;
+            ahead.b[k][1] = there ? __ldg(at + 24) : zero;
+            ahead.b[k][2] = there ? __ldg(at + 48) : zero;
+        }
     };
     struct OctetShape { int first, steps, streamed, degree; };
     auto octet_shape = [&](int o) {
@@ -1403,20 +1406,36 @@ __device__ __forceinline__ void pcg_solve(const WrapDev& w, const WrapControl& c
                 const int streamed = min(shape.streamed, shape.degree);
                 for (int t = 0; t < streamed; t += kStepsAhead) {
                     add_steps(t, streamed, [&](int k) {
-                        return t + k < streamed ? row_pair_dot<false>(ahead.b[k][0], ahead.b[k][1], ahead.b[k][2],
-                                                                      U + ahead.node[k] * 6)
-                                                : RowPair{0.0f, 0.0f};
+                        return row_pair_dot<false>(ahead.b[k][0], ahead.b[k][1], ahead.b[k][2],
+                                                   U + ahead.node[k] * 6);
                     });
                     fetch(shape.first, t + kStepsAhead, streamed);
                 }
                 const int* const node = listed_at + i_node;
                 const int end = shape.degree - shape.streamed;
-                for (int t = 0; t < end; t += kStepsAhead)
+                for (int t = 0; t < end; t += kStepsAhead) {
+                    // every load of the group before its first product
+                    int at[kStepsAhead], other[kStepsAhead];
+#pragma unroll
+                    for (int k = 0; k < kStepsAhead; ++k) at[k] = min(t + k, end - 1);  // past the end: not added
+#pragma unroll
+                    for (int k = 0; k < kStepsAhead; ++k) other[k] = node[at[k] * kOctet] * 6;
+                    float4 b[kStepsAhead][3];
+                    float2 u[kStepsAhead][3];
+#pragma unroll
+                    for (int k = 0; k < kStepsAhead; ++k)
+#pragma unroll
+                        for (int j = 0; j < 3; ++j) {
+                            b[k][j] = cached_at[at[k] * kStepFloat4s + 24 * j];
+                            u[k][j] = reinterpret_cast<const float2*>(U + other[k])[j];
+                        }
                     add_steps(t, end, [&](int k) {
-                        const int tk = min(t + k, end - 1);  // past the end: the last one again, not added
-                        return row_pair_dot<false>(cached_at[tk * kStepFloat4s], cached_at[tk * kStepFloat4s + 24],
-                                                   cached_at[tk * kStepFloat4s + 48], U + node[tk * kOctet] * 6);
+                        return RowPair{row_dot<false>(b[k][0].x, b[k][0].y, b[k][0].z, b[k][0].w, b[k][1].x, b[k][1].y,
+                                                      u[k][0], u[k][1], u[k][2]),
+                                       row_dot<false>(b[k][1].z, b[k][1].w, b[k][2].x, b[k][2].y, b[k][2].z, b[k][2].w,
+                                                      u[k][0], u[k][1], u[k][2])};
                     });
+                }
             }
             const int first_row = (o * kOctet - n0) * 6;
             if (on) *reinterpret_cast<float2*>(Wv + first_row + 2 * lane) = make_float2(y.a, y.b);
