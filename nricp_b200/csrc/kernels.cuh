@@ -86,6 +86,10 @@ int pcg_cluster_size(int max_nodes, int wraps, int sm_count);
 // Sets the shape's grid solve from its wraps and max_nodes.
 void grid_solve_shape(TickShape& shape);
 int pcg_max_nodes();
+// The vertices of `wrap` (device descriptor) under state buffer `buffer` of a
+// level, in the caller's units, into `out` (device, vertices x 3).
+void launch_caller_vertices(const WrapDev* wrap, int vertices, int level, int buffer, const double center[3],
+                            double scale, double* out, cudaStream_t stream);
 // The weighted rigid fit of n point pairs (device arrays); out = R (row-major
 // 3x3), t.
 void launch_fit_rigid(const double* src, const double* dst, const double* weights, int n, double* out,

@@ -1165,12 +1165,15 @@ WrapDownload download_result(const Wrap& w, const WrapControl& c, cudaStream_t s
 
 // Result of one wrap in the caller's units (route_result_to_dict,
 // src/python/bindings.cpp:674-710), from its downloaded state; host only.
-void compose_result(const Wrap& w, const WrapDownload& d, NricpResult* out) {
+// The vertices are evaluated here unless `vertices_done`.
+void compose_result(const Wrap& w, const WrapDownload& d, NricpResult* out, bool vertices_done = false) {
     const WrapControl& c = d.control;
     const int level = std::min(c.level, w.levels - 1);
     const int N = w.layouts[level].node_count;
-    const std::vector<double> vertices = evaluate_host(w, d.rot, d.trans, level);
-    if (out->vertices) std::memcpy(out->vertices, vertices.data(), sizeof(double) * vertices.size());
+    if (out->vertices && !vertices_done) {
+        const std::vector<double> vertices = evaluate_host(w, d.rot, d.trans, level);
+        std::memcpy(out->vertices, vertices.data(), sizeof(double) * vertices.size());
+    }
     if (out->rotations) std::memcpy(out->rotations, d.rot.data(), sizeof(double) * d.rot.size());
     if (out->translations) std::memcpy(out->translations, d.trans.data(), sizeof(double) * d.trans.size());
     if (out->node_positions)
@@ -1200,36 +1203,30 @@ void compose_result(const Wrap& w, const WrapDownload& d, NricpResult* out) {
     }
 }
 
-void write_result(const Wrap& w, const WrapControl& c, cudaStream_t stream, NricpResult* out) {
-    compose_result(w, download_result(w, c, stream), out);
-}
-
 }  // namespace
 
-void Batch::result(int i, NricpResult* out) { write_result(*wraps_[i], host_controls_[i], stream_, out); }
+// Wrap i's vertices under state buffer `buffer` of `level` into host memory,
+// evaluated on the device.  Between ticks the template normals' array is free:
+// every query writes it anew.
+void Batch::download_vertices(int i, int level, int buffer, double* out) {
+    const Wrap& w = *wraps_[i];
+    launch_caller_vertices(dev_wraps_ + i, w.V, level, buffer, w.graph.center, w.graph.scale, w.dev.qnormals, stream_);
+    check(cudaGetLastError(), "vertices");
+    check(cudaMemcpyAsync(out, w.dev.qnormals, sizeof(double) * 3 * w.V, cudaMemcpyDeviceToHost, stream_),
+          "download vertices");
+    g_transfers.d2h += sizeof(double) * 3 * w.V;
+}
+
+void Batch::result(int i, NricpResult* out) {
+    const Wrap& w = *wraps_[i];
+    const WrapControl& c = host_controls_[i];
+    if (out->vertices) download_vertices(i, std::min(c.level, w.levels - 1), c.state, out->vertices);
+    compose_result(w, download_result(w, c, stream_), out, true);
+}
 
 void Batch::results(NricpResult* outs) {
     const int W = static_cast<int>(wraps_.size());
-    std::vector<WrapDownload> downloads;
-    downloads.reserve(W);
-    for (int i = 0; i < W; ++i) downloads.push_back(download_result(*wraps_[i], host_controls_[i], stream_));
-    // vertices in FP64 and the reports, on the host's cores
-    std::vector<std::string> failure(W);
-#pragma omp parallel for schedule(dynamic, 1) if (W > 1)
-    for (int i = 0; i < W; ++i) {
-        try {
-            compose_result(*wraps_[i], downloads[i], &outs[i]);
-        } catch (const std::exception& e) {
-            failure[i] = e.what();
-        }
-    }
-    for (int i = 0; i < W; ++i)
-        if (!failure[i].empty()) throw std::runtime_error(failure[i]);
-}
-
-std::vector<double> Batch::evaluate_host(int i, const std::vector<double>& rot,
-                                         const std::vector<double>& trans, int level) const {
-    return nricp_b200::evaluate_host(*wraps_[i], rot, trans, level);
+    for (int i = 0; i < W; ++i) result(i, &outs[i]);
 }
 
 int Batch::finest_nodes(int i) const { return wraps_[i]->layouts.back().node_count; }
@@ -1239,19 +1236,10 @@ int Batch::vertices(int i) const { return wraps_[i]->V; }
 void Batch::current_vertices(int i, double* out) {
     pull_controls();
     const WrapControl& c = host_controls_[i];
-    Wrap& w = *wraps_[i];
-    const int level = std::min(c.level, w.levels - 1);
+    const int level = std::min(c.level, wraps_[i]->levels - 1);
     // a level whose warm start has not run yet still holds the previous one
-    const int shown = c.phase == kPhaseTransfer ? level - 1 : level;
-    const int N = w.layouts[shown].node_count;
-    std::vector<double> rot(static_cast<size_t>(N) * 9), trans(static_cast<size_t>(N) * 3);
-    check(cudaMemcpyAsync(rot.data(), w.dev.rot[c.state], sizeof(double) * rot.size(),
-                          cudaMemcpyDeviceToHost, stream_), "download rot");
-    check(cudaMemcpyAsync(trans.data(), w.dev.trans[c.state], sizeof(double) * trans.size(),
-                          cudaMemcpyDeviceToHost, stream_), "download trans");
+    download_vertices(i, c.phase == kPhaseTransfer ? level - 1 : level, c.state, out);
     check(cudaStreamSynchronize(stream_), "download");
-    const std::vector<double> v = evaluate_host(i, rot, trans, shown);
-    std::memcpy(out, v.data(), sizeof(double) * v.size());
 }
 
 const WrapDev* Batch::device_wrap(int i) const { return dev_wraps_ + i; }

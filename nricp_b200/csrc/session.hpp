@@ -95,8 +95,7 @@ public:
     const WrapDev* device_wrap(int i) const;
 
 private:
-    std::vector<double> evaluate_host(int i, const std::vector<double>& rot,
-                                      const std::vector<double>& trans, int level) const;
+    void download_vertices(int i, int level, int buffer, double* out);
 
     std::vector<std::unique_ptr<Wrap>> wraps_;
     StreamLease stream_;

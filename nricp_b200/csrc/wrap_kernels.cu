@@ -2528,6 +2528,37 @@ void grid_solve_shape(TickShape& shape) {
 
 int pcg_max_nodes() { return 32768; }
 
+// A wrap's template vertices under a state, in the caller's units
+// (mesh.cpp:189-193): the operations of the host's evaluation, each rounded on
+// its own, so the bits are the host's.  (The host took 2 ms for 25,000 vertices
+// on one core, and as long again at every step a session redraws.)
+__global__ void __launch_bounds__(kVertexThreads) k_caller_vertices(const WrapDev* __restrict__ wrap, int level,
+                                                                    int buffer, double cx, double cy, double cz,
+                                                                    double scale, double* __restrict__ out) {
+    const WrapDev& w = *wrap;
+    const int v = blockIdx.x * kVertexThreads + threadIdx.x;
+    if (v >= w.V) return;
+    const LevelDev& L = w.levels[level];
+    const double* R = w.rot[buffer];
+    const double* T = w.trans[buffer];
+    const D3 p = load_d3(w.tpl, v);
+    D3 sum = {0.0, 0.0, 0.0};
+    const int count = L.bind_counts[v];
+    for (int s = 0; s < count; ++s) {
+        const int j = L.bind_nodes[v * kMaxSlots + s];
+        const D3 g = load_d3(L.rest, j);
+        const D3 applied = radd(radd(rmat(R + j * 9, rsub(p, g)), g), load_d3(T, j));
+        sum = radd(sum, rmul(applied, L.bind_weights[v * kMaxSlots + s]));
+    }
+    store_d3(out, v, {da(__ddiv_rn(sum.x, scale), cx), da(__ddiv_rn(sum.y, scale), cy), da(__ddiv_rn(sum.z, scale), cz)});
+}
+
+void launch_caller_vertices(const WrapDev* wrap, int vertices, int level, int buffer, const double center[3],
+                            double scale, double* out, cudaStream_t stream) {
+    k_caller_vertices<<<(vertices + kVertexThreads - 1) / kVertexThreads, kVertexThreads, 0, stream>>>(
+        wrap, level, buffer, center[0], center[1], center[2], scale, out);
+}
+
 void launch_fit_rigid(const double* src, const double* dst, const double* weights, int n, double* out,
                       cudaStream_t stream) {
     k_fit_rigid<<<1, kRigidThreads, 0, stream>>>(src, dst, weights, n, out);
