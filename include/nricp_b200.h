@@ -254,7 +254,7 @@ int nricp_batch_step(NricpBatch* batch, double* device_ms);
  * 0 gives each wrap its own size (about 128 nodes per CTA), one launch per
  * size class, the classes running side by side; -s (s = 1..4) halves those
  * per-wrap sizes s times.  A new batch starts at the smallest s whose classes
- * need at most three CTAs per SM.  Every choice gives bit-identical results;
+ * need at most three CTAs per SM (unhalved if they fit one per SM).  Every choice gives bit-identical results;
  * it trades one wrap's latency against the batch's throughput.
  * *cluster_out (may be NULL) receives the largest size in effect. */
 int nricp_batch_tune(NricpBatch* batch, int pcg_cluster, int* cluster_out);
@@ -297,7 +297,7 @@ typedef struct NricpServerConfig {
     int prep_threads;            /* host threads preparing requests; 0: half the cores */
     int pcg_cluster;             /* solve cluster: > 0 one size (a power of two up to 16) for every
                                     slot; 0 (the default) per-wrap latency classes, halved once
-                                    when the running wraps would need more than three CTAs per
+                                    when the running wraps would need more than one CTA per
                                     SM; -s (1..4) latency classes always halved s times */
     int ticks_per_poll;          /* ticks launched between looks at the wraps' progress */
     int large_face_threshold;    /* requests whose target has at least this many triangles run

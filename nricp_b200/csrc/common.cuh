@@ -177,8 +177,8 @@ struct WrapDev {
     uint8_t* long_flag;           // 2 x V
     uint8_t* corr_code;           // V rejection code
     double* robust;               // V
-    float4* residual32;           // V: (o.x, o.y, o.z, plane value scale) per vertex
-    float4* resid_aux32;          // V: (n.x, n.y, n.z, p2p scale)
+    float4* residual32;           // V: (offset xyz, point weight)
+    float4* resid_aux32;          // V: (normal xyz, plane weight)
     float4* lm_resid32;           // V: landmark offset (xyz), w
     float4* offsets32;            // V x kMaxSlots: each binding's node-local offset R (p - g), FP32,
                                   // and its FP32 weight, for the tick's assembly

@@ -838,11 +838,11 @@ bool Batch::all_done() const {
     return true;
 }
 
-// Per-wrap latency classes, halved until every class launch together needs
-// at most three CTAs per SM (-s for nricp_batch_tune).  On the 64 uneven
-// wraps of the benchmark that is one halving: the classes' CTAs then run in
-// under three rounds of the SMs, while a second halving lengthens every
-// solve iteration more than it saves.
+// Per-wrap latency classes while their CTAs fit on the SMs at once; else
+// halved until they need at most three per SM (-s for nricp_batch_tune).
+// Uneven wraps of the benchmark's sizes, ms per step unhalved / halved / halved
+// twice: 8 wraps (88 CTAs) 77.7 / 77.7 / 91.4, 16 (180) 133 / 127 / 150, 32
+// (360) 228 / 217 / 248, 64 (728) 434 / 403 / 447.
 int Batch::default_pcg_cluster() const {
     int device = 0, sms = 148;
     check(cudaGetDevice(&device), "device");
@@ -850,7 +850,7 @@ int Batch::default_pcg_cluster() const {
     for (int shift = 0; shift < 4; ++shift) {
         long ctas = 0;
         for (const auto& w : wraps_) ctas += std::max(1, pcg_latency_cluster(w->max_nodes) >> shift);
-        if (ctas <= 3L * sms) return -shift;
+        if (ctas <= (shift == 0 ? 1L : 3L) * sms) return -shift;
     }
     return -4;
 }
@@ -1573,13 +1573,13 @@ struct Server::Impl {
 
     // A wrap's class is its latency cluster halved `shift` times: a fixed
     // shift (pcg_cluster < 0), or by load (0) -- none while the running
-    // wraps' latency clusters fit three CTAs per SM, else one.
+    // wraps' latency clusters fit one CTA per SM, else one.
     int max_shift() const { return cfg.pcg_cluster < 0 ? -cfg.pcg_cluster : 1; }
     int shift_for(int count) const {
         if (cfg.pcg_cluster < 0) return -cfg.pcg_cluster;
         long ctas = 0;
         for (int i = 0; i < count; ++i) ctas += pcg_latency_cluster(slot_nodes[i]);
-        return ctas <= 3L * sms ? 0 : 1;
+        return ctas <= sms ? 0 : 1;
     }
     static int class_of(int nodes, int shift) { return std::max(1, pcg_latency_cluster(nodes) >> shift); }
     // Rewrites the class rows for the running wraps in slots 0 .. count-1
