@@ -1898,13 +1898,59 @@ __device__ __forceinline__ NodeEntry load_entry(const WrapDev& w, int entry, boo
     return x;
 }
 
+// One incident smoothness edge as a node sees it: its energy is stored if the
+// node is its first (the decision kernel sums them), and what the block and the
+// right-hand side need of it is returned.
+struct EdgeTerms {
+    F3 difference, arm;
+    int role;  // 0 none, 1 the edge's first node, 2 its second
+};
+__device__ __forceinline__ EdgeTerms edge_terms(const WrapDev& w, const WrapControl& c, const LevelDev& L, int e,
+                                                int a, int b, int node, bool build) {
+    EdgeTerms t;
+    t.role = 0;
+    t.difference = t.arm = F3{0.0f, 0.0f, 0.0f};
+    const double weight = w.weights[c.level][2];
+    double energy = 0.0;
+    if (weight > 0.0) {
+        const int buf = eval_buffer(c);
+        const double* R = w.rot[buf];
+        const double* T = w.trans[buf];
+        const D3 ga = load_d3(L.rest, a), gb = load_d3(L.rest, b);
+        const D3 gd = rsub(gb, ga);
+        const D3 field_a = radd(radd(rmat(R + a * 9, gd), ga), load_d3(T, a));
+        const D3 field_b = radd(gb, load_d3(T, b));
+        const D3 diff = rsub(field_a, field_b);
+        const D3 scaled = rmul(diff, sqrt(weight));
+        energy = da(da(dm(scaled.x, scaled.x), dm(scaled.y, scaled.y)), dm(scaled.z, scaled.z));
+        if (build) {
+            t.difference = F3{(float)diff.x, (float)diff.y, (float)diff.z};
+            t.role = 2;
+            if (a == node) {
+                t.role = 1;
+                t.arm = mul3f(w.rot32 + a * 9, {(float)gd.x, (float)gd.y, (float)gd.z});
+            }
+        }
+    }
+    if (a == node) w.edge_partials[e] = energy;
+    return t;
+}
+
+// What the node's loop over its bindings has nothing to do with is loaded ahead
+// of it: the lane's first edge (few nodes have more than 32) is reduced to six
+// numbers while the first binding's data are on their way, so that the chain
+// list -> edge -> positions and rotations does not follow the loop's own.
 __device__ __forceinline__ void assemble_node(const WrapDev& w, const WrapControl& c, int node) {
     const bool build = assembles(c);
     const LevelDev& L = w.levels[c.level];
     const int lane = threadIdx.x & 31;
     const double* wt = w.weights[c.level];
-    const int buf = eval_buffer(c);
     const int next = 1 - c.system;
+    const int edge_first = L.node_edge_begin[node] + lane, edge_end = L.node_edge_begin[node + 1];
+    const int edge = edge_first < edge_end ? L.node_edge_list[edge_first] : -1;
+    EdgeTerms near;
+    near.role = 0;
+    near.difference = near.arm = F3{0.0f, 0.0f, 0.0f};
     float d[21], g[6];
     for (int i = 0; i < 21; ++i) d[i] = 0.0f;
     for (int i = 0; i < 6; ++i) g[i] = 0.0f;
@@ -1914,7 +1960,10 @@ __device__ __forceinline__ void assemble_node(const WrapDev& w, const WrapContro
         int i = L.gather_begin[node] + lane;
         int after = i + 32 < end ? L.gather_entry[i + 32] : 0;
         NodeEntry ahead;
-        if (i < end) ahead = load_entry(w, L.gather_entry[i], landmarks);
+        const int entry = i < end ? L.gather_entry[i] : 0;
+        const int ea = edge >= 0 ? L.edges[edge * 2] : 0, eb = edge >= 0 ? L.edges[edge * 2 + 1] : 0;
+        if (i < end) ahead = load_entry(w, entry, landmarks);
+        if (edge >= 0) near = edge_terms(w, c, L, edge, ea, eb, node, true);
         for (; i < end; i += 32) {
             const NodeEntry x = ahead;
             if (i + 32 < end) ahead = load_entry(w, after, landmarks);
@@ -1947,40 +1996,28 @@ __device__ __forceinline__ void assemble_node(const WrapDev& w, const WrapContro
                 g[3] -= s * o.x; g[4] -= s * o.y; g[5] -= s * o.z;
             }
         }
+    } else if (edge >= 0) {
+        edge_terms(w, c, L, edge, L.edges[edge * 2], L.edges[edge * 2 + 1], node, false);
     }
-    // the incident smoothness edges; each edge's energy is its first node's
-    // to store (the decision kernel sums them)
+    // the incident smoothness edges
     const float ws = (float)wt[2];
-    const double sc = sqrt(wt[2]);
-    const double* R = w.rot[buf];
-    const double* T = w.trans[buf];
-    for (int i = L.node_edge_begin[node] + lane; i < L.node_edge_begin[node + 1]; i += 32) {
-        const int e = L.node_edge_list[i];
-        const int a = L.edges[e * 2], b = L.edges[e * 2 + 1];
-        double energy = 0.0;
-        if (wt[2] > 0.0) {
-            const D3 ga = load_d3(L.rest, a), gb = load_d3(L.rest, b);
-            const D3 gd = rsub(gb, ga);
-            const D3 field_a = radd(radd(rmat(R + a * 9, gd), ga), load_d3(T, a));
-            const D3 field_b = radd(gb, load_d3(T, b));
-            const D3 diff = rsub(field_a, field_b);
-            const D3 scaled = rmul(diff, sc);
-            energy = da(da(dm(scaled.x, scaled.x), dm(scaled.y, scaled.y)), dm(scaled.z, scaled.z));
-            if (build) {
-                const F3 dv = {(float)diff.x, (float)diff.y, (float)diff.z};
-                if (a == node) {
-                    const F3 cv = mul3f(w.rot32 + a * 9, {(float)gd.x, (float)gd.y, (float)gd.z});
-                    add_offset_block(d, cv, ws);
-                    const F3 cd = cross(cv, dv);
-                    g[0] -= ws * cd.x; g[1] -= ws * cd.y; g[2] -= ws * cd.z;
-                    g[3] -= ws * dv.x; g[4] -= ws * dv.y; g[5] -= ws * dv.z;
-                } else {
-                    d[tri_index(3, 3)] += ws; d[tri_index(4, 4)] += ws; d[tri_index(5, 5)] += ws;
-                    g[3] += ws * dv.x; g[4] += ws * dv.y; g[5] += ws * dv.z;
-                }
-            }
+    auto add_edge = [&](const EdgeTerms& t) {
+        if (t.role == 0) return;
+        const F3 dv = t.difference;
+        if (t.role == 1) {
+            add_offset_block(d, t.arm, ws);
+            const F3 cd = cross(t.arm, dv);
+            g[0] -= ws * cd.x; g[1] -= ws * cd.y; g[2] -= ws * cd.z;
+            g[3] -= ws * dv.x; g[4] -= ws * dv.y; g[5] -= ws * dv.z;
+        } else {
+            d[tri_index(3, 3)] += ws; d[tri_index(4, 4)] += ws; d[tri_index(5, 5)] += ws;
+            g[3] += ws * dv.x; g[4] += ws * dv.y; g[5] += ws * dv.z;
         }
-        if (a == node) w.edge_partials[e] = energy;
+    };
+    add_edge(near);
+    for (int i = edge_first + 32; i < edge_end; i += 32) {
+        const int e = L.node_edge_list[i];
+        add_edge(edge_terms(w, c, L, e, L.edges[e * 2], L.edges[e * 2 + 1], node, build));
     }
     if (!build) return;
     if (lane == 0 && wt[3] > 0.0) {  // the anchor term, formed with the residuals
@@ -2046,13 +2083,27 @@ __device__ __forceinline__ void assemble_block(const WrapDev& w, const WrapContr
     float blk[36];
     for (int i = 0; i < 36; ++i) blk[i] = 0.0f;
     const bool pair = k < L.pair_count;
+    // what the loop has nothing to do with is loaded ahead of it
+    const int edge = L.block_edge[k];
+    const int slot = L.sell_slots[k * 2], mirror = L.sell_slots[k * 2 + 1];
+    const float ws = edge >= 0 && w.weights[c.level][2] > 0.0 ? (float)w.weights[c.level][2] : 0.0f;
+    const bool arm = ws > 0.0f && c.route == 0;
+    F3 cv = {0.0f, 0.0f, 0.0f};
+    // of the smoothness edge's term, ws * [[0, -[c]x], [0, -I]]: c = R_a (g_b - g_a)
+    auto edge_arm = [&](int a, int b) {
+        const D3 gd = rsub(load_d3(L.rest, b), load_d3(L.rest, a));
+        cv = mul3f(w.rot32 + a * 9, {(float)gd.x, (float)gd.y, (float)gd.z});
+    };
     if (pair) {
         const int end = L.pair_begin[k + 1];
         const bool landmarks = w.L > 0;
         int i = L.pair_begin[k] + lane;
         int after = i + 32 < end ? L.pair_entry[i + 32] : 0;
         PairEntry ahead;
-        if (i < end) ahead = load_pair(w, L.pair_entry[i], landmarks);
+        const int entry = i < end ? L.pair_entry[i] : 0;
+        const int ea = arm ? L.edges[edge * 2] : 0, eb = arm ? L.edges[edge * 2 + 1] : 0;
+        if (i < end) ahead = load_pair(w, entry, landmarks);
+        if (arm) edge_arm(ea, eb);
         for (; i < end; i += 32) {
             const PairEntry x = ahead;
             if (i + 32 < end) ahead = load_pair(w, after, landmarks);
@@ -2087,23 +2138,16 @@ __device__ __forceinline__ void assemble_block(const WrapDev& w, const WrapContr
                     for (int q = 0; q < 6; ++q) blk[r * 6 + q] += s * ua[r] * ub[q];
             }
         }
-    }
-    // the smoothness edge's term, ws * [[0, -[c]x], [0, -I]], c = R_a (g_b - g_a)
-    const int edge = L.block_edge[k];
-    const float ws = edge >= 0 && w.weights[c.level][2] > 0.0 ? (float)w.weights[c.level][2] : 0.0f;
-    F3 cv = {0.0f, 0.0f, 0.0f};
-    if (ws > 0.0f && c.route == 0) {
-        const int a = L.edges[edge * 2], b = L.edges[edge * 2 + 1];
-        const D3 gd = rsub(load_d3(L.rest, b), load_d3(L.rest, a));
-        cv = mul3f(w.rot32 + a * 9, {(float)gd.x, (float)gd.y, (float)gd.z});
+    } else if (arm) {
+        edge_arm(L.edges[edge * 2], L.edges[edge * 2 + 1]);
     }
     // the 36 sums spread over the lanes (two each at most); each lane stores
     // what it holds, both ways
     int first = 0, count = 36;
     if (pair) warp_sum_halving<36>(blk, lane, first, count);
     else halving_place<36>(lane, first, count);
-    float* A = w.offdiag[1 - c.system] + block_base(L.sell_slots[k * 2]);
-    float* T = w.offdiag[1 - c.system] + block_base(L.sell_slots[k * 2 + 1]);
+    float* A = w.offdiag[1 - c.system] + block_base(slot);
+    float* T = w.offdiag[1 - c.system] + block_base(mirror);
 #pragma unroll
     for (int i = 0; i < 2; ++i) {
         if (i >= count) break;
