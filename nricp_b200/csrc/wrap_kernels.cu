@@ -671,14 +671,29 @@ __device__ __forceinline__ void k_c_fit_body(const WrapDev& w, int part, int bx)
     const D3 tn = load_d3(T, node);
     double S[9];
     for (int i = 0; i < 9; ++i) S[i] = 0.0;
+    // the lane's first edge, read while its first binding is on its way
+    const int edge_first = L.node_edge_begin[node] + lane, edge_end = L.node_edge_begin[node + 1];
+    D3 edge_src, edge_dst;
+    auto load_edge = [&](int i) {  // false: the node is the edge's second
+        const int e = L.node_edge_list[i];
+        const int a = L.edges[e * 2], b = L.edges[e * 2 + 1];
+        if (a != node) return false;
+        const D3 gb = load_d3(L.rest, b);
+        edge_src = gb - g;
+        edge_dst = gb + load_d3(T, b) - g - tn;
+        return true;
+    };
+    const bool near = edge_first < edge_end && load_edge(edge_first);
     for (int i = L.gather_begin[node] + lane; i < L.gather_begin[node + 1]; i += 32) {
         const int entry = L.gather_entry[i];
         const int v = entry / kMaxSlots;
         const double own = L.bind_weights[entry];
         const D3 src = load_d3(w.tpl, v) - g;
+        const D3 point = load_d3(w.corr_point, v);
+        const double robust = w.robust[v];
         if (w.corr_code[v] == 0) {
-            const D3 dst = load_d3(w.corr_point, v) - g - tn;
-            const double s = data_weight * w.robust[v] * own;
+            const D3 dst = point - g - tn;
+            const double s = data_weight * robust * own;
             const double xs[3] = {src.x, src.y, src.z}, ys[3] = {dst.x, dst.y, dst.z};
             for (int r = 0; r < 3; ++r)
                 for (int q = 0; q < 3; ++q) S[r * 3 + q] += s * xs[r] * ys[q];
@@ -691,17 +706,14 @@ __device__ __forceinline__ void k_c_fit_body(const WrapDev& w, int part, int bx)
                 for (int q = 0; q < 3; ++q) S[r * 3 + q] += s * xs[r] * ys[q];
         }
     }
-    for (int i = L.node_edge_begin[node] + lane; i < L.node_edge_begin[node + 1]; i += 32) {
-        const int e = L.node_edge_list[i];
-        const int a = L.edges[e * 2], b = L.edges[e * 2 + 1];
-        if (a != node) continue;
-        const D3 gb = load_d3(L.rest, b);
-        const D3 src = gb - g;
-        const D3 dst = gb + load_d3(T, b) - g - tn;
-        const double xs[3] = {src.x, src.y, src.z}, ys[3] = {dst.x, dst.y, dst.z};
+    auto add_edge = [&] {
+        const double xs[3] = {edge_src.x, edge_src.y, edge_src.z}, ys[3] = {edge_dst.x, edge_dst.y, edge_dst.z};
         for (int r = 0; r < 3; ++r)
             for (int q = 0; q < 3; ++q) S[r * 3 + q] += wt[2] * xs[r] * ys[q];
-    }
+    };
+    if (near) add_edge();
+    for (int i = edge_first + 32; i < edge_end; i += 32)
+        if (load_edge(i)) add_edge();
     for (int i = 0; i < 9; ++i) S[i] = warp_sum(S[i]);
     if (lane == 0) {
         double fit[9], cur[9], curT[9], rel[9], step[9], out[9];
@@ -728,6 +740,42 @@ __global__ void k_c_fit(const WrapDev* __restrict__ wraps, int wrap_count, int p
         [&](int wi, int bx) { k_c_fit_body(wraps[wi], part, bx); });
 }
 
+// Every vertex deformed by the fitted rotations, once for the right-hand side
+// that follows (the candidate's evaluation overwrites it).  The nodes' warps
+// did this for each binding again: up to eight dependent reads of a rotation
+// per entry.  8k vertices, 130 ticks: a step 23.8 -> 22.2 ms, with the fit's and
+// this kernel's first edges read beside the bindings.
+__device__ __forceinline__ void k_c_deform_body(const WrapDev& w, int part, int bx) {
+    const WrapControl c = *w.control;
+    if (!in_part(c, part)) return;
+    if (c.phase != kPhaseSolve || c.route != 1) return;
+    const LevelDev& L = w.levels[c.level];
+    const int v = bx * blockDim.x + threadIdx.x;
+    if (v >= w.V) return;
+    const double* Rc = w.rot[1 - c.state];
+    const double* Tc = w.trans[1 - c.state];
+    const D3 p = load_d3(w.tpl, v);
+    D3 deformed = {0.0, 0.0, 0.0};
+    const int count = L.bind_counts[v];
+    for (int s = 0; s < count; ++s) {
+        const int j = L.bind_nodes[v * kMaxSlots + s];
+        const double ws = L.bind_weights[v * kMaxSlots + s];
+        const D3 gj = load_d3(L.rest, j);
+        deformed = deformed + (mul3(Rc + j * 9, p - gj) + gj + load_d3(Tc, j)) * ws;
+    }
+    store_d3(w.deformed, v, deformed);
+}
+
+__global__ void __launch_bounds__(kVertexThreads) k_c_deform(const WrapDev* __restrict__ wraps, int wrap_count, int part) {
+    over_virtual_blocks<false>(
+        wraps, wrap_count,
+        [&](const WrapDev& w) {
+            const WrapControl c = *w.control;
+            return in_part(c, part) && c.phase == kPhaseSolve && c.route == 1 ? blocks_of_dev(w.V, kVertexThreads) : 0;
+        },
+        [&](int wi, int bx) { k_c_deform_body(wraps[wi], part, bx); });
+}
+
 // Warp per node: the translation-only right-hand side with the fitted
 // rotations (local_global.cu:317-438); the rotation half is exactly zero.
 __device__ __forceinline__ void k_c_rhs_body(const WrapDev& w, int part, int bx) {
@@ -742,28 +790,33 @@ __device__ __forceinline__ void k_c_rhs_body(const WrapDev& w, int part, int bx)
     const double* Rc = w.rot[1 - c.state];
     const double* Tc = w.trans[1 - c.state];
     double local[3] = {0.0, 0.0, 0.0};
+    // the lane's first edge, read while its first binding is on its way
+    const int edge_first = L.node_edge_begin[node] + lane, edge_end = L.node_edge_begin[node + 1];
+    double sign = 0.0;
+    auto edge_difference = [&](int i) {
+        const int e = L.node_edge_list[i];
+        const int a = L.edges[e * 2], b = L.edges[e * 2 + 1];
+        const D3 ga = load_d3(L.rest, a), gb = load_d3(L.rest, b);
+        sign = a == node ? 1.0 : -1.0;
+        return mul3(Rc + a * 9, gb - ga) + ga + load_d3(Tc, a) - gb - load_d3(Tc, b);
+    };
+    D3 diff = {0.0, 0.0, 0.0};
+    if (edge_first < edge_end) diff = edge_difference(edge_first);
     for (int i = L.gather_begin[node] + lane; i < L.gather_begin[node + 1]; i += 32) {
         const int entry = L.gather_entry[i];
         const int v = entry / kMaxSlots;
         const double own = L.bind_weights[entry];
-        const D3 p = load_d3(w.tpl, v);
-        D3 deformed = {0.0, 0.0, 0.0};
-        const int count = L.bind_counts[v];
-        for (int s = 0; s < count; ++s) {
-            const int j = L.bind_nodes[v * kMaxSlots + s];
-            const double ws = L.bind_weights[v * kMaxSlots + s];
-            const D3 gj = load_d3(L.rest, j);
-            deformed = deformed + (mul3(Rc + j * 9, p - gj) + gj + load_d3(Tc, j)) * ws;
-        }
+        const D3 deformed = load_d3(w.deformed, v);
+        const D3 point = load_d3(w.corr_point, v);
+        const D3 n = load_d3(w.corr_normal, v);
+        const double u = w.robust[v];
         if (w.corr_code[v] == 0) {
-            const D3 off = deformed - load_d3(w.corr_point, v);
-            const double u = w.robust[v];
+            const D3 off = deformed - point;
             if (wt[0] > 0.0) {
                 const double s = wt[0] * u * own;
                 local[0] -= s * off.x; local[1] -= s * off.y; local[2] -= s * off.z;
             }
             if (wt[1] > 0.0) {
-                const D3 n = load_d3(w.corr_normal, v);
                 const double s = wt[1] * u * own * dot(n, off);
                 local[0] -= s * n.x; local[1] -= s * n.y; local[2] -= s * n.z;
             }
@@ -774,12 +827,8 @@ __device__ __forceinline__ void k_c_rhs_body(const WrapDev& w, int part, int bx)
             local[0] -= s * o.x; local[1] -= s * o.y; local[2] -= s * o.z;
         }
     }
-    for (int i = L.node_edge_begin[node] + lane; i < L.node_edge_begin[node + 1]; i += 32) {
-        const int e = L.node_edge_list[i];
-        const int a = L.edges[e * 2], b = L.edges[e * 2 + 1];
-        const D3 ga = load_d3(L.rest, a), gb = load_d3(L.rest, b);
-        const D3 diff = mul3(Rc + a * 9, gb - ga) + ga + load_d3(Tc, a) - gb - load_d3(Tc, b);
-        const double sign = a == node ? 1.0 : -1.0;
+    for (int i = edge_first; i < edge_end; i += 32) {
+        if (i != edge_first) diff = edge_difference(i);
         local[0] -= sign * wt[2] * diff.x;
         local[1] -= sign * wt[2] * diff.y;
         local[2] -= sign * wt[2] * diff.z;
@@ -2380,7 +2429,7 @@ __global__ void __launch_bounds__(kDecideThreads) k_decide(const WrapDev* __rest
 // Grids of the virtual-block kernels: as many blocks as fit on the device
 // at once (occupancy of each kernel at its block size, times the SMs).
 struct VirtualGrids {
-    int prologue, c_fit, c_rhs, evaluate, normals, residual, candidate, assemble;
+    int prologue, c_fit, c_deform, c_rhs, evaluate, normals, residual, candidate, assemble;
 };
 const VirtualGrids& virtual_grids() {
     static const VirtualGrids grids = [] {
@@ -2395,6 +2444,7 @@ const VirtualGrids& virtual_grids() {
         VirtualGrids g;
         g.prologue = fit(k_prologue, 128);
         g.c_fit = fit(k_c_fit, kNodeThreads);
+        g.c_deform = fit(k_c_deform, kVertexThreads);
         g.c_rhs = fit(k_c_rhs, kNodeThreads);
         g.evaluate = fit(k_evaluate, kVertexThreads);
         g.normals = fit(k_normals, kVertexThreads);
@@ -2445,6 +2495,7 @@ void launch_tick(const WrapDev* wraps, const TickShape& s, cudaStream_t stream,
     // ---- the solve chain ----
     if (s.route_c) {
         k_c_fit<<<grids.c_fit, kNodeThreads, virtual_smem, stream>>>(wraps, W, solve_part);
+        k_c_deform<<<grids.c_deform, kVertexThreads, virtual_smem, stream>>>(wraps, W, solve_part);
         k_c_rhs<<<grids.c_rhs, kNodeThreads, virtual_smem, stream>>>(wraps, W, solve_part);
     }
     if (timed) cudaEventRecord(timers->pcg_begin, stream);
@@ -2508,10 +2559,10 @@ void launch_tick(const WrapDev* wraps, const TickShape& s, cudaStream_t stream,
 }
 
 int tick_kernel_launches(const TickShape& s, bool timed) {
-    // stats twice, [fit, rhs,] solve launches, prologue, evaluate, normals,
+    // stats twice, [fit, deform, rhs,] solve launches, prologue, evaluate, normals,
     // query, residual, assembly, decision; an untimed tick with a side stream
     // runs the last three in each branch
-    return 9 + (s.route_c ? 2 : 0) + (s.grid_nodes > 0 ? 1 : 0) + (s.pcg_groups > 0 ? s.pcg_groups : 1) + (s.side_stream && !timed ? 3 : 0);
+    return 9 + (s.route_c ? 3 : 0) + (s.grid_nodes > 0 ? 1 : 0) + (s.pcg_groups > 0 ? s.pcg_groups : 1) + (s.side_stream && !timed ? 3 : 0);
 }
 
 // Cluster size of the solve for one wrap of `nodes` nodes on its own: a
