@@ -54,8 +54,7 @@ struct LevelDev {
     const int32_t* node_edge_begin;
     const int32_t* node_edge_list;
     const int32_t* edges;          // edge_count x 2
-    // pair groups: (a, b) and their (vertex, slot_a, slot_b) entries
-    const int32_t* pair_nodes;     // pair_count x 2
+    // pair groups: their (vertex, slot_a, slot_b) entries
     const int32_t* pair_begin;     // pair_count + 1
     const int32_t* pair_entry;     // vertex * 64 + slot_a * 8 + slot_b
     // off-diagonal row lists for the matvec, by octets of nodes: step t of an
@@ -63,8 +62,7 @@ struct LevelDev {
     const int32_t* row_begin;      // N + 1: a node's entries are counted by row_begin[n + 1] - row_begin[n]
     const int32_t* sell_begin;     // octets + 1: first step of each octet
     const int32_t* sell_nodes;     // steps x 8: the other node of each block (0: none)
-    const int32_t* offdiag_nodes;  // offdiag_count x 2 (pair groups first, then edge-only pairs)
-    const int32_t* block_edge;     // offdiag_count: the smoothness edge that adds to the block, or -1
+    const int32_t* block_edge;     // offdiag_count (pair groups first, then edge-only pairs): the smoothness edge that adds to the block, or -1
     const int32_t* sell_slots;     // offdiag_count x 2: places (step * 8 + node of the octet) of B (a) and B^T (b)
     // warm start from the previous level (level > 0): 4 source nodes + weights
     const int32_t* transfer_nodes;   // N x 4
@@ -120,7 +118,7 @@ struct WrapControl {
 struct WrapDev {
     // sizes
     int V, T, Vt, F, L;
-    int max_nodes, max_offdiag, max_pairs, max_edges;
+    int max_nodes, max_offdiag, max_edges;
     int energy_blocks;    // partial records written by the vertex pass
     // settings (per level where they vary)
     double weights[kMaxLevels][kEnergyKinds];

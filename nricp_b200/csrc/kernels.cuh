@@ -44,8 +44,6 @@ struct TickShape {
     int wraps;
     int max_vertices;
     int max_nodes;
-    int max_edges;
-    int max_pairs;
     int route_c;         // some wrap solves by route C (else its Horn-fit kernels are not launched)
     int energy_blocks;   // vertex-pass blocks per wrap (partials written)
     int edge_blocks;

@@ -148,7 +148,7 @@ struct Wrap {
     TemplateGraph graph;
     std::vector<LevelLayout> layouts;
     int V = 0, T = 0, Vt = 0, F = 0, L = 0, levels = 0;
-    int max_nodes = 0, max_edges = 0, max_pairs = 0, max_offdiag = 0, max_steps = 0;
+    int max_nodes = 0, max_edges = 0, max_offdiag = 0, max_steps = 0;
     double setup_seconds = 0.0, solve_started = 0.0, solve_seconds = 0.0;
     Arena arena;
     WrapDev dev{};        // host copy of the descriptor
@@ -224,7 +224,6 @@ void envelope(Wrap& w) {
     for (const LevelLayout& L : w.layouts) {
         w.max_nodes = std::max(w.max_nodes, L.node_count);
         w.max_edges = std::max(w.max_edges, L.edge_count);
-        w.max_pairs = std::max(w.max_pairs, L.pair_count);
         w.max_offdiag = std::max(w.max_offdiag, static_cast<int>(L.offdiag_nodes.size() / 2));
         w.max_steps = std::max(w.max_steps, static_cast<int>(L.sell_begin.back()));
     }
@@ -251,9 +250,9 @@ size_t bytes_of_layout(const LevelLayout& L) {
     return 256 * 27 + sizeof(double) * (L.rest.size() + L.bind_weights.size() + L.transfer_weights.size()) +
            sizeof(int32_t) * (L.bind_nodes.size() + L.bind_counts.size() + L.gather_begin.size() +
                               L.gather_entry.size() + L.node_edge_begin.size() +
-                              L.node_edge_list.size() + L.edges.size() + L.pair_nodes.size() +
+                              L.node_edge_list.size() + L.edges.size() +
                               L.pair_begin.size() + L.pair_entry.size() + L.row_begin.size() +
-                              L.sell_begin.size() + L.sell_nodes.size() + L.offdiag_nodes.size() + L.sell_slots.size() +
+                              L.sell_begin.size() + L.sell_nodes.size() + L.sell_slots.size() +
                               L.offdiag_nodes.size() / 2 +
                               L.transfer_nodes.size() +
                               L.transfer_counts.size());
@@ -369,7 +368,7 @@ size_t prepare_device(Wrap& w, WrapControl* control, cudaStream_t stream, bool p
     WrapDev& D = w.dev;
     std::memset(&D, 0, sizeof D);
     D.V = V; D.T = w.T; D.Vt = w.Vt; D.F = w.F; D.L = w.L;
-    D.max_nodes = w.max_nodes; D.max_offdiag = w.max_offdiag; D.max_pairs = w.max_pairs;
+    D.max_nodes = w.max_nodes; D.max_offdiag = w.max_offdiag;
     D.max_edges = w.max_edges; D.energy_blocks = vblocks;
     const double units = w.graph.scale;
     for (int l = 0; l < kMaxLevels; ++l) {
@@ -466,13 +465,11 @@ size_t prepare_device(Wrap& w, WrapControl* control, cudaStream_t stream, bool p
         G.node_edge_begin = put(L.node_edge_begin);
         G.node_edge_list = put(L.node_edge_list);
         G.edges = put(L.edges);
-        G.pair_nodes = put(L.pair_nodes);
         G.pair_begin = put(L.pair_begin);
         G.pair_entry = put(L.pair_entry);
         G.row_begin = put(L.row_begin);
         G.sell_begin = put(L.sell_begin);
         G.sell_nodes = put(L.sell_nodes);
-        G.offdiag_nodes = put(L.offdiag_nodes);
         G.sell_slots = put(L.sell_slots);
         {
             std::vector<int32_t> block_edge(L.offdiag_nodes.size() / 2, -1);
@@ -774,8 +771,6 @@ void Batch::upload_all(LbvhExport* lbvh_out) {
         g_transfers.h2d += w.input_bytes;
         shape_.max_vertices = std::max(shape_.max_vertices, w.V);
         shape_.max_nodes = std::max(shape_.max_nodes, w.max_nodes);
-        shape_.max_edges = std::max(shape_.max_edges, w.max_edges);
-        shape_.max_pairs = std::max(shape_.max_pairs, w.max_pairs);
         if (w.desc.route == NRICP_ROUTE_C) shape_.route_c = 1;
     }
     set_pcg_cluster(default_pcg_cluster());
@@ -1255,7 +1250,7 @@ namespace {
 struct TemplateEntry {
     TemplateGraph graph;
     std::vector<LevelLayout> layouts;
-    int levels = 0, max_nodes = 0, max_edges = 0, max_pairs = 0, max_offdiag = 0, max_steps = 0;
+    int levels = 0, max_nodes = 0, max_edges = 0, max_offdiag = 0, max_steps = 0;
 };
 
 uint64_t fnv1a(const void* data, size_t bytes, uint64_t h) {
@@ -1377,7 +1372,6 @@ struct Server::Impl {
             fresh->levels = w.levels;
             fresh->max_nodes = w.max_nodes;
             fresh->max_edges = w.max_edges;
-            fresh->max_pairs = w.max_pairs;
             fresh->max_offdiag = w.max_offdiag;
             fresh->max_steps = w.max_steps;
             std::lock_guard<std::mutex> lk(cache_mu);
@@ -1389,7 +1383,6 @@ struct Server::Impl {
         w.levels = entry->levels;
         w.max_nodes = entry->max_nodes;
         w.max_edges = entry->max_edges;
-        w.max_pairs = entry->max_pairs;
         w.max_offdiag = entry->max_offdiag;
         w.max_steps = entry->max_steps;
     }
@@ -1522,8 +1515,6 @@ struct Server::Impl {
         const TickShape before = shape;
         shape.max_vertices = std::max(shape.max_vertices, w.V);
         shape.max_nodes = std::max(shape.max_nodes, w.max_nodes);
-        shape.max_edges = std::max(shape.max_edges, w.max_edges);
-        shape.max_pairs = std::max(shape.max_pairs, w.max_pairs);
         if (w.desc.route == NRICP_ROUTE_C) shape.route_c = 1;
         if (std::memcmp(&before, &shape, sizeof shape) != 0) {
             for (auto& [count, g] : graphs) cudaGraphExecDestroy(g);
