@@ -253,8 +253,9 @@ int nricp_batch_step(NricpBatch* batch, double* device_ms);
  * power of two from 1 to 16 gives every wrap that many CTAs in one launch;
  * 0 gives each wrap its own size (about 128 nodes per CTA), one launch per
  * size class, the classes running side by side; -s (s = 1..4) halves those
- * per-wrap sizes s times.  A new batch starts at the smallest s whose classes
- * need at most three CTAs per SM (unhalved if they fit one per SM).  Every choice gives bit-identical results;
+ * per-wrap sizes s times.  A new batch starts with about 64 nodes per CTA or
+ * with s = 0 if those clusters run at once, else at the smallest s > 0 whose
+ * classes need at most three CTAs per SM.  Every choice gives bit-identical results;
  * it trades one wrap's latency against the batch's throughput.
  * *cluster_out (may be NULL) receives the largest size in effect. */
 int nricp_batch_tune(NricpBatch* batch, int pcg_cluster, int* cluster_out);
@@ -296,9 +297,9 @@ typedef struct NricpServerConfig {
     int max_slots;               /* wraps resident at once (1..1024) */
     int prep_threads;            /* host threads preparing requests; 0: half the cores */
     int pcg_cluster;             /* solve cluster: > 0 one size (a power of two up to 16) for every
-                                    slot; 0 (the default) per-wrap latency classes, halved once
-                                    when the running wraps would need more than one CTA per
-                                    SM; -s (1..4) latency classes always halved s times */
+                                    slot; 0 (the default) per-wrap latency classes, of about 64
+                                    or 128 nodes per CTA while the running wraps' clusters run
+                                    at once, else halved once; -s (1..4) latency classes always halved s times */
     int ticks_per_poll;          /* ticks launched between looks at the wraps' progress */
     int large_face_threshold;    /* requests whose target has at least this many triangles run
                                     in a lane of their own, with its own slots, stream and

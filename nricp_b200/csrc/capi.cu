@@ -300,7 +300,7 @@ int nricp_batch_step(NricpBatch* b, double* device_ms) {
 
 int nricp_batch_tune(NricpBatch* b, int pcg_cluster, int* cluster_out) {
     return guarded([&] {
-        b->batch.set_pcg_cluster(pcg_cluster);
+        b->batch.tune(pcg_cluster);
         if (cluster_out) *cluster_out = b->batch.shape().pcg_cluster;
     });
 }

@@ -79,7 +79,9 @@ void launch_tick(const WrapDev* wraps, const TickShape& shape, cudaStream_t stre
 // Kernels one tick launches (a timed tick runs its branches one after the
 // other, with one assembly).
 int tick_kernel_launches(const TickShape& shape, bool timed = false);
-int pcg_latency_cluster(int nodes);
+int pcg_class_cluster(int nodes, int shift);
+// The share of the device that one solve cluster of this size takes.
+double pcg_cluster_share(int cluster);
 int pcg_cluster_size(int max_nodes, int wraps, int sm_count);
 // Sets the shape's grid solve from its wraps and max_nodes.
 void grid_solve_shape(TickShape& shape);

@@ -833,21 +833,34 @@ bool Batch::all_done() const {
     return true;
 }
 
-// Per-wrap latency classes while their CTAs fit on the SMs at once; else
-// halved until they need at most three per SM (-s for nricp_batch_tune).
-// Uneven wraps of the benchmark's sizes, ms per step unhalved / halved / halved
-// twice: 8 wraps (88 CTAs) 77.7 / 77.7 / 91.4, 16 (180) 133 / 127 / 150, 32
-// (360) 228 / 217 / 248, 64 (728) 434 / 403 / 447.
+// The finest classes whose clusters run at once, about 64 or about 128
+// nodes per CTA; else the latter halved until they need at most three CTAs per
+// SM (-s for nricp_batch_tune).  Uneven wraps of the benchmark's sizes, ms per step
+// with 128 nodes per CTA / halved / halved twice: 8 wraps (88 CTAs) 77.7 / 77.7 /
+// 91.4, 16 (180) 133 / 127 / 150, 32 (360) 228 / 217 / 248, 64 (728) 434 / 403 /
+// 447.  (These and the server's rule count clusters, not CTAs: eight or nine
+// clusters of sixteen are all that run at once.)  One wrap of 200 nodes, 64 / 128 nodes per CTA: 12.5 / 13.2, of 544 nodes
+// by route C 21.9 / 22.3.
 int Batch::default_pcg_cluster() const {
     int device = 0, sms = 148;
     check(cudaGetDevice(&device), "device");
     check(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device), "device");
-    for (int shift = 0; shift < 4; ++shift) {
+    for (int shift = -1; shift < 4; ++shift) {
         long ctas = 0;
-        for (const auto& w : wraps_) ctas += std::max(1, pcg_latency_cluster(w->max_nodes) >> shift);
-        if (ctas <= (shift == 0 ? 1L : 3L) * sms) return -shift;
+        double share = 0.0;
+        for (const auto& w : wraps_) {
+            const int cluster = pcg_class_cluster(w->max_nodes, shift);
+            ctas += cluster;
+            share += pcg_cluster_share(cluster);
+        }
+        if (shift <= 0 ? share <= 1.0 : ctas <= 3L * sms) return shift < 0 ? kFineClasses : -shift;
     }
     return -4;
+}
+
+void Batch::tune(int cluster) {
+    if (cluster > 16) throw InvalidArgument("the solve's cluster size is a power of two from 1 to 16");
+    set_pcg_cluster(cluster);
 }
 
 void Batch::set_pcg_cluster(int cluster) {
@@ -863,9 +876,10 @@ void Batch::set_pcg_cluster(int cluster) {
     tail_ready_ = tail_on_ = false;
     grid_solve_shape(shape_);
     solve_shape(cluster, shape_, pcg_index_, nullptr);
-    if (cluster < 0) {  // halved classes: halved once less for the tail
+    if (cluster <= 0) {  // classes one step finer for the tail
         tail_shape_ = shape_;
-        solve_shape(cluster + 1, tail_shape_, tail_index_, &tail_cls_);
+        tail_fine_ = cluster == 0;
+        solve_shape(cluster < 0 ? cluster + 1 : kFineClasses, tail_shape_, tail_index_, &tail_cls_);
         tail_ready_ = true;
     }
 }
@@ -875,7 +889,7 @@ void Batch::solve_shape(int cluster, TickShape& shape, int* index, std::vector<i
     std::vector<int> nodes(W);
     for (int i = 0; i < W; ++i) nodes[i] = wraps_[i]->max_nodes;
     shape.pcg_groups = 0;
-    if (cluster > 0) {
+    if (cluster > 0 && cluster != kFineClasses) {
         if (cluster > 16 || (cluster & (cluster - 1)) != 0)
             throw InvalidArgument("the solve's cluster size is a power of two from 1 to 16");
         shape.pcg_cluster = cluster;
@@ -884,9 +898,9 @@ void Batch::solve_shape(int cluster, TickShape& shape, int* index, std::vector<i
     }
     if (cluster < -4) throw InvalidArgument("the solve's class shift is 0 to 4");
     // one class per wrap: its own latency cluster, halved `shift` times
-    const int shift = -cluster;
+    const int shift = cluster == kFineClasses ? -1 : -cluster;
     std::vector<int> cls(W);
-    for (int i = 0; i < W; ++i) cls[i] = std::max(1, pcg_latency_cluster(nodes[i]) >> shift);
+    for (int i = 0; i < W; ++i) cls[i] = pcg_class_cluster(nodes[i], shift);
     if (cls_out) *cls_out = cls;
     std::vector<int> sizes;
     for (int c = 16; c >= 1; c /= 2)
@@ -920,11 +934,19 @@ void Batch::solve_shape(int cluster, TickShape& shape, int* index, std::vector<i
     shape.pcg_cluster = sizes[0];
 }
 
+// The finest classes pay only once all their clusters run at once (12 wraps of
+// 400 nodes, by CTAs: 43.0 ms a step, by clusters 36.4); the coarser ones gain
+// from the moment their CTAs would fit (14 uneven wraps 106.6 / 109.9, 64 wraps
+// 393.8 / 399.6).
 bool Batch::tail_due() const {
     long ctas = 0;
+    double share = 0.0;
     for (size_t i = 0; i < wraps_.size(); ++i)
-        if (host_controls_[i].phase != kPhaseDone) ctas += tail_cls_[i];
-    return ctas <= sms_;
+        if (host_controls_[i].phase != kPhaseDone) {
+            ctas += tail_cls_[i];
+            share += pcg_cluster_share(tail_cls_[i]);
+        }
+    return tail_fine_ ? share <= 1.0 : ctas <= sms_;
 }
 
 cudaGraphExec_t Batch::capture(const TickShape& shape) {
@@ -1563,16 +1585,18 @@ struct Server::Impl {
     std::map<int, int> launches_per_tick;
 
     // A wrap's class is its latency cluster halved `shift` times: a fixed
-    // shift (pcg_cluster < 0), or by load (0) -- none while the running
-    // wraps' latency clusters fit one CTA per SM, else one.
+    // shift (pcg_cluster < 0), or by load (0) -- the finest of -1, 0 and 1
+    // whose clusters for the running wraps run at once, else 1.
     int max_shift() const { return cfg.pcg_cluster < 0 ? -cfg.pcg_cluster : 1; }
     int shift_for(int count) const {
         if (cfg.pcg_cluster < 0) return -cfg.pcg_cluster;
-        long ctas = 0;
-        for (int i = 0; i < count; ++i) ctas += pcg_latency_cluster(slot_nodes[i]);
-        return ctas <= sms ? 0 : 1;
+        for (int shift = -1; shift < 1; ++shift) {
+            double share = 0.0;
+            for (int i = 0; i < count; ++i) share += pcg_cluster_share(pcg_class_cluster(slot_nodes[i], shift));
+            if (share <= 1.0) return shift;
+        }
+        return 1;
     }
-    static int class_of(int nodes, int shift) { return std::max(1, pcg_latency_cluster(nodes) >> shift); }
     // Rewrites the class rows for the running wraps in slots 0 .. count-1
     // (tick stream order: the next tick reads them).
     void upload_classes(int count) {
@@ -1582,7 +1606,7 @@ struct Server::Impl {
         const int shift = shift_for(count);
         for (int i = 0; i < count; ++i) {
             int g = 0;
-            while ((class_top >> g) > class_of(slot_nodes[i], shift)) ++g;
+            while ((class_top >> g) > pcg_class_cluster(slot_nodes[i], shift)) ++g;
             rows[static_cast<size_t>(g) * cfg.max_slots + fill[g]++] = i;
         }
         if (rows == class_rows) return;

@@ -70,7 +70,10 @@ public:
     // Cluster size of the solve launch.  > 0: that size for every wrap; 0:
     // each wrap its own latency cluster (about 128 nodes per CTA), one launch
     // per size class, the classes in parallel; -s: the same classes halved s
-    // times.  Every choice gives bit-identical results.
+    // times; kFineClasses (a new batch's own choice, not a caller's): about 64
+    // nodes per CTA.  Every choice gives bit-identical results.
+    static constexpr int kFineClasses = 1 << 16;
+    void tune(int cluster);  // a caller's choice
     void set_pcg_cluster(int cluster);
     int default_pcg_cluster() const;
     void pull_controls();
@@ -126,15 +129,14 @@ private:
     // set_pcg_cluster takes it), its class lists in `index` (device); `cls` (if given) receives each wrap's cluster size.
     void solve_shape(int cluster, TickShape& shape, int* index, std::vector<int>* cls);
     cudaGraphExec_t capture(const TickShape& shape);
-    // The batch's tail.  With halved classes, once the wraps still running
-    // would fit on the SMs in one round at one halving less, their ticks run
-    // with that shape: few wraps left, each gets more CTAs.  Results do not
-    // depend on the cluster size.
+    // The batch's tail.  Once the wraps still running would fit on the SMs in
+    // one round at classes one step finer, their ticks run from a second graph
+    // of those classes.
     bool tail_due() const;
     TickShape tail_shape_{};
     int* tail_index_ = nullptr;
     std::vector<int> tail_cls_;
-    bool tail_ready_ = false, tail_on_ = false;
+    bool tail_ready_ = false, tail_on_ = false, tail_fine_ = false;
     cudaGraphExec_t tail_graph_ = nullptr;
     int sms_ = 148;
     std::vector<TickRecord> records_;

@@ -2565,13 +2565,17 @@ int tick_kernel_launches(const TickShape& s, bool timed) {
     return 9 + (s.route_c ? 3 : 0) + (s.grid_nodes > 0 ? 1 : 0) + (s.pcg_groups > 0 ? s.pcg_groups : 1) + (s.side_stream && !timed ? 3 : 0);
 }
 
-// Cluster size of the solve for one wrap of `nodes` nodes on its own: a
-// power of two with about 128 nodes (32 segments, two per warp) per CTA, at
-// most 16 CTAs (the non-portable maximum, enabled here).
-int pcg_latency_cluster(int nodes) {
+// Cluster size of the solve for a wrap of `nodes` nodes in a class: a power of
+// two with about 128 nodes (an octet per warp) per CTA, at most 16 CTAs (the
+// non-portable maximum, enabled here), halved `shift` times; shift -1: about 64
+// nodes.  An iteration's shared-memory reads fall with the rows per CTA: us per
+// iteration with 64 / 128 nodes a CTA: 200 nodes 4.40 / 5.51, 544 nodes 4.97 /
+// 5.48; with 32 nodes a CTA 200 nodes take 4.15, the whole step no less.
+int pcg_class_cluster(int nodes, int shift) {
+    const int per_cta = shift < 0 ? 64 : 128;
     int ranks = 1;
-    while (ranks < 16 && ranks * 128 < nodes) ranks *= 2;
-    return ranks;
+    while (ranks < 16 && ranks * per_cta < nodes) ranks *= 2;
+    return std::max(1, shift > 0 ? ranks >> shift : ranks);
 }
 
 void pcg_enable() {
@@ -2584,12 +2588,44 @@ void pcg_enable() {
     (void)enabled;
 }
 
+// One over the clusters that run at once: a cluster's CTAs sit in one group of
+// SMs, so that, say, twelve clusters of sixteen do not fit on 148 SMs.
+double pcg_cluster_share(int cluster) {
+    struct Shares {
+        double of[5];
+    };
+    static const Shares shares = [] {
+        pcg_enable();
+        Shares s{};
+        for (int i = 0; i < 5; ++i) {
+            cudaLaunchConfig_t config = {};
+            config.gridDim = dim3(1 << i);
+            config.blockDim = dim3(kPcgThreads);
+            config.dynamicSmemBytes = kPcgMaxSmemBytes;
+            cudaLaunchAttribute attribute[1];
+            attribute[0].id = cudaLaunchAttributeClusterDimension;
+            attribute[0].val.clusterDim.x = 1 << i;
+            attribute[0].val.clusterDim.y = 1;
+            attribute[0].val.clusterDim.z = 1;
+            config.attrs = attribute;
+            config.numAttrs = 1;
+            int clusters = 0;
+            cudaOccupancyMaxActiveClusters(&clusters, k_pcg, &config);
+            s.of[i] = 1.0 / std::max(1, clusters);
+        }
+        return s;
+    }();
+    int i = 0;
+    while (i < 4 && (1 << i) < cluster) ++i;
+    return shares.of[i];
+}
+
 // Default cluster size for a batch: one wrap takes its latency cluster; many
 // wraps share the SMs, so the cluster shrinks until one CTA per SM holds the
 // whole batch (the result does not depend on the choice).
 int pcg_cluster_size(int max_nodes, int wraps, int sm_count) {
     pcg_enable();
-    int ranks = pcg_latency_cluster(max_nodes);
+    int ranks = pcg_class_cluster(max_nodes, 0);
     while (ranks > 1 && (long)ranks * wraps > sm_count) ranks /= 2;
     return ranks;
 }
