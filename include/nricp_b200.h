@@ -255,8 +255,11 @@ int nricp_batch_step(NricpBatch* batch, double* device_ms);
  * size class, the classes running side by side; -s (s = 1..4) halves those
  * per-wrap sizes s times.  A new batch starts with about 64 nodes per CTA or
  * with s = 0 if those clusters run at once, else at the smallest s > 0 whose
- * classes need at most three CTAs per SM.  Every choice gives bit-identical results;
- * it trades one wrap's latency against the batch's throughput.
+ * classes need at most three CTAs per SM.  With classes (0 or -s), graphs of
+ * more than 2,000 nodes in a batch of at most eight wraps are solved by the
+ * whole device while no smaller graph is being solved; a uniform size applies
+ * to every graph.  Every choice gives bit-identical results; it trades one
+ * wrap's latency against the batch's throughput.
  * *cluster_out (may be NULL) receives the largest size in effect. */
 int nricp_batch_tune(NricpBatch* batch, int pcg_cluster, int* cluster_out);
 /* Per-tick records of wrap 0 from the last nricp_batch_profile. */
@@ -299,7 +302,8 @@ typedef struct NricpServerConfig {
     int pcg_cluster;             /* solve cluster: > 0 one size (a power of two up to 16) for every
                                     slot; 0 (the default) per-wrap latency classes, of about 64
                                     or 128 nodes per CTA while the running wraps' clusters run
-                                    at once, else halved once; -s (1..4) latency classes always halved s times */
+                                    at once, else halved once; -s (1..4) latency classes always
+                                    halved s times; large graphs as nricp_batch_tune's */
     int ticks_per_poll;          /* ticks launched between looks at the wraps' progress */
     int large_face_threshold;    /* requests whose target has at least this many triangles run
                                     in a lane of their own, with its own slots, stream and

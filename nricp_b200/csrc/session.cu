@@ -874,8 +874,11 @@ void Batch::set_pcg_cluster(int cluster) {
             *g = nullptr;
         }
     tail_ready_ = tail_on_ = false;
-    grid_solve_shape(shape_);
     solve_shape(cluster, shape_, pcg_index_, nullptr);
+    // a uniform size is the caller's for every graph; with classes the largest
+    // graphs may be the whole device's
+    shape_.grid_nodes = shape_.grid_ctas = 0;
+    if (cluster <= 0 || cluster == kFineClasses) grid_solve_shape(shape_);
     if (cluster <= 0) {  // classes one step finer for the tail
         tail_shape_ = shape_;
         tail_fine_ = cluster == 0;
@@ -1551,7 +1554,7 @@ struct Server::Impl {
         if (it != graphs.end()) return it->second;
         TickShape t = shape;
         t.wraps = count;
-        grid_solve_shape(t);
+        if (cfg.pcg_cluster <= 0) grid_solve_shape(t);  // one size for every slot: no grid
         t.pcg_groups = 0;
         pcg_cluster_size(t.max_nodes, count, sms);  // enables the launch attributes
         if (class_count == 0) {

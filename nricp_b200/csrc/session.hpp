@@ -71,7 +71,8 @@ public:
     // each wrap its own latency cluster (about 128 nodes per CTA), one launch
     // per size class, the classes in parallel; -s: the same classes halved s
     // times; kFineClasses (a new batch's own choice, not a caller's): about 64
-    // nodes per CTA.  Every choice gives bit-identical results.
+    // nodes per CTA.  With classes the whole device may take a large graph's
+    // solve (grid_solve_shape).  Every choice gives bit-identical results.
     static constexpr int kFineClasses = 1 << 16;
     void tune(int cluster);  // a caller's choice
     void set_pcg_cluster(int cluster);
@@ -85,7 +86,7 @@ public:
     // The current system of wrap `i` and the state it was assembled at.
     void inspect(int i, NricpInspect* out);
     void result(int i, NricpResult* out);
-    // Every wrap's result: downloads in turn, then the host work in parallel.
+    // Every wrap's result, one after the other.
     void results(NricpResult* outs);
     void current_vertices(int i, double* out);
     int finest_nodes(int i) const;

@@ -138,7 +138,9 @@ class WrapBatch:
         wrap, 0 for each wrap's own size in per-class launches, -s for those
         sizes halved s times (a new batch starts with finer sizes yet, or with
         0, where their clusters run at once, else with the smallest s whose
-        classes need at most three CTAs per SM).  Returns the largest size
+        classes need at most three CTAs per SM).  With classes, the graphs of
+        more than 2,000 nodes in a batch of at most eight wraps are solved by
+        the whole device while no smaller graph is.  Returns the largest size
         in effect; results are bit-identical for every choice."""
         out = C.c_int()
         check(load().nricp_batch_tune(self._handle, int(pcg_cluster), C.byref(out)))
