@@ -262,6 +262,12 @@ int nricp_batch_step(NricpBatch* batch, double* device_ms);
  * wrap's latency against the batch's throughput.
  * *cluster_out (may be NULL) receives the largest size in effect. */
 int nricp_batch_tune(NricpBatch* batch, int pcg_cluster, int* cluster_out);
+/* No reference counterpart.  How often a CTA of the linear solve looks for data
+ * of its own copies or of the CTAs it solves with before it gives up: tries of
+ * about 4 us, 2^19 (2 s) unless set, 0 to give up at once.  A wrap whose wait
+ * ran out ends there, and the call that ran it reports the error; the batch
+ * can be reset and run again. */
+int nricp_batch_wait_limit(NricpBatch* batch, int tries);
 /* Per-tick records of wrap 0 from the last nricp_batch_profile. */
 typedef struct NricpTickRecord {
     int phase;          /* 0 transfer, 1 refresh, 2 solve, 3 final */

@@ -4,6 +4,8 @@
 #include <cstdint>
 #include <cuda_runtime.h>
 
+#include "common.cuh"
+
 namespace nricp_b200 {
 
 __device__ __forceinline__ uint32_t shared_address(const void* p) {
@@ -25,12 +27,11 @@ __device__ __forceinline__ void mbar_arrive_expect(void* bar, int bytes) {
     asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(shared_address(bar)), "r"(bytes)
                  : "memory");
 }
-// Waits for the phase of this parity, with a limit (about a second): false if
-// it ran out.
-constexpr int kWaitLimit = 1 << 20;
-__device__ __forceinline__ bool mbar_wait(void* bar, int parity) {
+// Waits for the phase of this parity, at most `tries` times (kWaitTries): false
+// if they ran out.
+__device__ __forceinline__ bool mbar_wait(void* bar, int parity, int tries) {
     const uint32_t at = shared_address(bar);
-    for (int i = 0; i < kWaitLimit; ++i) {
+    for (int i = 0; i < tries; ++i) {
         uint32_t done;
         asm volatile("{\n.reg .pred p;\n"
                      "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n"

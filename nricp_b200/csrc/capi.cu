@@ -305,6 +305,10 @@ int nricp_batch_tune(NricpBatch* b, int pcg_cluster, int* cluster_out) {
     });
 }
 
+int nricp_batch_wait_limit(NricpBatch* b, int tries) {
+    return guarded([&] { b->batch.set_wait_tries(tries); });
+}
+
 int nricp_batch_tick_records(NricpBatch* b, NricpTickRecord* out, int capacity, int* count) {
     return guarded([&] {
         const auto& records = b->batch.tick_records();

@@ -26,6 +26,17 @@ constexpr int kPartialStride = 8;   // doubles per energy partial record
 constexpr int kErrorTraversal = 1;  // a closest-point walk overflowed its stack
 constexpr int kErrorSolveWait = 2;  // a wait inside the linear solve ran out
 
+// The limit of every wait inside a kernel for its own copies or for CTAs that
+// run at the same time: tries of an mbarrier, each of which the hardware
+// suspends for 3.95 us when nothing comes -- 2.1 s; or 32 times as many plain
+// polls of a word in global memory (150 ns each) -- 2.5 s.  The CTAs of a
+// cluster and of a cooperative grid start together, so a foreign kernel that
+// holds SMs delays them all and no wait begins before it has left.  Counted
+// in tries and not in time, so that a context which was paused meanwhile does
+// not give up when it goes on.
+constexpr int kWaitTries = 1 << 19;
+constexpr int kPollsPerTry = 32;
+
 // Device phases of one wrap.  They mirror the reference session's
 // BeginLevel / Refresh / InnerStep / CloseOuter / EndLevel
 // (src/cuda/session.cu:504-542); CloseOuter folds into the decision kernel.

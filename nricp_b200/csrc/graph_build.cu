@@ -162,7 +162,7 @@ __global__ void __launch_bounds__(kFpsThreads, 1) k_fps(const double* __restrict
         }
         int win = 0;
         if (ranks > 1) {
-            if (!mbar_wait(&arrived[set], (s >> 1) & 1)) timed_out = true;
+            if (!mbar_wait(&arrived[set], (s >> 1) & 1, kWaitTries)) timed_out = true;
             key = lane < ranks ? slots[set][lane].key : 0;
             index = lane < ranks ? (int)slots[set][lane].index : INT_MAX;
             const int own = index;

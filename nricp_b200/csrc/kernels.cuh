@@ -59,6 +59,7 @@ struct TickShape {
     cudaEvent_t pcg_fork, pcg_join[5];
     int grid_nodes;  // graphs above this may be solved by the whole device (0: no such launch)
     int grid_ctas;
+    int wait_tries = kWaitTries;         // limit of the waits inside the solve
     int* query_counter;                  // device: the query queues' heads, 2 ints
     // The refresh chain's branch (null: one chain on the tick's stream).
     cudaStream_t side_stream;

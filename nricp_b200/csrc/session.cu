@@ -858,6 +858,20 @@ int Batch::default_pcg_cluster() const {
     return -4;
 }
 
+void Batch::drop_graphs() {
+    for (cudaGraphExec_t* g : {&graph_exec_, &tail_graph_})
+        if (*g) {
+            cudaGraphExecDestroy(*g);
+            *g = nullptr;
+        }
+}
+
+void Batch::set_wait_tries(int tries) {
+    if (tries < 0 || tries > kWaitTries) throw InvalidArgument("the solve's wait limit is 0 to 2^19 tries");
+    drop_graphs();
+    shape_.wait_tries = tail_shape_.wait_tries = tries;
+}
+
 void Batch::tune(int cluster) {
     if (cluster > 16) throw InvalidArgument("the solve's cluster size is a power of two from 1 to 16");
     set_pcg_cluster(cluster);
@@ -868,11 +882,7 @@ void Batch::set_pcg_cluster(int cluster) {
     check(cudaGetDevice(&device), "device");
     check(cudaDeviceGetAttribute(&sms_, cudaDevAttrMultiProcessorCount, device), "device");
     pcg_cluster_size(shape_.max_nodes, static_cast<int>(wraps_.size()), sms_);  // enables the launch attributes
-    for (cudaGraphExec_t* g : {&graph_exec_, &tail_graph_})
-        if (*g) {
-            cudaGraphExecDestroy(*g);
-            *g = nullptr;
-        }
+    drop_graphs();
     tail_ready_ = tail_on_ = false;
     solve_shape(cluster, shape_, pcg_index_, nullptr);
     // a uniform size is the caller's for every graph; with classes the largest

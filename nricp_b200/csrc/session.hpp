@@ -75,6 +75,7 @@ public:
     // solve (grid_solve_shape).  Every choice gives bit-identical results.
     static constexpr int kFineClasses = 1 << 16;
     void tune(int cluster);  // a caller's choice
+    void set_wait_tries(int tries);  // limit of the waits inside the solve (0 .. kWaitTries)
     void set_pcg_cluster(int cluster);
     int default_pcg_cluster() const;
     void pull_controls();
@@ -130,6 +131,7 @@ private:
     // set_pcg_cluster takes it), its class lists in `index` (device); `cls` (if given) receives each wrap's cluster size.
     void solve_shape(int cluster, TickShape& shape, int* index, std::vector<int>* cls);
     cudaGraphExec_t capture(const TickShape& shape);
+    void drop_graphs();
     // The batch's tail.  Once the wraps still running would fit on the SMs in
     // one round at classes one step finer, their ticks run from a second graph
     // of those classes.

@@ -1020,12 +1020,12 @@ __device__ __forceinline__ void wait_copies() { asm volatile("cp.async.wait_all;
 constexpr int kGatherSteps = 16;  // steps whose u a warp of a grid solve gathers at a time
 
 // One thread's part of a meeting of a cooperative grid's CTAs: counts its CTA
-// in and waits, with a limit (about a second), until `target` have come.
-__device__ __forceinline__ bool grid_arrive_and_wait(unsigned* arrivals, unsigned target) {
+// in and waits, at most `polls` times, until `target` have come.
+__device__ __forceinline__ bool grid_arrive_and_wait(unsigned* arrivals, unsigned target, int polls) {
     // the release covers what the CTA's threads wrote before the block barrier;
     // the polls are plain, and one fence after the last orders what follows
     asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(arrivals) : "memory");
-    for (int i = 0; i < kWaitLimit; ++i) {
+    for (int i = 0; i < polls; ++i) {
         unsigned seen;
         asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(seen) : "l"(arrivals) : "memory");
         if (seen >= target) {
@@ -1075,9 +1075,13 @@ struct StepBlocks {
 // (eight floats a node) and the segments' sums are then in global memory, and
 // the CTAs meet at a counter in global memory twice per iteration; a CTA holds
 // so few rows that its own arrays are always in shared memory.
+//
+// Every wait has a limit (`tries`).  A CTA whose wait ran out sets
+// kErrorSolveWait, upon which the decision kernel ends the wrap; it first waits
+// for the copies it has started, and its peers' waits run out in turn.
 template <bool kAllShared, bool kGrid>
 __device__ __forceinline__ void pcg_solve(const WrapDev& w, const WrapControl& c, const PcgPlacement& place,
-                                          int budget_floats) {
+                                          int budget_floats, int tries) {
     static_assert(kAllShared || !kGrid, "the grid's own rows fit");
     cg::cluster_group cluster = cg::this_cluster();
     const LevelDev& L = w.levels[c.level];
@@ -1260,7 +1264,15 @@ __device__ __forceinline__ void pcg_solve(const WrapDev& w, const WrapControl& c
     const int cached = cached_s, listed = listed_s;
     const float4* cached_blocks = reinterpret_cast<const float4*>(cursor);
     const int* cached_nodes = reinterpret_cast<const int*>(cursor + (long)(o1 - o0) * cached * kStepFloats);
-    if (!mbar_wait(&blocks_arrived, 0)) timed_out = true;
+    // The lists of nodes among what was copied are indices: without them no
+    // product is formed.
+    const bool incomplete = __syncthreads_or(!mbar_wait(&blocks_arrived, 0, tries));
+    auto give_up = [&]() {
+        if (threadIdx.x == 0) atomicOr(&w.control->error, kErrorSolveWait);
+        mbar_wait(&blocks_arrived, 0, kWaitTries);  // this CTA's own copies
+        for (int i = 0; i < 256; ++i) __nanosleep(10000);  // and those it sent to its peers (2.6 ms)
+    };
+    if (incomplete) give_up();
 
     // The CTAs that own rows; the others only wait at the end.  (Where u is
     // global the loop meets at cluster barriers, and a graph that large gives
@@ -1276,7 +1288,8 @@ __device__ __forceinline__ void pcg_solve(const WrapDev& w, const WrapControl& c
     auto meet = [&]() {     // every active CTA's writes before it are visible after it
         __syncthreads();
         ++meetings;
-        if (threadIdx.x == 0 && !grid_arrive_and_wait(w.grid_arrivals, meetings * (unsigned)active)) timed_out = true;
+        if (threadIdx.x == 0 && !grid_arrive_and_wait(w.grid_arrivals, meetings * (unsigned)active, tries * kPollsPerTry))
+            timed_out = true;
         // the other threads learn of a wait that ran out at the totals' barrier
         __syncthreads();
     };
@@ -1365,7 +1378,8 @@ __device__ __forceinline__ void pcg_solve(const WrapDev& w, const WrapControl& c
             if (!kGrid) fetch(shape.first, 0, min(shape.streamed, shape.degree));
         }
     };
-    if (own > 0) {
+    const bool solving = own > 0 && !incomplete;
+    if (solving) {
         segment_rows([](int) {});
         share_u();
         fetch_first();
@@ -1374,8 +1388,8 @@ __device__ __forceinline__ void pcg_solve(const WrapDev& w, const WrapControl& c
     double gamma_prev = 0.0, alpha_prev = 0.0, bnorm = 0.0, residual = 0.0, surely_above = 0.0;
     int iterations = 0;
     bool converged = false;
-    for (int it = 0; own > 0; ++it) {
-        if (u_shared && active > 1 && !mbar_wait(&u_arrived, it & 1)) timed_out = true;
+    for (int it = 0; solving; ++it) {
+        if (u_shared && active > 1 && !mbar_wait(&u_arrived, it & 1, tries)) timed_out = true;
         // ---- w = A u for the owned rows, an octet per warp at a time: lane
         //      3i + p multiplies rows 2p and 2p + 1 of the octet's node i ----
         for (int o = o0 + warp; o < o1; o += kPcgWarps) {
@@ -1535,7 +1549,7 @@ __device__ __forceinline__ void pcg_solve(const WrapDev& w, const WrapControl& c
             } else if (lane == 0) {
                 mbar_arrive(&sums_arrived);
             }
-            if (!mbar_wait(&sums_arrived, it & 1)) timed_out = true;
+            if (!mbar_wait(&sums_arrived, it & 1, tries)) timed_out = true;
         }
         // ---- totals over every segment, in one fixed order in every CTA:
         //      each warp its stride of the segments, then every warp the same
@@ -1564,8 +1578,7 @@ __device__ __forceinline__ void pcg_solve(const WrapDev& w, const WrapControl& c
             delta = __shfl_sync(0xffffffffu, a, 16);
             rr_total = b2;
             if (failed) {  // uniform over the CTA; its peers' waits run out in turn
-                if (threadIdx.x == 0) atomicOr(&w.control->error, kErrorSolveWait);
-                for (int i = 0; i < 256; ++i) __nanosleep(10000);  // the copies in flight
+                give_up();
                 break;
             }
         }
@@ -1659,7 +1672,7 @@ __device__ inline bool grid_takes(const WrapDev* wraps, int wrap_count, int node
 
 // The wraps the grid takes, one after the other over the whole device.
 __global__ void __launch_bounds__(kPcgThreads, 1) k_pcg_grid(const WrapDev* __restrict__ wraps, int wrap_count,
-                                                          int grid_nodes, int budget_floats) {
+                                                          int grid_nodes, int budget_floats, int tries) {
     for (int i = 0; i < wrap_count; ++i) {
         const WrapDev& w = wraps[i];
         const WrapControl c = *w.control;
@@ -1669,14 +1682,14 @@ __global__ void __launch_bounds__(kPcgThreads, 1) k_pcg_grid(const WrapDev* __re
         PcgPlacement place = {};
         place.floats = pcg_owned_capacity(N, (int)gridDim.x) * (6 + kPcgVectorFloats + 2 * kPcgBlockFloats) +
                        kPcgWarps * kGatherSteps * 64;
-        pcg_solve<true, true>(w, c, place, budget_floats);
+        pcg_solve<true, true>(w, c, place, budget_floats, tries);
         __syncthreads();  // shared memory of one wrap before the next
     }
 }
 
 __global__ void __launch_bounds__(kPcgThreads, 1) k_pcg(const WrapDev* __restrict__ wraps,
                                                      const int* __restrict__ index,
-                                                     int budget_floats, int wrap_count, int grid_nodes) {
+                                                     int budget_floats, int wrap_count, int grid_nodes, int tries) {
     const int slot = index ? index[blockIdx.y] : (int)blockIdx.y;
     if (slot < 0) return;  // an empty entry of a class launch; uniform across the cluster
     const WrapDev& w = wraps[slot];
@@ -1686,9 +1699,9 @@ __global__ void __launch_bounds__(kPcgThreads, 1) k_pcg(const WrapDev* __restric
     const PcgPlacement place =
         pcg_place(w.levels[c.level].node_count, (int)cg::this_cluster().num_blocks(), budget_floats);
     if (place.all()) {
-        pcg_solve<true, false>(w, c, place, budget_floats);
+        pcg_solve<true, false>(w, c, place, budget_floats, tries);
     } else {
-        pcg_solve<false, false>(w, c, place, budget_floats);
+        pcg_solve<false, false>(w, c, place, budget_floats, tries);
     }
 }
 
@@ -2420,6 +2433,7 @@ __global__ void __launch_bounds__(kDecideThreads) k_decide(const WrapDev* __rest
         c.inner = 0;
         c.attempt = 0;
     }
+    if (c.error & kErrorSolveWait) c.phase = kPhaseDone;  // the host reports it
     *ctl = c;
 }
 
@@ -2512,7 +2526,8 @@ void launch_tick(const WrapDev* wraps, const TickShape& s, cudaStream_t stream,
         attribute[0].val.clusterDim.z = 1;
         config.attrs = attribute;
         config.numAttrs = 1;
-        cudaLaunchKernelEx(&config, k_pcg, wraps, index, kPcgMaxSmemBytes / (int)sizeof(float), W, s.grid_nodes);
+        cudaLaunchKernelEx(&config, k_pcg, wraps, index, kPcgMaxSmemBytes / (int)sizeof(float), W, s.grid_nodes,
+                           s.wait_tries);
     };
     if (s.grid_nodes > 0) {
         cudaLaunchConfig_t config = {};
@@ -2525,7 +2540,8 @@ void launch_tick(const WrapDev* wraps, const TickShape& s, cudaStream_t stream,
         attribute[0].val.cooperative = 1;
         config.attrs = attribute;
         config.numAttrs = 1;
-        cudaLaunchKernelEx(&config, k_pcg_grid, wraps, W, s.grid_nodes, kPcgMaxSmemBytes / (int)sizeof(float));
+        cudaLaunchKernelEx(&config, k_pcg_grid, wraps, W, s.grid_nodes, kPcgMaxSmemBytes / (int)sizeof(float),
+                           s.wait_tries);
     }
     if (s.pcg_groups <= 0) {
         launch_pcg(s.pcg_cluster, W, nullptr, stream);

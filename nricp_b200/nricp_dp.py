@@ -146,6 +146,12 @@ class WrapBatch:
         check(load().nricp_batch_tune(self._handle, int(pcg_cluster), C.byref(out)))
         return out.value
 
+    def wait_limit(self, tries: int) -> None:
+        """How often a CTA of the linear solve looks for the data of the CTAs
+        it solves with before it gives up (tries of about 4 us; 2^19 unless
+        set, 0 to give up at once) and its wrap is reported failed."""
+        check(load().nricp_batch_wait_limit(self._handle, int(tries)))
+
     # Candidate cluster settings of the linear solve that autotune() times:
     # per-wrap classes halved once, unhalved, halved twice, and uniform sizes.
     TUNE_CANDIDATES = (-1, 0, -2, 8, 16, 4)
