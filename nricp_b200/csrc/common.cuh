@@ -207,7 +207,7 @@ struct WrapDev {
     float* pcg_s;                 // N x 6: s = A p (by recurrence)
     float* pcg_u;                 // N x 8: u = M^-1 r, every node (six floats a node, eight in a grid solve)
     double* pcg_sums;             // 6 per octet: a grid solve's partial sums
-    unsigned* grid_arrivals;      // its CTAs' meetings this tick
+    unsigned* solve_arrivals;     // this tick's: a grid's CTAs at their meetings, or a cluster's that left the loop
     // reductions
     double* partials;             // energy_blocks x kPartialStride
     double* edge_partials;        // edges: each edge's smoothness energy (the decision kernel sums them)

@@ -514,7 +514,7 @@ size_t prepare_device(Wrap& w, WrapControl* control, cudaStream_t stream, bool p
     D.pcg_s = a.at<float>(o_s);
     D.pcg_u = a.at<float>(o_u);
     D.pcg_sums = a.at<double>(o_sums);
-    D.grid_arrivals = a.at<unsigned>(o_arrivals);
+    D.solve_arrivals = a.at<unsigned>(o_arrivals);
     D.partials = a.at<double>(o_part);
     D.edge_partials = a.at<double>(o_epart);
     D.node_partials = a.at<double>(o_npart);

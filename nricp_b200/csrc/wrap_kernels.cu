@@ -316,7 +316,7 @@ __global__ void __launch_bounds__(kStatsThreads) k_stats(const WrapDev* __restri
     const WrapControl c = *w.control;
     if (!final_mode && threadIdx.x == 0) {
         w.control->tick_phase = c.phase;
-        *w.grid_arrivals = 0;  // the grid solve's meetings of this tick
+        *w.solve_arrivals = 0;
     }
     CorrStats* target = nullptr;
     int level = -1;
@@ -1275,8 +1275,7 @@ __device__ __forceinline__ void pcg_solve(const WrapDev& w, const WrapControl& c
     if (incomplete) give_up();
 
     // The CTAs that own rows; the others only wait at the end.  (Where u is
-    // global the loop meets at cluster barriers, and a graph that large gives
-    // every CTA rows.)
+    // global the loop meets at cluster barriers, and so does the end.)
     const int active = (octets * kOctet + cap - 1) / cap;
     const bool u_shared = !kGrid && (kAllShared || place.u_shared);
     const int u_bytes = ((N * 6 + 3) & ~3) * (int)sizeof(float);  // of every row
@@ -1288,7 +1287,7 @@ __device__ __forceinline__ void pcg_solve(const WrapDev& w, const WrapControl& c
     auto meet = [&]() {     // every active CTA's writes before it are visible after it
         __syncthreads();
         ++meetings;
-        if (threadIdx.x == 0 && !grid_arrive_and_wait(w.grid_arrivals, meetings * (unsigned)active, tries * kPollsPerTry))
+        if (threadIdx.x == 0 && !grid_arrive_and_wait(w.solve_arrivals, meetings * (unsigned)active, tries * kPollsPerTry))
             timed_out = true;
         // the other threads learn of a wait that ran out at the totals' barrier
         __syncthreads();
@@ -1646,8 +1645,25 @@ __device__ __forceinline__ void pcg_solve(const WrapDev& w, const WrapControl& c
         }
     }
     // no CTA may exit while another can still write into its shared memory
-    if (!kGrid) {
+    if (!kGrid && u_shared) {
         cluster.sync();
+    } else if (!kGrid) {
+        // The loop has met at this barrier, so a CTA whose wait ran out would
+        // pair with the others' next meeting and exit while they go on to send
+        // it their sums.  It meets them until every CTA has left the loop,
+        // which their waits for its own sums see to.
+        __shared__ int all_left_s;
+        if (threadIdx.x == 0) atomicAdd(w.solve_arrivals, 1u);  // after the last that this CTA has sent
+        for (;;) {
+            cluster.sync();
+            if (threadIdx.x == 0) {
+                unsigned left;
+                asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(left) : "l"(w.solve_arrivals) : "memory");
+                all_left_s = left >= (unsigned)ranks;
+            }
+            __syncthreads();
+            if (all_left_s) break;
+        }
     } else {
         __syncthreads();
         if (threadIdx.x == 0)  // initialised again for the block's next wrap

@@ -49,6 +49,13 @@ def test_a_solve_that_waits_in_vain_is_reported(dp, device, nodes, cluster):
     _solve_gives_up_and_recovers(dp, _large(nodes), cluster)
 
 
+# u in global memory (above 7,680 nodes): the loop meets at cluster barriers, and
+# a CTA that leaves it early stays until every CTA has left
+@pytest.mark.parametrize("cluster", [16, 4, 1])
+def test_a_solve_that_meets_at_barriers_gives_up_together(dp, device, cluster):
+    _solve_gives_up_and_recovers(dp, _large(8_200), cluster)
+
+
 def test_a_limit_out_of_range_is_refused(dp, device):
     case = S.small_case(seed=3)
     batch = dp.WrapBatch([(*case.args(), case.options)])
