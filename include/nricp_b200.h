@@ -384,6 +384,12 @@ typedef struct NricpGraphLevel {
 int nricp_template_graph(const double* points, int count, int levels, int nodes_initial, int growth,
                          int max_nodes, int edge_neighbours, double* center, double* scale,
                          NricpGraphLevel* out, int use_device);
+/* No reference counterpart.  The same build on the device with a limit of
+ * 0 to 2^19 tries of about 4 us (2^19 otherwise) for each of the waits inside
+ * the farthest-point seeds; an error is reported where one runs out. */
+int nricp_template_graph_within(const double* points, int count, int levels, int nodes_initial, int growth,
+                                int max_nodes, int edge_neighbours, double* center, double* scale,
+                                NricpGraphLevel* out, int wait_tries);
 
 /* farthest_point_seeds(points, count, first_index) (bindings.cpp:796-804,
  * src/core/sampling.cpp:47-88): deterministic farthest-point sampling, ties

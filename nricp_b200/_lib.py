@@ -76,6 +76,8 @@ def _declare(lib: C.CDLL) -> None:
                                                  i32p, C.c_int, P(C.c_int), C.c_int]),
         "nricp_template_graph": (C.c_int, [dp, C.c_int, C.c_int, C.c_int, C.c_int, C.c_int, C.c_int, dp, dp,
                                            P(_abi.GraphLevel), C.c_int]),
+        "nricp_template_graph_within": (C.c_int, [dp, C.c_int, C.c_int, C.c_int, C.c_int, C.c_int, C.c_int, dp, dp,
+                                                  P(_abi.GraphLevel), C.c_int]),
         "nricp_closest_points": (C.c_int, [dp, C.c_int, i32p, C.c_int, dp, C.c_int, dp, dp, dp, i32p]),
         "nricp_fit_rigid": (C.c_int, [dp, dp, dp, C.c_int, dp, dp]),
         "nricp_farthest_point_seeds": (C.c_int, [dp, C.c_int, C.c_int, C.c_int, i32p, P(C.c_int)]),

@@ -354,14 +354,15 @@ int nricp_batch_solve(const NricpSolveDesc* descs, int count, NricpResult* resul
 namespace {
 
 TemplateGraph template_graph(const double* points, int count, int levels, int nodes_initial, int growth, int max_nodes,
-                             int edge_neighbours, bool use_device) {
+                             int edge_neighbours, bool use_device, int wait_tries = kWaitTries) {
     if (count <= 0) throw InvalidArgument("invalid mesh: mesh has no vertices");
     if (max_nodes > NRICP_MAX_SLOTS) throw InvalidArgument("max_nodes_per_vertex exceeds 8");
     if (use_device && device_graph_supported(edge_neighbours)) {
         require_device();
         const StreamLease stream = StreamLease::take();
         return std::move(device_template_graphs(
-            {GraphRequest{points, count, levels, nodes_initial, growth, max_nodes, edge_neighbours}}, stream)[0]);
+            {GraphRequest{points, count, levels, nodes_initial, growth, max_nodes, edge_neighbours}}, stream,
+            wait_tries)[0]);
     }
     return build_template_graph(points, count, levels, nodes_initial, growth, max_nodes, edge_neighbours);
 }
@@ -383,6 +384,16 @@ void copy_level(const GraphLevel& L, int count, int32_t* template_indices, doubl
     *edge_count = E;
     if (E > edge_capacity) throw InvalidArgument("edge buffer too small");
     std::memcpy(edges, L.edges.data(), sizeof(int32_t) * 2 * E);
+}
+
+void copy_graph(const TemplateGraph& g, int count, double* center, double* scale, NricpGraphLevel* out) {
+    for (int k = 0; k < 3; ++k) center[k] = g.center[k];
+    *scale = g.scale;
+    for (size_t l = 0; l < g.levels.size(); ++l) {
+        NricpGraphLevel& o = out[l];
+        copy_level(g.levels[l], count, o.template_indices, o.node_positions, o.bind_nodes, o.bind_weights,
+                   o.bind_counts, o.edges, o.edge_capacity, &o.edge_count);
+    }
 }
 
 }  // namespace
@@ -408,15 +419,18 @@ int nricp_template_graph_level(const double* points, int count, int levels, int 
 int nricp_template_graph(const double* points, int count, int levels, int nodes_initial, int growth, int max_nodes,
                          int edge_neighbours, double* center, double* scale, NricpGraphLevel* out, int use_device) {
     return guarded([&] {
-        const TemplateGraph g =
-            template_graph(points, count, levels, nodes_initial, growth, max_nodes, edge_neighbours, use_device != 0);
-        for (int k = 0; k < 3; ++k) center[k] = g.center[k];
-        *scale = g.scale;
-        for (size_t l = 0; l < g.levels.size(); ++l) {
-            NricpGraphLevel& o = out[l];
-            copy_level(g.levels[l], count, o.template_indices, o.node_positions, o.bind_nodes, o.bind_weights,
-                       o.bind_counts, o.edges, o.edge_capacity, &o.edge_count);
-        }
+        copy_graph(template_graph(points, count, levels, nodes_initial, growth, max_nodes, edge_neighbours,
+                                  use_device != 0), count, center, scale, out);
+    });
+}
+
+int nricp_template_graph_within(const double* points, int count, int levels, int nodes_initial, int growth,
+                                int max_nodes, int edge_neighbours, double* center, double* scale,
+                                NricpGraphLevel* out, int wait_tries) {
+    return guarded([&] {
+        if (wait_tries < 0 || wait_tries > kWaitTries) throw InvalidArgument("the wait limit is 0 to 2^19 tries");
+        copy_graph(template_graph(points, count, levels, nodes_initial, growth, max_nodes, edge_neighbours, true,
+                                  wait_tries), count, center, scale, out);
     });
 }
 

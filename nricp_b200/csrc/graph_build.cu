@@ -78,7 +78,7 @@ __global__ void __launch_bounds__(kFpsThreads, 1) k_fps(const double* __restrict
                                                      const int* __restrict__ seed_count,
                                                      const long* __restrict__ seed_offset,
                                                      const int* __restrict__ templates, int* __restrict__ seeds_all,
-                                                     int* __restrict__ failed) {
+                                                     int* __restrict__ failed, int tries) {
     cg::cluster_group cluster = cg::this_cluster();
     const int t = templates[blockIdx.y];
     const int n = point_count[t];
@@ -138,11 +138,7 @@ __global__ void __launch_bounds__(kFpsThreads, 1) k_fps(const double* __restrict
             warp_key[warp] = key;
             warp_index[warp] = index;
         }
-        if (__syncthreads_or(timed_out)) {
-            if (threadIdx.x == 0) atomicOr(failed, 1);
-            for (int i = 0; i < 256; ++i) __nanosleep(10000);  // the stores in flight
-            break;
-        }
+        if (__syncthreads_or(timed_out)) break;
         if (warp == 0) {
             key = warp_key[lane];  // 32 warps
             index = warp_index[lane];
@@ -162,7 +158,7 @@ __global__ void __launch_bounds__(kFpsThreads, 1) k_fps(const double* __restrict
         }
         int win = 0;
         if (ranks > 1) {
-            if (!mbar_wait(&arrived[set], (s >> 1) & 1, kWaitTries)) timed_out = true;
+            if (!mbar_wait(&arrived[set], (s >> 1) & 1, tries)) timed_out = true;
             key = lane < ranks ? slots[set][lane].key : 0;
             index = lane < ranks ? (int)slots[set][lane].index : INT_MAX;
             const int own = index;
@@ -172,10 +168,15 @@ __global__ void __launch_bounds__(kFpsThreads, 1) k_fps(const double* __restrict
             __syncthreads();
         }
         const FpsCandidate& w = slots[set][max(win, 0)];
-        if (rank == 0 && threadIdx.x == 0) seeds[s + 1] = (int)w.index;
+        if (rank == 0 && threadIdx.x == 0 && !timed_out) seeds[s + 1] = (int)w.index;
         c[0] = w.x;
         c[1] = w.y;
         c[2] = w.z;
+    }
+    // a wait that ran out, the last step's too; the peers' run out in turn
+    if (__syncthreads_or(timed_out)) {
+        if (threadIdx.x == 0) atomicOr(failed, 1);
+        for (int i = 0; i < 256; ++i) __nanosleep(10000);  // the stores in flight (2.6 ms)
     }
     // no CTA leaves while another may still write into its shared memory
     cluster.sync();
@@ -482,7 +483,7 @@ private:
 bool device_graph_supported(int edge_neighbours) { return edge_neighbours <= kMaxEdgeNeighbours; }
 
 std::vector<TemplateGraph> device_template_graphs(const std::vector<GraphRequest>& requests,
-                                                  cudaStream_t stream) {
+                                                  cudaStream_t stream, int wait_tries) {
     const int W = static_cast<int>(requests.size());
     std::vector<TemplateGraph> out(W);
     if (W == 0) return out;
@@ -654,6 +655,9 @@ std::vector<TemplateGraph> device_template_graphs(const std::vector<GraphRequest
         }();
         (void)enabled;
         check(cudaMemsetAsync(d_failed, 0, sizeof(int), stream), "farthest-point seeds");
+        // where a wait runs out the rest of the seeds stay the first point:
+        // the kernels that follow read points by them before the host knows
+        check(cudaMemsetAsync(d_seeds, 0, seed_bytes, stream), "farthest-point seeds");
         cudaEvent_t fork = nullptr;
         check(cudaEventCreateWithFlags(&fork, cudaEventDisableTiming), "event");
         check(cudaEventRecord(fork, stream), "event");
@@ -686,7 +690,7 @@ std::vector<TemplateGraph> device_template_graphs(const std::vector<GraphRequest
                 config.numAttrs = 1;
                 check(cudaLaunchKernelEx(&config, kernels[k % 4], (const double*)d_points,
                                          longs(o_point_offset), ints(o_point_count), ints(o_seed_count),
-                                         longs(o_seed_offset), ints(o_class[k]), d_seeds, d_failed),
+                                         longs(o_seed_offset), ints(o_class[k]), d_seeds, d_failed, wait_tries),
                       "farthest-point seeds");
             });
         }

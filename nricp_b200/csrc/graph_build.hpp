@@ -6,6 +6,7 @@
 
 #include <cuda_runtime.h>
 
+#include "common.cuh"
 #include "host.hpp"
 
 namespace nricp_b200 {
@@ -20,7 +21,8 @@ struct GraphRequest {
 bool device_graph_supported(int edge_neighbours);
 
 // One graph per request, in order; runs on `stream` and returns when done.
+// `wait_tries`: limit of the waits inside the seeds' kernel (StateError).
 std::vector<TemplateGraph> device_template_graphs(const std::vector<GraphRequest>& requests,
-                                                  cudaStream_t stream);
+                                                  cudaStream_t stream, int wait_tries = kWaitTries);
 
 }  // namespace nricp_b200

@@ -6,12 +6,15 @@ arrive.
 
 from __future__ import annotations
 
+import ctypes as C
 import time
 
 import numpy as np
 import pytest
 
+from nricp_b200 import _abi
 from nricp_b200 import synthetic as S
+from nricp_b200._lib import check, load
 
 pytestmark = pytest.mark.gpu
 
@@ -62,3 +65,29 @@ def test_a_limit_out_of_range_is_refused(dp, device):
     for tries in (-1, (1 << 19) + 1):
         with pytest.raises(ValueError):
             batch.wait_limit(tries)
+
+
+def _seeds_within(points, nodes, tries):
+    """The seeds of one level of `nodes` nodes, built with this wait limit."""
+    n = len(points)
+    P = lambda a, t: a.ctypes.data_as(C.POINTER(t))  # noqa: E731
+    level = {"indices": np.full(nodes, -1, dtype=np.int32), "positions": np.empty((nodes, 3)),
+             "nodes": np.empty((n, _abi.MAX_SLOTS), dtype=np.int32), "weights": np.empty((n, _abi.MAX_SLOTS)),
+             "counts": np.empty(n, dtype=np.int32), "edges": np.empty((nodes * 4, 2), dtype=np.int32)}
+    out = _abi.GraphLevel(P(level["indices"], C.c_int32), P(level["positions"], C.c_double),
+                          P(level["nodes"], C.c_int32), P(level["weights"], C.c_double),
+                          P(level["counts"], C.c_int32), P(level["edges"], C.c_int32), nodes * 4, 0)
+    center, scale = np.zeros(3), C.c_double()
+    check(load().nricp_template_graph_within(P(points, C.c_double), n, 1, nodes, 2, 4, 4, P(center, C.c_double),
+                                             C.byref(scale), C.byref(out), tries))
+    return level["indices"]
+
+
+# 2 seeds: the only wait is the last step's
+@pytest.mark.parametrize("points, nodes", [(3_000, 2), (3_000, 3), (30_000, 40), (100_000, 2)])
+def test_seeds_that_wait_in_vain_are_reported(dp, device, points, nodes):
+    p = np.random.default_rng(points).normal(size=(points, 3))
+    with pytest.raises(RuntimeError, match="a wait inside the farthest-point seeds ran out"):
+        _seeds_within(p, nodes, 0)
+    after = _seeds_within(p, nodes, 1 << 19)
+    assert np.array_equal(after, dp.farthest_point_seeds(p, nodes))
