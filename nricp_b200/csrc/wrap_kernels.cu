@@ -16,6 +16,7 @@
 #include "async.cuh"
 #include "common.cuh"
 #include "kernels.cuh"
+#include "solve_layout.hpp"
 
 #include <cooperative_groups.h>
 
@@ -28,7 +29,6 @@ namespace {
 constexpr int kVertexThreads = 256;
 constexpr int kNodeThreads = 256;   // 8 warps = 8 nodes per block
 constexpr int kEdgeSums = 128;      // edges per partial sum of the smoothness energy
-constexpr int kPcgThreads = 512;
 constexpr int kStatsThreads = 512;
 
 // Which branch of a tick handles a wrap: part 0 every wrap (one chain), 1 the
@@ -888,19 +888,6 @@ __device__ inline void solve6(const float* l, const double* rhs, double* x) {
     for (int r = 0; r < 6; ++r) x[r] = z[r];
 }
 
-// ---- the solve's partition and shared-memory layout ------------------------
-//
-// Rows are grouped into segments of kSegNodes nodes (24 rows: one pass of a
-// warp; 4-node segments balance the warps better than 8-node ones, 0.90 s
-// against 0.93 s per 64-wrap batch, and 16-node ones are slower).  A segment is
-// the unit of ownership and of reduction: one warp forms the segment's FP64
-// partial dot products in a fixed lane order, and the cluster sums the
-// segments' partials in a fixed order.  A CTA owns a contiguous run of
-// segments, so the cluster size only decides which CTA computes which
-// segment, never the order of any sum: a wrap's solve is bit-identical for
-// every cluster size, and with it alone and in any batch.
-constexpr int kSegNodes = 4;
-
 // The solve's reductions -- the dot products, the residual norm, the Krylov
 // scalars and the x and r vectors -- are FP64.  A build with
 // NRICP_FP32_REDUCTIONS defined rounds every one of those operations to FP32
@@ -916,56 +903,6 @@ __device__ __forceinline__ double warp_sum_rnd(double v) {
     for (int o = 16; o > 0; o >>= 1) v = rnd(v + __shfl_xor_sync(0xffffffffu, v, o));
     return v;
 }
-constexpr int kPcgWarps = kPcgThreads / 32;
-// Shared floats per owned node: X, R (2 x 6 FP64), P, S, W (18), its row's
-// entry count and (one per octet each) the octet's first step and steps, padded.
-constexpr int kPcgVectorFloats = 44;
-constexpr int kPcgBlockFloats = 36;   // its damped diagonal block; and its inverse
-// Dynamic shared memory of every solve launch: all there is.  A solve CTA holds
-// its SM alone (512 threads of 128 registers), and what the vectors leave
-// holds off-diagonal blocks.
-constexpr int kPcgMaxSmemBytes = 225 * 1024;
-constexpr int kOctet = 8;             // nodes a warp multiplies at a time (24 of its lanes)
-
-__host__ __device__ inline int pcg_segments(int nodes) { return (nodes + kSegNodes - 1) / kSegNodes; }
-__host__ __device__ inline int pcg_octets(int nodes) { return (nodes + kOctet - 1) / kOctet; }
-// FP64 slots for the segments' three partials (two segments per octet)
-__host__ __device__ inline int pcg_slot_doubles(int nodes) { return 6 * pcg_octets(nodes); }
-
-// Owned-node capacity of one CTA when `ranks` CTAs share the solve.
-__host__ __device__ inline int pcg_owned_capacity(int nodes, int ranks) {
-    return (pcg_octets(nodes) + ranks - 1) / ranks * kOctet;
-}
-
-// Placement for one wrap within the launch's shared memory, in this order:
-// the segment slots always, the all-node direction copy U if it fits (the
-// matvec reads it ~20 times per row), the owned rows' vectors, their diagonal
-// blocks, the inverses of those, and what is left for the last steps of every
-// owned octet's off-diagonal blocks.  Whatever does not fit lives in the wrap's
-// global scratch; the arithmetic is the same.
-struct PcgPlacement {
-    bool u_shared, vectors_shared, diagonal_shared, inverse_shared;
-    __device__ bool all() const { return u_shared && vectors_shared && diagonal_shared && inverse_shared; }
-    int floats;  // shared floats used before the blocks
-};
-__device__ inline PcgPlacement pcg_place(int nodes, int ranks, int budget_floats) {
-    PcgPlacement p;
-    int used = pcg_slot_doubles(nodes) * 2;
-    const int u = (nodes * 6 + 3) & ~3;
-    const int cap = pcg_owned_capacity(nodes, ranks);
-    auto take = [&](int floats) {
-        const bool fits = used + floats <= budget_floats;
-        if (fits) used += floats;
-        return fits;
-    };
-    p.u_shared = take(u);
-    p.vectors_shared = take(cap * kPcgVectorFloats);
-    p.diagonal_shared = take(cap * kPcgBlockFloats);
-    p.inverse_shared = take(cap * kPcgBlockFloats);
-    p.floats = used;
-    return p;
-}
-
 // Inverse of a 6x6 SPD block from its Cholesky factor L (lower): L^-T L^-1.
 __device__ inline void cholesky_inverse6(const float* l, float* inv) {
     float li[36];
@@ -1017,7 +954,6 @@ __device__ __forceinline__ void copy_16_async(void* dst, const void* src) {
                  : "memory");
 }
 __device__ __forceinline__ void wait_copies() { asm volatile("cp.async.wait_all;" ::: "memory"); }
-constexpr int kGatherSteps = 16;  // steps whose u a warp of a grid solve gathers at a time
 
 // One thread's part of a meeting of a cooperative grid's CTAs: counts its CTA
 // in and waits, at most `polls` times, until `target` have come.
@@ -1082,7 +1018,7 @@ struct StepBlocks {
 template <bool kAllShared, bool kGrid>
 __device__ __forceinline__ void pcg_solve(const WrapDev& w, const WrapControl& c, const PcgPlacement& place,
                                           int budget_floats, int tries) {
-    static_assert(kAllShared || !kGrid, "the grid's own rows fit");
+    static_assert(kAllShared || !kGrid, "a grid whose rows would not fit is not launched (pcg_grid_fits)");
     cg::cluster_group cluster = cg::this_cluster();
     const LevelDev& L = w.levels[c.level];
     const int N = L.node_count;
@@ -1696,8 +1632,7 @@ __global__ void __launch_bounds__(kPcgThreads, 1) k_pcg_grid(const WrapDev* __re
         const int N = w.levels[c.level].node_count;
         if (!grid_takes(wraps, wrap_count, N, grid_nodes)) continue;
         PcgPlacement place = {};
-        place.floats = pcg_owned_capacity(N, (int)gridDim.x) * (6 + kPcgVectorFloats + 2 * kPcgBlockFloats) +
-                       kPcgWarps * kGatherSteps * 64;
+        place.floats = pcg_grid_floats(N, (int)gridDim.x);
         pcg_solve<true, true>(w, c, place, budget_floats, tries);
         __syncthreads();  // shared memory of one wrap before the next
     }
@@ -2542,7 +2477,7 @@ void launch_tick(const WrapDev* wraps, const TickShape& s, cudaStream_t stream,
         attribute[0].val.clusterDim.z = 1;
         config.attrs = attribute;
         config.numAttrs = 1;
-        cudaLaunchKernelEx(&config, k_pcg, wraps, index, kPcgMaxSmemBytes / (int)sizeof(float), W, s.grid_nodes,
+        cudaLaunchKernelEx(&config, k_pcg, wraps, index, kPcgMaxSmemFloats, W, s.grid_nodes,
                            s.wait_tries);
     };
     if (s.grid_nodes > 0) {
@@ -2556,7 +2491,7 @@ void launch_tick(const WrapDev* wraps, const TickShape& s, cudaStream_t stream,
         attribute[0].val.cooperative = 1;
         config.attrs = attribute;
         config.numAttrs = 1;
-        cudaLaunchKernelEx(&config, k_pcg_grid, wraps, W, s.grid_nodes, kPcgMaxSmemBytes / (int)sizeof(float),
+        cudaLaunchKernelEx(&config, k_pcg_grid, wraps, W, s.grid_nodes, kPcgMaxSmemFloats,
                            s.wait_tries);
     }
     if (s.pcg_groups <= 0) {
@@ -2682,7 +2617,7 @@ void grid_solve_shape(TickShape& shape) {
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
     cudaDeviceGetAttribute(&cooperative, cudaDevAttrCooperativeLaunch, device);
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_pcg_grid, kPcgThreads, kPcgMaxSmemBytes);
-    if (!cooperative || per_sm < 1) {
+    if (!cooperative || per_sm < 1 || !pcg_grid_fits(shape.max_nodes, sms)) {
         shape.grid_nodes = 0;
         return;
     }
