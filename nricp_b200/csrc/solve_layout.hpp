@@ -47,14 +47,18 @@ NRICP_HOST_DEVICE inline int pcg_owned_capacity(int nodes, int ranks) {
 
 // Placement for one wrap within the launch's shared memory, in this order:
 // the segment slots always, the all-node direction copy U if it fits (the
-// matvec reads it ~20 times per row), the owned rows' vectors, their diagonal
-// blocks, the inverses of those, and what is left for the last steps of every
-// owned octet's off-diagonal blocks.  Whatever does not fit lives in the wrap's
-// global scratch; the arithmetic is the same.
+// matvec reads it ~20 times per row), the owned rows' vectors, the inverses of
+// their diagonal blocks, if all of these fit those blocks themselves, and what
+// is left for the last steps of every owned octet's off-diagonal blocks.
+// Whatever does not fit lives in the wrap's global scratch, and the diagonal
+// blocks are then read from the system; the arithmetic is the same.  (The
+// instance without all arrays in shared memory never reads the blocks there.
+// With their 36 to 54 KB left to off-diagonal steps an iteration takes, 3,000
+// nodes on 8 CTAs, 26.4 -> 25.2 us; 3,100 30.3 -> 28.9; 4,200 on 16 25.6 -> 24.9.)
 struct PcgPlacement {
     bool u_shared, vectors_shared, diagonal_shared, inverse_shared;
     int floats;  // shared floats used before the blocks
-    NRICP_HOST_DEVICE bool all() const { return u_shared && vectors_shared && diagonal_shared && inverse_shared; }
+    NRICP_HOST_DEVICE bool all() const { return diagonal_shared; }
 };
 NRICP_HOST_DEVICE inline PcgPlacement pcg_place(int nodes, int ranks, int budget_floats) {
     PcgPlacement p;
@@ -68,8 +72,8 @@ NRICP_HOST_DEVICE inline PcgPlacement pcg_place(int nodes, int ranks, int budget
     };
     p.u_shared = take(u);
     p.vectors_shared = take(cap * kPcgVectorFloats);
-    p.diagonal_shared = take(cap * kPcgBlockFloats);
     p.inverse_shared = take(cap * kPcgBlockFloats);
+    p.diagonal_shared = p.u_shared && p.vectors_shared && p.inverse_shared && take(cap * kPcgBlockFloats);
     p.floats = used;
     return p;
 }

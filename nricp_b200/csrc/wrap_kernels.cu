@@ -1077,7 +1077,7 @@ __device__ __forceinline__ void pcg_solve(const WrapDev& w, const WrapControl& c
         S = w.pcg_s + n0 * 6;
         Wv = w.pcg_ap + n0 * 6;
     }
-    if (kAllShared || place.diagonal_shared) {
+    if (kAllShared) {
         diagonal = cursor;
         cursor += cap * kPcgBlockFloats;
     }

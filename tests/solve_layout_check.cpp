@@ -26,6 +26,13 @@ int main() {
             expect(cap % 8 == 0 && (long)cap * ctas >= n, "every node is owned", n, ctas);
             const PcgPlacement p = pcg_place(n, ctas, kPcgMaxSmemFloats);
             expect(p.floats <= kPcgMaxSmemFloats, "a cluster's arrays fit", n, ctas);
+            // only what the instance reads is taken: the damped diagonal blocks
+            // are in shared memory with everything else or not at all
+            const int slots = 12 * ((n + 7) / 8), u = (n * 6 + 3) / 4 * 4;
+            const int read = slots + (p.u_shared ? u : 0) + (p.vectors_shared ? cap * 44 : 0) +
+                             (p.inverse_shared ? cap * 36 : 0) + (p.all() ? cap * 36 : 0);
+            expect(p.floats == read, "nothing is taken that is not read", n, ctas);
+            expect(p.all() == (slots + u + cap * (44 + 72) <= kPcgMaxSmemFloats), "all arrays where they fit", n, ctas);
         }
         // the whole device: what the kernel carves, array by array
         for (int ctas : {16, 64, 97, 98, 132, 148, 160}) {
