@@ -1031,7 +1031,7 @@ __device__ __forceinline__ void pcg_solve(const WrapDev& w, const WrapControl& c
     const int o1 = min(octets, o0 + cap / kOctet);
     const int n0 = o0 * kOctet;
     const int n1 = min(N, o1 * kOctet);
-    const int own = n1 > n0 ? n1 - n0 : 0;
+    int own = n1 > n0 ? n1 - n0 : 0;
     const int rows = own * 6;
 
     extern __shared__ float4 dynamic_shared[];
@@ -1208,7 +1208,10 @@ __device__ __forceinline__ void pcg_solve(const WrapDev& w, const WrapControl& c
         mbar_wait(&blocks_arrived, 0, kWaitTries);  // this CTA's own copies
         for (int i = 0; i < 256; ++i) __nanosleep(10000);  // and those it sent to its peers (2.6 ms)
     };
-    if (incomplete) give_up();
+    if (incomplete) {
+        give_up();
+        own = 0;  // skips the loop
+    }
 
     // The CTAs that own rows; the others only wait at the end.  (Where u is
     // global the loop meets at cluster barriers, and so does the end.)
@@ -1313,8 +1316,7 @@ __device__ __forceinline__ void pcg_solve(const WrapDev& w, const WrapControl& c
             if (!kGrid) fetch(shape.first, 0, min(shape.streamed, shape.degree));
         }
     };
-    const bool solving = own > 0 && !incomplete;
-    if (solving) {
+    if (own > 0) {
         segment_rows([](int) {});
         share_u();
         fetch_first();
@@ -1323,7 +1325,7 @@ __device__ __forceinline__ void pcg_solve(const WrapDev& w, const WrapControl& c
     double gamma_prev = 0.0, alpha_prev = 0.0, bnorm = 0.0, residual = 0.0, surely_above = 0.0;
     int iterations = 0;
     bool converged = false;
-    for (int it = 0; solving; ++it) {
+    for (int it = 0; own > 0; ++it) {
         if (u_shared && active > 1 && !mbar_wait(&u_arrived, it & 1, tries)) timed_out = true;
         // ---- w = A u for the owned rows, an octet per warp at a time: lane
         //      3i + p multiplies rows 2p and 2p + 1 of the octet's node i ----
