@@ -18,7 +18,7 @@ LIB = HERE / "libnricp_b200.so"
 SOURCES = ["host.cpp", "lbvh.cu", "wrap_kernels.cu", "graph_build.cu", "session.cu", "capi.cu",
            "static_scratch.cu"]
 HEADERS = ["async.cuh", "common.cuh", "kernels.cuh", "host.hpp", "session.hpp", "graph_build.hpp",
-           "resources.hpp", "solve_layout.hpp", "staging.hpp"]
+           "per_device.hpp", "resources.hpp", "solve_layout.hpp", "staging.hpp"]
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 
 

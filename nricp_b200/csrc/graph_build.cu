@@ -17,6 +17,7 @@
 
 #include "async.cuh"
 #include "graph_build.hpp"
+#include "per_device.hpp"
 #include "resources.hpp"
 #include "session.hpp"
 #include "staging.hpp"
@@ -645,15 +646,16 @@ std::vector<TemplateGraph> device_template_graphs(const std::vector<GraphRequest
     {
         using FpsKernel = decltype(&k_fps<1>);
         static const FpsKernel kernels[4] = {k_fps<1>, k_fps<2>, k_fps<4>, k_fps<8>};
-        static const bool enabled = [] {
+        static PerDevice<bool>& enabled = *new PerDevice<bool>;
+        enabled.of(device, [] {
             for (int k = 0; k < 4; ++k) {
-                cudaFuncSetAttribute(kernels[k], cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
-                cudaFuncSetAttribute(kernels[k], cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     24 * kFpsThreads * (1 << k));
+                check(cudaFuncSetAttribute(kernels[k], cudaFuncAttributeNonPortableClusterSizeAllowed, 1),
+                      "farthest-point seeds' attributes");
+                check(cudaFuncSetAttribute(kernels[k], cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                           24 * kFpsThreads * (1 << k)), "farthest-point seeds' attributes");
             }
             return true;
-        }();
-        (void)enabled;
+        });
         check(cudaMemsetAsync(d_failed, 0, sizeof(int), stream), "farthest-point seeds");
         // where a wait runs out the rest of the seeds stay the first point:
         // the kernels that follow read points by them before the host knows

@@ -19,8 +19,11 @@
 
 #include "common.cuh"
 #include "kernels.cuh"
+#include "per_device.hpp"
 
 namespace nricp_b200 {
+
+void check(cudaError_t status, const char* what);  // throws CudaError (session.cu)
 
 namespace {
 
@@ -1173,18 +1176,25 @@ __global__ void __launch_bounds__(128) k_closest_points(const WrapDev* __restric
     out_triangles[i] = tri;
 }
 
+// Blocks of 128 threads of `kernel` that fit on the current device at once.
+template <typename Kernel>
+static int resident_blocks(PerDevice<int>& of_device, Kernel kernel, size_t shared_bytes) {
+    int device = 0;
+    check(cudaGetDevice(&device), "device");
+    return of_device.of(device, [&] {
+        int sms = 0, per_sm = 0;
+        check(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device), "device");
+        check(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, 128, shared_bytes), "occupancy");
+        const int blocks = sms * (per_sm > 0 ? per_sm : 1);
+        return blocks > 0 ? blocks : 1;
+    });
+}
+
 void launch_query(const WrapDev* wraps, int wrap_count, cudaStream_t stream, int* counter) {
     // the warps' stacks, then two scans over the wraps (1024 at most)
     constexpr size_t kStackBytes = (sizeof(uint32_t) + sizeof(float)) * kWarpStack * 4;
-    static const int resident = [] {  // blocks of the queue that fit on the device at once
-        int device = 0, sms = 0, per_sm = 0;
-        cudaGetDevice(&device);
-        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_query_queue, 128,
-                                                      kStackBytes + 2 * sizeof(int) * 1025);
-        const int blocks = sms * (per_sm > 0 ? per_sm : 1);
-        return blocks > 0 ? blocks : 1;
-    }();
+    static PerDevice<int>& of_device = *new PerDevice<int>;
+    const int resident = resident_blocks(of_device, k_query_queue, kStackBytes + 2 * sizeof(int) * 1025);
     cudaMemsetAsync(counter, 0, 2 * sizeof(int), stream);
     k_query_queue<<<resident, 128, kStackBytes + 2 * sizeof(int) * (wrap_count + 1), stream>>>(
         wraps, wrap_count, counter);
@@ -1193,13 +1203,8 @@ void launch_query(const WrapDev* wraps, int wrap_count, cudaStream_t stream, int
 void launch_closest_points(const WrapDev* wrap, const double* queries, int count,
                            double* points, double* normals, double* distances, int32_t* triangles,
                            int* overflow, cudaStream_t stream) {
-    static const long resident = [] {
-        int device = 0, sms = 148, per_sm = 0;
-        cudaGetDevice(&device);
-        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_closest_points<8>, 128, 0);
-        return 128L * sms * (per_sm > 0 ? per_sm : 1);
-    }();
+    static PerDevice<int>& of_device = *new PerDevice<int>;
+    const long resident = 128L * resident_blocks(of_device, k_closest_points<8>, 0);
     auto launch = [&](auto kernel, int lanes) {
         kernel<<<blocks_for((long)count * lanes, 128), 128, 0, stream>>>(wrap, queries, count, points, normals, distances,
                                                                    triangles, overflow);
@@ -1231,8 +1236,6 @@ __global__ void k_check_faces(const int32_t* __restrict__ faces, int count, int 
 }
 
 }  // namespace
-
-void check(cudaError_t status, const char* what);  // throws CudaError (session.cu)
 
 size_t lbvh_export_scratch_bytes(int n) {
     const size_t pieces[] = {

@@ -16,15 +16,24 @@
 #include "async.cuh"
 #include "common.cuh"
 #include "kernels.cuh"
+#include "per_device.hpp"
 #include "solve_layout.hpp"
 
 #include <cooperative_groups.h>
 
 namespace nricp_b200 {
 
+void check(cudaError_t status, const char* what);  // throws CudaError (session.cu)
+
 namespace cg = cooperative_groups;
 
 namespace {
+
+int current_device() {
+    int device = 0;
+    check(cudaGetDevice(&device), "device");
+    return device;
+}
 
 constexpr int kVertexThreads = 256;
 constexpr int kNodeThreads = 256;   // 8 warps = 8 nodes per block
@@ -2399,13 +2408,15 @@ struct VirtualGrids {
     int prologue, c_fit, c_deform, c_rhs, evaluate, normals, residual, candidate, assemble;
 };
 const VirtualGrids& virtual_grids() {
-    static const VirtualGrids grids = [] {
-        int device = 0, sms = 148;
-        cudaGetDevice(&device);
-        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
+    static PerDevice<VirtualGrids>& grids = *new PerDevice<VirtualGrids>;
+    const int device = current_device();
+    return grids.of(device, [device] {
+        int sms = 148;
+        check(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device), "device");
         auto fit = [sms](auto kernel, int threads) {
             int per_sm = 0;
-            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, threads, sizeof(int) * 1025);
+            check(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, threads, sizeof(int) * 1025),
+                  "occupancy");
             return sms * (per_sm > 0 ? per_sm : 1);
         };
         VirtualGrids g;
@@ -2419,8 +2430,7 @@ const VirtualGrids& virtual_grids() {
         g.candidate = fit(k_residual<true>, kVertexThreads);
         g.assemble = fit(k_assemble, kNodeThreads);
         return g;
-    }();
-    return grids;
+    });
 }
 
 void launch_tick(const WrapDev* wraps, const TickShape& s, cudaStream_t stream,
@@ -2547,14 +2557,17 @@ int pcg_class_cluster(int nodes, int shift) {
     return std::max(1, shift > 0 ? ranks >> shift : ranks);
 }
 
+// The solve kernels' launch attributes, on the current device.
 void pcg_enable() {
-    static const bool enabled = [] {  // once per process, thread-safe
-        cudaFuncSetAttribute(k_pcg, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
-        cudaFuncSetAttribute(k_pcg, cudaFuncAttributeMaxDynamicSharedMemorySize, kPcgMaxSmemBytes);
-        cudaFuncSetAttribute(k_pcg_grid, cudaFuncAttributeMaxDynamicSharedMemorySize, kPcgMaxSmemBytes);
+    static PerDevice<bool>& enabled = *new PerDevice<bool>;
+    enabled.of(current_device(), [] {
+        check(cudaFuncSetAttribute(k_pcg, cudaFuncAttributeNonPortableClusterSizeAllowed, 1), "solve attributes");
+        check(cudaFuncSetAttribute(k_pcg, cudaFuncAttributeMaxDynamicSharedMemorySize, kPcgMaxSmemBytes),
+              "solve attributes");
+        check(cudaFuncSetAttribute(k_pcg_grid, cudaFuncAttributeMaxDynamicSharedMemorySize, kPcgMaxSmemBytes),
+              "solve attributes");
         return true;
-    }();
-    (void)enabled;
+    });
 }
 
 // One over the clusters that run at once: a cluster's CTAs sit in one group of
@@ -2563,7 +2576,8 @@ double pcg_cluster_share(int cluster) {
     struct Shares {
         double of[5];
     };
-    static const Shares shares = [] {
+    static PerDevice<Shares>& of_device = *new PerDevice<Shares>;
+    const Shares& shares = of_device.of(current_device(), [] {
         pcg_enable();
         Shares s{};
         for (int i = 0; i < 5; ++i) {
@@ -2579,11 +2593,14 @@ double pcg_cluster_share(int cluster) {
             config.attrs = attribute;
             config.numAttrs = 1;
             int clusters = 0;
-            cudaOccupancyMaxActiveClusters(&clusters, k_pcg, &config);
+            if (cudaOccupancyMaxActiveClusters(&clusters, k_pcg, &config) != cudaSuccess) {
+                cudaGetLastError();  // not a size for this device: it takes all of it
+                clusters = 0;
+            }
             s.of[i] = 1.0 / std::max(1, clusters);
         }
         return s;
-    }();
+    });
     int i = 0;
     while (i < 4 && (1 << i) < cluster) ++i;
     return shares.of[i];
@@ -2614,11 +2631,12 @@ void grid_solve_shape(TickShape& shape) {
     shape.grid_ctas = 0;
     if (!shape.grid_nodes) return;
     pcg_enable();
-    int device = 0, sms = 0, cooperative = 0, per_sm = 0;
-    cudaGetDevice(&device);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
-    cudaDeviceGetAttribute(&cooperative, cudaDevAttrCooperativeLaunch, device);
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_pcg_grid, kPcgThreads, kPcgMaxSmemBytes);
+    const int device = current_device();
+    int sms = 0, cooperative = 0, per_sm = 0;
+    check(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device), "device");
+    check(cudaDeviceGetAttribute(&cooperative, cudaDevAttrCooperativeLaunch, device), "device");
+    check(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_pcg_grid, kPcgThreads, kPcgMaxSmemBytes),
+          "occupancy");
     if (!cooperative || per_sm < 1 || !pcg_grid_fits(shape.max_nodes, sms)) {
         shape.grid_nodes = 0;
         return;
