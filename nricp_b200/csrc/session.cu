@@ -36,8 +36,9 @@ thread_local std::string g_last_error;
 thread_local TransferCounters g_transfers;
 
 void check(cudaError_t status, const char* what) {
-    if (status != cudaSuccess)
-        throw CudaError(std::string("CUDA error in ") + what + ": " + cudaGetErrorString(status));
+    if (status == cudaSuccess) return;
+    cudaGetLastError();  // reported here: not again by the thread's next look at its last error
+    throw CudaError(std::string("CUDA error in ") + what + ": " + cudaGetErrorString(status));
 }
 
 namespace {
@@ -582,6 +583,35 @@ int target_build_launches(const Wrap& w) { return lbvh_build_launches(w.F); }
 // ---------------------------------------------------------------------------
 // Batch
 // ---------------------------------------------------------------------------
+namespace {
+
+// The tick as a graph.  A launch that is refused spoils the capture, which is
+// ended all the same, and is what is reported.
+cudaGraphExec_t capture_tick(const WrapDev* wraps, const TickShape& shape, cudaStream_t stream) {
+    cudaGraph_t graph = nullptr;
+    cudaGraphExec_t exec = nullptr;
+    cudaGetLastError();  // an earlier call's, of whoever shares this thread
+    check(cudaStreamBeginCapture(stream, cudaStreamCaptureModeThreadLocal), "capture");
+    std::string thrown;
+    try {
+        launch_tick(wraps, shape, stream, nullptr);
+    } catch (const std::exception& e) {
+        thrown = e.what();
+    }
+    const cudaError_t launched = cudaGetLastError();
+    cudaError_t status = cudaStreamEndCapture(stream, &graph);
+    if (thrown.empty() && launched == cudaSuccess && status == cudaSuccess)
+        status = cudaGraphInstantiate(&exec, graph, 0);
+    if (graph) cudaGraphDestroy(graph);
+    if (status != cudaSuccess) cudaGetLastError();
+    if (!thrown.empty()) throw CudaError(thrown);
+    check(launched, "tick launch");
+    check(status, "tick graph");
+    return exec;
+}
+
+}  // namespace
+
 Batch::Batch() : stream_(StreamLease::take()) {}
 
 Batch::~Batch() {
@@ -962,19 +992,8 @@ bool Batch::tail_due() const {
     return tail_fine_ ? share <= 1.0 : ctas <= sms_;
 }
 
-cudaGraphExec_t Batch::capture(const TickShape& shape) {
-    cudaGraph_t graph = nullptr;
-    cudaGraphExec_t exec = nullptr;
-    check(cudaStreamBeginCapture(stream_, cudaStreamCaptureModeThreadLocal), "capture");
-    launch_tick(dev_wraps_, shape, stream_, nullptr);
-    check(cudaStreamEndCapture(stream_, &graph), "capture end");
-    check(cudaGraphInstantiate(&exec, graph, 0), "graph instantiate");
-    cudaGraphDestroy(graph);
-    return exec;
-}
-
 void Batch::run(int max_ticks) {
-    if (!graph_exec_) graph_exec_ = capture(shape_);
+    if (!graph_exec_) graph_exec_ = capture_tick(dev_wraps_, shape_, stream_);
     pull_controls();
     tail_on_ = false;
     int chunk = 4;
@@ -982,7 +1001,7 @@ void Batch::run(int max_ticks) {
         if (ticks_ >= max_ticks) throw StateError("the schedule did not finish within the tick limit");
         if (!tail_on_ && tail_ready_ && tail_due()) {
             tail_on_ = true;
-            if (!tail_graph_) tail_graph_ = capture(tail_shape_);
+            if (!tail_graph_) tail_graph_ = capture_tick(dev_wraps_, tail_shape_, stream_);
         }
         for (int i = 0; i < chunk; ++i) {
             check(cudaGraphLaunch(tail_on_ ? tail_graph_ : graph_exec_, stream_), "graph launch");
@@ -1583,13 +1602,7 @@ struct Server::Impl {
             t.pcg_groups = class_count;
             t.pcg_cluster = class_top;
         }
-        cudaGraph_t g = nullptr;
-        cudaGraphExec_t exec = nullptr;
-        check(cudaStreamBeginCapture(stream, cudaStreamCaptureModeThreadLocal), "capture");
-        launch_tick(dev_wraps, t, stream, nullptr);
-        check(cudaStreamEndCapture(stream, &g), "capture end");
-        check(cudaGraphInstantiate(&exec, g, 0), "graph instantiate");
-        cudaGraphDestroy(g);
+        const cudaGraphExec_t exec = capture_tick(dev_wraps, t, stream);
         captures += 1;
         launches_per_tick[count] = tick_kernel_launches(t);
         graphs[count] = exec;

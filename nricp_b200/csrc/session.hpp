@@ -130,7 +130,6 @@ private:
     // Solve launch fields of `shape` for the cluster setting `cluster` (as
     // set_pcg_cluster takes it), its class lists in `index` (device); `cls` (if given) receives each wrap's cluster size.
     void solve_shape(int cluster, TickShape& shape, int* index, std::vector<int>* cls);
-    cudaGraphExec_t capture(const TickShape& shape);
     void drop_graphs();
     // The batch's tail.  Once the wraps still running would fit on the SMs in
     // one round at classes one step finer, their ticks run from a second graph
