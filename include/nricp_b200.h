@@ -150,6 +150,12 @@ int nricp_transfer_counters(unsigned long long* h2d, unsigned long long* d2h, in
 /* device_info(), src/python/bindings.cpp:1614-1622. */
 int nricp_device_info(int* available, char* description, size_t capacity);
 
+/* No reference counterpart.  Every call that uses the device takes its memory
+ * from a pool per device that keeps up to 8 GB between calls; this gives back
+ * what no batch, session or call holds, after waiting for the device (a
+ * server's own pool is given back with the server). */
+int nricp_release_memory(void);
+
 /* Node count per level for a descriptor (src/core/graph.cpp:52-57): sizes the
  * caller's result buffers.  `level_count` receives the number of levels. */
 int nricp_plan(const NricpSolveDesc* desc, int32_t* level_nodes, int capacity,

@@ -47,6 +47,7 @@ def _declare(lib: C.CDLL) -> None:
         "nricp_last_error": (C.c_char_p, []),
         "nricp_transfer_counters": (C.c_int, [P(C.c_ulonglong), P(C.c_ulonglong), C.c_int]),
         "nricp_device_info": (C.c_int, [P(C.c_int), C.c_char_p, C.c_size_t]),
+        "nricp_release_memory": (C.c_int, []),
         "nricp_plan": (C.c_int, [desc_p, i32p, C.c_int, P(C.c_int)]),
         "nricp_solve": (C.c_int, [desc_p, result_p]),
         "nricp_session_create": (C.c_int, [desc_p, P(C.c_void_p)]),

@@ -149,6 +149,10 @@ int nricp_device_info(int* available, char* description, size_t capacity) {
     });
 }
 
+int nricp_release_memory(void) {
+    return guarded([&] { release_pools(); });
+}
+
 int nricp_plan(const NricpSolveDesc* desc, int32_t* level_nodes, int capacity, int* level_count) {
     return guarded([&] {
         const int levels = desc->graph_levels > 1 ? desc->graph_levels : 1;

@@ -22,13 +22,20 @@ void check(cudaError_t status, const char* what);  // throws CudaError (session.
 
 // Device memory: a stream-ordered pool per device that keeps up to 8 GB
 // between calls, so that repeated calls allocate and free without waiting for
-// the device.
+// the device; release_pools gives back what no call holds.
+struct DevicePools {
+    std::mutex mu;
+    std::map<int, cudaMemPool_t> of_device;
+    static DevicePools& all() {
+        static DevicePools& pools = *new DevicePools;
+        return pools;
+    }
+};
 inline cudaMemPool_t batch_pool(int device) {
-    static std::mutex& mu = *new std::mutex;
-    static std::map<int, cudaMemPool_t>& pools = *new std::map<int, cudaMemPool_t>;
-    std::lock_guard<std::mutex> lk(mu);
-    auto it = pools.find(device);
-    if (it != pools.end()) return it->second;
+    DevicePools& pools = DevicePools::all();
+    std::lock_guard<std::mutex> lk(pools.mu);
+    auto it = pools.of_device.find(device);
+    if (it != pools.of_device.end()) return it->second;
     cudaMemPoolProps props = {};
     props.allocType = cudaMemAllocationTypePinned;
     props.location.type = cudaMemLocationTypeDevice;
@@ -37,8 +44,24 @@ inline cudaMemPool_t batch_pool(int device) {
     check(cudaMemPoolCreate(&pool, &props), "cudaMemPoolCreate");
     uint64_t keep = 8ull << 30;
     check(cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep), "pool");
-    pools[device] = pool;
+    pools.of_device[device] = pool;
     return pool;
+}
+
+// Waits for each device that has a pool, so that every free has taken place.
+inline void release_pools() {
+    DevicePools& pools = DevicePools::all();
+    std::lock_guard<std::mutex> lk(pools.mu);
+    int current = 0;
+    if (!pools.of_device.empty()) check(cudaGetDevice(&current), "device");
+    for (const auto& [device, pool] : pools.of_device) {
+        check(cudaSetDevice(device), "cudaSetDevice");
+        const cudaError_t done = cudaDeviceSynchronize();
+        const cudaError_t trimmed = cudaMemPoolTrimTo(pool, 0);
+        check(cudaSetDevice(current), "cudaSetDevice");
+        check(done, "release memory");
+        check(trimmed, "release memory");
+    }
 }
 
 inline cudaMemPool_t current_pool() {

@@ -418,6 +418,13 @@ def device_info() -> dict:
     return {"available": bool(available.value), "device": text.value.decode()}
 
 
+def release_memory() -> None:
+    """Gives back the device memory that the library keeps between calls (up
+    to 8 GB per device) and that no batch, session or call holds.  No
+    reference counterpart."""
+    check(load().nricp_release_memory())
+
+
 def build_info() -> dict:
     """The reference's keys (bindings.cpp:723-737); pybind11_version names the
     binding layer, here ctypes over the C ABI."""
