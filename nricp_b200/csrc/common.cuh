@@ -129,8 +129,6 @@ struct WrapControl {
 struct WrapDev {
     // sizes
     int V, T, Vt, F, L;
-    int max_nodes, max_offdiag, max_edges;
-    int energy_blocks;    // partial records written by the vertex pass
     // settings (per level where they vary)
     double weights[kMaxLevels][kEnergyKinds];
     int robust_kernel[kMaxLevels];
@@ -209,10 +207,9 @@ struct WrapDev {
     double* pcg_sums;             // 6 per octet: a grid solve's partial sums
     unsigned* solve_arrivals;     // this tick's: a grid's CTAs at their meetings, or a cluster's that left the loop
     // reductions
-    double* partials;             // energy_blocks x kPartialStride
+    double* partials;             // vertex blocks x kPartialStride
     double* edge_partials;        // edges: each edge's smoothness energy (the decision kernel sums them)
     double* node_partials;        // N: each node's anchor energy (the decision kernel sums them)
-    int* counts;                  // stats scratch
     // report
     LevelRecord* records;         // level_count
     CorrStats* level_stats;       // level_count

@@ -42,12 +42,8 @@ void launch_closest_points(const WrapDev* wrap, const double* queries, int count
 // Launch shape of one tick, sized for the largest wrap of the batch.
 struct TickShape {
     int wraps;
-    int max_vertices;
     int max_nodes;
     int route_c;         // some wrap solves by route C (else its Horn-fit kernels are not launched)
-    int energy_blocks;   // vertex-pass blocks per wrap (partials written)
-    int edge_blocks;
-    int node_blocks;
     int pcg_cluster;       // CTAs per wrap in the cluster solve (any value gives the same result)
     // The solve may instead be split into launches by cluster class, each over
     // a list of wraps (device array), run as parallel branches of the tick.
@@ -83,7 +79,8 @@ int tick_kernel_launches(const TickShape& shape, bool timed = false);
 int pcg_class_cluster(int nodes, int shift);
 // The share of the device that one solve cluster of this size takes.
 double pcg_cluster_share(int cluster);
-int pcg_cluster_size(int max_nodes, int wraps, int sm_count);
+// The solve kernels' launch attributes, on the current device; before any tick.
+void pcg_enable();
 // Sets the shape's grid solve from its wraps and max_nodes.
 void grid_solve_shape(TickShape& shape);
 int pcg_max_nodes();
@@ -95,6 +92,5 @@ void launch_caller_vertices(const WrapDev* wrap, int vertices, int level, int bu
 // 3x3), t.
 void launch_fit_rigid(const double* src, const double* dst, const double* weights, int n, double* out,
                       cudaStream_t stream);
-void launch_evaluate_state(const WrapDev* wraps, const TickShape& shape, cudaStream_t stream);
 
 }  // namespace nricp_b200

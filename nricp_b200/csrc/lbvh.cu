@@ -707,10 +707,8 @@ __device__ inline double leaf_distance(const WrapDev& w, int leaf, D3 q, int* tr
 // boxes and query; every triangle reached is measured in FP64 -- an FP32
 // closest-point routine can misplace its point on thin sliver triangles by
 // far more than any fixed window.  `seed` is a triangle whose distance bounds
-// the search from the start.  Returns the winner, or -1; `steps_taken` (if
-// given) receives the nodes and leaves visited.
-__device__ int nearest_triangle(const WrapDev& w, F3 q, D3 q64, int seed, int* overflow,
-                                long* steps_taken = nullptr) {
+// the search from the start.  Returns the winner, or -1.
+__device__ int nearest_triangle(const WrapDev& w, F3 q, D3 q64, int seed, int* overflow) {
     const double slack = (double)w.rank_window;
     double best = 1e300;     // FP64 squared distance of the best triangle so far
     float bound = 3.4e38f;   // FP32 pruning radius^2: (sqrt(best) + slack)^2, rounded up
@@ -771,7 +769,6 @@ __device__ int nearest_triangle(const WrapDev& w, F3 q, D3 q64, int seed, int* o
         }
         if (!found) break;
     }
-    if (steps_taken) *steps_taken = steps;
     return best_tri;
 }
 

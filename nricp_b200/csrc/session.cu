@@ -149,7 +149,7 @@ struct Wrap {
     TemplateGraph graph;
     std::vector<LevelLayout> layouts;
     int V = 0, T = 0, Vt = 0, F = 0, L = 0, levels = 0;
-    int max_nodes = 0, max_edges = 0, max_offdiag = 0, max_steps = 0;
+    int max_nodes = 0, max_edges = 0, max_steps = 0;
     double setup_seconds = 0.0, solve_started = 0.0, solve_seconds = 0.0;
     Arena arena;
     WrapDev dev{};        // host copy of the descriptor
@@ -225,7 +225,6 @@ void envelope(Wrap& w) {
     for (const LevelLayout& L : w.layouts) {
         w.max_nodes = std::max(w.max_nodes, L.node_count);
         w.max_edges = std::max(w.max_edges, L.edge_count);
-        w.max_offdiag = std::max(w.max_offdiag, static_cast<int>(L.offdiag_nodes.size() / 2));
         w.max_steps = std::max(w.max_steps, static_cast<int>(L.sell_begin.back()));
     }
 }
@@ -369,8 +368,6 @@ size_t prepare_device(Wrap& w, WrapControl* control, cudaStream_t stream, bool p
     WrapDev& D = w.dev;
     std::memset(&D, 0, sizeof D);
     D.V = V; D.T = w.T; D.Vt = w.Vt; D.F = w.F; D.L = w.L;
-    D.max_nodes = w.max_nodes; D.max_offdiag = w.max_offdiag;
-    D.max_edges = w.max_edges; D.energy_blocks = vblocks;
     const double units = w.graph.scale;
     for (int l = 0; l < kMaxLevels; ++l) {
         const NricpLevelSettings& s =
@@ -799,7 +796,6 @@ void Batch::upload_all(LbvhExport* lbvh_out) {
     for (int i = 0; i < W; ++i) {
         Wrap& w = *wraps_[i];
         g_transfers.h2d += w.input_bytes;
-        shape_.max_vertices = std::max(shape_.max_vertices, w.V);
         shape_.max_nodes = std::max(shape_.max_nodes, w.max_nodes);
         if (w.desc.route == NRICP_ROUTE_C) shape_.route_c = 1;
     }
@@ -911,7 +907,7 @@ void Batch::set_pcg_cluster(int cluster) {
     int device = 0;
     check(cudaGetDevice(&device), "device");
     check(cudaDeviceGetAttribute(&sms_, cudaDevAttrMultiProcessorCount, device), "device");
-    pcg_cluster_size(shape_.max_nodes, static_cast<int>(wraps_.size()), sms_);  // enables the launch attributes
+    pcg_enable();
     drop_graphs();
     tail_ready_ = tail_on_ = false;
     solve_shape(cluster, shape_, pcg_index_, nullptr);
@@ -1304,7 +1300,7 @@ namespace {
 struct TemplateEntry {
     TemplateGraph graph;
     std::vector<LevelLayout> layouts;
-    int levels = 0, max_nodes = 0, max_edges = 0, max_offdiag = 0, max_steps = 0;
+    int levels = 0, max_nodes = 0, max_edges = 0, max_steps = 0;
 };
 
 uint64_t fnv1a(const void* data, size_t bytes, uint64_t h) {
@@ -1426,7 +1422,6 @@ struct Server::Impl {
             fresh->levels = w.levels;
             fresh->max_nodes = w.max_nodes;
             fresh->max_edges = w.max_edges;
-            fresh->max_offdiag = w.max_offdiag;
             fresh->max_steps = w.max_steps;
             std::lock_guard<std::mutex> lk(cache_mu);
             cache.emplace(key, std::move(fresh));
@@ -1437,7 +1432,6 @@ struct Server::Impl {
         w.levels = entry->levels;
         w.max_nodes = entry->max_nodes;
         w.max_edges = entry->max_edges;
-        w.max_offdiag = entry->max_offdiag;
         w.max_steps = entry->max_steps;
     }
 
@@ -1567,7 +1561,6 @@ struct Server::Impl {
 
     void grow_shape(const Wrap& w) {
         const TickShape before = shape;
-        shape.max_vertices = std::max(shape.max_vertices, w.V);
         shape.max_nodes = std::max(shape.max_nodes, w.max_nodes);
         if (w.desc.route == NRICP_ROUTE_C) shape.route_c = 1;
         if (std::memcmp(&before, &shape, sizeof shape) != 0) {
@@ -1585,7 +1578,7 @@ struct Server::Impl {
         t.wraps = count;
         if (cfg.pcg_cluster <= 0) grid_solve_shape(t);  // one size for every slot: no grid
         t.pcg_groups = 0;
-        pcg_cluster_size(t.max_nodes, count, sms);  // enables the launch attributes
+        pcg_enable();
         if (class_count == 0) {
             t.pcg_cluster = cfg.pcg_cluster;
         } else {

@@ -881,21 +881,6 @@ __device__ inline bool cholesky6(float* a) {
         }
     return true;
 }
-__device__ inline void solve6(const float* l, const double* rhs, double* x) {
-    float y[6];
-    for (int r = 0; r < 6; ++r) {
-        float s = (float)rhs[r];
-        for (int k = 0; k < r; ++k) s -= l[r * 6 + k] * y[k];
-        y[r] = s / l[r * 6 + r];
-    }
-    float z[6];
-    for (int r = 5; r >= 0; --r) {
-        float s = y[r];
-        for (int k = r + 1; k < 6; ++k) s -= l[k * 6 + r] * z[k];
-        z[r] = s / l[r * 6 + r];
-    }
-    for (int r = 0; r < 6; ++r) x[r] = z[r];
-}
 
 // The solve's reductions -- the dot products, the residual norm, the Krylov
 // scalars and the x and r vectors -- are FP64.  A build with
@@ -2557,7 +2542,6 @@ int pcg_class_cluster(int nodes, int shift) {
     return std::max(1, shift > 0 ? ranks >> shift : ranks);
 }
 
-// The solve kernels' launch attributes, on the current device.
 void pcg_enable() {
     static PerDevice<bool>& enabled = *new PerDevice<bool>;
     enabled.of(current_device(), [] {
@@ -2604,16 +2588,6 @@ double pcg_cluster_share(int cluster) {
     int i = 0;
     while (i < 4 && (1 << i) < cluster) ++i;
     return shares.of[i];
-}
-
-// Default cluster size for a batch: one wrap takes its latency cluster; many
-// wraps share the SMs, so the cluster shrinks until one CTA per SM holds the
-// whole batch (the result does not depend on the choice).
-int pcg_cluster_size(int max_nodes, int wraps, int sm_count) {
-    pcg_enable();
-    int ranks = pcg_class_cluster(max_nodes, 0);
-    while (ranks > 1 && (long)ranks * wraps > sm_count) ranks /= 2;
-    return ranks;
 }
 
 // Graphs above this many nodes (per wrap the grid takes) are solved by the
