@@ -1367,7 +1367,6 @@ struct Server::Impl {
     WrapControl* staging_controls = nullptr;  // where each loader's reset writes its wrap's control
     std::vector<WrapDev> host_wraps;
     std::vector<RequestPtr> slot_req;    // the running request of each slot, or null
-    std::vector<int> slot_nodes;
     int slots_used = 0;
     size_t resident = 0, peak = 0;
     void* lbvh_scratch[kLoaders] = {};   // each loader's, on its stream, from the pool
@@ -1603,6 +1602,8 @@ struct Server::Impl {
     }
     std::map<int, int> launches_per_tick;
 
+    // The nodes of the wrap in `slot`, wherever it was placed first.
+    int nodes_of(int slot) const { return slot_req[slot] ? slot_req[slot]->wrap->max_nodes : 0; }
     // A wrap's class is its latency cluster halved `shift` times: a fixed
     // shift (pcg_cluster < 0), or by load (0) -- the finest of -1, 0 and 1
     // whose clusters for the running wraps run at once, else 1.
@@ -1611,7 +1612,7 @@ struct Server::Impl {
         if (cfg.pcg_cluster < 0) return -cfg.pcg_cluster;
         for (int shift = -1; shift < 1; ++shift) {
             double share = 0.0;
-            for (int i = 0; i < count; ++i) share += pcg_cluster_share(pcg_class_cluster(slot_nodes[i], shift));
+            for (int i = 0; i < count; ++i) share += pcg_cluster_share(pcg_class_cluster(nodes_of(i), shift));
             if (share <= 1.0) return shift;
         }
         return 1;
@@ -1625,7 +1626,7 @@ struct Server::Impl {
         const int shift = shift_for(count);
         for (int i = 0; i < count; ++i) {
             int g = 0;
-            while ((class_top >> g) > pcg_class_cluster(slot_nodes[i], shift)) ++g;
+            while ((class_top >> g) > pcg_class_cluster(nodes_of(i), shift)) ++g;
             rows[static_cast<size_t>(g) * cfg.max_slots + fill[g]++] = i;
         }
         if (rows == class_rows) return;
@@ -1760,7 +1761,6 @@ struct Server::Impl {
                                           cudaMemcpyHostToDevice, stream), "slot control");
                     check(cudaMemcpyAsync(dev_wraps + slot, &host_wraps[slot], sizeof(WrapDev),
                                           cudaMemcpyHostToDevice, stream), "slot descriptor");
-                    slot_nodes[slot] = w.max_nodes;
                     grow_shape(w);
                 }
                 count = running_snapshot();
@@ -1901,7 +1901,6 @@ Server::Server(const NricpServerConfig& config) : impl_(std::make_unique<Impl>()
     check(cudaMallocHost(&m.host_controls, sizeof(WrapControl) * m.cfg.max_slots), "cudaMallocHost(controls)");
     m.host_wraps.assign(m.cfg.max_slots, WrapDev{});
     m.slot_req.assign(m.cfg.max_slots, nullptr);
-    m.slot_nodes.assign(m.cfg.max_slots, 0);
     int threads = m.cfg.prep_threads;
     if (threads <= 0) threads = std::max(1, static_cast<int>(std::thread::hardware_concurrency()) / 2);
     for (int i = 0; i < threads; ++i) m.preppers.emplace_back([&m] { m.prep_loop(); });
