@@ -864,7 +864,8 @@ __global__ void k_c_rhs(const WrapDev* __restrict__ wraps, int wrap_count, int p
 }
 
 // ---------------------------------------------------------------------------
-// the damped solve: block-Jacobi PCG in one CTA per wrap (pcg_solver.cu:15-241)
+// the damped solve: block-Jacobi PCG by a cluster of CTAs per wrap, or by the whole
+// device (pcg_solver.cu:15-241)
 // FP32 blocks and matvec, FP64 solution / residual / dots.
 // ---------------------------------------------------------------------------
 __device__ inline bool cholesky6(float* a) {
@@ -2598,7 +2599,14 @@ double pcg_cluster_share(int cluster) {
 // 10,000.
 constexpr int kGridNodes = 2000;
 // Wraps a tick may hold with the grid solve among its launches: it is of use to
-// few large wraps only, and a launch without work costs each tick 3 us.
+// few large wraps only, and a launch without work costs each tick 3 us.  A
+// batch's step with / without it, ms (6 bindings): 2,500 + 200 nodes 40.5 /
+// 42.8; 5,000 + 1,000 68.3 / 93.1; 2,500 + 3 of 800 46.3 / 47.1; 5,000 + 3 of
+// 1,500 86.5 / 102.3; 2,500 + 7 of 500 48.6 / 48.8; 5,000 + 7 of 1,200 90.2 /
+// 111.0; 2 of 5,000 + 6 of 500 104.0 / 110.9; and where it is of least use, 4 of
+// 4,000 107.8 / 109.4, 3 of 5,000 121.7 / 120.9, 8 of 2,100 124.3 / 122.2.  A
+// server's two lanes, a request of 2,500 nodes in one and five small ones in the
+// other, 99 / 98; of 5,000 nodes 167 / 192.
 constexpr int kGridWraps = 8;
 void grid_solve_shape(TickShape& shape) {
     shape.grid_nodes = shape.max_nodes > kGridNodes && shape.wraps <= kGridWraps ? kGridNodes : 0;
